@@ -247,7 +247,7 @@ struct b2_ctx {
     // fused, it is integer-multiply work) though a lone key switch gains 8 us; batched calls gain 1 %. So it is on for
     // batched calls and off for single ones unless B2_KS_FUSED_WIDE = 0 | 1 says otherwise.
     int mac_wide = -1;
-    bool use_mac = false;          // N = 2^16: ModUp's last forward pass carries the inner product (off with B2_KS_FUSED_IP=0)
+    bool use_mac = false;          // N = 2^15, 2^16: ModUp's last forward pass carries the inner product (off with B2_KS_FUSED_IP=0)
     int sm_count = 148;
     // RNS-limb sharding of one ciphertext over `shard_world` GPUs: this rank's slice of every list
     int shard_rank = 0, shard_world = 1;
@@ -739,9 +739,9 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
             b2_ctx_destroy(c);
             return fail(B2_ENOMEM, "ctx_create: cudaMalloc(status word) failed");
         }
-        if (c->logN == 16) {
+        if (c->logN == 15 || c->logN == 16) {
             // per device: the fused row pass stages a key tile next to its exchange buffer (49 KB, above the 48 KB default)
-            // <8, 4, 3> = the row-pass configuration of N = 2^16 (PassCfg<8>, asserted where the kernel is launched)
+            // <8, 4, 3> = the row-pass configuration of N = 2^15 and 2^16 (PassCfg<8>, asserted where the kernel is launched)
             cudaError_t em = cudaFuncSetAttribute(ntt_fwd_rows_mac<8, 4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)mac_smem_bytes<8, 4, 3>());
             if (em != cudaSuccess) {
@@ -770,7 +770,7 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
     const char *env_mac = getenv("B2_KS_FUSED_IP");
     if (const char *e = getenv("B2_KS_FUSED_WIDE")) c->mac_wide = e[0] != '0' ? 1 : 0;
     if (const char *e = getenv("B2_KS_FUSED_ORDER")) c->mac_interleave = e[0] == '1';
-    c->use_mac = (c->logN == 16) && !c->use_cluster && !c->use_pipe && !(env_mac && env_mac[0] == '0');
+    c->use_mac = (c->logN == 15 || c->logN == 16) && !c->use_cluster && !c->use_pipe && !(env_mac && env_mac[0] == '0');
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
     if (c->sm_count < 1) c->sm_count = 148;
     c->plan.resize(sQ + 1);
@@ -861,6 +861,19 @@ static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const 
     const dim3 grid = pass_grid(b, njobs * (N >> (LOG_B + B::LOG_C)), batch);
     LaunchScope ls(c, s, "ntt_fwd_rows");
     ntt_fwd_pass<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi><<<grid, pass_threads<LOG_B>(), 0, s>>>(b, epi);
+}
+
+// the forward column pass alone, for the rings whose row pass has 256 points (2^15, 2^16)
+template <int LOG_A>
+static void launch_fwd_cols_n(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
+    using A = PassCfg<LOG_A>;
+    LaunchScope ls(c, s, "ntt_fwd_cols");
+    ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore>
+        <<<dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s>>>(a, EpiStore{});
+}
+static void launch_fwd_cols(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
+    if (a.logN == 16) launch_fwd_cols_n<8>(c, a, njobs, s, batch);
+    else launch_fwd_cols_n<7>(c, a, njobs, s, batch);
 }
 
 template <int LOG_A, int LOG_B>
@@ -1760,8 +1773,11 @@ static int ks_tail_fused(b2_ctx *c, size_t l, const uint64_t *digits, const uint
     return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
 }
 
-// ModUp and inner product of the fused key switch with the FP64 limbs' inner product inside the last forward pass.
-// Applies at N = 2^16 when the level's Q limbs are FP64 primes behind a prefix of wide ones; *done tells whether it ran.
+// ModUp and inner product of the fused key switch. At N = 2^16 (batched calls: 2^15 too) the inner product of the FP64 limbs
+// runs inside the last forward pass when the level's Q limbs are FP64 primes behind a prefix of wide ones; batched calls in
+// the other rings store both passes and run the stand-alone inner product, every kernel one launch over the batch
+// (N = 2^14, 8 limbs, 2 special primes, 32 products and rescales: 3045 us one set after another, 822 us so).
+// *done tells whether it ran.
 // ct [2][l][N] += (inner product) * P^-1 on the Q limbs; cxP [2][alpha][N] = (acc_p: +=) the P limbs of the inner product.
 // A batch of key switches with one key, every kernel one launch over the batch: set b's input, ciphertext, and its scratch
 // blocks t [l], up [beta][l+alpha], cxP [2][alpha] start b * c2_bs / ct_bs / l / beta (l+alpha) / 2 alpha limbs further.
@@ -1774,15 +1790,17 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     const size_t N = c->N, lP = l + c->size_P, beta = c->plan[l].beta;
     const LevelPlan &pl = c->plan[l];
     *done = false;
-    const bool wide = (c->mac_wide < 0 ? kb.batch > 1 : c->mac_wide == 1) && beta <= B2_MAC_MAX_BETA;
-    if (!(c->use_mac && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP))) return B2_OK;
+    const bool batched = kb.batch != 1;
+    const bool wide = (c->mac_wide < 0 ? batched : c->mac_wide == 1) && beta <= B2_MAC_MAX_BETA;
+    // single calls at 2^15 run the stored row pass and the stand-alone inner product: the split by prime class costs two
+    // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853)
+    const bool mac = c->use_mac && (batched || c->logN == 16 || c->mac_wide == 1) && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
+    if (!mac && !batched) return B2_OK;
+    if (batched && (!c->bconv_tc || c->tc_simple || c->use_cluster || c->use_pipe || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
+        return B2_OK;  // the caller falls back to one key switch at a time
     {
-        // ModUp up to the column pass for every limb; the row pass is stored only for the limbs the stand-alone inner
-        // product still handles (wide Q primes and P); for the FP64 limbs of Q it runs inside ntt_fwd_rows_mac
         using Cfg = PassCfg<8>;
         const uint32_t B = kb.batch, per = (uint32_t)(beta * lP), a2 = (uint32_t)(2 * c->size_P);
-        const bool batched = B != 1;
-        if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs)) return B2_OK;  // the caller falls back to one key switch at a time
         int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, kb.c2_bs, 0, (uint32_t)l});
         if (rc) return rc;
         if (batched) {
@@ -1792,15 +1810,23 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             rc = run_bconv(c, false, t, up, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)lP, true, s, &pl.tc_up);
         }
         if (rc) return rc;
+        if (!mac) {
+            // rings whose row pass is not the 256-point one (and keys of more than B2_MAC_MAX_BETA digits): both passes
+            // stored for every limb, then the stand-alone inner product, each one launch over the batch
+            rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            if (rc) return rc;
+            const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
+            rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib);
+            if (rc) return rc;
+            *done = true;
+            return B2_OK;
+        }
+        // ModUp up to the column pass for every limb; the row pass is stored only for the limbs the stand-alone inner
+        // product still handles (wide Q primes and P); for the FP64 limbs of Q it runs inside ntt_fwd_rows_mac
         NttArgs a{up, up, pl.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
         a.src_bs = a.dst_bs = batched ? per : 0;
-        {
-            NttArgs a1 = a;
-            const dim3 grid = pass_grid(a1, pl.n_up_ntt * (uint32_t)(N >> (8 + Cfg::LOG_CC)), B);
-            LaunchScope ls(c, s, "ntt_fwd_cols");
-            ntt_fwd_pass<8, Cfg::R_STRIDED, Cfg::R_CONTIG, Cfg::LOG_CC, true, false, EpiStore><<<grid, pass_threads<8, true>(), 0, s>>>(a1, EpiStore{});
-            LAUNCH_CHECK("ntt_fwd_pass");
-        }
+        launch_fwd_cols(c, a, pl.n_up_ntt, s, B);
+        LAUNCH_CHECK("ntt_fwd_pass");
         // the limbs on 60-bit primes (q0, P) either ride on the fused pass too (integer arithmetic) or, mac_wide off,
         // keep the stored row pass and the stand-alone inner product
         if (!wide && pl.n_up_rows) {
@@ -1882,8 +1908,8 @@ extern "C" size_t b2_keyswitch_batch_workspace_bytes(const b2_ctx *c, size_t l, 
 }
 
 // `batch` key switches with ONE key: ct_b [2][l][N] += ModDown(<ModUp(c2_b), key>), set b's input at d_c2 + b * c2_stride
-// limbs and its ciphertext at d_ct + b * ct_stride limbs. Where the fused pipeline applies (N = 2^16, tensor-core base
-// conversion) every kernel is one launch over the whole batch - 10 to 12 launches for the batch instead of per key
+// limbs and its ciphertext at d_ct + b * ct_stride limbs. With the tensor-core base
+// conversion every kernel is one launch over the whole batch - 10 to 12 launches for the batch instead of per key
 // switch, grids that fill the GPU at every level, and the key read from HBM once per batch: the fused inner product
 // puts the sets that share a key tile next to one another in the grid, so all but the first find it in L2. Elsewhere the
 // key switches run one after another on the same stream. Workspace: t [batch][l] | up [batch][beta][l+alpha] | cxP [batch][2][alpha].
@@ -2936,9 +2962,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 NttArgs na{UP, UP, sp.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
                 na.src_bs = na.dst_bs = per;
                 if (sp.n_up_ntt) {
-                    LaunchScope ls(c, s, "ntt_fwd_cols");
-                    ntt_fwd_pass<8, Cfg::R_STRIDED, Cfg::R_CONTIG, Cfg::LOG_CC, true, false, EpiStore>
-                        <<<dim3(sp.n_up_ntt * (uint32_t)(N >> (8 + Cfg::LOG_CC)), B), pass_threads<8, true>(), 0, s>>>(na, EpiStore{});
+                    launch_fwd_cols(c, na, sp.n_up_ntt, s, B);
                     LAUNCH_CHECK("ntt_fwd_pass");
                 }
                 MacArgs m{};
