@@ -300,6 +300,23 @@ struct LaunchScope {
     }
 };
 
+// Every kernel of the library is launched with the programmatic-serialisation attribute and begins with pdl_enter()
+// (modarith.cuh): the next kernel's launch and block scheduling overlap the end of the previous one, and its CTAs wait until
+// that kernel has completed and its writes are visible. At small sizes a key switch is a chain of a dozen kernels of 2 to 5
+// us, where launch latency is a third of the time (one transform pair of 8 limbs at N = 2^14: 30.7 -> 22.1 us; a rotation at
+// N = 2^13: 74 -> 54). No kernel signals before it ends (griddepcontrol.launch_dependents): CTAs that are scheduled early
+// take SM slots from the running grid and bunch up on the SMs that empty first (signalled on entry, eight hoisted rotations
+// at N = 2^15 take 708 us; before the exchange of the transforms 597; never 599; without the attribute 670).
+template <class... P, class... A>
+static void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = s, cfg.attrs = &at, cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);  // LAUNCH_CHECK reads the error
+}
+
 template <typename T>
 static T *blob_take(char *&cur, size_t count) {
     uintptr_t p = (reinterpret_cast<uintptr_t>(cur) + 15) & ~uintptr_t(15);
@@ -839,13 +856,12 @@ static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const 
             const uint32_t total = njobs * (N >> (LOG_A + A::LOG_C));
             {
                 LaunchScope ls(c, s, "ntt_fwd_cols");
-                ntt_fwd_pipe<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_C, true, false, EpiStore>
-                    <<<pipe_grid(c, total), pass_threads<LOG_A>(), 0, s>>>(a, EpiStore{}, total);  // the pipelined passes keep 8 columns
+                launch_k(ntt_fwd_pipe<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_C, true, false, EpiStore>, pipe_grid(c, total), pass_threads<LOG_A>(), 0, s, a, EpiStore{}, total);  // the pipelined passes keep 8 columns
             }
             NttArgs b = a;
             b.src = a.dst;
             LaunchScope ls(c, s, "ntt_fwd_rows");
-            ntt_fwd_pipe<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi><<<pipe_grid(c, total), pass_threads<LOG_B>(), 0, s>>>(b, epi, total);
+            launch_k(ntt_fwd_pipe<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi>, pipe_grid(c, total), pass_threads<LOG_B>(), 0, s, b, epi, total);
             return;
         }
     }
@@ -853,14 +869,14 @@ static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const 
         NttArgs a1 = a;
         const dim3 grid = pass_grid(a1, njobs * (N >> (LOG_A + A::LOG_CC)), batch);
         LaunchScope ls(c, s, "ntt_fwd_cols");
-        ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC><<<grid, pass_threads<LOG_A, true>(), 0, s>>>(a1, EpiStore{});
+        launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC>, grid, pass_threads<LOG_A, true>(), 0, s, a1, EpiStore{});
     }
     NttArgs b = a;
     b.src = a.dst;  // second pass works in place on the first pass's output
     b.src_lm1 = a.dst_lm1, b.src_bs = a.dst_bs;
     const dim3 grid = pass_grid(b, njobs * (N >> (LOG_B + B::LOG_C)), batch);
     LaunchScope ls(c, s, "ntt_fwd_rows");
-    ntt_fwd_pass<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi><<<grid, pass_threads<LOG_B>(), 0, s>>>(b, epi);
+    launch_k(ntt_fwd_pass<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi>, grid, pass_threads<LOG_B>(), 0, s, b, epi);
 }
 
 // the forward column pass alone, for the rings whose row pass has 256 points (2^15, 2^16)
@@ -868,8 +884,7 @@ template <int LOG_A>
 static void launch_fwd_cols_n(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
     using A = PassCfg<LOG_A>;
     LaunchScope ls(c, s, "ntt_fwd_cols");
-    ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore>
-        <<<dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s>>>(a, EpiStore{});
+    launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore>, dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
 }
 static void launch_fwd_cols(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
     if (a.logN == 16) launch_fwd_cols_n<8>(c, a, njobs, s, batch);
@@ -886,12 +901,12 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
             const uint32_t total = njobs * (N >> (LOG_B + B::LOG_C));
             {
                 LaunchScope ls(c, s, "ntt_inv_rows");
-                ntt_inv_pipe<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false><<<pipe_grid(c, total), pass_threads<LOG_B>(), 0, s>>>(a, total);
+                launch_k(ntt_inv_pipe<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false>, pipe_grid(c, total), pass_threads<LOG_B>(), 0, s, a, total);
             }
             NttArgs b = a;
             b.src = a.dst;
             LaunchScope ls(c, s, "ntt_inv_cols");
-            ntt_inv_pipe<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_C, true, true><<<pipe_grid(c, total), pass_threads<LOG_A>(), 0, s>>>(b, total);
+            launch_k(ntt_inv_pipe<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_C, true, true>, pipe_grid(c, total), pass_threads<LOG_A>(), 0, s, b, total);
             return;
         }
     }
@@ -899,14 +914,14 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
         NttArgs a1 = a;
         const dim3 grid = pass_grid(a1, njobs * (N >> (LOG_B + B::LOG_C)), batch);
         LaunchScope ls(c, s, "ntt_inv_rows");
-        ntt_inv_pass<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false><<<grid, pass_threads<LOG_B>(), 0, s>>>(a1);
+        launch_k(ntt_inv_pass<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false>, grid, pass_threads<LOG_B>(), 0, s, a1);
     }
     NttArgs b = a;
     b.src = a.dst;
     b.src_lm1 = a.dst_lm1, b.src_bs = a.dst_bs;
     const dim3 grid = pass_grid(b, njobs * (N >> (LOG_A + A::LOG_CC)), batch);
     LaunchScope ls(c, s, "ntt_inv_cols");
-    ntt_inv_pass<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_CC, true, true><<<grid, pass_threads<LOG_A, true>(), 0, s>>>(b);
+    launch_k(ntt_inv_pass<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_CC, true, true>, grid, pass_threads<LOG_A, true>(), 0, s, b);
 }
 
 // SRC != 0: the column pass makes limb job.x from slot job.x / src_div of src (words mod src_q) instead of reading it
@@ -928,7 +943,7 @@ static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
         // rather than remembered per thread (a thread may drive contexts on several devices)
         CUDA_TRY(cudaFuncSetAttribute(ntt_fwd_cluster<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM));
         LaunchScope ls(c, s, "ntt_fwd_cluster");
-        ntt_fwd_cluster<Epi><<<njobs * CL_SIZE, CL_THREADS, CL_SMEM, s>>>(a, epi);
+        launch_k(ntt_fwd_cluster<Epi>, njobs * CL_SIZE, CL_THREADS, CL_SMEM, s, a, epi);
         LAUNCH_CHECK("ntt_fwd_cluster");
         return B2_OK;
     }
@@ -954,7 +969,7 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if (c->use_cluster) {
         CUDA_TRY(cudaFuncSetAttribute(ntt_inv_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM));
         LaunchScope ls(c, s, "ntt_inv_cluster");
-        ntt_inv_cluster<<<njobs * CL_SIZE, CL_THREADS, CL_SMEM, s>>>(a);
+        launch_k(ntt_inv_cluster, njobs * CL_SIZE, CL_THREADS, CL_SMEM, s, a);
         LAUNCH_CHECK("ntt_inv_cluster");
         return B2_OK;
     }
@@ -988,6 +1003,7 @@ template <int MAX_NI, bool COPY>
 __global__ void __launch_bounds__(128) bconv_kernel(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
                                                     const uint64_t *__restrict__ copy_src, const BconvGroup *groups,
                                                     const uint2 *outs, const uint64_t *mats, const Mod *mod, uint32_t N) {
+    pdl_enter();
     extern __shared__ __align__(16) uint64_t s_raw[];
     const BconvGroup g = groups[blockIdx.y];
     BconvOut *s_out = reinterpret_cast<BconvOut *>(s_raw);          // [n_out]
@@ -1133,6 +1149,7 @@ template <bool COPY>
 __global__ void __launch_bounds__(128) bconv_fp_kernel(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
                                                        const uint64_t *__restrict__ copy_src, const BconvGroup *groups, const uint2 *outs,
                                                        const double *matd, const b2_ctx::RedcMeta *redc, uint32_t N) {
+    pdl_enter();
     extern __shared__ __align__(16) uint64_t s_raw[];
     const BconvGroup g = groups[blockIdx.y];
     BconvMetaS *s_meta = reinterpret_cast<BconvMetaS *>(s_raw);                      // [n_out]
@@ -1183,6 +1200,7 @@ __global__ void __launch_bounds__(256) ks_inner_prod_kernel(const uint64_t *__re
                                                            const W2 *__restrict__ pinv, const Mod *mod, const b2_ctx::RedcMeta *redc,
                                                            uint32_t N, uint32_t l, uint32_t lP, uint32_t size_Q, uint32_t size_QP,
                                                            uint32_t beta, uint4 own_range, const IpBatch ib, const uint32_t *__restrict__ perm) {
+    pdl_enter();
     // perm (optional): the digits are read through the NTT-domain permutation of a Galois element, digit[perm[n]] - hoisted
     // rotations, whose permuted copy of the ModUp digits is then never written (src/evaluate.cu:2041-2045 permutes into a buffer)
     // own_range = (first Q limb, number of Q limbs, first P limb, number of P limbs) this launch
@@ -1325,6 +1343,7 @@ __global__ void __launch_bounds__(256) ks_inner_prod_kernel(const uint64_t *__re
 // A batch in one launch: blockIdx.y = pair b, whose operands, result and d2 start b * bs.x / .y / .z / .w limbs further.
 __global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *__restrict__ a, const uint64_t *__restrict__ b, uint64_t *__restrict__ out,
                                                         uint64_t *__restrict__ out2, const Mod *mod, uint32_t N, uint32_t l, uint4 bs) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t S = (size_t)l * N;
     if (idx >= S) return;
@@ -1351,6 +1370,7 @@ __global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *__restr
 // ciphertext. b_wrap: the second operand is one polynomial shared by all (a plaintext).
 __global__ void __launch_bounds__(256) poly_op_kernel(int op, const uint64_t *a, const uint64_t *b, uint64_t *out, const Mod *mod,
                                                      uint32_t N, uint32_t n_limbs, uint32_t period, int b_wrap) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_limbs * N) return;
     const Mod md = mod[(idx / N) % period];
@@ -1372,6 +1392,7 @@ __global__ void __launch_bounds__(256) poly_op_kernel(int op, const uint64_t *a,
 struct ScalarTab { uint64_t v[64]; };
 __global__ void __launch_bounds__(256) poly_scalar_kernel(int op, const uint64_t *a, ScalarTab tab, uint64_t *out, const Mod *mod,
                                                         uint32_t N, uint32_t n_limbs, uint32_t period) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_limbs * N) return;
     const uint32_t limb = (uint32_t)((idx / N) % period);
@@ -1391,6 +1412,7 @@ __global__ void __launch_bounds__(256) poly_scalar_kernel(int op, const uint64_t
 // Optional second operand pair so that c0 and c1 (or several digit buffers) go in one launch.
 __global__ void __launch_bounds__(256) galois_gather_kernel(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst,
                                                            const uint32_t *__restrict__ perm, uint32_t N, uint32_t n_limbs) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_limbs * N) return;
     const size_t limb = idx / N;
@@ -1402,6 +1424,7 @@ __global__ void __launch_bounds__(256) galois_gather_kernel(const uint64_t *__re
 template <bool ACC>
 __global__ void __launch_bounds__(256) galois_split_kernel(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst0, uint64_t *__restrict__ dst1,
                                                           const uint32_t *__restrict__ perm, const Mod *mod, uint32_t N, uint32_t l) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t S = (size_t)l * N;
     if (idx >= 2 * S) return;
@@ -1420,6 +1443,7 @@ __global__ void __launch_bounds__(256) galois_split_kernel(const uint64_t *__res
 // one signed, centred int64 coefficient vector -> its residue in each of n_limbs primes.
 __global__ void __launch_bounds__(256) expand_signed_kernel(const int64_t *__restrict__ src, uint64_t *__restrict__ dst, const Mod *mod, uint32_t N,
                                                            uint32_t n_limbs, uint32_t first_prime) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_limbs * N) return;
     const Mod md = mod[first_prime + idx / N];
@@ -1434,6 +1458,7 @@ __global__ void __launch_bounds__(256) expand_signed_kernel(const int64_t *__res
 // rounds to nearest instead of flooring. r: [n_poly][N] coefficient form mod q_last.
 __global__ void __launch_bounds__(256) rescale_centre_kernel(const uint64_t *__restrict__ r, uint64_t *__restrict__ out, const Mod *mod, uint32_t N,
                                                             uint32_t n_out, uint32_t n_poly) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_poly * n_out * N) return;
     const uint32_t i = (uint32_t)(idx % N), j = (uint32_t)((idx / N) % n_out), p = (uint32_t)(idx / ((size_t)N * n_out));
@@ -1457,6 +1482,7 @@ struct LincombArgs {
 };
 __global__ void __launch_bounds__(256) lincomb_kernel(const __grid_constant__ LincombArgs a, uint64_t *out, const Mod *mod, uint32_t N, uint32_t l,
                                                      uint32_t n_poly, uint32_t n_terms) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_poly * l * N) return;
     const uint32_t i = (uint32_t)(idx % N), limb = (uint32_t)((idx / N) % l), p = (uint32_t)(idx / ((size_t)N * l));
@@ -1469,6 +1495,7 @@ __global__ void __launch_bounds__(256) lincomb_kernel(const __grid_constant__ Li
 // M signed coefficient vectors at once: src [M][N] -> dst [M][l][N] (limb j of every polynomial on prime j)
 __global__ void __launch_bounds__(256) expand_signed_batch_kernel(const int64_t *__restrict__ src, uint64_t *__restrict__ dst, const Mod *mod, uint32_t N,
                                                                  uint32_t l, uint32_t M) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)M * l * N) return;
     const uint32_t i = (uint32_t)(idx % N), limb = (uint32_t)((idx / N) % l), m = (uint32_t)(idx / ((size_t)N * l));
@@ -1489,6 +1516,7 @@ struct MacPtrs {
 // The reference reduces after every term; the sum of canonical products is the same residue.
 __global__ void __launch_bounds__(256) bsgs_mac_kernel(const uint64_t *const *pts, const uint64_t *const *babies, uint64_t *out, const Mod *mod,
                                                       uint32_t N, uint32_t l, uint32_t M) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t S = (size_t)l * N;
     if (idx >= S) return;
@@ -1518,6 +1546,7 @@ __global__ void __launch_bounds__(256) bsgs_mac_kernel(const uint64_t *const *pt
 template <int G>
 __global__ void __launch_bounds__(256) bsgs_mac_multi_kernel(const uint64_t *const *pts, const uint64_t *const *babies, uint64_t *const *outs,
                                                             const Mod *mod, uint32_t N, uint32_t l, uint32_t M, uint32_t n_g) {
+    pdl_enter();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t S = (size_t)l * N;
     if (idx >= S) return;
@@ -1580,9 +1609,9 @@ static int run_bconv_tc(const b2_ctx *c, bool copy, const uint64_t *in, uint64_t
         const dim3 grid(N / 128, n_jobs);
         const uint32_t smem = tc_smem_request(tc.max_alloc, TC_SMEM_BYTES);
         switch (c->tc_wg) {
-            case 1: bconv_tc_kernel<1><<<grid, 128, smem, s>>>(in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
-            case 4: bconv_tc_kernel<4><<<grid, 512, smem, s>>>(in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
-            default: bconv_tc_kernel<2><<<grid, 256, smem, s>>>(in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
+            case 1: launch_k(bconv_tc_kernel<1>, grid, 128, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
+            case 4: launch_k(bconv_tc_kernel<4>, grid, 512, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
+            default: launch_k(bconv_tc_kernel<2>, grid, 256, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
         }
         LAUNCH_CHECK("bconv_tc_kernel");
         return B2_OK;
@@ -1594,9 +1623,9 @@ static int run_bconv_tc(const b2_ctx *c, bool copy, const uint64_t *in, uint64_t
     const uint32_t grid = std::min(total, fit * (uint32_t)c->sm_count);
     const uint32_t smem = tc_smem_request(tc.max_alloc, TCP_SMEM_BYTES);
     switch (c->tc_wg) {
-        case 1: bconv_tc_persist<1><<<grid, 128, smem, s>>>(in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
-        case 2: bconv_tc_persist<2><<<grid, 256, smem, s>>>(in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
-        default: bconv_tc_persist<4><<<grid, 512, smem, s>>>(in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
+        case 1: launch_k(bconv_tc_persist<1>, grid, 128, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
+        case 2: launch_k(bconv_tc_persist<2>, grid, 256, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
+        default: launch_k(bconv_tc_persist<4>, grid, 512, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
     }
     LAUNCH_CHECK("bconv_tc_persist");
     return B2_OK;
@@ -1613,19 +1642,19 @@ static int run_bconv(const b2_ctx *c, bool copy, const uint64_t *in, uint64_t *o
         dim3 grid(N / 128, n_groups);
         const size_t smem = (size_t)max_out * sizeof(BconvMetaS) + (size_t)max_out * 24 * 8;
         (void)in3;
-        if (copy) bconv_fp_kernel<true><<<grid, 128, smem, s>>>(in, out, copy_src, groups, outs, matd, c->d_redc, N);
-        else bconv_fp_kernel<false><<<grid, 128, smem, s>>>(in, out, copy_src, groups, outs, matd, c->d_redc, N);
+        if (copy) launch_k(bconv_fp_kernel<true>, grid, 128, smem, s, in, out, copy_src, groups, outs, matd, c->d_redc, N);
+        else launch_k(bconv_fp_kernel<false>, grid, 128, smem, s, in, out, copy_src, groups, outs, matd, c->d_redc, N);
         LAUNCH_CHECK("bconv_fp_kernel");
         return B2_OK;
     }
     dim3 grid(N / 2 / 128, n_groups);
     const size_t smem = ((size_t)max_ni + 4) * max_out * 8;
     if (copy) {
-        if (max_ni <= 8) bconv_kernel<8, true><<<grid, 128, smem, s>>>(in, out, copy_src, groups, outs, mats, c->d_mod, N);
-        else bconv_kernel<16, true><<<grid, 128, smem, s>>>(in, out, copy_src, groups, outs, mats, c->d_mod, N);
+        if (max_ni <= 8) launch_k(bconv_kernel<8, true>, grid, 128, smem, s, in, out, copy_src, groups, outs, mats, c->d_mod, N);
+        else launch_k(bconv_kernel<16, true>, grid, 128, smem, s, in, out, copy_src, groups, outs, mats, c->d_mod, N);
     } else {
-        if (max_ni <= 8) bconv_kernel<8, false><<<grid, 128, smem, s>>>(in, out, copy_src, groups, outs, mats, c->d_mod, N);
-        else bconv_kernel<16, false><<<grid, 128, smem, s>>>(in, out, copy_src, groups, outs, mats, c->d_mod, N);
+        if (max_ni <= 8) launch_k(bconv_kernel<8, false>, grid, 128, smem, s, in, out, copy_src, groups, outs, mats, c->d_mod, N);
+        else launch_k(bconv_kernel<16, false>, grid, 128, smem, s, in, out, copy_src, groups, outs, mats, c->d_mod, N);
     }
     LAUNCH_CHECK("bconv_kernel");
     return B2_OK;
@@ -1708,13 +1737,13 @@ static int inner_prod_impl(b2_ctx *c, size_t l, const uint64_t *digits, const ui
     const IpBatch ib = ipb ? *ipb : IpBatch{0, 0, 0, 1, (uint32_t)c->size_P, 0, 0};
     LaunchScope ls(c, s, "ks_inner_prod");
     if (fused && acc_p)
-        ks_inner_prod_kernel<3, true, true><<<grid, 256, 0, s>>>(digits, own, ep, out, ct, c->d_Pinv, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l,
+        launch_k(ks_inner_prod_kernel<3, true, true>, grid, 256, 0, s, digits, own, ep, out, ct, c->d_Pinv, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l,
                                                                (uint32_t)lP, (uint32_t)c->size_Q, (uint32_t)c->size_QP, (uint32_t)beta, rg, ib, perm);
     else if (fused)
-        ks_inner_prod_kernel<3, true><<<grid, 256, 0, s>>>(digits, own, ep, out, ct, c->d_Pinv, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l, (uint32_t)lP,
+        launch_k(ks_inner_prod_kernel<3, true>, grid, 256, 0, s, digits, own, ep, out, ct, c->d_Pinv, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l, (uint32_t)lP,
                                                          (uint32_t)c->size_Q, (uint32_t)c->size_QP, (uint32_t)beta, rg, ib, perm);
     else
-        ks_inner_prod_kernel<3, false><<<grid, 256, 0, s>>>(digits, own, ep, out, nullptr, nullptr, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l, (uint32_t)lP,
+        launch_k(ks_inner_prod_kernel<3, false>, grid, 256, 0, s, digits, own, ep, out, nullptr, nullptr, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l, (uint32_t)lP,
                                                           (uint32_t)c->size_Q, (uint32_t)c->size_QP, (uint32_t)beta, rg, ib, perm);
     LAUNCH_CHECK("ks_inner_prod_kernel");
     return B2_OK;
@@ -1834,7 +1863,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             b.jobs = pl.jobs_up_rows;
             const dim3 grid = pass_grid(b, pl.n_up_rows * (uint32_t)(N >> (8 + Cfg::LOG_C)), B);
             LaunchScope ls(c, s, "ntt_fwd_rows");
-            ntt_fwd_pass<8, Cfg::R_STRIDED, Cfg::R_CONTIG, Cfg::LOG_C, false, true, EpiStore><<<grid, pass_threads<8>(), 0, s>>>(b, EpiStore{});
+            launch_k(ntt_fwd_pass<8, Cfg::R_STRIDED, Cfg::R_CONTIG, Cfg::LOG_C, false, true, EpiStore>, grid, pass_threads<8>(), 0, s, b, EpiStore{});
             LAUNCH_CHECK("ntt_fwd_pass");
         }
         if (!wide) {
@@ -1861,8 +1890,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             LaunchScope ls(c, s, "ntt_fwd_rows_mac");
             static_assert(Cfg::R_STRIDED == Cfg::R_CONTIG, "the fused pass wants equal stage groups");
             static_assert(Cfg::R_CONTIG == 4 && Cfg::LOG_C == 3, "b2_ctx_create raises the shared-memory limit of this instantiation");
-            ntt_fwd_rows_mac<8, Cfg::R_CONTIG, Cfg::LOG_C>
-                <<<dim3(B, n_limbs * (uint32_t)(N >> (8 + Cfg::LOG_C))), pass_threads<8>(), mac_smem_bytes<8, Cfg::R_CONTIG, Cfg::LOG_C>(), s>>>(a, m);
+            launch_k(ntt_fwd_rows_mac<8, Cfg::R_CONTIG, Cfg::LOG_C>, dim3(B, n_limbs * (uint32_t)(N >> (8 + Cfg::LOG_C))), pass_threads<8>(), mac_smem_bytes<8, Cfg::R_CONTIG, Cfg::LOG_C>(), s, a, m);
             LAUNCH_CHECK("ntt_fwd_rows_mac");
         }
     }
@@ -1960,7 +1988,7 @@ extern "C" int b2_tensor_mul(b2_ctx *c, size_t l, const uint64_t *d_a, const uin
     if (!d_a || !d_b || !d_out) return fail(B2_EINVAL, "tensor_mul: null pointer");
     const size_t n = l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "tensor_mul");
-    tensor_mul_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_a, d_b, d_out, d_out + 2 * n, c->d_mod, (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
+    launch_k(tensor_mul_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, d_a, d_b, d_out, d_out + 2 * n, c->d_mod, (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
     LAUNCH_CHECK("tensor_mul_kernel");
     return B2_OK;
 }
@@ -1978,7 +2006,7 @@ extern "C" int b2_multiply_and_relin(b2_ctx *c, size_t l, const uint64_t *d_a, c
         // d0, d1 straight into the result, d2 into scratch for the key switch (every thread reads its own position of
         // the operands before it writes, so the result may alias an operand)
         LaunchScope ls(c, s, "tensor_mul");
-        tensor_mul_kernel<<<(unsigned)((S + 255) / 256), 256, 0, s>>>(d_a, d_b, d_out, t3 + 2 * S, c->d_mod, (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
+        launch_k(tensor_mul_kernel, (unsigned)((S + 255) / 256), 256, 0, s, d_a, d_b, d_out, t3 + 2 * S, c->d_mod, (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
         LAUNCH_CHECK("tensor_mul_kernel");
     }
     return keyswitch_impl(c, l, t3 + 2 * S, rlk, n_evk, d_out, ws, s);
@@ -2002,7 +2030,7 @@ static int rescale_tail(const b2_ctx *c, size_t l, size_t n_poly, const uint64_t
     } else {
         const size_t n = n_poly * (l - 1) * c->N;
         LaunchScope ls(c, s, "rescale_centre");
-        rescale_centre_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(r, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(l - 1), (uint32_t)n_poly);
+        launch_k(rescale_centre_kernel, (unsigned)((n + 255) / 256), 256, 0, s, r, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(l - 1), (uint32_t)n_poly);
         LAUNCH_CHECK("rescale_centre_kernel");
     }
     return run_fwd(c, d_out, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s);
@@ -2073,7 +2101,7 @@ extern "C" int b2_multiply_relin_rescale_batch(b2_ctx *c, size_t l, size_t batch
     uint64_t *prod = (uint64_t *)d_ws, *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
     {
         LaunchScope ls(c, s, "tensor_mul");
-        tensor_mul_kernel<<<dim3((unsigned)((S + 255) / 256), B), 256, 0, s>>>(d_a, d_b, prod, prod + 2 * S, c->d_mod, (uint32_t)N, (uint32_t)l,
+        launch_k(tensor_mul_kernel, dim3((unsigned)((S + 255) / 256), B), 256, 0, s, d_a, d_b, prod, prod + 2 * S, c->d_mod, (uint32_t)N, (uint32_t)l,
                                                                              make_uint4((uint32_t)a_stride, (uint32_t)b_stride, (uint32_t)(3 * l), (uint32_t)(3 * l)));
         LAUNCH_CHECK("tensor_mul_kernel");
     }
@@ -2202,7 +2230,7 @@ extern "C" int b2_galois_prepare(b2_ctx *c, uint32_t elt) {
 static int gather_impl(b2_ctx *c, const uint32_t *perm, const uint64_t *src, uint64_t *dst, size_t n_limbs, cudaStream_t s) {
     const size_t n = n_limbs * c->N;
     LaunchScope ls(c, s, "galois_gather");
-    galois_gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, perm, (uint32_t)c->N, (uint32_t)n_limbs);
+    launch_k(galois_gather_kernel, (unsigned)((n + 255) / 256), 256, 0, s, src, dst, perm, (uint32_t)c->N, (uint32_t)n_limbs);
     LAUNCH_CHECK("galois_gather_kernel");
     return B2_OK;
 }
@@ -2210,8 +2238,8 @@ static int gather_impl(b2_ctx *c, const uint32_t *perm, const uint64_t *src, uin
 static int gather_split_impl(b2_ctx *c, const uint32_t *perm, const uint64_t *src, uint64_t *dst0, uint64_t *dst1, size_t l, bool acc, cudaStream_t s) {
     const size_t n = 2 * l * c->N;
     LaunchScope ls(c, s, "galois_gather");
-    if (acc) galois_split_kernel<true><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst0, dst1, perm, c->d_mod, (uint32_t)c->N, (uint32_t)l);
-    else galois_split_kernel<false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst0, dst1, perm, c->d_mod, (uint32_t)c->N, (uint32_t)l);
+    if (acc) launch_k(galois_split_kernel<true>, (unsigned)((n + 255) / 256), 256, 0, s, src, dst0, dst1, perm, c->d_mod, (uint32_t)c->N, (uint32_t)l);
+    else launch_k(galois_split_kernel<false>, (unsigned)((n + 255) / 256), 256, 0, s, src, dst0, dst1, perm, c->d_mod, (uint32_t)c->N, (uint32_t)l);
     LAUNCH_CHECK("galois_split_kernel");
     return B2_OK;
 }
@@ -2388,7 +2416,7 @@ extern "C" int b2_bsgs_mac(b2_ctx *c, size_t l, size_t M, const uint64_t *const 
     if (!pts || !babies || !d_out || M == 0) return fail(B2_EINVAL, "bsgs_mac: bad argument");
     const size_t n = l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "bsgs_mac");
-    bsgs_mac_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(pts, babies, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)M);
+    launch_k(bsgs_mac_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, pts, babies, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)M);
     LAUNCH_CHECK("bsgs_mac_kernel");
     return B2_OK;
 }
@@ -2400,7 +2428,7 @@ extern "C" int b2_bsgs_mac_multi(b2_ctx *c, size_t l, size_t M, size_t n_giants,
     if (!pts || !babies || !outs || M == 0 || n_giants < 1 || n_giants > 4) return fail(B2_EINVAL, "bsgs_mac_multi: bad argument (1 to 4 giants)");
     const size_t n = l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "bsgs_mac");
-    bsgs_mac_multi_kernel<4><<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(pts, babies, outs, c->d_mod, (uint32_t)c->N, (uint32_t)l,
+    launch_k(bsgs_mac_multi_kernel<4>, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, pts, babies, outs, c->d_mod, (uint32_t)c->N, (uint32_t)l,
                                                                                             (uint32_t)M, (uint32_t)n_giants);
     LAUNCH_CHECK("bsgs_mac_multi_kernel");
     return B2_OK;
@@ -2415,7 +2443,7 @@ extern "C" int b2_expand_signed(b2_ctx *c, size_t first_prime, size_t n_limbs, c
     const size_t n = n_limbs * c->N;
     {
         LaunchScope ls(c, s, "expand_signed");
-        expand_signed_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_signed, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
+        launch_k(expand_signed_kernel, (unsigned)((n + 255) / 256), 256, 0, s, d_signed, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
                                                                         (uint32_t)first_prime);
         LAUNCH_CHECK("expand_signed_kernel");
     }
@@ -2435,12 +2463,12 @@ extern "C" int b2_special_fft(b2_ctx *c, void *d_vals, void *d_out, const uint32
     LaunchScope ls(c, s, "special_fft");
     if (inverse) {
         for (uint32_t len = n; len >= 2; len >>= 1)
-            b2::cfft_stage_kernel<<<(n / 2 + 255) / 256, 256, 0, s>>>(v, n, len, d_rot, (const double2 *)d_ksi, M, 1);
-        b2::cfft_bitrev_kernel<<<(n + 255) / 256, 256, 0, s>>>(o, v, n, logn, scale);
+            launch_k(b2::cfft_stage_kernel, (n / 2 + 255) / 256, 256, 0, s, v, n, len, d_rot, (const double2 *)d_ksi, M, 1);
+        launch_k(b2::cfft_bitrev_kernel, (n + 255) / 256, 256, 0, s, o, v, n, logn, scale);
     } else {
-        b2::cfft_bitrev_kernel<<<(n + 255) / 256, 256, 0, s>>>(o, v, n, logn, scale);
+        launch_k(b2::cfft_bitrev_kernel, (n + 255) / 256, 256, 0, s, o, v, n, logn, scale);
         for (uint32_t len = 2; len <= n; len <<= 1)
-            b2::cfft_stage_kernel<<<(n / 2 + 255) / 256, 256, 0, s>>>(o, n, len, d_rot, (const double2 *)d_ksi, M, 0);
+            launch_k(b2::cfft_stage_kernel, (n / 2 + 255) / 256, 256, 0, s, o, n, len, d_rot, (const double2 *)d_ksi, M, 0);
     }
     LAUNCH_CHECK("special_fft kernels");
     return B2_OK;
@@ -2453,7 +2481,7 @@ extern "C" int b2_encode_round(b2_ctx *c, const void *d_u, int64_t *d_coeffs, vo
     if (!d_u || !d_coeffs) return fail(B2_EINVAL, "encode_round: null pointer");
     const uint32_t n = (uint32_t)(c->N / 2);
     LaunchScope ls(c, (cudaStream_t)stream, "encode_round");
-    b2::encode_round_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>((const double2 *)d_u, n, d_coeffs);
+    launch_k(b2::encode_round_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, (const double2 *)d_u, n, d_coeffs);
     LAUNCH_CHECK("encode_round_kernel");
     return B2_OK;
 }
@@ -2467,7 +2495,7 @@ extern "C" int b2_decode_compose(b2_ctx *c, size_t l, const uint64_t *d_res, con
     if (!d_res || !d_tab || !d_out) return fail(B2_EINVAL, "decode_compose: null pointer");
     if (l > (size_t)b2::B2_CRT_MAX_LIMBS) return fail(B2_ESIZE, "decode_compose: more than 64 limbs");
     LaunchScope ls(c, (cudaStream_t)stream, "decode_compose");
-    b2::decode_compose_kernel<<<(unsigned)((c->N + 127) / 128), 128, 0, (cudaStream_t)stream>>>(d_res, d_tab, c->d_mod, (uint32_t)c->N, (uint32_t)l, inv_scale,
+    launch_k(b2::decode_compose_kernel, (unsigned)((c->N + 127) / 128), 128, 0, (cudaStream_t)stream, d_res, d_tab, c->d_mod, (uint32_t)c->N, (uint32_t)l, inv_scale,
                                                                                               (double2 *)d_out);
     LAUNCH_CHECK("decode_compose_kernel");
     return B2_OK;
@@ -2490,10 +2518,10 @@ extern "C" int b2_sample(b2_ctx *c, int kind, const uint8_t *key32, const uint8_
     if (blocks * (size_t)(b2::B2_SAMPLE_RESERVE + 1) > 0xFFFFFFFFull) return fail(B2_ESIZE, "sample: the draw does not fit the block counter");
     LaunchScope ls(c, s, "sample");
     if (kind == 0)
-        b2::sample_uniform_kernel<<<(unsigned)((blocks + 127) / 128), 128, 0, s>>>((uint64_t *)d_out, k, c->d_mod, (uint32_t)first_prime, (uint32_t)c->N,
+        launch_k(b2::sample_uniform_kernel, (unsigned)((blocks + 127) / 128), 128, 0, s, (uint64_t *)d_out, k, c->d_mod, (uint32_t)first_prime, (uint32_t)c->N,
                                                                                   (uint32_t)blocks);
     else
-        b2::sample_small_kernel<<<(unsigned)((blocks + 127) / 128), 128, 0, s>>>((int64_t *)d_out, k, kind, (uint32_t)blocks);
+        launch_k(b2::sample_small_kernel, (unsigned)((blocks + 127) / 128), 128, 0, s, (int64_t *)d_out, k, kind, (uint32_t)blocks);
     LAUNCH_CHECK("sample kernel");
     return B2_OK;
 }
@@ -2512,7 +2540,7 @@ extern "C" int b2_expand_single_chain_batch(b2_ctx *c, size_t l, size_t M, const
     const size_t n = M * l * c->N;
     {
         LaunchScope ls(c, s, "expand_signed");
-        expand_signed_batch_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_signed, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)M);
+        launch_k(expand_signed_batch_kernel, (unsigned)((n + 255) / 256), 256, 0, s, d_signed, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)M);
         LAUNCH_CHECK("expand_signed_batch_kernel");
     }
     return run_fwd(c, d_out, d_out, nullptr, (uint32_t)(M * l), 0, EpiStore{}, s, (uint32_t)l);
@@ -2523,7 +2551,7 @@ extern "C" int b2_poly_op(b2_ctx *c, int op, size_t n_limbs, const uint64_t *d_a
     if (op < 0 || op > 3 || !d_a || !d_out || (op != 3 && !d_b) || n_limbs < 1 || n_limbs > c->size_QP) return fail(B2_EINVAL, "poly_op: bad argument");
     const size_t n = n_limbs * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_op");
-    poly_op_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
+    launch_k(poly_op_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
                                                                                    (uint32_t)n_limbs, 0);
     LAUNCH_CHECK("poly_op_kernel");
     return B2_OK;
@@ -2535,7 +2563,7 @@ extern "C" int b2_ct_op(b2_ctx *c, int op, size_t l, size_t n_poly, const uint64
         return fail(B2_EINVAL, "ct_op: bad argument");
     const size_t n = n_poly * l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_op");
-    poly_op_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(n_poly * l),
+    launch_k(poly_op_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(n_poly * l),
                                                                                    (uint32_t)l, op == 2);
     LAUNCH_CHECK("poly_op_kernel");
     return B2_OK;
@@ -2552,7 +2580,7 @@ extern "C" int b2_poly_scalar(b2_ctx *c, int op, size_t n_limbs, const uint64_t 
     }
     const size_t n = n_limbs * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_scalar");
-    poly_scalar_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(op, d_a, tab, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
+    launch_k(poly_scalar_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, op, d_a, tab, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
                                                                                        (uint32_t)n_limbs);
     LAUNCH_CHECK("poly_scalar_kernel");
     return B2_OK;
@@ -2568,7 +2596,7 @@ extern "C" int b2_ct_scalar(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *
     }
     const size_t n = n_poly * l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_scalar");
-    poly_scalar_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(1, d_a, tab, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(n_poly * l),
+    launch_k(poly_scalar_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, 1, d_a, tab, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(n_poly * l),
                                                                                        (uint32_t)l);
     LAUNCH_CHECK("poly_scalar_kernel");
     return B2_OK;
@@ -2597,7 +2625,7 @@ extern "C" int b2_ct_lincomb(b2_ctx *c, size_t l, size_t n_poly, size_t n_terms,
     }
     const size_t n = n_poly * l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "lincomb");
-    lincomb_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)n_poly,
+    launch_k(lincomb_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, a, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)n_poly,
                                                                                    (uint32_t)n_terms);
     LAUNCH_CHECK("lincomb_kernel");
     return B2_OK;
@@ -2978,8 +3006,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 m.dig_bs = per, m.own_bs = (uint32_t)l, m.ct_bs = (uint32_t)(2 * l);
                 m.cxp_i = 2 * B, m.cxp_k = B, m.cxp_bs = 1;
                 LaunchScope ls(c, s, "ntt_fwd_rows_mac");
-                ntt_fwd_rows_mac<8, Cfg::R_CONTIG, Cfg::LOG_C>
-                    <<<dim3(B, (sp.nq + sp.np) * (uint32_t)(N >> (8 + Cfg::LOG_C))), pass_threads<8>(), mac_smem_bytes<8, Cfg::R_CONTIG, Cfg::LOG_C>(), s>>>(na, m);
+                launch_k(ntt_fwd_rows_mac<8, Cfg::R_CONTIG, Cfg::LOG_C>, dim3(B, (sp.nq + sp.np) * (uint32_t)(N >> (8 + Cfg::LOG_C))), pass_threads<8>(), mac_smem_bytes<8, Cfg::R_CONTIG, Cfg::LOG_C>(), s, na, m);
                 LAUNCH_CHECK("ntt_fwd_rows_mac");
             } else {
                 rc = run_fwd(c, UP, UP, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});

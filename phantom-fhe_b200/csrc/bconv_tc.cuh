@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "bconv_tc_plan.h"
+#include "modarith.cuh"
 
 namespace b2 {
 
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(128 * WG) bconv_tc_kernel(const uint64_t *__re
                                                             const uint64_t *__restrict__ copy_src, const TcJob *__restrict__ jobs,
                                                             const TcGroup *__restrict__ groups, const uint8_t *__restrict__ images, uint32_t N,
                                                             uint32_t *err) {
+    pdl_enter();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t *sA = tc_smem, *sB = tc_smem + TC_SMEM_A;
     uint64_t *bar = reinterpret_cast<uint64_t *>(tc_smem + TC_SMEM_CTRL);
@@ -316,6 +318,7 @@ __global__ void __launch_bounds__(128 * WG) bconv_tc_persist(const uint64_t *__r
                                                              const uint64_t *__restrict__ copy_src, const TcJob *__restrict__ jobs,
                                                              const TcGroup *__restrict__ groups, const uint8_t *__restrict__ images, uint32_t N,
                                                              uint32_t n_jobs, uint32_t alloc_cols, uint32_t *err, const TcBatch tb) {
+    pdl_enter();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t *sB = tc_smem + TCP_SMEM_B;
     TcOutS *sOut = reinterpret_cast<TcOutS *>(tc_smem + TCP_SMEM_GRP);              // [16][4]

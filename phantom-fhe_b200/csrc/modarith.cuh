@@ -11,6 +11,10 @@
 
 namespace b2 {
 
+// First statement of every kernel: waits for the previous kernel of the stream to have completed (see launch_k). Nothing a
+// kernel of the stream writes may be read before it.
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // {w, floor(w * 2^64 / q)}
 struct __align__(16) W2 {
     uint64_t w, ws;

@@ -440,6 +440,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
 template <int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, int SRC = 0>
 __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2)), 1 << (R1 > R2 ? R1 : R2)))
 ntt_fwd_pass(NttArgs a, Epi epi) {
+    pdl_enter();
     static_assert(R1 + R2 == LOG_T, "stage split");
     constexpr int TT = 1 << LOG_T, C = 1 << LOG_C;
     __shared__ uint64_t sm[C * (TT + (TT >> R2))];
@@ -666,6 +667,7 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
 
 template <int LOG_T, int R, int LOG_C>
 __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) >> R, 3) ntt_fwd_rows_mac(NttArgs a, const __grid_constant__ MacArgs m) {
+    pdl_enter();
     static_assert(2 * R == LOG_T, "equal stage groups: one register group per thread in both");
     constexpr int TT = 1 << LOG_T, C = 1 << LOG_C;
     constexpr int TPAD = TT + (TT >> R);
@@ -786,6 +788,7 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
 template <int LOG_T, int RA, int RB, int LOG_C, bool COLS, bool LAST>
 __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (RA > RB ? RA : RB)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (RA > RB ? RA : RB)), 1 << (RA > RB ? RA : RB)))
 ntt_inv_pass(NttArgs a) {
+    pdl_enter();
     static_assert(RA + RB == LOG_T, "stage split");
     constexpr int TT = 1 << LOG_T, C = 1 << LOG_C;
     __shared__ uint64_t sm[C * (TT + (TT >> RA))];
@@ -824,6 +827,7 @@ __device__ __forceinline__ void stage_tile(uint64_t *buf, const uint64_t *src, s
 template <int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi>
 __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2))))
 ntt_fwd_pipe(NttArgs a, Epi epi, uint32_t total) {
+    pdl_enter();
     static_assert(R1 == R2, "pipelined passes are built for equal stage groups");
     constexpr int TT = 1 << LOG_T, C = 1 << LOG_C, THREADS = (C * TT) >> R1;
     __shared__ __align__(16) uint64_t buf[2][C * (TT + (TT >> R2))];
@@ -853,6 +857,7 @@ ntt_fwd_pipe(NttArgs a, Epi epi, uint32_t total) {
 template <int LOG_T, int RA, int RB, int LOG_C, bool COLS, bool LAST>
 __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (RA > RB ? RA : RB)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (RA > RB ? RA : RB))))
 ntt_inv_pipe(NttArgs a, uint32_t total) {
+    pdl_enter();
     static_assert(RA == RB, "pipelined passes are built for equal stage groups");
     constexpr int TT = 1 << LOG_T, C = 1 << LOG_C, THREADS = (C * TT) >> RA;
     constexpr bool FIRST = !COLS;
@@ -989,6 +994,7 @@ __device__ __forceinline__ void fwd_cluster_body(const NttArgs &a, const Epi &ep
 
 template <class Epi>
 __global__ void __cluster_dims__(CL_SIZE, 1, 1) __launch_bounds__(CL_THREADS, 2) ntt_fwd_cluster(NttArgs a, Epi epi) {
+    pdl_enter();
     extern __shared__ __align__(16) uint64_t cl_smem[];
     const Job job = get_job(a, blockIdx.x / CL_SIZE);
     const Mod md = a.mod[job.y];
@@ -1073,6 +1079,7 @@ __device__ __forceinline__ void inv_cluster_body(const NttArgs &a, uint64_t *sme
 }
 
 __global__ void __cluster_dims__(CL_SIZE, 1, 1) __launch_bounds__(CL_THREADS, 2) ntt_inv_cluster(NttArgs a) {
+    pdl_enter();
     extern __shared__ __align__(16) uint64_t cl_smem[];
     const Job job = get_job(a, blockIdx.x / CL_SIZE);
     const Mod md = a.mod[job.y];

@@ -60,6 +60,7 @@ __device__ __forceinline__ uint64_t word_of(const uint32_t (&b)[16], int i) { re
 // grid: one thread per block of the keystream = 8 coefficients; total_blocks = n_limbs * N / 8
 __global__ void __launch_bounds__(128) sample_uniform_kernel(uint64_t *__restrict__ out, const ChaChaKey key, const Mod *mod, uint32_t first_prime,
                                                              uint32_t N, uint32_t total_blocks) {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total_blocks) return;
     const Mod md = mod[first_prime + t / (N >> 3)];
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(128) sample_uniform_kernel(uint64_t *__restric
 
 // kind 1: centred binomial with 21 coin pairs; kind 2: uniform ternary. One thread per block = 8 signed coefficients.
 __global__ void __launch_bounds__(128) sample_small_kernel(int64_t *__restrict__ out, const ChaChaKey key, int kind, uint32_t n_blocks) {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_blocks) return;
     uint32_t blk[16];
