@@ -198,8 +198,6 @@ struct LevelPlan {
     double *matd_up = nullptr;     // mat_up as 21-bit pieces of (entry * 2^64 mod p), [..][3]
     BconvGroup *grp_dn = nullptr;  // 2 (one per polynomial)
     uint2 *outs_dn = nullptr;      // l entries shared by both groups
-    BconvGroup *grp_rs = nullptr;  // 3
-    uint2 *outs_rs = nullptr;      // l-1
     void *blob = nullptr;
     TcSet tc_up, tc_dn, tc_dnf;    // tensor-core form of the ModUp / ModDown / fused-ModDown conversions
     void *tc_blob = nullptr;
@@ -220,8 +218,7 @@ struct b2_ctx {
     W2 *d_macfin = nullptr;     // [size_QP] closing constant of the fused inner product's Montgomery sums: P^-1 * 2^64 mod q_j, 2^64 mod p_i
     uint64_t *d_mat_dn = nullptr;  // [size_Q][size_P]: (P/p_i) mod q_j
     uint64_t *d_mat_dn_pinv = nullptr;  // the same times P^-1 mod q_j (fused key switch)
-    uint64_t *d_one = nullptr;     // [size_QP] ones: the [n_out][1] "matrix" of the rescale reduction
-    double *d_matd_dn = nullptr, *d_matd_dn_pinv = nullptr, *d_matd_one = nullptr;  // FP64 piece forms
+    double *d_matd_dn = nullptr, *d_matd_dn_pinv = nullptr;  // FP64 piece forms
     struct RedcMeta {
         uint64_t p, ninv;  // ninv = -p^-1 mod 2^64
         uint32_t pieces, pad;
@@ -238,8 +235,6 @@ struct b2_ctx {
     uint32_t tc_max_groups = 16;   // B2_BCONV_GROUPS: column groups per conversion job (8: at most 128 TMEM columns, four CTAs per SM)
     uint32_t *d_err = nullptr;     // device status word: set by a kernel whose bounded wait ran out
     std::vector<uint64_t> h_mat_dn, h_mat_dn_pinv;  // host copies of the ModDown matrices [size_Q][size_P]
-    bool use_cluster = false;      // N = 2^16: single-launch transforms on 8-CTA clusters
-    bool use_pipe = false;         // N = 2^16: persistent passes with asynchronous double-buffered tile loads
     bool mac_interleave = false;   // B2_KS_FUSED_ORDER=1: consecutive CTAs of the fused pass walk limbs, not tiles (measured slower)
     // The fused pass may also take the limbs on primes of 41 bits and more (q0 and P at the usual parameters): 10 launches
     // instead of 12 and no stored digits at all. Measured on B200 at N = 2^16, l = 24: single calls lose 4 % of their
@@ -397,8 +392,6 @@ static int build_level(b2_ctx *c, size_t l) {
     auto *matd_up = blob_take<double>(cur, mat_up_words * 3);
     auto *grp_dn = blob_take<BconvGroup>(cur, 2);
     auto *outs_dn = blob_take<uint2>(cur, l);
-    auto *grp_rs = blob_take<BconvGroup>(cur, 3);
-    auto *outs_rs = blob_take<uint2>(cur, l);
     const size_t used = cur - host.data();
     if (used > bytes) return fail(B2_ENOMEM, "level blob overflow");
 
@@ -463,14 +456,12 @@ static int build_level(b2_ctx *c, size_t l) {
         const uint64_t ql = c->q[l - 1];
         for (size_t j = 0; j + 1 < l; j++) {
             qlast_inv[j] = h_w2(h_invmod(ql % c->q[j], c->q[j]), c->q[j]);
-            outs_rs[j] = make_uint2((uint32_t)j, (uint32_t)j);
         }
         for (size_t p = 0; p < 3; p++) {
             jobs_rs_intt[p] = make_uint4((uint32_t)(p * l + l - 1), (uint32_t)(l - 1), (uint32_t)(l - 1), (uint32_t)p);
             for (size_t j = 0; j + 1 < l; j++)
                 jobs_rs_ntt[p * (l - 1) + j] =
                     make_uint4((uint32_t)(p * (l - 1) + j), (uint32_t)j, (uint32_t)(p * l + j), (uint32_t)(p * (l - 1) + j));
-            grp_rs[p] = BconvGroup{(uint32_t)p, 1, 0, 0, (uint32_t)(l - 1), (uint32_t)(p * (l - 1)), 0, h_npieces(ql)};
         }
     }
     if (cudaMalloc(&pl.blob, used) != cudaSuccess) return fail(B2_ENOMEM, "cudaMalloc(level plan) failed");
@@ -499,8 +490,6 @@ static int build_level(b2_ctx *c, size_t l) {
     pl.matd_up = (double *)dev(matd_up);
     pl.grp_dn = (BconvGroup *)dev(grp_dn);
     pl.outs_dn = (uint2 *)dev(outs_dn);
-    pl.grp_rs = (BconvGroup *)dev(grp_rs);
-    pl.outs_rs = (uint2 *)dev(outs_rs);
     if (c->bconv_tc) {
         // the same conversions as tensor-core jobs: ModUp digits, then ModDown of up to two polynomials with the plain
         // matrix (cx layout [2][lP]) and with the P^-1-carrying one (compact P limbs [2][alpha])
@@ -548,10 +537,8 @@ extern "C" void b2_ctx_destroy(b2_ctx *c) {
     cudaFree(c->d_macfin);
     cudaFree(c->d_mat_dn);
     cudaFree(c->d_mat_dn_pinv);
-    cudaFree(c->d_one);
     cudaFree(c->d_matd_dn);
     cudaFree(c->d_matd_dn_pinv);
-    cudaFree(c->d_matd_one);
     cudaFree(c->d_redc);
     for (auto &pl : c->plan) {
         cudaFree(pl.blob);
@@ -651,8 +638,7 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
         Pinv[j] = h_w2(h_invmod(P, qj), qj);
         for (size_t i = 0; i < sP; i++) mat_dn_pinv[j * sP + i] = h_mulmod(mat_dn[j * sP + i], Pinv[j].w, qj);
     }
-    const std::vector<uint64_t> ones(size_QP, 1);
-    std::vector<double> matd_dn(3 * sQ * sP), matd_dn_pinv(3 * sQ * sP), matd_one(3 * size_QP);
+    std::vector<double> matd_dn(3 * sQ * sP), matd_dn_pinv(3 * sQ * sP);
     std::vector<b2_ctx::RedcMeta> redc(size_QP);
     for (size_t j = 0; j < sQ; j++)
         for (size_t i = 0; i < sP; i++) {
@@ -660,7 +646,6 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
             h_pieces(mat_dn_pinv[j * sP + i], c->q[j], &matd_dn_pinv[3 * (j * sP + i)]);
         }
     for (size_t j = 0; j < size_QP; j++) {
-        h_pieces(1, c->q[j], &matd_one[3 * j]);
         uint64_t inv = 1;  // Newton: inv = q^-1 mod 2^64
         for (int it = 0; it < 6; it++) inv *= 2 - c->q[j] * inv;
         redc[j] = b2_ctx::RedcMeta{c->q[j], (uint64_t)(0 - inv), h_npieces(c->q[j]), 0, 0, {0, 0, 0, 0}, {0, 0, 0, 0}};
@@ -721,18 +706,13 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
     }
     if (e == cudaSuccess) e = up((void **)&c->d_mat_dn, mat_dn.data(), 8 * sQ * sP);
     if (e == cudaSuccess) e = up((void **)&c->d_mat_dn_pinv, mat_dn_pinv.data(), 8 * sQ * sP);
-    if (e == cudaSuccess) e = up((void **)&c->d_one, ones.data(), 8 * size_QP);
     if (e == cudaSuccess) e = up((void **)&c->d_matd_dn, matd_dn.data(), 8 * matd_dn.size());
     if (e == cudaSuccess) e = up((void **)&c->d_matd_dn_pinv, matd_dn_pinv.data(), 8 * matd_dn_pinv.size());
-    if (e == cudaSuccess) e = up((void **)&c->d_matd_one, matd_one.data(), 8 * matd_one.size());
     if (e == cudaSuccess) e = up((void **)&c->d_redc, redc.data(), sizeof(b2_ctx::RedcMeta) * size_QP);
     if (e != cudaSuccess) {
         b2_ctx_destroy(c);
         return fail((int)e, std::string("ctx_create: table upload failed: ") + cudaGetErrorString(e));
     }
-    // B2_NTT_CLUSTER=1 selects the single-launch cluster transforms at N = 2^16. They are bit-exact
-    // but measured slower than the two-launch transforms on B200 (register pressure, two CTAs per
-    // SM), so they stay opt-in.
     c->h_mat_dn = mat_dn;
     c->h_mat_dn_pinv = mat_dn_pinv;
     {
@@ -780,14 +760,10 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
             }
         }
     }
-    const char *env_cl = getenv("B2_NTT_CLUSTER");
-    c->use_cluster = (c->logN == 16) && env_cl && env_cl[0] == '1';
-    const char *env_pipe = getenv("B2_NTT_PIPE");
-    c->use_pipe = (c->logN == 16) && env_pipe && env_pipe[0] == '1';
     const char *env_mac = getenv("B2_KS_FUSED_IP");
     if (const char *e = getenv("B2_KS_FUSED_WIDE")) c->mac_wide = e[0] != '0' ? 1 : 0;
     if (const char *e = getenv("B2_KS_FUSED_ORDER")) c->mac_interleave = e[0] == '1';
-    c->use_mac = (c->logN == 15 || c->logN == 16) && !c->use_cluster && !c->use_pipe && !(env_mac && env_mac[0] == '0');
+    c->use_mac = (c->logN == 15 || c->logN == 16) && !(env_mac && env_mac[0] == '0');
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
     if (c->sm_count < 1) c->sm_count = 148;
     c->plan.resize(sQ + 1);
@@ -836,13 +812,6 @@ static constexpr int pass_threads() {
     return (1 << ((COLS ? P::LOG_CC : P::LOG_C) + LOG_T)) >> (P::R_STRIDED > P::R_CONTIG ? P::R_STRIDED : P::R_CONTIG);
 }
 
-// grid of a pipelined pass: every CTA gets the same number of tiles (as far as divisibility allows)
-static uint32_t pipe_grid(const b2_ctx *c, uint32_t total) {
-    const uint32_t slots = (uint32_t)c->sm_count * 6;
-    const uint32_t per_cta = (total + slots - 1) / slots;
-    return (total + per_cta - 1) / per_cta;
-}
-
 // grid of a two-pass transform kernel over `work` tiles and `batch` sets
 static dim3 pass_grid(NttArgs &, uint32_t work, uint32_t batch) { return dim3(work, batch); }
 
@@ -851,20 +820,6 @@ static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const 
     using A = PassCfg<LOG_A>;
     using B = PassCfg<LOG_B>;
     const uint32_t N = 1u << a.logN;
-    if constexpr (LOG_A == 8 && LOG_B == 8 && SRC == 0) {
-        if (c->use_pipe) {
-            const uint32_t total = njobs * (N >> (LOG_A + A::LOG_C));
-            {
-                LaunchScope ls(c, s, "ntt_fwd_cols");
-                launch_k(ntt_fwd_pipe<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_C, true, false, EpiStore>, pipe_grid(c, total), pass_threads<LOG_A>(), 0, s, a, EpiStore{}, total);  // the pipelined passes keep 8 columns
-            }
-            NttArgs b = a;
-            b.src = a.dst;
-            LaunchScope ls(c, s, "ntt_fwd_rows");
-            launch_k(ntt_fwd_pipe<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi>, pipe_grid(c, total), pass_threads<LOG_B>(), 0, s, b, epi, total);
-            return;
-        }
-    }
     {
         NttArgs a1 = a;
         const dim3 grid = pass_grid(a1, njobs * (N >> (LOG_A + A::LOG_CC)), batch);
@@ -896,20 +851,6 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
     using A = PassCfg<LOG_A>;
     using B = PassCfg<LOG_B>;
     const uint32_t N = 1u << a.logN;
-    if constexpr (LOG_A == 8 && LOG_B == 8) {
-        if (c->use_pipe) {
-            const uint32_t total = njobs * (N >> (LOG_B + B::LOG_C));
-            {
-                LaunchScope ls(c, s, "ntt_inv_rows");
-                launch_k(ntt_inv_pipe<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false>, pipe_grid(c, total), pass_threads<LOG_B>(), 0, s, a, total);
-            }
-            NttArgs b = a;
-            b.src = a.dst;
-            LaunchScope ls(c, s, "ntt_inv_cols");
-            launch_k(ntt_inv_pipe<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_C, true, true>, pipe_grid(c, total), pass_threads<LOG_A>(), 0, s, b, total);
-            return;
-        }
-    }
     {
         NttArgs a1 = a;
         const dim3 grid = pass_grid(a1, njobs * (N >> (LOG_B + B::LOG_C)), batch);
@@ -936,17 +877,7 @@ static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
     NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, period, src_div, src_q, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
-    if (bd.batch != 1 && (c->use_cluster || c->use_pipe)) return fail(B2_EINVAL, "batched transforms need the two-pass kernels");
-    if (SRC != 0 && (c->use_cluster || src_div == 0)) return fail(B2_EINVAL, "the on-the-fly source needs the two-pass transform");
-    if (c->use_cluster) {
-        // the attribute belongs to the (function, device) pair; setting it is cheap, so it is set on every launch path
-        // rather than remembered per thread (a thread may drive contexts on several devices)
-        CUDA_TRY(cudaFuncSetAttribute(ntt_fwd_cluster<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM));
-        LaunchScope ls(c, s, "ntt_fwd_cluster");
-        launch_k(ntt_fwd_cluster<Epi>, njobs * CL_SIZE, CL_THREADS, CL_SMEM, s, a, epi);
-        LAUNCH_CHECK("ntt_fwd_cluster");
-        return B2_OK;
-    }
+    if (SRC != 0 && src_div == 0) return fail(B2_EINVAL, "the on-the-fly source needs its divisor");
     switch (c->logN) {
         case 17: launch_fwd<8, 9, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
         case 16: launch_fwd<8, 8, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
@@ -965,14 +896,6 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
     NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
-    if (bd.batch != 1 && (c->use_cluster || c->use_pipe)) return fail(B2_EINVAL, "batched transforms need the two-pass kernels");
-    if (c->use_cluster) {
-        CUDA_TRY(cudaFuncSetAttribute(ntt_inv_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM));
-        LaunchScope ls(c, s, "ntt_inv_cluster");
-        launch_k(ntt_inv_cluster, njobs * CL_SIZE, CL_THREADS, CL_SMEM, s, a);
-        LAUNCH_CHECK("ntt_inv_cluster");
-        return B2_OK;
-    }
     switch (c->logN) {
         case 17: launch_inv<8, 9>(c, a, njobs, s, bd.batch); break;
         case 16: launch_inv<8, 8>(c, a, njobs, s, bd.batch); break;
@@ -1221,7 +1144,7 @@ __global__ void __launch_bounds__(256) ks_inner_prod_kernel(const uint64_t *__re
     // (src/rns_bconv.cu:522-528), so the digit buffer need not hold a copy of it
     const uint32_t own_d = (own && t < l) ? t / (lP - l) : 0xFFFFFFFFu;
     const uint2 p2 = perm ? *reinterpret_cast<const uint2 *>(perm + n) : make_uint2(0, 0);
-    if (md.q < b2::FP_LIMIT) {
+    if (md.q < b2::FP_SMALL_LIMIT) {
         // Small prime (uniform over the block): digits and key words are below 2^41, so each product
         // is four exact FP64 FMAs on 21-bit pieces instead of five wide integer multiplies, and the
         // reduction of sum_w A_w 2^(21 w) stays in FP64 too. Same residues as the integer path.
@@ -1452,22 +1375,6 @@ __global__ void __launch_bounds__(256) expand_signed_kernel(const int64_t *__res
     u128 v{mag, 0};
     const uint64_t r = barrett128(v, md.q, md.r0, md.r1);
     dst[idx] = (c >= 0 || r == 0) ? r : md.q - r;
-}
-
-// Centred remainder of the dropped limb, reduced into every remaining prime: with it the rescale
-// rounds to nearest instead of flooring. r: [n_poly][N] coefficient form mod q_last.
-__global__ void __launch_bounds__(256) rescale_centre_kernel(const uint64_t *__restrict__ r, uint64_t *__restrict__ out, const Mod *mod, uint32_t N,
-                                                            uint32_t n_out, uint32_t n_poly) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_poly * n_out * N) return;
-    const uint32_t i = (uint32_t)(idx % N), j = (uint32_t)((idx / N) % n_out), p = (uint32_t)(idx / ((size_t)N * n_out));
-    const Mod md = mod[j];
-    const uint64_t ql = mod[n_out].q, half = ql >> 1;
-    const uint64_t v = r[(size_t)p * N + i];
-    uint64_t d = barrett64(v, md.q, md.r1);
-    if (v > half) d = sub_mod(d, barrett64(ql, md.q, md.r1), md.q);  // v - q_last, the negative representative
-    out[idx] = d;
 }
 
 // out = sum_t x_t * s_t (+ c on polynomial 0): per-limb integer weights, one reduction per value. The terms may
@@ -1825,7 +1732,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853)
     const bool mac = c->use_mac && (batched || c->logN == 16 || c->mac_wide == 1) && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
     if (!mac && !batched) return B2_OK;
-    if (batched && (!c->bconv_tc || c->tc_simple || c->use_cluster || c->use_pipe || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
+    if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
         return B2_OK;  // the caller falls back to one key switch at a time
     {
         using Cfg = PassCfg<8>;
@@ -2015,25 +1922,13 @@ extern "C" int b2_multiply_and_relin(b2_ctx *c, size_t l, const uint64_t *d_a, c
 // Second half of a rescale. r [n_poly][N]: the dropped limb of every polynomial in coefficient form. Every remaining
 // limb j gets (in_j - NTT_j(rem mod q_j)) * q_last^-1 with rem = r (MODE 1, the reference's floor: src/rns.cu:1128-1183)
 // or its centred representative (MODE 2, round to nearest). The forward column pass reduces r into q_j as it loads, so
-// the (l-1) reduced copies are never written out; the one-launch and pipelined transform variants have no such load and
-// go through a reduction kernel first.
+// the (l-1) reduced copies are never written out.
 template <int MODE>
 static int rescale_tail(const b2_ctx *c, size_t l, size_t n_poly, const uint64_t *r, const uint64_t *d_in, uint64_t *d_out, cudaStream_t s) {
     const LevelPlan &pl = c->plan[l];
     EpiSubMul<false> epi{d_in, d_out, pl.qlast_inv};
     const uint32_t njobs = (uint32_t)(n_poly * (l - 1));
-    if (!c->use_cluster && !c->use_pipe) return run_fwd<EpiSubMul<false>, MODE>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, (uint32_t)(l - 1), c->q[l - 1]);
-    if (MODE == 1) {
-        // r mod q_j for every remaining prime: a base conversion with one input and the matrix [1]
-        int rc = run_bconv(c, false, r, d_out, nullptr, pl.grp_rs, (uint32_t)n_poly, pl.outs_rs, c->d_one, c->d_matd_one, 1, (uint32_t)(l - 1), true, s);
-        if (rc) return rc;
-    } else {
-        const size_t n = n_poly * (l - 1) * c->N;
-        LaunchScope ls(c, s, "rescale_centre");
-        launch_k(rescale_centre_kernel, (unsigned)((n + 255) / 256), 256, 0, s, r, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(l - 1), (uint32_t)n_poly);
-        LAUNCH_CHECK("rescale_centre_kernel");
-    }
-    return run_fwd(c, d_out, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s);
+    return run_fwd<EpiSubMul<false>, MODE>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, (uint32_t)(l - 1), c->q[l - 1]);
 }
 
 extern "C" int b2_rescale(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *d_in, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
@@ -2110,15 +2005,6 @@ extern "C" int b2_multiply_relin_rescale_batch(b2_ctx *c, size_t l, size_t batch
     if (!rescale) {
         for (size_t b = 0; b < batch; b++)
             CUDA_TRY(cudaMemcpyAsync(d_out + b * out_stride * N, prod + b * 3 * S, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
-        return B2_OK;
-    }
-    if (c->use_cluster || c->use_pipe) {
-        for (size_t b = 0; b < batch; b++) {
-            rc = run_inv(c, prod + b * 3 * S, r, c->plan[l].jobs_rs_intt, 2, 0, c->d_fin_plain, s);
-            if (rc) return rc;
-            rc = rescale_tail<1>(c, l, 2, r, prod + b * 3 * S, d_out + b * out_stride * N, s);
-            if (rc) return rc;
-        }
         return B2_OK;
     }
     const LevelPlan &pl = c->plan[l];

@@ -314,7 +314,7 @@ __device__ __forceinline__ void tcp_fetch_a(uint8_t *sA, const uint64_t *__restr
 }
 
 template <int WG>
-__global__ void __launch_bounds__(128 * WG) bconv_tc_persist(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
+__global__ void __launch_bounds__(128 * WG, 8 / WG) bconv_tc_persist(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
                                                              const uint64_t *__restrict__ copy_src, const TcJob *__restrict__ jobs,
                                                              const TcGroup *__restrict__ groups, const uint8_t *__restrict__ images, uint32_t N,
                                                              uint32_t n_jobs, uint32_t alloc_cols, uint32_t *err, const TcBatch tb) {

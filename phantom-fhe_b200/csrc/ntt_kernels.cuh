@@ -182,70 +182,137 @@ __device__ __forceinline__ int pad_idx(int e) { return e + (e >> RC); }
 // ================================================================================================
 // arithmetic policies
 // ================================================================================================
-// On B200 a 32x32->64-bit integer multiply issues at a quarter of the rate of a double-precision
-// FMA (measured: ~16 vs 64 lanes per clock per SM), and a 64-bit Shoup product needs six of them.
-// Primes below 2^41 therefore run their butterflies in FP64: residues are held as doubles with
+// On B200 a 32x32->64-bit integer multiply issues at less than half the rate of a double-precision
+// FMA (measured: ~26 against ~62 lanes per clock per SM), and a 64-bit Shoup product needs six of
+// them. Primes below 2^50 therefore run their butterflies in FP64: residues are held as doubles with
 // exact integer values, a modular product is
 //     h = y*w,  l = fma(y,w,-h)            (h + l = y*w exactly)
-//     c = rint(y * (w/q))                  (quotient estimate, off by at most one)
-//     r = fma(-c, q, h) + l                (exact: |h - c q| < 2^53), r = y*w (mod q), |r| < q
-// and a butterfly costs 8 FP64 instructions and no integer multiply. Ranges: a forward stage grows
-// a residue by < q (|x| < 17q after 16 stages); an inverse stage doubles the bound and every pass
-// renormalises once, so products never see |y| >= 2^50. Results are converted back to canonical
-// uint64 at the end, so outputs are bit-identical to the integer path.
-// Larger primes use 64-bit Shoup/Harvey butterflies; below 2^46 without any conditional
-// subtraction (forward: < 33q after 16 stages; inverse: < 2^17 q), above with one per butterfly.
-constexpr uint64_t FP_LIMIT = 1ull << 41;
-constexpr uint64_t WIDE_LIMIT = 1ull << 46;
+//     c = rint(y * (w/q))                  (quotient estimate)
+//     r = fma(-c, q, h) + l                (exact: |h - c q| < 2^53), r = y*w (mod q)
+// and a butterfly costs 8 FP64 instructions and no integer multiply. Results are converted back to
+// canonical uint64 at the end, so outputs are bit-identical to the integer path.
+//
+// Every policy says how large a residue may be where, in units of its own, and the stage runners below
+// evaluate those rules at compile time: a correction is emitted only where a bound would be passed.
+//   ct_out(B)          bound after a forward stage whose inputs are bounded by B; ct<B> is that butterfly
+//   gs_sum / gs_prod   bounds of the two outputs of an inverse butterfly; gs(.., ba, bb) is that butterfly
+//   group_end          what is done to a residue that changes thread between two stage groups of a pass
+//   pass_end           what is done to a residue that is stored between the passes of an inverse transform
+//   B_CANON / B_PASS / GS_PASS   bounds of canonical input, of what a forward / an inverse pass stores
+constexpr uint64_t FP_SMALL_LIMIT = 1ull << 41;
+constexpr uint64_t FP_LIMIT = 1ull << 50;
+constexpr uint64_t INT_LAZY_LIMIT = 1ull << 60;
 constexpr double FP_MAGIC = 6755399441055744.0;  // 1.5 * 2^52: (v + M) - M = rint(v) for |v| < 2^51
 constexpr double FP_2_52 = 4503599627370496.0;
 
-template <bool WIDE>
-struct ArithInt {
+// Primes of [2^50, 2^60): residues run up to 16 q in a 64-bit word, bounds in units of q. The quotient of the Shoup product
+// leaves out the lowest of its four partial products (one low at most, so the product is below 3 q), and instead of a
+// conditional subtraction per butterfly (six ALU instructions on 64-bit words) a residue is brought below 2 q by a 32-bit
+// quotient estimate (four instructions) every fourth stage or so. Inverse passes over 60-bit primes, N = 2^16, on B200: see
+// launch_inv.
+struct ArithIntLazy {
     using T = uint64_t;
     using Tw = W2;
     struct K {
-        uint64_t q, q2, r1;
-        int logN;
+        uint64_t q, nq;   // nq = -q mod 2^64
+        uint32_t m, s;    // floor(2^(64 + s) / q), normalised to 32 bits
     };
-    __device__ __forceinline__ static K make(const Mod &md, int logN) { return K{md.q, 2 * md.q, md.r1, logN}; }
+    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_PASS = 16, GS_PASS = 6;
+    __device__ __forceinline__ static K make(const Mod &md, int) {
+        const uint32_t s = __clz((uint32_t)md.r1);  // r1 = floor(2^64 / q), in [2^4, 2^14]
+        return K{md.q, 0 - md.q, (uint32_t)((md.r1 << s) | (md.r0 >> (64 - s))), s};
+    }
     __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &) { return ldg_w2(tw + idx); }
     __device__ __forceinline__ static Tw ldfin(const W2 *p, const K &) { return ldg_w2(p); }
     __device__ __forceinline__ static T from_u64(uint64_t v, const K &) { return v; }
     __device__ __forceinline__ static T from_raw(uint64_t v) { return v; }
     __device__ __forceinline__ static uint64_t to_raw(T v) { return v; }
+    // x - k q with k = floor(x / q) or one less: below 2 q for any x
+    __device__ __forceinline__ static T reduce(T x, const K &k) {
+        const uint32_t c = __umulhi((uint32_t)(x >> 32), k.m) >> k.s;
+        return x + (uint64_t)c * k.nq;
+    }
+    __device__ __forceinline__ static T mul(T x, W2 w, const K &k) {  // below 3 q for any x
+        const uint32_t xl = (uint32_t)x, xh = (uint32_t)(x >> 32), sl = (uint32_t)w.ws, sh = (uint32_t)(w.ws >> 32);
+        const uint64_t t = (uint64_t)xh * sl, u = (uint64_t)xl * sh + (uint32_t)t;
+        const uint64_t h = (uint64_t)xh * sh + (t >> 32) + (u >> 32);
+        return x * w.w + h * k.nq;
+    }
+    __host__ __device__ static constexpr int ct_out(int B) { return (B + PROD > LIM ? RED : B) + PROD; }
+    template <int B>
     __device__ __forceinline__ static void ct(T &a, T &b, W2 w, const K &k) {
-        if (WIDE) {
-            const uint64_t t = mul_shoup_lazy(b, w, k.q);
-            b = a + k.q2 - t;
-            a = a + t;
-        } else {
-            ct_bfly(a, b, w, k.q, k.q2);
-        }
+        const uint64_t t = mul(b, w, k);
+        if (B + PROD > LIM) a = reduce(a, k);
+        b = a + (uint64_t)PROD * k.q - t;
+        a = a + t;
     }
-    // g = number of stages of the whole inverse transform already done
-    __device__ __forceinline__ static void gs(T &a, T &b, W2 w, const K &k, int g) {
-        if (WIDE) {
-            const uint64_t d = a - b + (k.q << (g + 1));
-            a = a + b;
-            b = mul_shoup_lazy(d, w, k.q);
-        } else {
-            gs_bfly(a, b, w, k.q, k.q2);
-        }
+    // a sum over the limit is avoided by reducing the larger operand, then the other one if that is not enough
+    __host__ __device__ static constexpr int red_a(int ba, int bb) { return ba + bb > LIM && (ba >= bb || bb + RED > LIM) ? RED : ba; }
+    __host__ __device__ static constexpr int red_b(int ba, int bb) { return red_a(ba, bb) + bb > LIM ? RED : bb; }
+    __host__ __device__ static constexpr int gs_sum(int ba, int bb) { return red_a(ba, bb) + red_b(ba, bb); }
+    __host__ __device__ static constexpr int gs_prod(int, int) { return PROD; }
+    __device__ __forceinline__ static void gs_in(T &a, T &b, const K &k, int ba, int bb) {
+        if (red_a(ba, bb) != ba) a = reduce(a, k);
+        if (red_b(ba, bb) != bb) b = reduce(b, k);
     }
-    __device__ __forceinline__ static void gs_last(T &a, T &b, W2 sx, W2 sy, const K &k) {
-        const uint64_t s = a + b;
-        const uint64_t d = a - b + (WIDE ? (k.q << k.logN) : k.q2);
+    __device__ __forceinline__ static void gs(T &a, T &b, W2 w, const K &k, int ba, int bb) {
+        gs_in(a, b, k, ba, bb);
+        const uint64_t d = a + (uint64_t)red_b(ba, bb) * k.q - b;
+        a = a + b;
+        b = mul(d, w, k);
+    }
+    __device__ __forceinline__ static void gs_last(T &a, T &b, W2 sx, W2 sy, const K &k, int ba, int bb) {
+        gs_in(a, b, k, ba, bb);
+        const uint64_t d = a + (uint64_t)red_b(ba, bb) * k.q - b, s = a + b;
         a = mul_shoup(s, sx, k.q);
         b = mul_shoup(d, sy, k.q);
     }
-    __device__ __forceinline__ static T pass_end(T v, const K &) { return v; }  // nothing to renormalise
-    __device__ __forceinline__ static uint64_t canon_fwd(T v, const K &k) {
-        return WIDE ? barrett64(v, k.q, k.r1) : csub(csub(v, k.q2), k.q);
-    }
+    __host__ __device__ static constexpr int group_end_out(int B) { return B > GS_PASS ? RED : B; }
+    __device__ __forceinline__ static T group_end(T v, const K &k, int B) { return B > GS_PASS ? reduce(v, k) : v; }
+    __device__ __forceinline__ static T pass_end(T v, const K &k, int B) { return group_end(v, k, B); }
+    __device__ __forceinline__ static uint64_t canon_fwd(T v, const K &k) { return csub(reduce(v, k), k.q); }
     __device__ __forceinline__ static uint64_t canon_inv(T v, const K &) { return v; }  // gs_last is canonical
 };
 
+// Primes of 61 bits (and whatever else does not fit above): Harvey butterflies, one conditional subtraction each; forward
+// residues stay below 4 q, inverse ones below 2 q, and no bound needs tracking
+struct ArithInt {
+    using T = uint64_t;
+    using Tw = W2;
+    struct K {
+        uint64_t q, q2;
+    };
+    static constexpr int B_CANON = 0, B_PASS = 0, GS_PASS = 0;
+    __device__ __forceinline__ static K make(const Mod &md, int) { return K{md.q, 2 * md.q}; }
+    __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &) { return ldg_w2(tw + idx); }
+    __device__ __forceinline__ static Tw ldfin(const W2 *p, const K &) { return ldg_w2(p); }
+    __device__ __forceinline__ static T from_u64(uint64_t v, const K &) { return v; }
+    __device__ __forceinline__ static T from_raw(uint64_t v) { return v; }
+    __device__ __forceinline__ static uint64_t to_raw(T v) { return v; }
+    __host__ __device__ static constexpr int ct_out(int) { return 0; }
+    template <int B>
+    __device__ __forceinline__ static void ct(T &a, T &b, W2 w, const K &k) { ct_bfly(a, b, w, k.q, k.q2); }
+    __host__ __device__ static constexpr int gs_sum(int, int) { return 0; }
+    __host__ __device__ static constexpr int gs_prod(int, int) { return 0; }
+    __device__ __forceinline__ static void gs(T &a, T &b, W2 w, const K &k, int, int) { gs_bfly(a, b, w, k.q, k.q2); }
+    __device__ __forceinline__ static void gs_last(T &a, T &b, W2 sx, W2 sy, const K &k, int, int) {
+        const uint64_t s = a + b, d = a - b + k.q2;
+        a = mul_shoup(s, sx, k.q);
+        b = mul_shoup(d, sy, k.q);
+    }
+    __host__ __device__ static constexpr int group_end_out(int) { return 0; }
+    __device__ __forceinline__ static T group_end(T v, const K &, int) { return v; }
+    __device__ __forceinline__ static T pass_end(T v, const K &, int) { return v; }
+    __device__ __forceinline__ static uint64_t canon_fwd(T v, const K &k) { return csub(csub(v, k.q2), k.q); }
+    __device__ __forceinline__ static uint64_t canon_inv(T v, const K &) { return v; }
+};
+
+// FP64 residues. BIG = false: primes below 2^41, where no residue needs a correction inside a pass (a forward stage grows a
+// residue by less than q, 18 q after 17 stages; an inverse pass doubles its bound 9 times at most and is renormalised at its
+// end, so products never see |y| >= 2^51).
+// BIG = true: primes below 2^50, bounds in sixteenths of q. A factor may be 2 q at most (|y| < 2^51, so that the quotient is
+// rounded right), a sum 8 q (2^53, exact); a product of |y| <= B is below (1/2 + B/4) q.
+template <bool BIG>
 struct ArithFp {
     using T = double;
     struct Tw {
@@ -253,10 +320,12 @@ struct ArithFp {
     };
     struct K {
         double q, qinv;
-        int logN;
     };
+    static constexpr int FACTOR = 32, LIM = 128, RED = 9;
+    static constexpr int B_CANON = BIG ? 16 : 0, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0;
+    __host__ __device__ static constexpr int prod(int B) { return 9 + (B + 3) / 4; }
     // table entry i of an FP64 prime is one double (8 bytes); w / q is rebuilt as w * (1/q), whose
-    // relative error of 2^-52 is far inside the slack of the quotient estimate
+    // relative error of 2^-52 is inside the slack of the quotient estimate
     __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &k) {
         const double w = __ldg(reinterpret_cast<const double *>(tw) + idx);
         return Tw{w, __dmul_rn(w, k.qinv)};
@@ -265,9 +334,9 @@ struct ArithFp {
         const W2 v = ldg_w2(p);
         return Tw{__longlong_as_double((long long)v.w), __longlong_as_double((long long)v.ws)};
     }
-    __device__ __forceinline__ static K make(const Mod &md, int logN) {
+    __device__ __forceinline__ static K make(const Mod &md, int) {
         const double q = (double)md.q;
-        return K{q, 1.0 / q, logN};
+        return K{q, 1.0 / q};
     }
     __device__ __forceinline__ static T from_u64(uint64_t v, const K &) {
         return __dsub_rn(__longlong_as_double((long long)(v | 0x4330000000000000ull)), FP_2_52);
@@ -281,26 +350,47 @@ struct ArithFp {
         const double c = __dsub_rn(__fma_rn(y, wq, FP_MAGIC), FP_MAGIC);
         return __dadd_rn(__fma_rn(-c, k.q, h), l);
     }
+    // the representative of least magnitude (|v| <= 2^53)
     __device__ __forceinline__ static T reduce(T v, const K &k) {
         const double c = __dsub_rn(__fma_rn(v, k.qinv, FP_MAGIC), FP_MAGIC);
         return __fma_rn(-c, k.q, v);
     }
+    __host__ __device__ static constexpr int factor(int B) { return B > FACTOR ? RED : B; }
+    __host__ __device__ static constexpr int ct_out(int B) {
+        if (!BIG) return 0;
+        return (B + prod(factor(B)) > LIM ? RED : B) + prod(factor(B));
+    }
+    template <int B>
     __device__ __forceinline__ static void ct(T &a, T &b, Tw w, const K &k) {
+        if (BIG && B > FACTOR) b = reduce(b, k);
+        if (BIG && B + prod(factor(B)) > LIM) a = reduce(a, k);
         const double t = mulmod(b, w, k);
         b = __dsub_rn(a, t);
         a = __dadd_rn(a, t);
     }
-    __device__ __forceinline__ static void gs(T &a, T &b, Tw w, const K &k, int) {
-        const double d = __dsub_rn(a, b);
+    __host__ __device__ static constexpr int gs_in_bound(int ba, int bb) { return ba + bb > LIM ? 2 * RED : ba + bb; }
+    __host__ __device__ static constexpr int gs_sum(int ba, int bb) { return BIG ? gs_in_bound(ba, bb) : 0; }
+    __host__ __device__ static constexpr int gs_prod(int ba, int bb) { return BIG ? prod(factor(gs_in_bound(ba, bb))) : 0; }
+    __device__ __forceinline__ static void gs_in(T &a, T &b, const K &k, int ba, int bb) {
+        if (BIG && ba + bb > LIM) a = reduce(a, k), b = reduce(b, k);
+    }
+    __device__ __forceinline__ static void gs(T &a, T &b, Tw w, const K &k, int ba, int bb) {
+        gs_in(a, b, k, ba, bb);
+        double d = __dsub_rn(a, b);
         a = __dadd_rn(a, b);
+        if (BIG && gs_in_bound(ba, bb) > FACTOR) d = reduce(d, k);
         b = mulmod(d, w, k);
     }
-    __device__ __forceinline__ static void gs_last(T &a, T &b, Tw sx, Tw sy, const K &k) {
-        const double s = __dadd_rn(a, b), d = __dsub_rn(a, b);
+    __device__ __forceinline__ static void gs_last(T &a, T &b, Tw sx, Tw sy, const K &k, int ba, int bb) {
+        gs_in(a, b, k, ba, bb);
+        double s = __dadd_rn(a, b), d = __dsub_rn(a, b);
+        if (BIG && gs_in_bound(ba, bb) > FACTOR) s = reduce(s, k), d = reduce(d, k);
         a = mulmod(s, sx, k);
         b = mulmod(d, sy, k);
     }
-    __device__ __forceinline__ static T pass_end(T v, const K &k) { return reduce(v, k); }
+    __host__ __device__ static constexpr int group_end_out(int B) { return B; }
+    __device__ __forceinline__ static T group_end(T v, const K &, int) { return v; }
+    __device__ __forceinline__ static T pass_end(T v, const K &k, int) { return reduce(v, k); }
     __device__ __forceinline__ static uint64_t to_canon(T v, const K &k) {  // |v| < q
         if (v < 0.0) v = __dadd_rn(v, k.q);
         return (uint64_t)__double_as_longlong(__dadd_rn(v, FP_2_52)) & 0x000FFFFFFFFFFFFFull;
@@ -309,10 +399,19 @@ struct ArithFp {
     __device__ __forceinline__ static uint64_t canon_inv(T v, const K &k) { return to_canon(v, k); }
 };
 
+// calls f with the policy of the prime (uniform over a CTA)
+template <class F>
+__device__ __forceinline__ void with_arith(uint64_t q, F &&f) {
+    if (q < FP_SMALL_LIMIT) f(ArithFp<false>{});
+    else if (q < FP_LIMIT) f(ArithFp<true>{});
+    else if (q < INT_LAZY_LIMIT) f(ArithIntLazy{});
+    else f(ArithInt{});
+}
+
 // ---- stage runners: compile-time recursion keeps every register index a constant --------------
-// forward: E residues x[], local stages S..R-1 of this stage group; twiddle index
+// forward: E residues x[] bounded by B, local stages S..R-1 of this stage group; twiddle index
 // (P << (shift + S)) + (k0 << S) + g.
-template <class A, int S, int R, int E>
+template <class A, int S, int R, int E, int B>
 __device__ __forceinline__ void ct_stages(typename A::T (&x)[E], const W2 *tw, size_t P, int shift, size_t k0, const typename A::K &k) {
     if constexpr (S < R) {
         constexpr int half = E >> (S + 1);
@@ -320,26 +419,61 @@ __device__ __forceinline__ void ct_stages(typename A::T (&x)[E], const W2 *tw, s
         for (int g = 0; g < (1 << S); g++) {
             const typename A::Tw w = A::ldtw(tw, (P << (shift + S)) + (k0 << S) + g, k);
 #pragma unroll
-            for (int j = 0; j < half; j++) A::ct(x[g * 2 * half + j], x[g * 2 * half + j + half], w, k);
+            for (int j = 0; j < half; j++) A::template ct<B>(x[g * 2 * half + j], x[g * 2 * half + j + half], w, k);
         }
-        ct_stages<A, S + 1, R, E>(x, tw, P, shift, k0, k);
+        ct_stages<A, S + 1, R, E, A::ct_out(B)>(x, tw, P, shift, k0, k);
     }
 }
+// bound after R forward stages
+template <class A>
+__host__ __device__ constexpr int ct_bound(int B, int R) {
+    for (int i = 0; i < R; i++) B = A::ct_out(B);
+    return B;
+}
 
-// inverse: local stages U..R-1 (gap 2^U); twiddle index (m0 >> U) * P + (k0 >> U) + g with
-// m0 = sub-transform size >> (1 + stages already done), k0 = first pair group of this thread at
-// U = 0. g0 = stages of the whole transform already done.
-template <class A, int U, int R, int E>
-__device__ __forceinline__ void gs_stages(typename A::T (&x)[E], const W2 *tw, size_t P, int m0, size_t k0, int g0, const typename A::K &k) {
+// bounds of the E residues of a thread before local stage U of an inverse stage group that starts at bound B everywhere
+template <int E>
+struct GsBounds {
+    int v[E];
+};
+template <class A, int E>
+__host__ __device__ constexpr GsBounds<E> gs_bounds(int B, int U) {
+    GsBounds<E> r{};
+    for (int i = 0; i < E; i++) r.v[i] = B;
+    for (int u = 0; u < U; u++)
+        for (int i = 0; i < E; i++)
+            if (!(i & (1 << u))) {
+                const int j = i | (1 << u), s = A::gs_sum(r.v[i], r.v[j]), p = A::gs_prod(r.v[i], r.v[j]);
+                r.v[i] = s, r.v[j] = p;
+            }
+    return r;
+}
+// bound of what a stage group of R stages hands to the next one
+template <class A, int E>
+__host__ __device__ constexpr int gs_group_bound(int B, int R) {
+    const GsBounds<E> b = gs_bounds<A, E>(B, R);
+    int m = 0;
+    for (int i = 0; i < E; i++) m = m > A::group_end_out(b.v[i]) ? m : A::group_end_out(b.v[i]);
+    return m;
+}
+
+// inverse: local stages U..R-1 (gap 2^U) of a group that starts at bound B; twiddle index (m0 >> U) * P + (k0 >> U) + g
+// with m0 = sub-transform size >> (1 + stages already done), k0 = first pair group of this thread at U = 0.
+template <class A, int U, int R, int E, int B>
+__device__ __forceinline__ void gs_stages(typename A::T (&x)[E], const W2 *tw, size_t P, int m0, size_t k0, const typename A::K &k) {
     if constexpr (U < R) {
         constexpr int gap = 1 << U;
+        constexpr GsBounds<E> bd = gs_bounds<A, E>(B, U);
 #pragma unroll
         for (int g = 0; g < (E >> (U + 1)); g++) {
             const typename A::Tw w = A::ldtw(tw, (size_t)(m0 >> U) * P + (k0 >> U) + g, k);
 #pragma unroll
-            for (int j = 0; j < gap; j++) A::gs(x[g * 2 * gap + j], x[g * 2 * gap + j + gap], w, k, g0 + U);
+            for (int j = 0; j < gap; j++) {
+                const int i = g * 2 * gap + j;
+                A::gs(x[i], x[i + gap], w, k, bd.v[i], bd.v[i + gap]);
+            }
         }
-        gs_stages<A, U + 1, R, E>(x, tw, P, m0, k0, g0, k);
+        gs_stages<A, U + 1, R, E, B>(x, tw, P, m0, k0, k);
     }
 }
 
@@ -347,15 +481,14 @@ __device__ __forceinline__ void gs_stages(typename A::T (&x)[E], const W2 *tw, s
 // forward pass: R1 strided stages, exchange, R2 contiguous stages
 // FIRST: the input holds canonical residues (else the raw lazy values of the previous pass)
 // ================================================================================================
-// STAGED: the tile's input already sits in `sm` itself, dense ([e][c] for the column pass, [c][e] for the row
-// pass), put there by asynchronous copies; it is read into registers, and after a barrier the same buffer
-// serves as the exchange buffer.
 // SRC (column pass only): 1 = the input word reduced into the limb's prime, 2 = its centred representative
 // (word - src_q when the word exceeds src_q / 2) reduced: the remainder a rescale subtracts, floor or nearest.
-template <class A, int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, bool STAGED = false, int SRC = 0>
+template <class A, int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, int SRC = 0>
 __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint64_t *sm, const Job &job, const Mod &md, uint32_t tile) {
     using T = typename A::T;
-    static_assert(SRC == 0 || (COLS && !STAGED), "the on-the-fly source belongs to the plain column pass");
+    static_assert(SRC == 0 || COLS, "the on-the-fly source belongs to the column pass");
+    constexpr int B0 = COLS ? A::B_CANON : A::B_PASS, B1 = ct_bound<A>(B0, R1);
+    static_assert(ct_bound<A>(B1, R2) <= A::B_PASS, "a forward pass stores residues within B_PASS");
     constexpr bool FIRST = COLS;
     constexpr int TT = 1 << LOG_T, E1 = 1 << R1, E2 = 1 << R2, C = 1 << LOG_C;
     constexpr int EPT = E1 > E2 ? E1 : E2;
@@ -383,8 +516,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
         const uint64_t *p = src + base + (size_t)c * cstride + (size_t)elo * estride;
 #pragma unroll
         for (int i = 0; i < E1; i++) {
-            const int e = elo + i * E2;
-            uint64_t v = STAGED ? sm[COLS ? (e * C + c) : (c * TT + e)] : p[(size_t)i * E2 * estride];
+            uint64_t v = p[(size_t)i * E2 * estride];
             if (SRC) {
                 const uint64_t word = v;
                 v = barrett64(word, md.q, md.r1);
@@ -392,11 +524,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
             }
             x[i] = FIRST ? A::from_u64(v, k) : A::from_raw(v);
         }
-        if (STAGED) {
-            static_assert(!STAGED || E1 == EPT, "staged input wants one register group per thread");
-            __syncthreads();  // every staged value is in registers: the buffer may now take the exchange
-        }
-        ct_stages<A, 0, R1, E1>(x, tw, P, 0, 0, k);
+        ct_stages<A, 0, R1, E1, B0>(x, tw, P, 0, 0, k);
 #pragma unroll
         for (int i = 0; i < E1; i++) {
             const int pe = pad_idx<LOG_T, R2>(elo + i * E2);
@@ -423,7 +551,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
             const int pe = pad_idx<LOG_T, R2>(ehi * E2 + i);
             x[i] = A::from_raw(sm[COLS ? (pe * C + c) : (c * TPAD + pe)]);
         }
-        ct_stages<A, 0, R2, E2>(x, tw, P, R1, ehi, k);
+        ct_stages<A, 0, R2, E2, B1>(x, tw, P, R1, ehi, k);
         if (LAST) {
             static_assert(!LAST || !COLS, "the last forward pass is the row pass");
             uint64_t y[E2];
@@ -448,9 +576,7 @@ ntt_fwd_pass(NttArgs a, Epi epi) {
     const uint32_t jobi = work_idx(a) / tiles, tile = work_idx(a) % tiles;
     const Job job = get_job(a, jobi);
     const Mod md = a.mod[job.y];
-    if (md.q < FP_LIMIT) fwd_body<ArithFp, LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, false, SRC>(a, epi, sm, job, md, tile);
-    else if (md.q < WIDE_LIMIT) fwd_body<ArithInt<true>, LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, false, SRC>(a, epi, sm, job, md, tile);
-    else fwd_body<ArithInt<false>, LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, false, SRC>(a, epi, sm, job, md, tile);
+    with_arith(md.q, [&](auto A) { fwd_body<decltype(A), LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, SRC>(a, epi, sm, job, md, tile); });
 }
 
 // ================================================================================================
@@ -509,24 +635,9 @@ constexpr size_t mac_smem_bytes() {
 // below q, so any 64-bit y gives a value below 2q) summed in one 64-bit word - 128-bit accumulators for sixteen residues
 // times two polynomials would not fit the register file, and a Barrett reduction per product costs twice the multiplies.
 // The factor 2^-64 is undone by the constant of the final multiplication (MacArgs::fin).
-template <class A> struct MacAcc;
-template <> struct MacAcc<ArithFp> {
-    using T = double;
-    using K = ArithFp::K;
-    struct C {};
-    __device__ __forceinline__ static C make(const Mod &) { return C{}; }
-    __device__ __forceinline__ static T zero() { return 0.0; }
-    __device__ __forceinline__ static double operand(double y, const K &k) { return ArithFp::reduce(y, k); }
-    __device__ __forceinline__ static void mac(T &acc, double y, uint64_t key, const K &k, const C &) {
-        const double w = ArithFp::from_u64(key, k);
-        acc = __dadd_rn(acc, ArithFp::mulmod(y, ArithFp::Tw{w, __dmul_rn(w, k.qinv)}, k));
-    }
-    // canonical residue of the sum
-    __device__ __forceinline__ static uint64_t finish(T acc, W2, const K &k, const C &) { return ArithFp::canon_fwd(acc, k); }
-};
-template <bool WIDE> struct MacAcc<ArithInt<WIDE>> {
+template <class A> struct MacAcc {
     using T = uint64_t;
-    using K = typename ArithInt<WIDE>::K;
+    using K = typename A::K;
     struct C {
         uint64_t q, q2, ninv;  // ninv = -q^-1 mod 2^64
         bool tight;            // 2 * beta * q could pass 2^64: keep the sum below 2q after every term
@@ -538,7 +649,7 @@ template <bool WIDE> struct MacAcc<ArithInt<WIDE>> {
         return C{md.q, 2 * md.q, 0 - x, (md.q >> 59) != 0};
     }
     __device__ __forceinline__ static T zero() { return 0; }
-    __device__ __forceinline__ static uint64_t operand(uint64_t y, const K &) { return y; }  // lazy values (below 2^63) do
+    __device__ __forceinline__ static uint64_t operand(uint64_t y, const K &) { return y; }  // any lazy value does
     __device__ __forceinline__ static void mac(T &acc, uint64_t y, uint64_t key, const K &, const C &c) {
         const uint64_t lo = y * key, hi = __umul64hi(y, key);
         const uint64_t m = lo * c.ninv;
@@ -548,6 +659,21 @@ template <bool WIDE> struct MacAcc<ArithInt<WIDE>> {
     }
     // sum * 2^-64 times the limb's closing constant, canonical
     __device__ __forceinline__ static uint64_t finish(T acc, W2 fin, const K &, const C &c) { return mul_shoup(acc, fin, c.q); }
+};
+template <bool BIG> struct MacAcc<ArithFp<BIG>> {
+    using Fp = ArithFp<BIG>;
+    using T = double;
+    using K = typename Fp::K;
+    struct C {};
+    __device__ __forceinline__ static C make(const Mod &) { return C{}; }
+    __device__ __forceinline__ static T zero() { return 0.0; }
+    __device__ __forceinline__ static double operand(double y, const K &k) { return Fp::reduce(y, k); }
+    __device__ __forceinline__ static void mac(T &acc, double y, uint64_t key, const K &k, const C &) {
+        const double w = Fp::from_u64(key, k);
+        acc = __dadd_rn(acc, Fp::mulmod(y, typename Fp::Tw{w, __dmul_rn(w, k.qinv)}, k));
+    }
+    // canonical residue of the sum
+    __device__ __forceinline__ static uint64_t finish(T acc, W2, const K &k, const C &) { return Fp::canon_fwd(acc, k); }
 };
 
 // One tile of one output limb t (logical index: Q limbs 0 .. l-1, then the P limbs) through all digits.
@@ -598,13 +724,13 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
             const uint64_t *src = a.src + ((size_t)bset * m.dig_bs + (size_t)d * m.lP + t) * N + base + (size_t)c * TT + e;
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = A::from_raw(src[i * E]);
-            ct_stages<A, 0, R, E>(y, tw, P, 0, 0, k);
+            ct_stages<A, 0, R, E, A::B_PASS>(y, tw, P, 0, 0, k);
 #pragma unroll
             for (int i = 0; i < E; i++) sm[c * TPAD + pad_idx<LOG_T, R>(e + i * E)] = A::to_raw(y[i]);
             __syncthreads();
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = A::from_raw(sm[c * TPAD + pad_idx<LOG_T, R>(e * E + i)]);
-            ct_stages<A, 0, R, E>(y, tw, P, R, e, k);
+            ct_stages<A, 0, R, E, ct_bound<A>(A::B_PASS, R)>(y, tw, P, R, e, k);
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = Acc::operand(y[i], k);
         }
@@ -625,7 +751,7 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
     if (t < m.l) {
         // a Q limb: ct[k][t] += sum * P^-1. FP64 sums are canonical first and take P^-1; integer sums carry 2^-64 and
         // take P^-1 * 2^64 in the same single multiplication.
-        constexpr bool FP = std::is_same<A, ArithFp>::value;
+        constexpr bool FP = std::is_same<typename A::T, double>::value;
         const W2 pi = FP ? m.pinv[pp] : m.fin[pp];
         uint64_t *c0 = m.ct + ((size_t)bset * m.ct_bs + t) * N + o, *c1 = c0 + (size_t)m.l * N;
 #pragma unroll
@@ -681,15 +807,13 @@ __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) >> R, 3) ntt_fwd_rows_m
     const uint32_t t = i < m.p_first ? m.l + m.p_off + i : m.first_limb + (i - m.p_first);
     const uint32_t pp = t < m.l ? t : m.size_Q + (t - m.l);  // the limb's prime
     const Mod md = a.mod[pp];
-    if (md.q < FP_LIMIT) mac_body<ArithFp, LOG_T, R, LOG_C>(a, m, sm, kb, t, pp, tile, bset, md);
-    else if (md.q < WIDE_LIMIT) mac_body<ArithInt<true>, LOG_T, R, LOG_C>(a, m, sm, kb, t, pp, tile, bset, md);
-    else mac_body<ArithInt<false>, LOG_T, R, LOG_C>(a, m, sm, kb, t, pp, tile, bset, md);
+    with_arith(md.q, [&](auto A) { mac_body<decltype(A), LOG_T, R, LOG_C>(a, m, sm, kb, t, pp, tile, bset, md); });
 }
 
 // ================================================================================================
 // inverse pass: RA contiguous stages, exchange, RB strided stages
 // ================================================================================================
-template <class A, int LOG_T, int RA, int RB, int LOG_C, bool COLS, bool LAST, bool STAGED = false>
+template <class A, int LOG_T, int RA, int RB, int LOG_C, bool COLS, bool LAST>
 __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const Job &job, const Mod &md, uint32_t tile) {
     using T = typename A::T;
     constexpr bool FIRST = !COLS;
@@ -707,8 +831,8 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
     const size_t base = COLS ? (size_t)tile * C : (size_t)tile * C * TT;
     const uint32_t n1 = (uint32_t)(N >> LOG_T);
     const int tid = threadIdx.x;
-    // stages of the whole transform done before this pass: the row pass comes first
-    const int g_pass = COLS ? ((int)a.logN - LOG_T) : 0;
+    constexpr int B0 = FIRST ? A::B_CANON : A::GS_PASS, B1 = gs_group_bound<A, EA>(B0, RA);
+    constexpr GsBounds<EA> end_a = gs_bounds<A, EA>(B0, RA);
 
     // ---- stage group 1: contiguous runs of EA residues ----------------------------------------------
 #pragma unroll
@@ -719,16 +843,7 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
         const uint32_t P = COLS ? 1u : (n1 + tile * C + c);
         T x[EA];
         const uint64_t *p = src + base + (size_t)c * cstride + (size_t)ehi * EA * estride;
-        if (STAGED) {
-            static_assert(!STAGED || EA == EPT, "staged input wants one register group per thread");
-#pragma unroll
-            for (int i = 0; i < EA; i++) {
-                const int e = ehi * EA + i;
-                const uint64_t v = sm[COLS ? (e * C + c) : (c * TT + e)];
-                x[i] = FIRST ? A::from_u64(v, k) : A::from_raw(v);
-            }
-            __syncthreads();
-        } else if (COLS) {
+        if (COLS) {
 #pragma unroll
             for (int i = 0; i < EA; i++) {
                 const uint64_t v = p[(size_t)i * estride];
@@ -744,11 +859,11 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
                 x[i + 3] = FIRST ? A::from_u64(v.d, k) : A::from_raw(v.d);
             }
         }
-        gs_stages<A, 0, RA, EA>(x, tw, P, TT >> 1, (size_t)ehi * (EA >> 1), g_pass, k);
+        gs_stages<A, 0, RA, EA, B0>(x, tw, P, TT >> 1, (size_t)ehi * (EA >> 1), k);
 #pragma unroll
         for (int i = 0; i < EA; i++) {
             const int pe = pad_idx<LOG_T, RA>(ehi * EA + i);
-            sm[COLS ? (pe * C + c) : (c * TPAD + pe)] = A::to_raw(x[i]);
+            sm[COLS ? (pe * C + c) : (c * TPAD + pe)] = A::to_raw(A::group_end(x[i], k, end_a.v[i]));
         }
     }
     __syncthreads();
@@ -765,7 +880,8 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
             const int pe = pad_idx<LOG_T, RA>(elo + i * EA);
             x[i] = A::from_raw(sm[COLS ? (pe * C + c) : (c * TPAD + pe)]);
         }
-        gs_stages<A, 0, (LAST ? RB - 1 : RB), EB>(x, tw, P, TT >> (RA + 1), 0, g_pass + RA, k);
+        gs_stages<A, 0, (LAST ? RB - 1 : RB), EB, B1>(x, tw, P, TT >> (RA + 1), 0, k);
+        constexpr GsBounds<EB> end_b = gs_bounds<A, EB>(B1, LAST ? RB - 1 : RB);
         uint64_t *o = dst + base + (size_t)c * cstride + (size_t)elo * estride;
         if (LAST) {
             // last stage of the whole transform (twiddle index 1): the x outputs take the scale,
@@ -775,12 +891,12 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
             const typename A::Tw sx = A::ldfin(a.fin + 2 * (size_t)job.z, k);
             const typename A::Tw sy = A::ldfin(a.fin + 2 * (size_t)job.z + 1, k);
 #pragma unroll
-            for (int j = 0; j < gap; j++) A::gs_last(x[j], x[j + gap], sx, sy, k);
+            for (int j = 0; j < gap; j++) A::gs_last(x[j], x[j + gap], sx, sy, k, end_b.v[j], end_b.v[j + gap]);
 #pragma unroll
             for (int i = 0; i < EB; i++) o[(size_t)i * EA * estride] = A::canon_inv(x[i], k);
         } else {
 #pragma unroll
-            for (int i = 0; i < EB; i++) o[(size_t)i * EA * estride] = A::to_raw(A::pass_end(x[i], k));
+            for (int i = 0; i < EB; i++) o[(size_t)i * EA * estride] = A::to_raw(A::pass_end(x[i], k, end_b.v[i]));
         }
     }
 }
@@ -796,296 +912,7 @@ ntt_inv_pass(NttArgs a) {
     const uint32_t jobi = work_idx(a) / tiles, tile = work_idx(a) % tiles;
     const Job job = get_job(a, jobi);
     const Mod md = a.mod[job.y];
-    if (md.q < FP_LIMIT) inv_body<ArithFp, LOG_T, RA, RB, LOG_C, COLS, LAST>(a, sm, job, md, tile);
-    else if (md.q < WIDE_LIMIT) inv_body<ArithInt<true>, LOG_T, RA, RB, LOG_C, COLS, LAST>(a, sm, job, md, tile);
-    else inv_body<ArithInt<false>, LOG_T, RA, RB, LOG_C, COLS, LAST>(a, sm, job, md, tile);
-}
-
-// ================================================================================================
-// pipelined passes: a resident CTA walks over several tiles, and while it transforms one tile the next one
-// is already on its way from global memory into the second shared-memory buffer (cp.async, 16 bytes per
-// copy, L1 bypassed). The plain kernels above have bytes in flight only during the load phase of each CTA,
-// which bounds them near 2.5 TB/s; here every resident CTA always has a whole tile in flight.
-// ================================================================================================
-// tile `tile` of limb slot `slot` of src -> dense buffer ([e][c] or [c][e])
-template <int LOG_T, int LOG_C, bool COLS, int THREADS>
-__device__ __forceinline__ void stage_tile(uint64_t *buf, const uint64_t *src, size_t N, uint32_t slot, uint32_t tile) {
-    constexpr int TT = 1 << LOG_T, C = 1 << LOG_C;
-    constexpr int GRAN = C * TT / 2;  // 16-byte granules per tile
-    const uint64_t *s = src + (size_t)slot * N + (COLS ? (size_t)tile * C : (size_t)tile * C * TT);
-#pragma unroll
-    for (int g = threadIdx.x; g < GRAN; g += THREADS) {
-        if (COLS) {
-            const int row = g / (C / 2), part = g % (C / 2);
-            cp_async16(buf + row * C + part * 2, s + (size_t)row * (N >> LOG_T) + part * 2);
-        } else {
-            cp_async16(buf + g * 2, s + (size_t)g * 2);
-        }
-    }
-}
-
-template <int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi>
-__global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2))))
-ntt_fwd_pipe(NttArgs a, Epi epi, uint32_t total) {
-    pdl_enter();
-    static_assert(R1 == R2, "pipelined passes are built for equal stage groups");
-    constexpr int TT = 1 << LOG_T, C = 1 << LOG_C, THREADS = (C * TT) >> R1;
-    __shared__ __align__(16) uint64_t buf[2][C * (TT + (TT >> R2))];
-    const size_t N = (size_t)1 << a.logN;
-    const uint32_t tiles = (uint32_t)(N >> (LOG_T + LOG_C));
-    uint32_t item = blockIdx.x;
-    if (item < total) stage_tile<LOG_T, LOG_C, COLS, THREADS>(buf[0], a.src, N, get_job(a, item / tiles).x, item % tiles);
-    cp_async_commit();
-    for (uint32_t it = 0; item < total; it++, item += gridDim.x) {
-        const uint32_t nxt = item + gridDim.x;
-        if (nxt < total) stage_tile<LOG_T, LOG_C, COLS, THREADS>(buf[(it + 1) & 1], a.src, N, get_job(a, nxt / tiles).x, nxt % tiles);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        uint64_t *sm = buf[it & 1];
-        const Job job = get_job(a, item / tiles);
-        const Mod md = a.mod[job.y];
-        const uint32_t tile = item % tiles;
-        if (md.q < FP_LIMIT) fwd_body<ArithFp, LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, true>(a, epi, sm, job, md, tile);
-        else if (md.q < WIDE_LIMIT) fwd_body<ArithInt<true>, LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, true>(a, epi, sm, job, md, tile);
-        else fwd_body<ArithInt<false>, LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, true>(a, epi, sm, job, md, tile);
-        __syncthreads();  // the buffer is refilled two iterations from now, by the prefetch of the next one
-    }
-    cp_async_wait<0>();
-}
-
-template <int LOG_T, int RA, int RB, int LOG_C, bool COLS, bool LAST>
-__global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (RA > RB ? RA : RB)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (RA > RB ? RA : RB))))
-ntt_inv_pipe(NttArgs a, uint32_t total) {
-    pdl_enter();
-    static_assert(RA == RB, "pipelined passes are built for equal stage groups");
-    constexpr int TT = 1 << LOG_T, C = 1 << LOG_C, THREADS = (C * TT) >> RA;
-    constexpr bool FIRST = !COLS;
-    __shared__ __align__(16) uint64_t buf[2][C * (TT + (TT >> RA))];
-    const size_t N = (size_t)1 << a.logN;
-    const uint32_t tiles = (uint32_t)(N >> (LOG_T + LOG_C));
-    uint32_t item = blockIdx.x;
-    if (item < total) {
-        const Job j0 = get_job(a, item / tiles);
-        stage_tile<LOG_T, LOG_C, COLS, THREADS>(buf[0], a.src, N, FIRST ? j0.x : j0.w, item % tiles);
-    }
-    cp_async_commit();
-    for (uint32_t it = 0; item < total; it++, item += gridDim.x) {
-        const uint32_t nxt = item + gridDim.x;
-        if (nxt < total) {
-            const Job jn = get_job(a, nxt / tiles);
-            stage_tile<LOG_T, LOG_C, COLS, THREADS>(buf[(it + 1) & 1], a.src, N, FIRST ? jn.x : jn.w, nxt % tiles);
-        }
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        uint64_t *sm = buf[it & 1];
-        const Job job = get_job(a, item / tiles);
-        const Mod md = a.mod[job.y];
-        const uint32_t tile = item % tiles;
-        if (md.q < FP_LIMIT) inv_body<ArithFp, LOG_T, RA, RB, LOG_C, COLS, LAST, true>(a, sm, job, md, tile);
-        else if (md.q < WIDE_LIMIT) inv_body<ArithInt<true>, LOG_T, RA, RB, LOG_C, COLS, LAST, true>(a, sm, job, md, tile);
-        else inv_body<ArithInt<false>, LOG_T, RA, RB, LOG_C, COLS, LAST, true>(a, sm, job, md, tile);
-        __syncthreads();
-    }
-    cp_async_wait<0>();
-}
-
-}  // namespace b2
-
-// ================================================================================================
-// single-launch transforms for N = 2^16 on a thread-block cluster
-// ================================================================================================
-// A cluster of 8 CTAs owns one limb (256 x 256 residues, 512 KiB). The two passes exchange through
-// distributed shared memory instead of global memory: every CTA keeps a 256 x 32 (forward: its
-// column block after the column pass) or 32 x 256 (inverse: its row block after the row pass)
-// slab of 64 KiB in shared memory, the cluster synchronises with the hardware cluster barrier, and
-// the second pass gathers its inputs from the eight slabs. A limb therefore crosses global memory
-// once in and once out. No flag or spin wait is involved: cluster.sync() is the only rendezvous
-// and every thread of every CTA reaches it unconditionally.
-#include <cooperative_groups.h>
-
-namespace b2 {
-namespace cg = cooperative_groups;
-
-constexpr int CL_SIZE = 8;        // CTAs per cluster
-constexpr int CL_THREADS = 256;   // two tile groups of 128 threads
-constexpr int CL_SLAB = 256 * 32; // residues per slab
-constexpr int CL_EX = 8 * (256 + 16);
-constexpr size_t CL_SMEM = (size_t)(CL_SLAB + 2 * CL_EX) * 8;
-
-// slab indexing with a rotation of the 8-column groups by (row >> 4): rows 16 apart fall into
-// different bank groups, which is what the two access patterns below need
-__device__ __forceinline__ int slab_fwd(int row, int col32) { return row * 32 + ((col32 + 8 * (row >> 4)) & 31); }
-__device__ __forceinline__ int slab_inv(int row32, int col) { return row32 * 256 + (col ^ (8 * ((row32 >> 4) & 1))); }
-
-template <class A, class Epi>
-__device__ __forceinline__ void fwd_cluster_body(const NttArgs &a, const Epi &epi, uint64_t *smem, const Job &job, const Mod &md) {
-    using T = typename A::T;
-    constexpr int LOG_T = 8, R1 = 4, R2 = 4, E = 16, C = 8, TPAD = 256 + 16;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const size_t N = 65536;
-    const typename A::K k = A::make(md, 16);
-    const W2 *tw = a.tw + (size_t)job.y * N;
-    const uint64_t *src = a.src + (size_t)job.x * N;
-    uint64_t *slab = smem;
-    const int tg = threadIdx.x >> 7, t = threadIdx.x & 127;
-    uint64_t *ex = smem + CL_SLAB + tg * CL_EX;
-
-    // ---- column pass on this CTA's 32 columns: 4 tiles of 8, two at a time -------------------
-#pragma unroll 1
-    for (int it = 0; it < 2; it++) {
-        const int ti = it * 2 + tg;
-        const int c = t % C, e_lo = t / C;
-        T x[E];
-        const uint64_t *p = src + (size_t)e_lo * 256 + rank * 32 + ti * 8 + c;
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = A::from_u64(p[(size_t)i * 16 * 256], k);
-        ct_stages<A, 0, R1, E>(x, tw, 1, 0, 0, k);
-#pragma unroll
-        for (int i = 0; i < E; i++) ex[pad_idx<LOG_T, R2>(e_lo + i * 16) * C + c] = A::to_raw(x[i]);
-        __syncthreads();
-        const int e_hi = t / C;
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = A::from_raw(ex[pad_idx<LOG_T, R2>(e_hi * 16 + i) * C + c]);
-        ct_stages<A, 0, R2, E>(x, tw, 1, R1, e_hi, k);
-#pragma unroll
-        for (int i = 0; i < E; i++) slab[slab_fwd(e_hi * 16 + i, ti * 8 + c)] = A::to_raw(x[i]);
-        __syncthreads();
-    }
-    cluster.sync();
-    // ---- row pass on this CTA's 32 rows, inputs gathered from the eight slabs -------------------
-    Epi e = epi;
-    e.init(a, job, N);
-    (void)TPAD;
-#pragma unroll 1
-    for (int it = 0; it < 2; it++) {
-        const int ti = it * 2 + tg;
-        const int ch = t / 16, e_lo = t % 16;
-        const int row = rank * 32 + ti * 8 + ch;
-        const uint32_t P = 256u + (uint32_t)row;
-        T x[E];
-#pragma unroll
-        for (int i = 0; i < E; i++) {
-            const int col = e_lo + 16 * i;
-            const uint64_t *peer = cluster.map_shared_rank(slab, col >> 5);
-            x[i] = A::from_raw(peer[slab_fwd(row, col & 31)]);
-        }
-        ct_stages<A, 0, R1, E>(x, tw, P, 0, 0, k);
-#pragma unroll
-        for (int i = 0; i < E; i++) ex[ch * TPAD + pad_idx<LOG_T, R2>(e_lo + i * 16)] = A::to_raw(x[i]);
-        __syncthreads();
-        const int e_hi = t % 16;
-        const size_t o = (size_t)row * 256 + (size_t)e_hi * 16;
-        typename Epi::template Regs<E> regs;
-        e.template preload<E>(regs, o);
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = A::from_raw(ex[ch * TPAD + pad_idx<LOG_T, R2>(e_hi * 16 + i)]);
-        ct_stages<A, 0, R2, E>(x, tw, P, R1, e_hi, k);
-        uint64_t y[E];
-#pragma unroll
-        for (int i = 0; i < E; i++) y[i] = A::canon_fwd(x[i], k);
-        e.template finish<E>(regs, o, y, md.q);
-        __syncthreads();
-    }
-    cluster.sync();  // nobody leaves while a peer may still read its slab
-}
-
-template <class Epi>
-__global__ void __cluster_dims__(CL_SIZE, 1, 1) __launch_bounds__(CL_THREADS, 2) ntt_fwd_cluster(NttArgs a, Epi epi) {
-    pdl_enter();
-    extern __shared__ __align__(16) uint64_t cl_smem[];
-    const Job job = get_job(a, blockIdx.x / CL_SIZE);
-    const Mod md = a.mod[job.y];
-    if (md.q < FP_LIMIT) fwd_cluster_body<ArithFp, Epi>(a, epi, cl_smem, job, md);
-    else if (md.q < WIDE_LIMIT) fwd_cluster_body<ArithInt<true>, Epi>(a, epi, cl_smem, job, md);
-    else fwd_cluster_body<ArithInt<false>, Epi>(a, epi, cl_smem, job, md);
-}
-
-template <class A>
-__device__ __forceinline__ void inv_cluster_body(const NttArgs &a, uint64_t *smem, const Job &job, const Mod &md) {
-    using T = typename A::T;
-    constexpr int LOG_T = 8, RA = 4, RB = 4, E = 16, C = 8, TPAD = 256 + 16;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const size_t N = 65536;
-    const typename A::K k = A::make(md, 16);
-    const W2 *tw = a.tw + (size_t)job.y * N;
-    const uint64_t *src = a.src + (size_t)job.x * N;
-    uint64_t *dst = a.dst + (size_t)job.w * N;
-    uint64_t *slab = smem;
-    const int tg = threadIdx.x >> 7, t = threadIdx.x & 127;
-    uint64_t *ex = smem + CL_SLAB + tg * CL_EX;
-
-    // ---- row pass on this CTA's 32 rows (bit-reversed input, contiguous) ------------------------
-#pragma unroll 1
-    for (int it = 0; it < 2; it++) {
-        const int ti = it * 2 + tg;
-        const int ch = t / 16, e_hi = t % 16;
-        const int row32 = ti * 8 + ch;
-        const uint32_t P = 256u + (uint32_t)(rank * 32 + row32);
-        T x[E];
-        const uint64_t *p = src + (size_t)(rank * 32 + row32) * 256 + (size_t)e_hi * 16;
-#pragma unroll
-        for (int i = 0; i < E; i += 2) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p + i);
-            x[i] = A::from_u64(v.x, k);
-            x[i + 1] = A::from_u64(v.y, k);
-        }
-        gs_stages<A, 0, RA, E>(x, tw, P, 128, (size_t)e_hi * 8, 0, k);
-#pragma unroll
-        for (int i = 0; i < E; i++) ex[ch * TPAD + pad_idx<LOG_T, RA>(e_hi * 16 + i)] = A::to_raw(x[i]);
-        __syncthreads();
-        const int e_lo = t % 16;
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = A::from_raw(ex[ch * TPAD + pad_idx<LOG_T, RA>(e_lo + i * 16)]);
-        gs_stages<A, 0, RB, E>(x, tw, P, 128 >> RA, 0, RA, k);
-#pragma unroll
-        for (int i = 0; i < E; i++) slab[slab_inv(row32, e_lo + 16 * i)] = A::to_raw(A::pass_end(x[i], k));
-        __syncthreads();
-    }
-    cluster.sync();
-    // ---- column pass on this CTA's 32 columns, inputs gathered from the eight slabs ----------------
-#pragma unroll 1
-    for (int it = 0; it < 2; it++) {
-        const int ti = it * 2 + tg;
-        const int c = t % C, e_hi = t / C;
-        const int col = rank * 32 + ti * 8 + c;
-        T x[E];
-        {
-            const uint64_t *peer = cluster.map_shared_rank(slab, e_hi >> 1);
-#pragma unroll
-            for (int i = 0; i < E; i++) x[i] = A::from_raw(peer[slab_inv((e_hi & 1) * 16 + i, col)]);
-        }
-        gs_stages<A, 0, RA, E>(x, tw, 1, 128, (size_t)e_hi * 8, 8, k);
-#pragma unroll
-        for (int i = 0; i < E; i++) ex[pad_idx<LOG_T, RA>(e_hi * 16 + i) * C + c] = A::to_raw(x[i]);
-        __syncthreads();
-        const int e_lo = t / C;
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = A::from_raw(ex[pad_idx<LOG_T, RA>(e_lo + i * 16) * C + c]);
-        gs_stages<A, 0, RB - 1, E>(x, tw, 1, 128 >> RA, 0, 8 + RA, k);
-        const typename A::Tw sx = A::ldfin(a.fin + 2 * (size_t)job.z, k);
-        const typename A::Tw sy = A::ldfin(a.fin + 2 * (size_t)job.z + 1, k);
-#pragma unroll
-        for (int j = 0; j < E / 2; j++) A::gs_last(x[j], x[j + E / 2], sx, sy, k);
-        uint64_t *o = dst + (size_t)e_lo * 256 + col;
-#pragma unroll
-        for (int i = 0; i < E; i++) o[(size_t)i * 16 * 256] = A::canon_inv(x[i], k);
-        __syncthreads();
-    }
-    cluster.sync();
-}
-
-__global__ void __cluster_dims__(CL_SIZE, 1, 1) __launch_bounds__(CL_THREADS, 2) ntt_inv_cluster(NttArgs a) {
-    pdl_enter();
-    extern __shared__ __align__(16) uint64_t cl_smem[];
-    const Job job = get_job(a, blockIdx.x / CL_SIZE);
-    const Mod md = a.mod[job.y];
-    if (md.q < FP_LIMIT) inv_cluster_body<ArithFp>(a, cl_smem, job, md);
-    else if (md.q < WIDE_LIMIT) inv_cluster_body<ArithInt<true>>(a, cl_smem, job, md);
-    else inv_cluster_body<ArithInt<false>>(a, cl_smem, job, md);
+    with_arith(md.q, [&](auto A) { inv_body<decltype(A), LOG_T, RA, RB, LOG_C, COLS, LAST>(a, sm, job, md, tile); });
 }
 
 }  // namespace b2
