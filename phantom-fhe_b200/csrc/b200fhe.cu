@@ -21,6 +21,7 @@
 #include "sampler.cuh"
 #include "encoder.cuh"
 #include "bconv_tc.cuh"
+#include "elementwise.cuh"
 
 using namespace b2;
 typedef unsigned __int128 u128_t;
@@ -616,7 +617,9 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
         uint64_t r1 = (uint64_t)(hi / q);
         u128_t rem = hi % q;
         uint64_t r0 = (uint64_t)((rem << 64) / q);
-        mods[l] = Mod{q, r0, r1, 0};
+        // floor(2^(62 + n) / q) for q of n bits: 62 + n <= 123, so the numerator fits
+        const uint64_t mu = (uint64_t)(((u128_t)1 << (62 + 64 - __builtin_clzll(q))) / q);
+        mods[l] = Mod{q, r0, r1, mu};
     }
     // ---- P-related constants (src/rns.cu:100-138, 192-194) ----
     const size_t sQ = c->size_Q, sP = size_P;
@@ -869,6 +872,7 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
 // A batched launch: `batch` polynomial sets, slot s of set b at s * (lm1 + 1) + b * bs of the source / destination
 struct BatchDims {
     uint32_t batch = 1, src_lm1 = 0, src_bs = 0, dst_lm1 = 0, dst_bs = 0;
+    const uint32_t *perm = nullptr;  // inverse transforms: the input is read through this permutation
 };
 
 template <class Epi, int SRC = 0>
@@ -895,7 +899,7 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
                    const W2 *fin, cudaStream_t s, const BatchDims &bd = BatchDims{}) {
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
+    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, bd.perm};
     switch (c->logN) {
         case 17: launch_inv<8, 9>(c, a, njobs, s, bd.batch); break;
         case 16: launch_inv<8, 8>(c, a, njobs, s, bd.batch); break;
@@ -1096,402 +1100,17 @@ __global__ void __launch_bounds__(128) bconv_fp_kernel(const uint64_t *__restric
     else bconv_fp_body<3, COPY>(in, out, copy_src, g, s_meta, s_m, N, n);
 }
 
-struct EvkPtrs {
-    const uint64_t *p[64];
-};
-
-// A batch of inner products in one launch (FUSED form): blockIdx.y = set b. Digits, the NTT-form input and the ciphertext
-// of set b start b * dig_bs / own_bs / ct_bs limbs further; P limb i of polynomial k lands at slot
-// (i * p_mul_i + k * p_mul_k) * (p_lm1 + 1) + b * p_bs of the P-limb buffer. One set: {0, 0, 0, 1, alpha, 0, 0}.
+// strides of a batch of fused inner products: see IpArgs. One set: {0, 0, 0, 1, alpha, 0, 0}.
 struct IpBatch {
     uint32_t dig_bs, own_bs, ct_bs, p_mul_i, p_mul_k, p_lm1, p_bs;
 };
 
-// Key-switch inner product (src/eval_key_switch.cu:175-230): for logical limb t (physical prime pp)
-//   acc[k][t][n] = (sum_d digits[d][t][n] * evk[d][k][pp][n]) mod q_pp,   k = 0, 1
-// accumulated in 128 bits and reduced once. Pure streaming: two coefficients per thread, 16-byte
-// loads, every load of a thread issued before the first multiply.
-// FUSED = false: out[k][t] = acc (the reference's cx buffer, [2][l+alpha][N]).
-// FUSED = true (whole key switch): Q limbs go straight into the ciphertext as
-//   ct[k][t] += acc * P^-1  and only the P limbs are kept, compactly, in outP [2][alpha][N];
-// together with a ModDown matrix that carries P^-1 this equals ct + (acc - delta) * P^-1.
-// ACCP (with FUSED): the P limbs are added to what outP already holds, so that several key switches share
-// one ModDown ("double hoisting": the Q limbs accumulate in ct anyway).
-template <int MAX_BETA, bool FUSED, bool ACCP = false>
-__global__ void __launch_bounds__(256) ks_inner_prod_kernel(const uint64_t *__restrict__ digits, const uint64_t *__restrict__ own,
-                                                           EvkPtrs evk, uint64_t *__restrict__ out, uint64_t *__restrict__ ct,
-                                                           const W2 *__restrict__ pinv, const Mod *mod, const b2_ctx::RedcMeta *redc,
-                                                           uint32_t N, uint32_t l, uint32_t lP, uint32_t size_Q, uint32_t size_QP,
-                                                           uint32_t beta, uint4 own_range, const IpBatch ib, const uint32_t *__restrict__ perm) {
-    pdl_enter();
-    // perm (optional): the digits are read through the NTT-domain permutation of a Galois element, digit[perm[n]] - hoisted
-    // rotations, whose permuted copy of the ModUp digits is then never written (src/evaluate.cu:2041-2045 permutes into a buffer)
-    // own_range = (first Q limb, number of Q limbs, first P limb, number of P limbs) this launch
-    // covers: everything on one GPU, the rank's slice under RNS-limb sharding
-    // The sets are the slow grid dimension: with the sets fastest (the CTAs that read one piece of the key next to one another) this
-    // kernel ran 13 % slower on B200.
-    digits += (size_t)blockIdx.y * ib.dig_bs * N;
-    if (own) own += (size_t)blockIdx.y * ib.own_bs * N;
-    if (FUSED) ct += (size_t)blockIdx.y * ib.ct_bs * N;
-    const size_t jdx = 2 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
-    if (jdx >= (size_t)(own_range.y + own_range.w) * N) return;
-    const uint32_t jl = (uint32_t)(jdx / N), n = (uint32_t)(jdx % N);
-    const uint32_t t = jl < own_range.y ? own_range.x + jl : l + own_range.z + (jl - own_range.y);
-    const size_t idx = (size_t)t * N + n;
-    const uint32_t pp = t < l ? t : size_Q + (t - l);
-    const Mod md = mod[pp];
-    // `own` (optional): the NTT-form input of ModUp; limb t of digit t / alpha is that input itself
-    // (src/rns_bconv.cu:522-528), so the digit buffer need not hold a copy of it
-    const uint32_t own_d = (own && t < l) ? t / (lP - l) : 0xFFFFFFFFu;
-    const uint2 p2 = perm ? *reinterpret_cast<const uint2 *>(perm + n) : make_uint2(0, 0);
-    if (md.q < b2::FP_SMALL_LIMIT) {
-        // Small prime (uniform over the block): digits and key words are below 2^41, so each product
-        // is four exact FP64 FMAs on 21-bit pieces instead of five wide integer multiplies, and the
-        // reduction of sum_w A_w 2^(21 w) stays in FP64 too. Same residues as the integer path.
-        const b2_ctx::RedcMeta rm = redc[pp];
-        const double qd = (double)md.q, qinv = 1.0 / qd;
-        double A[4][3];
-#pragma unroll
-        for (int o = 0; o < 4; o++) A[o][0] = A[o][1] = A[o][2] = 0.0;
-        auto lo = [](uint64_t v) { return __dsub_rn(__longlong_as_double((long long)((v & 0x1FFFFF) | 0x4330000000000000ull)), 4503599627370496.0); };
-        auto hi = [](uint64_t v) { return __dsub_rn(__longlong_as_double((long long)((v >> 21) | 0x4330000000000000ull)), 4503599627370496.0); };
-        for (uint32_t d = 0; d < beta; d++) {
-            ulonglong2 x;
-            if (perm) {
-                const uint64_t *dg = digits + ((size_t)d * lP + t) * N;
-                x = make_ulonglong2(dg[p2.x], dg[p2.y]);
-            } else {
-                x = (d == own_d) ? *reinterpret_cast<const ulonglong2 *>(own + (size_t)t * N + n)
-                                 : *reinterpret_cast<const ulonglong2 *>(digits + ((size_t)d * lP + t) * N + n);
-            }
-            const uint64_t *e = evk.p[d] + (size_t)pp * N + n;
-            const ulonglong2 e0 = __ldcs(reinterpret_cast<const ulonglong2 *>(e));
-            const ulonglong2 e1 = __ldcs(reinterpret_cast<const ulonglong2 *>(e + (size_t)size_QP * N));
-            const double xl[2] = {lo(x.x), lo(x.y)}, xh[2] = {hi(x.x), hi(x.y)};
-            const double el[4] = {lo(e0.x), lo(e0.y), lo(e1.x), lo(e1.y)}, eh[4] = {hi(e0.x), hi(e0.y), hi(e1.x), hi(e1.y)};
-#pragma unroll
-            for (int o = 0; o < 4; o++) {
-                const int c = o & 1;
-                A[o][0] = __fma_rn(xl[c], el[o], A[o][0]);
-                A[o][1] = __fma_rn(xl[c], eh[o], __fma_rn(xh[c], el[o], A[o][1]));
-                A[o][2] = __fma_rn(xh[c], eh[o], A[o][2]);
-            }
-        }
-        uint64_t r[4];
-        const W2 pi = FUSED && t < l ? pinv[pp] : W2{0, 0};
-        const double pid = (double)pi.w, piq = __dmul_rn(pid, qinv);
-#pragma unroll
-        for (int o = 0; o < 4; o++) {
-            double v = __dadd_rn(A[o][0], __dadd_rn(fp_mulmod(A[o][1], rm.cw[0], rm.cwq[0], qd), fp_mulmod(A[o][2], rm.cw[1], rm.cwq[1], qd)));
-            if (FUSED && t < l) v = fp_mulmod(v, pid, piq, qd);          // times P^-1 (|v| < 2^50)
-            else v = __fma_rn(-__dsub_rn(__fma_rn(v, qinv, b2::FP_MAGIC), b2::FP_MAGIC), qd, v);
-            if (v < 0.0) v = __dadd_rn(v, qd);
-            r[o] = (uint64_t)__double_as_longlong(__dadd_rn(v, 4503599627370496.0)) & 0x000FFFFFFFFFFFFFull;
-        }
-        if (!FUSED) {
-            *reinterpret_cast<ulonglong2 *>(out + idx) = make_ulonglong2(r[0], r[1]);
-            *reinterpret_cast<ulonglong2 *>(out + (size_t)lP * N + idx) = make_ulonglong2(r[2], r[3]);
-        } else if (t < l) {
-            uint64_t *c0 = ct + idx, *c1 = ct + (size_t)l * N + idx;
-            const ulonglong2 u0 = *reinterpret_cast<const ulonglong2 *>(c0), u1 = *reinterpret_cast<const ulonglong2 *>(c1);
-            *reinterpret_cast<ulonglong2 *>(c0) = make_ulonglong2(add_mod(u0.x, r[0], md.q), add_mod(u0.y, r[1], md.q));
-            *reinterpret_cast<ulonglong2 *>(c1) = make_ulonglong2(add_mod(u1.x, r[2], md.q), add_mod(u1.y, r[3], md.q));
-        } else {
-            const size_t o = ((size_t)(t - l) * ib.p_mul_i * (ib.p_lm1 + 1) + (size_t)blockIdx.y * ib.p_bs) * N + n;
-            const size_t o1 = o + (size_t)ib.p_mul_k * (ib.p_lm1 + 1) * N;
-            if (ACCP) {
-                const ulonglong2 p0 = *reinterpret_cast<const ulonglong2 *>(out + o), p1 = *reinterpret_cast<const ulonglong2 *>(out + o1);
-                r[0] = add_mod(r[0], p0.x, md.q), r[1] = add_mod(r[1], p0.y, md.q), r[2] = add_mod(r[2], p1.x, md.q), r[3] = add_mod(r[3], p1.y, md.q);
-            }
-            *reinterpret_cast<ulonglong2 *>(out + o) = make_ulonglong2(r[0], r[1]);
-            *reinterpret_cast<ulonglong2 *>(out + o1) = make_ulonglong2(r[2], r[3]);
-        }
-        return;
-    }
-    u128 a00{0, 0}, a01{0, 0}, a10{0, 0}, a11{0, 0};
-    for (uint32_t d0 = 0; d0 < beta; d0 += MAX_BETA) {
-        ulonglong2 x[MAX_BETA], e0[MAX_BETA], e1[MAX_BETA];
-#pragma unroll
-        for (int i = 0; i < MAX_BETA; i++) {
-            if (d0 + i < beta) {
-                if (perm) {
-                    const uint64_t *dg = digits + ((size_t)(d0 + i) * lP + t) * N;
-                    x[i] = make_ulonglong2(dg[p2.x], dg[p2.y]);
-                } else {
-                    x[i] = (d0 + i == own_d) ? *reinterpret_cast<const ulonglong2 *>(own + (size_t)t * N + n)
-                                             : *reinterpret_cast<const ulonglong2 *>(digits + ((size_t)(d0 + i) * lP + t) * N + n);
-                }
-                const uint64_t *e = evk.p[d0 + i] + (size_t)pp * N + n;
-                e0[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(e));
-                e1[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(e + (size_t)size_QP * N));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < MAX_BETA; i++) {
-            if (d0 + i < beta) {
-                mac128(a00, x[i].x, e0[i].x);
-                mac128(a01, x[i].y, e0[i].y);
-                mac128(a10, x[i].x, e1[i].x);
-                mac128(a11, x[i].y, e1[i].y);
-            }
-        }
-    }
-    uint64_t r00 = barrett128(a00, md.q, md.r0, md.r1), r01 = barrett128(a01, md.q, md.r0, md.r1);
-    uint64_t r10 = barrett128(a10, md.q, md.r0, md.r1), r11 = barrett128(a11, md.q, md.r0, md.r1);
-    if (!FUSED) {
-        *reinterpret_cast<ulonglong2 *>(out + idx) = make_ulonglong2(r00, r01);
-        *reinterpret_cast<ulonglong2 *>(out + (size_t)lP * N + idx) = make_ulonglong2(r10, r11);
-    } else if (t < l) {
-        const W2 pi = pinv[pp];
-        uint64_t *c0 = ct + idx, *c1 = ct + (size_t)l * N + idx;
-        const ulonglong2 u0 = *reinterpret_cast<const ulonglong2 *>(c0), u1 = *reinterpret_cast<const ulonglong2 *>(c1);
-        *reinterpret_cast<ulonglong2 *>(c0) =
-            make_ulonglong2(add_mod(u0.x, mul_shoup(r00, pi, md.q), md.q), add_mod(u0.y, mul_shoup(r01, pi, md.q), md.q));
-        *reinterpret_cast<ulonglong2 *>(c1) =
-            make_ulonglong2(add_mod(u1.x, mul_shoup(r10, pi, md.q), md.q), add_mod(u1.y, mul_shoup(r11, pi, md.q), md.q));
-    } else {
-        const size_t o = ((size_t)(t - l) * ib.p_mul_i * (ib.p_lm1 + 1) + (size_t)blockIdx.y * ib.p_bs) * N + n;
-        const size_t o1 = o + (size_t)ib.p_mul_k * (ib.p_lm1 + 1) * N;
-        if (ACCP) {
-            const ulonglong2 p0 = *reinterpret_cast<const ulonglong2 *>(out + o), p1 = *reinterpret_cast<const ulonglong2 *>(out + o1);
-            r00 = add_mod(r00, p0.x, md.q), r01 = add_mod(r01, p0.y, md.q), r10 = add_mod(r10, p1.x, md.q), r11 = add_mod(r11, p1.y, md.q);
-        }
-        *reinterpret_cast<ulonglong2 *>(out + o) = make_ulonglong2(r00, r01);
-        *reinterpret_cast<ulonglong2 *>(out + o1) = make_ulonglong2(r10, r11);
-    }
-}
-
-// HMult tensor product (src/polymath.cu:463-498): d0 = a0 b0, d2 = a1 b1, d1 = (a0+a1)(b0+b1) - d0 - d2
-// d0, d1 go to out[0..2S), d2 to out2[0..S): the relinearising caller keeps d2 in scratch and the rest in its result
-// A batch in one launch: blockIdx.y = pair b, whose operands, result and d2 start b * bs.x / .y / .z / .w limbs further.
-__global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *__restrict__ a, const uint64_t *__restrict__ b, uint64_t *__restrict__ out,
-                                                        uint64_t *__restrict__ out2, const Mod *mod, uint32_t N, uint32_t l, uint4 bs) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t S = (size_t)l * N;
-    if (idx >= S) return;
-    a += (size_t)blockIdx.y * bs.x * N, b += (size_t)blockIdx.y * bs.y * N, out += (size_t)blockIdx.y * bs.z * N, out2 += (size_t)blockIdx.y * bs.w * N;
-    const Mod md = mod[idx / N];
-    const uint64_t q = md.q;
-    const uint64_t a0 = a[idx], a1 = a[S + idx], b0 = b[idx], b1 = b[S + idx];
-    u128 p{0, 0};
-    mac128(p, a0, b0);
-    const uint64_t d0 = barrett128(p, q, md.r0, md.r1);
-    p = u128{0, 0};
-    mac128(p, a1, b1);
-    const uint64_t d2 = barrett128(p, q, md.r0, md.r1);
-    p = u128{0, 0};
-    mac128(p, add_mod(a0, a1, q), add_mod(b0, b1, q));
-    const uint64_t d1 = barrett128(p, q, md.r0, md.r1);
-    out[idx] = d0;
-    out[S + idx] = sub_mod(sub_mod(d1, d0, q), d2, q);
-    out2[idx] = d2;
-}
-
-// src/polymath.cu:17-180
-// `period` limbs per polynomial: limb t of the buffer uses prime t % period, so one launch covers a whole
-// ciphertext. b_wrap: the second operand is one polynomial shared by all (a plaintext).
-__global__ void __launch_bounds__(256) poly_op_kernel(int op, const uint64_t *a, const uint64_t *b, uint64_t *out, const Mod *mod,
-                                                     uint32_t N, uint32_t n_limbs, uint32_t period, int b_wrap) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_limbs * N) return;
-    const Mod md = mod[(idx / N) % period];
-    const uint64_t q = md.q, x = a[idx];
-    const size_t bi = b_wrap ? idx % ((size_t)period * N) : idx;
-    uint64_t r;
-    if (op == 0) r = add_mod(x, b[bi], q);
-    else if (op == 1) r = sub_mod(x, b[bi], q);
-    else if (op == 2) {
-        u128 p{0, 0};
-        mac128(p, x, b[bi]);
-        r = barrett128(p, q, md.r0, md.r1);
-    } else r = x ? q - x : 0;
-    out[idx] = r;
-}
-
-// Per-limb integer constants (src/bootstrap.cu:1535-1565, multiply_scalar_per_tower_kernel; adding
-// a constant polynomial c to NTT-form data adds c to every value of the limb).
-struct ScalarTab { uint64_t v[64]; };
-__global__ void __launch_bounds__(256) poly_scalar_kernel(int op, const uint64_t *a, ScalarTab tab, uint64_t *out, const Mod *mod,
-                                                        uint32_t N, uint32_t n_limbs, uint32_t period) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_limbs * N) return;
-    const uint32_t limb = (uint32_t)((idx / N) % period);
-    const Mod md = mod[limb];
-    const uint64_t q = md.q, x = a[idx], s = tab.v[limb];
-    uint64_t r;
-    if (op == 0) r = add_mod(x, s, q);
-    else {
-        u128 p{0, 0};
-        mac128(p, x, s);
-        r = barrett128(p, q, md.r0, md.r1);
-    }
-    out[idx] = r;
-}
-
-// NTT-domain automorphism (src/galois.cu:11-18): dst[l][i] = src[l][perm[i]].
-// Optional second operand pair so that c0 and c1 (or several digit buffers) go in one launch.
-__global__ void __launch_bounds__(256) galois_gather_kernel(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst,
-                                                           const uint32_t *__restrict__ perm, uint32_t N, uint32_t n_limbs) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_limbs * N) return;
-    const size_t limb = idx / N;
-    dst[idx] = src[limb * N + perm[idx % N]];
-}
-
-// The automorphism of a ciphertext (c0, c1) as a rotation needs it: perm(c0) goes straight into the result (added to it
-// when ACC: rotations that are summed), perm(c1) into the scratch the key switch reads. limbs [0, l) are c0, [l, 2l) c1.
-template <bool ACC>
-__global__ void __launch_bounds__(256) galois_split_kernel(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst0, uint64_t *__restrict__ dst1,
-                                                          const uint32_t *__restrict__ perm, const Mod *mod, uint32_t N, uint32_t l) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t S = (size_t)l * N;
-    if (idx >= 2 * S) return;
-    const size_t limb = idx / N;
-    const uint64_t v = src[limb * N + perm[idx % N]];
-    if (limb >= l) {
-        dst1[idx - S] = v;
-    } else if (ACC) {
-        dst0[idx] = add_mod(dst0[idx], v, mod[limb].q);
-    } else {
-        dst0[idx] = v;
-    }
-}
-
-// Single-chain plaintext expansion (src/bootstrap.cu:660-686, light_pt_expand_per_tower_kernel):
-// one signed, centred int64 coefficient vector -> its residue in each of n_limbs primes.
-__global__ void __launch_bounds__(256) expand_signed_kernel(const int64_t *__restrict__ src, uint64_t *__restrict__ dst, const Mod *mod, uint32_t N,
-                                                           uint32_t n_limbs, uint32_t first_prime) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_limbs * N) return;
-    const Mod md = mod[first_prime + idx / N];
-    const int64_t c = src[idx % N];
-    const uint64_t mag = c >= 0 ? (uint64_t)c : (uint64_t)0 - (uint64_t)c;
-    u128 v{mag, 0};
-    const uint64_t r = barrett128(v, md.q, md.r0, md.r1);
-    dst[idx] = (c >= 0 || r == 0) ? r : md.q - r;
-}
-
-// out = sum_t x_t * s_t (+ c on polynomial 0): per-limb integer weights, one reduction per value. The terms may
-// sit at higher levels than the output (more limbs per polynomial): lt[t] is term t's limb count.
-#define B2_LINCOMB_MAX_TERMS 8
-#define B2_LINCOMB_MAX_LIMBS 32
-struct LincombArgs {
-    const uint64_t *x[B2_LINCOMB_MAX_TERMS];
-    uint32_t lt[B2_LINCOMB_MAX_TERMS];
-    uint64_t s[B2_LINCOMB_MAX_TERMS][B2_LINCOMB_MAX_LIMBS];
-    uint64_t c[B2_LINCOMB_MAX_LIMBS];
-};
-__global__ void __launch_bounds__(256) lincomb_kernel(const __grid_constant__ LincombArgs a, uint64_t *out, const Mod *mod, uint32_t N, uint32_t l,
-                                                     uint32_t n_poly, uint32_t n_terms) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_poly * l * N) return;
-    const uint32_t i = (uint32_t)(idx % N), limb = (uint32_t)((idx / N) % l), p = (uint32_t)(idx / ((size_t)N * l));
-    const Mod md = mod[limb];
-    u128 acc{p == 0 ? a.c[limb] : 0, 0};
-    for (uint32_t t = 0; t < n_terms; t++) mac128(acc, a.x[t][((size_t)p * a.lt[t] + limb) * N + i], a.s[t][limb]);
-    out[idx] = barrett128(acc, md.q, md.r0, md.r1);
-}
-
-// M signed coefficient vectors at once: src [M][N] -> dst [M][l][N] (limb j of every polynomial on prime j)
-__global__ void __launch_bounds__(256) expand_signed_batch_kernel(const int64_t *__restrict__ src, uint64_t *__restrict__ dst, const Mod *mod, uint32_t N,
-                                                                 uint32_t l, uint32_t M) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)M * l * N) return;
-    const uint32_t i = (uint32_t)(idx % N), limb = (uint32_t)((idx / N) % l), m = (uint32_t)(idx / ((size_t)N * l));
-    const Mod md = mod[limb];
-    const int64_t c = src[(size_t)m * N + i];
-    const uint64_t mag = c >= 0 ? (uint64_t)c : (uint64_t)0 - (uint64_t)c;
-    u128 v{mag, 0};
-    const uint64_t r = barrett128(v, md.q, md.r0, md.r1);
-    dst[idx] = (c >= 0 || r == 0) ? r : md.q - r;
-}
-
-struct MacPtrs {
-    const uint64_t *const *pts;
-    const uint64_t *const *babies;
-};
-
-// BSGS giant-step multiply-accumulate (src/bsgs.cu:51-96): out_k = sum_b pt_b (.) baby_b[k].
-// The reference reduces after every term; the sum of canonical products is the same residue.
-__global__ void __launch_bounds__(256) bsgs_mac_kernel(const uint64_t *const *pts, const uint64_t *const *babies, uint64_t *out, const Mod *mod,
-                                                      uint32_t N, uint32_t l, uint32_t M) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t S = (size_t)l * N;
-    if (idx >= S) return;
-    const Mod md = mod[idx / N];
-    u128 a0{0, 0}, a1{0, 0};
-    uint32_t pending = 0;
-    uint64_t r0 = 0, r1 = 0;
-    for (uint32_t b = 0; b < M; b++) {
-        const uint64_t p = pts[b][idx];
-        mac128(a0, p, babies[b][idx]);
-        mac128(a1, p, babies[b][S + idx]);
-        if (++pending == 32) {  // 32 products of two 61-bit values stay below 2^128
-            a0 = u128{barrett128(a0, md.q, md.r0, md.r1), 0};
-            a1 = u128{barrett128(a1, md.q, md.r0, md.r1), 0};
-            pending = 1;
-        }
-    }
-    r0 = barrett128(a0, md.q, md.r0, md.r1);
-    r1 = barrett128(a1, md.q, md.r0, md.r1);
-    out[idx] = r0;
-    out[S + idx] = r1;
-}
-
-// Up to four giants at once: every baby value is loaded once and multiplied into each giant's own plaintext, so the
-// babies (two thirds of the bytes of the single-giant kernel) cross HBM once per group instead of once per giant.
-// pts[g * M + b] may be null: that giant has no diagonal for baby b.
-template <int G>
-__global__ void __launch_bounds__(256) bsgs_mac_multi_kernel(const uint64_t *const *pts, const uint64_t *const *babies, uint64_t *const *outs,
-                                                            const Mod *mod, uint32_t N, uint32_t l, uint32_t M, uint32_t n_g) {
-    pdl_enter();
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t S = (size_t)l * N;
-    if (idx >= S) return;
-    const Mod md = mod[idx / N];
-    u128 a[G][2];
-#pragma unroll
-    for (int g = 0; g < G; g++) a[g][0] = a[g][1] = u128{0, 0};
-    uint32_t pending = 0;
-    for (uint32_t b = 0; b < M; b++) {
-        const uint64_t *bb = babies[b];
-        const uint64_t y0 = bb[idx], y1 = bb[S + idx];
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            const uint64_t *pp = g < (int)n_g ? pts[(size_t)g * M + b] : nullptr;
-            if (pp) {
-                const uint64_t p = pp[idx];
-                mac128(a[g][0], p, y0);
-                mac128(a[g][1], p, y1);
-            }
-        }
-        if (++pending == 32) {  // 32 products of two 61-bit values stay below 2^128
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                a[g][0] = u128{barrett128(a[g][0], md.q, md.r0, md.r1), 0};
-                a[g][1] = u128{barrett128(a[g][1], md.q, md.r0, md.r1), 0};
-            }
-            pending = 1;
-        }
-    }
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        if (g < (int)n_g) {
-            uint64_t *o = outs[g];
-            o[idx] = barrett128(a[g][0], md.q, md.r0, md.r1);
-            o[S + idx] = barrett128(a[g][1], md.q, md.r0, md.r1);
-        }
-    }
-}
+// element-wise kernels: four words per thread where every buffer is 32-byte aligned, else one
+#define LAUNCH_V(kernel, wide, gy, gz, s, ...)                                                               \
+    do {                                                                                                     \
+        if (wide) launch_k(kernel<4>, dim3((unsigned)(c->N / 1024), gy, gz), 256, 0, s, __VA_ARGS__);        \
+        else launch_k(kernel<1>, dim3((unsigned)(c->N / 256), gy, gz), 256, 0, s, __VA_ARGS__);              \
+    } while (0)
 
 // Shared memory a conversion CTA asks for: what it uses, or enough that no more CTAs fit on an SM (228 KB) than its
 // 512 TMEM columns can serve, whichever is larger - so tcgen05.alloc finds its columns free and never waits.
@@ -1578,6 +1197,14 @@ static int run_bconv(const b2_ctx *c, bool copy, const uint64_t *in, uint64_t *o
 
 static inline size_t limb_bytes(const b2_ctx *c) { return c->N * 8; }
 
+// How many hoisted rotations go through each kernel together: as many as keep their P limbs and ModDown scratch (2 (l + alpha)
+// limbs each) within three quarters of the L2, two at least
+static size_t hoist_chunk(const b2_ctx *c, size_t l) {
+    const size_t one = 2 * (l + c->size_P) * limb_bytes(c), beta = (l + c->size_P - 1) / c->size_P;
+    const size_t fit = std::max<size_t>(2, (size_t(96) << 20) / one);
+    return std::max<size_t>(1, std::min({fit, (size_t)IP_MAX_STEPS, (size_t)EPI_TAB_MAX, IP_MAX_EVK / beta}));
+}
+
 extern "C" size_t b2_workspace_bytes(const b2_ctx *c, int op, size_t l) {
     if (!c || l < 1 || l > c->size_Q) return 0;
     const size_t a = c->size_P, beta = (l + a - 1) / a, lP = l + a, L = limb_bytes(c);
@@ -1588,7 +1215,7 @@ extern "C" size_t b2_workspace_bytes(const b2_ctx *c, int op, size_t l) {
         case B2_OP_RESCALE: return 3 * L;
         case B2_OP_MUL_RELIN: return (l + beta * lP + 2 * lP + 3 * l) * L;
         case B2_OP_ROTATE: return (l + beta * lP + 2 * lP + 2 * l) * L;
-        case B2_OP_HOIST: return (l + 2 * beta * lP + 2 * lP + l) * L;
+        case B2_OP_HOIST: return (3 * l + beta * lP + hoist_chunk(c, l) * 2 * lP) * L;
         default: return 0;
     }
 }
@@ -1606,9 +1233,12 @@ extern "C" int b2_ntt_inverse(b2_ctx *c, uint64_t *d, size_t n_limbs, size_t fir
 }
 
 // ModUp into `out`; `t` = l limbs of scratch for the scaled coefficient form
-static int modup_impl(b2_ctx *c, size_t l, const uint64_t *c2, uint64_t *out, uint64_t *t, bool copy_own, cudaStream_t s) {
+static int modup_impl(b2_ctx *c, size_t l, const uint64_t *c2, uint64_t *out, uint64_t *t, bool copy_own, cudaStream_t s,
+                      const uint32_t *perm = nullptr) {
     const LevelPlan &pl = c->plan[l];
-    int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s);
+    BatchDims bd;
+    bd.perm = perm;
+    int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, bd);
     if (rc) return rc;
     rc = run_bconv(c, copy_own, t, out, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)(l + c->size_P), true, s, &pl.tc_up);
     if (rc) return rc;
@@ -1623,37 +1253,50 @@ extern "C" int b2_modup(b2_ctx *c, size_t l, const uint64_t *d_c2, uint64_t *d_o
     return modup_impl(c, l, d_c2, d_out, (uint64_t *)d_ws, true, (cudaStream_t)stream);
 }
 
+// A rotation's part in a key switch: c2 (and c0, added to the first polynomial) are read through perm, and ct is overwritten
+// instead of added to.
+struct KsRot {
+    const uint32_t *perm = nullptr;
+    const uint64_t *c0 = nullptr;
+    bool ct_set = false;
+};
+
+static IpArgs ip_args(const b2_ctx *c, size_t l, const uint64_t *digits, const uint64_t *own, uint64_t *out, uint64_t *ct) {
+    IpArgs a{};
+    a.digits = digits, a.own = own, a.out = out, a.ct = ct, a.pinv = c->d_Pinv, a.mod = c->d_mod;
+    a.logN = (uint32_t)c->logN, a.l = (uint32_t)l, a.lP = (uint32_t)(l + c->size_P), a.size_Q = (uint32_t)c->size_Q, a.size_QP = (uint32_t)c->size_QP;
+    a.beta = c->plan[l].beta, a.nq = (uint32_t)l, a.np = (uint32_t)c->size_P;
+    a.ct_acc = 1, a.p_mul_i = 1, a.p_mul_k = (uint32_t)c->size_P;
+    return a;
+}
+
+// n_keys keys of n_evk digits each, one after another in evk
+static int run_inner_prod(const b2_ctx *c, IpArgs &a, const uint64_t *const *evk, size_t n_evk, size_t n_keys, uint32_t sets, cudaStream_t s) {
+    if (n_evk < a.beta) return fail(B2_EINVAL, "key has fewer digits than this level needs");
+    if (n_keys * a.beta > IP_MAX_EVK) return fail(B2_ESIZE, "inner product: too many digits in one launch");
+    for (size_t k = 0; k < n_keys; k++)
+        for (size_t d = 0; d < a.beta; d++) {
+            if (!evk[k * n_evk + d]) return fail(B2_EINVAL, "null evaluation-key digit");
+            a.evk[k * a.beta + d] = evk[k * n_evk + d];
+        }
+    if (a.nq + a.np == 0) return B2_OK;
+    LaunchScope ls(c, s, "ks_inner_prod");
+    launch_k(ks_inner_prod_kernel, dim3((unsigned)(c->N / 512), a.nq + a.np, sets), 256, 0, s, a);
+    LAUNCH_CHECK("ks_inner_prod_kernel");
+    return B2_OK;
+}
+
 // fused = false: out = cx [2][lP][N]. fused = true: Q limbs accumulate into ct, out = [2][alpha][N].
 static int inner_prod_impl(b2_ctx *c, size_t l, const uint64_t *digits, const uint64_t *own, const uint64_t *const *evk, size_t n_evk,
                            uint64_t *out, uint64_t *ct, bool fused, cudaStream_t s, const uint4 *range = nullptr, bool acc_p = false,
-                           uint32_t batch = 1, const IpBatch *ipb = nullptr, const uint32_t *perm = nullptr) {
-    const size_t beta = c->plan[l].beta, lP = l + c->size_P;
-    if (perm && own) return fail(B2_EINVAL, "a permuted inner product reads every limb from the digit buffer");
-    if (n_evk < beta) return fail(B2_EINVAL, "key has fewer digits than this level needs");
-    if (beta > 64) return fail(B2_ESIZE, "more than 64 digits");
-    EvkPtrs ep;
-    for (size_t d = 0; d < beta; d++) {
-        if (!evk[d]) return fail(B2_EINVAL, "null evaluation-key digit");
-        ep.p[d] = evk[d];
-    }
-    const uint4 rg = range ? *range : make_uint4(0, (uint32_t)l, 0, (uint32_t)c->size_P);
-    const size_t pairs = (size_t)(rg.y + rg.w) * c->N / 2;
-    if (pairs == 0) return B2_OK;
+                           uint32_t batch = 1, const IpBatch *ipb = nullptr, const KsRot &rot = KsRot{}) {
     if (batch != 1 && (!fused || !ipb)) return fail(B2_EINVAL, "a batched inner product runs in the fused form");
-    const dim3 grid((unsigned)((pairs + 255) / 256), batch);
-    const IpBatch ib = ipb ? *ipb : IpBatch{0, 0, 0, 1, (uint32_t)c->size_P, 0, 0};
-    LaunchScope ls(c, s, "ks_inner_prod");
-    if (fused && acc_p)
-        launch_k(ks_inner_prod_kernel<3, true, true>, grid, 256, 0, s, digits, own, ep, out, ct, c->d_Pinv, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l,
-                                                               (uint32_t)lP, (uint32_t)c->size_Q, (uint32_t)c->size_QP, (uint32_t)beta, rg, ib, perm);
-    else if (fused)
-        launch_k(ks_inner_prod_kernel<3, true>, grid, 256, 0, s, digits, own, ep, out, ct, c->d_Pinv, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l, (uint32_t)lP,
-                                                         (uint32_t)c->size_Q, (uint32_t)c->size_QP, (uint32_t)beta, rg, ib, perm);
-    else
-        launch_k(ks_inner_prod_kernel<3, false>, grid, 256, 0, s, digits, own, ep, out, nullptr, nullptr, c->d_mod, c->d_redc, (uint32_t)c->N, (uint32_t)l, (uint32_t)lP,
-                                                          (uint32_t)c->size_Q, (uint32_t)c->size_QP, (uint32_t)beta, rg, ib, perm);
-    LAUNCH_CHECK("ks_inner_prod_kernel");
-    return B2_OK;
+    IpArgs a = ip_args(c, l, digits, own, out, ct);
+    a.fused = fused, a.acc_p = acc_p;
+    if (range) a.q0 = range->x, a.nq = range->y, a.p0 = range->z, a.np = range->w;
+    if (ipb) a.dig_bs = ipb->dig_bs, a.own_bs = ipb->own_bs, a.ct_bs = ipb->ct_bs, a.p_mul_i = ipb->p_mul_i, a.p_mul_k = ipb->p_mul_k, a.p_lm1 = ipb->p_lm1, a.p_bs = ipb->p_bs;
+    a.perm[0] = rot.perm, a.c0 = rot.c0, a.ct_acc = !rot.ct_set;
+    return run_inner_prod(c, a, evk, n_evk, 1, batch, s);
 }
 
 extern "C" int b2_ks_inner_prod(b2_ctx *c, size_t l, const uint64_t *d_digits, const uint64_t *const *evk, size_t n_evk, uint64_t *d_out,
@@ -1692,17 +1335,13 @@ extern "C" int b2_moddown(b2_ctx *c, size_t l, size_t n_poly, uint64_t *d_cx, ui
     return moddown_impl(c, l, n_poly, d_cx, d_out, (uint64_t *)d_ws, false, (cudaStream_t)stream);
 }
 
-// Everything after ModUp, fused: ct += ModDown(<digits, evk>).
-// The inner product adds acc * P^-1 into the Q limbs of ct and keeps only the P limbs (cxP,
-// [2][alpha][N]); their inverse transform, the base conversion with the P^-1-carrying matrix and a
-// forward transform whose epilogue subtracts from ct finish the job. `delta`: 2*l limbs of scratch.
-static int ks_tail_fused(b2_ctx *c, size_t l, const uint64_t *digits, const uint64_t *own, const uint64_t *const *evk, size_t n_evk, uint64_t *ct,
-                         uint64_t *cxP, uint64_t *delta, cudaStream_t s, const uint32_t *perm = nullptr) {
+// The end of a fused key switch: the inner product has left acc * P^-1 in the Q limbs of the ciphertext and the P limbs in
+// cxP [2][alpha][N]. Their inverse transform, the base conversion with the P^-1-carrying matrix and a forward transform whose
+// epilogue subtracts from ct finish the job. `delta`: 2*l limbs of scratch.
+static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint64_t *ct, cudaStream_t s) {
     const LevelPlan &pl = c->plan[l];
     const size_t a = c->size_P;
-    int rc = inner_prod_impl(c, l, digits, own, evk, n_evk, cxP, ct, true, s, nullptr, false, 1, nullptr, perm);
-    if (rc) return rc;
-    rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
+    int rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
     if (rc) return rc;
     rc = run_bconv(c, false, cxP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
     if (rc) return rc;
@@ -1719,6 +1358,7 @@ static int ks_tail_fused(b2_ctx *c, size_t l, const uint64_t *digits, const uint
 // blocks t [l], up [beta][l+alpha], cxP [2][alpha] start b * c2_bs / ct_bs / l / beta (l+alpha) / 2 alpha limbs further.
 struct KsBatch {
     uint32_t batch = 1, c2_bs = 0, ct_bs = 0;
+    KsRot rot;
 };
 
 static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint64_t *const *evk, size_t n_evk, uint64_t *ct, uint64_t *cxP,
@@ -1737,7 +1377,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     {
         using Cfg = PassCfg<8>;
         const uint32_t B = kb.batch, per = (uint32_t)(beta * lP), a2 = (uint32_t)(2 * c->size_P);
-        int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, kb.c2_bs, 0, (uint32_t)l});
+        int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, kb.c2_bs, 0, (uint32_t)l, kb.rot.perm});
         if (rc) return rc;
         if (batched) {
             const TcBatch tb{B, 0, (uint32_t)l, 0, per, c->tc_serial_ld ? 1u : 0u};
@@ -1752,7 +1392,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
-            rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib);
+            rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib, kb.rot);
             if (rc) return rc;
             *done = true;
             return B2_OK;
@@ -1776,7 +1416,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (!wide) {
             const uint4 rest = make_uint4(0, pl.n_wideQ, 0, (uint32_t)c->size_P);
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
-            rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, &rest, acc_p, B, batched ? &ib : nullptr);
+            rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, &rest, acc_p, B, batched ? &ib : nullptr, kb.rot);
             if (rc) return rc;
         }
         {
@@ -1793,6 +1433,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             m.interleave = c->mac_interleave ? 1 : 0;
             m.dig_bs = per, m.own_bs = kb.c2_bs, m.ct_bs = kb.ct_bs, m.cxp_bs = a2;
             m.p_off = 0, m.cxp_i = 1, m.cxp_k = (uint32_t)c->size_P;
+            m.perm = kb.rot.perm, m.c0 = kb.rot.c0, m.ct_set = kb.rot.ct_set;
             const uint32_t n_limbs = (uint32_t)l - m.first_limb + m.p_first;
             LaunchScope ls(c, s, "ntt_fwd_rows_mac");
             static_assert(Cfg::R_STRIDED == Cfg::R_CONTIG, "the fused pass wants equal stage groups");
@@ -1807,24 +1448,19 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
 
 // ws layout of the key switch: t [l] | up [beta][lP] | cxP [2][alpha]; delta reuses `up`
 static int keyswitch_impl(b2_ctx *c, size_t l, const uint64_t *c2, const uint64_t *const *evk, size_t n_evk, uint64_t *ct, uint64_t *ws,
-                          cudaStream_t s) {
+                          cudaStream_t s, const KsRot &rot = KsRot{}) {
     const size_t N = c->N, lP = l + c->size_P, beta = c->plan[l].beta;
     uint64_t *t = ws, *up = t + l * N, *cxP = up + beta * lP * N;
-    const LevelPlan &pl = c->plan[l];
     bool done = false;
-    int rc = modup_inner_fused(c, l, c2, evk, n_evk, ct, cxP, t, up, false, s, &done);
+    int rc = modup_inner_fused(c, l, c2, evk, n_evk, ct, cxP, t, up, false, s, &done, KsBatch{1, 0, 0, rot});
     if (rc) return rc;
-    if (done) {
-        const size_t ap = c->size_P;
-        rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * ap), 0, c->d_fin_P, s);
+    if (!done) {
+        rc = modup_impl(c, l, c2, up, t, false, s, rot.perm);  // the inner product reads the own limbs from c2
         if (rc) return rc;
-        rc = run_bconv(c, false, cxP, up, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)ap, (uint32_t)l, true, s, &pl.tc_dnf);
+        rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, false, 1, nullptr, rot);
         if (rc) return rc;
-        return run_fwd(c, up, up, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
     }
-    rc = modup_impl(c, l, c2, up, t, false, s);  // the inner product reads the own limbs from c2
-    if (rc) return rc;
-    return ks_tail_fused(c, l, up, c2, evk, n_evk, ct, cxP, up, s);
+    return ks_moddown(c, l, cxP, up, ct, s);
 }
 
 extern "C" int b2_keyswitch(b2_ctx *c, size_t l, const uint64_t *d_c2, const uint64_t *const *evk, size_t n_evk, uint64_t *d_ct, void *d_ws,
@@ -1857,7 +1493,7 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     bool done = false;
     int rc = B2_OK;
     if (batch > 1) {
-        rc = modup_inner_fused(c, l, d_c2, evk, n_evk, d_ct, cxP, t, up, false, s, &done, KsBatch{B, (uint32_t)c2_stride, (uint32_t)ct_stride});
+        rc = modup_inner_fused(c, l, d_c2, evk, n_evk, d_ct, cxP, t, up, false, s, &done, KsBatch{B, (uint32_t)c2_stride, (uint32_t)ct_stride, KsRot{}});
         if (rc) return rc;
     }
     if (!done) {
@@ -1895,7 +1531,8 @@ extern "C" int b2_tensor_mul(b2_ctx *c, size_t l, const uint64_t *d_a, const uin
     if (!d_a || !d_b || !d_out) return fail(B2_EINVAL, "tensor_mul: null pointer");
     const size_t n = l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "tensor_mul");
-    launch_k(tensor_mul_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, d_a, d_b, d_out, d_out + 2 * n, c->d_mod, (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
+    LAUNCH_V(tensor_mul_kernel, aligned32(d_a) && aligned32(d_b) && aligned32(d_out), (unsigned)l, 1, (cudaStream_t)stream, d_a, d_b, d_out, d_out + 2 * n, c->d_mod,
+             (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
     LAUNCH_CHECK("tensor_mul_kernel");
     return B2_OK;
 }
@@ -1913,7 +1550,8 @@ extern "C" int b2_multiply_and_relin(b2_ctx *c, size_t l, const uint64_t *d_a, c
         // d0, d1 straight into the result, d2 into scratch for the key switch (every thread reads its own position of
         // the operands before it writes, so the result may alias an operand)
         LaunchScope ls(c, s, "tensor_mul");
-        launch_k(tensor_mul_kernel, (unsigned)((S + 255) / 256), 256, 0, s, d_a, d_b, d_out, t3 + 2 * S, c->d_mod, (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
+        LAUNCH_V(tensor_mul_kernel, aligned32(d_a) && aligned32(d_b) && aligned32(d_out) && aligned32(t3), (unsigned)l, 1, s, d_a, d_b, d_out, t3 + 2 * S, c->d_mod,
+                 (uint32_t)c->N, (uint32_t)l, make_uint4(0, 0, 0, 0));
         LAUNCH_CHECK("tensor_mul_kernel");
     }
     return keyswitch_impl(c, l, t3 + 2 * S, rlk, n_evk, d_out, ws, s);
@@ -1996,8 +1634,8 @@ extern "C" int b2_multiply_relin_rescale_batch(b2_ctx *c, size_t l, size_t batch
     uint64_t *prod = (uint64_t *)d_ws, *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
     {
         LaunchScope ls(c, s, "tensor_mul");
-        launch_k(tensor_mul_kernel, dim3((unsigned)((S + 255) / 256), B), 256, 0, s, d_a, d_b, prod, prod + 2 * S, c->d_mod, (uint32_t)N, (uint32_t)l,
-                                                                             make_uint4((uint32_t)a_stride, (uint32_t)b_stride, (uint32_t)(3 * l), (uint32_t)(3 * l)));
+        LAUNCH_V(tensor_mul_kernel, true, (unsigned)l, B, s, d_a, d_b, prod, prod + 2 * S, c->d_mod, (uint32_t)N, (uint32_t)l,
+                 make_uint4((uint32_t)a_stride, (uint32_t)b_stride, (uint32_t)(3 * l), (uint32_t)(3 * l)));
         LAUNCH_CHECK("tensor_mul_kernel");
     }
     int rc = keyswitch_batch_impl(c, l, batch, prod + 2 * S, 3 * l, rlk, n_evk, prod, 3 * l, ws, s);
@@ -2114,21 +1752,14 @@ extern "C" int b2_galois_prepare(b2_ctx *c, uint32_t elt) {
 }
 
 static int gather_impl(b2_ctx *c, const uint32_t *perm, const uint64_t *src, uint64_t *dst, size_t n_limbs, cudaStream_t s) {
-    const size_t n = n_limbs * c->N;
     LaunchScope ls(c, s, "galois_gather");
-    launch_k(galois_gather_kernel, (unsigned)((n + 255) / 256), 256, 0, s, src, dst, perm, (uint32_t)c->N, (uint32_t)n_limbs);
+    LAUNCH_V(galois_gather_kernel, aligned32(dst), (unsigned)n_limbs, 1, s, src, dst, perm, (uint32_t)c->N);
     LAUNCH_CHECK("galois_gather_kernel");
     return B2_OK;
 }
 
-static int gather_split_impl(b2_ctx *c, const uint32_t *perm, const uint64_t *src, uint64_t *dst0, uint64_t *dst1, size_t l, bool acc, cudaStream_t s) {
-    const size_t n = 2 * l * c->N;
-    LaunchScope ls(c, s, "galois_gather");
-    if (acc) launch_k(galois_split_kernel<true>, (unsigned)((n + 255) / 256), 256, 0, s, src, dst0, dst1, perm, c->d_mod, (uint32_t)c->N, (uint32_t)l);
-    else launch_k(galois_split_kernel<false>, (unsigned)((n + 255) / 256), 256, 0, s, src, dst0, dst1, perm, c->d_mod, (uint32_t)c->N, (uint32_t)l);
-    LAUNCH_CHECK("galois_split_kernel");
-    return B2_OK;
-}
+// whether [a, a + words) and [b, b + words) have a word in common
+static bool overlap(const uint64_t *a, const uint64_t *b, size_t words) { return a < b + words && b < a + words; }
 
 // tables must exist before an asynchronous sequence starts: creating one synchronises
 static int galois_lookup(b2_ctx *c, uint32_t elt, const uint32_t **out) {
@@ -2159,19 +1790,15 @@ extern "C" int b2_apply_galois(b2_ctx *c, size_t l, uint32_t elt, const uint64_t
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t S = l * c->N;
-    uint64_t *p = (uint64_t *)d_ws, *ws = p + 2 * S;  // permuted c0 | permuted c1
-    // (c0, c1) <- (perm(c0), 0) + key switch of perm(c1)   (src/evaluate.cu:1644-1655)
-    const bool apart = d_out + 2 * S <= d_ct || d_ct + 2 * S <= d_out;
-    if (apart) {
-        rc = gather_split_impl(c, perm, d_ct, d_out, p + S, l, false, s);  // perm(c0) lands in the result
-        if (rc) return rc;
-    } else {
-        rc = gather_impl(c, perm, d_ct, p, 2 * l, s);  // both polynomials: limb index only selects the row
-        if (rc) return rc;
-        CUDA_TRY(cudaMemcpyAsync(d_out, p, S * 8, cudaMemcpyDeviceToDevice, s));
+    uint64_t *p = (uint64_t *)d_ws, *ws = p + 2 * S;
+    // (c0, c1) <- (perm(c0), 0) + key switch of perm(c1)   (src/evaluate.cu:1644-1655): both polynomials are read through the
+    // permutation where they are needed; a result on top of its operand works on a copy
+    const uint64_t *ct = d_ct;
+    if (overlap(d_out, d_ct, 2 * S)) {
+        CUDA_TRY(cudaMemcpyAsync(p, d_ct, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
+        ct = p;
     }
-    CUDA_TRY(cudaMemsetAsync(d_out + S, 0, S * 8, s));
-    return keyswitch_impl(c, l, p + S, ksk, n_evk, d_out, ws, s);
+    return keyswitch_impl(c, l, ct + S, ksk, n_evk, d_out, ws, s, KsRot{perm, ct, true});
 }
 
 // Rotations whose results are summed share one ModDown: each call adds perm(c0) + (inner product) * P^-1 on the Q limbs
@@ -2186,32 +1813,20 @@ extern "C" int b2_apply_galois_accumulate(b2_ctx *c, size_t l, uint32_t elt, con
     int rc = galois_lookup(c, elt, &perm);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t N = c->N, S = l * N, lP = l + c->size_P, beta = c->plan[l].beta;
-    uint64_t *p = (uint64_t *)d_ws, *t = p + 2 * S, *up = t + S;  // permuted c0 | permuted c1 | t | up
-    if (d_acc + 2 * S <= d_ct || d_ct + 2 * S <= d_acc) {
-        // perm(c0) straight into (or onto) the accumulator, perm(c1) into scratch: one launch
-        rc = gather_split_impl(c, perm, d_ct, d_acc, p + S, l, !first, s);
-        if (rc) return rc;
-        if (first) CUDA_TRY(cudaMemsetAsync(d_acc + S, 0, S * 8, s));
-    } else {
-        rc = gather_impl(c, perm, d_ct, p, 2 * l, s);
-        if (rc) return rc;
-        if (first) {
-            CUDA_TRY(cudaMemcpyAsync(d_acc, p, S * 8, cudaMemcpyDeviceToDevice, s));
-            CUDA_TRY(cudaMemsetAsync(d_acc + S, 0, S * 8, s));
-        } else {
-            rc = b2_poly_op(c, 0, l, d_acc, p, d_acc, stream);
-            if (rc) return rc;
-        }
+    const size_t S = l * c->N;
+    uint64_t *p = (uint64_t *)d_ws, *t = p + 2 * S, *up = t + S;  // a copy of the operand where it is needed | t | up
+    const uint64_t *ct = d_ct;
+    if (overlap(d_acc, d_ct, 2 * S)) {
+        CUDA_TRY(cudaMemcpyAsync(p, d_ct, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
+        ct = p;
     }
-    (void)beta;
-    (void)lP;
+    const KsRot rot{perm, ct, first != 0};
     bool done = false;
-    rc = modup_inner_fused(c, l, p + S, ksk, n_evk, d_acc, d_accP, t, up, !first, s, &done);
+    rc = modup_inner_fused(c, l, ct + S, ksk, n_evk, d_acc, d_accP, t, up, !first, s, &done, KsBatch{1, 0, 0, rot});
     if (rc || done) return rc;
-    rc = modup_impl(c, l, p + S, up, t, false, s);
+    rc = modup_impl(c, l, ct + S, up, t, false, s, perm);
     if (rc) return rc;
-    return inner_prod_impl(c, l, up, p + S, ksk, n_evk, d_accP, d_acc, true, s, nullptr, !first);
+    return inner_prod_impl(c, l, up, ct + S, ksk, n_evk, d_accP, d_acc, true, s, nullptr, !first, 1, nullptr, rot);
 }
 
 extern "C" int b2_keyswitch_finish(b2_ctx *c, size_t l, uint64_t *d_accP, uint64_t *d_acc, void *d_ws, size_t ws_bytes, void *stream) {
@@ -2219,15 +1834,7 @@ extern "C" int b2_keyswitch_finish(b2_ctx *c, size_t l, uint64_t *d_accP, uint64
     CHECK_LEVEL(c, l);
     if (!d_accP || !d_acc || !d_ws) return fail(B2_EINVAL, "keyswitch_finish: null pointer");
     if (ws_bytes < 2 * l * c->N * sizeof(uint64_t)) return fail(B2_EWS, "keyswitch_finish: workspace too small (2 * size_Ql limbs)");
-    cudaStream_t s = (cudaStream_t)stream;
-    const LevelPlan &pl = c->plan[l];
-    const size_t a = c->size_P;
-    uint64_t *delta = (uint64_t *)d_ws;
-    int rc = run_inv(c, d_accP, d_accP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
-    if (rc) return rc;
-    rc = run_bconv(c, false, d_accP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
-    if (rc) return rc;
-    return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_acc}, s);
+    return ks_moddown(c, l, d_accP, (uint64_t *)d_ws, d_acc, (cudaStream_t)stream);
 }
 
 extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, const uint32_t *elts, size_t n_steps, const uint64_t *const *ksk,
@@ -2237,31 +1844,58 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
     if (!d_ct || !elts || !ksk || !d_outs || !d_ws) return fail(B2_EINVAL, "hoist_rotations: null pointer");
     if (ws_bytes < b2_workspace_bytes(c, B2_OP_HOIST, l)) return fail(B2_EWS, "hoist_rotations: workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t N = c->N, lP = l + c->size_P, beta = c->plan[l].beta, S = l * N;
+    const size_t N = c->N, a = c->size_P, lP = l + a, beta = c->plan[l].beta, S = l * N;
+    const LevelPlan &pl = c->plan[l];
     std::vector<const uint32_t *> perms(n_steps);
+    bool on_top = false;
     for (size_t i = 0; i < n_steps; i++) {
         int rc = galois_lookup(c, elts[i], &perms[i]);
         if (rc) return rc;
-    }
-    // ws: t [l] | up [beta][lP] | pup [beta][lP] | cx [2][lP] | pc0 [l]
-    uint64_t *t = (uint64_t *)d_ws, *up = t + S, *pup = up + beta * lP * N, *cx = pup + beta * lP * N, *pc0 = cx + 2 * lP * N;
-    int rc = modup_impl(c, l, d_ct + S, up, t, true, s);  // ModUp(c1) once (src/evaluate.cu:2013-2014)
-    if (rc) return rc;
-    for (size_t i = 0; i < n_steps; i++) {
         if (!d_outs[i]) return fail(B2_EINVAL, "hoist_rotations: null output");
-        rc = gather_impl(c, perms[i], d_ct, pc0, l, s);
+        on_top = on_top || overlap(d_outs[i], d_ct, 2 * S);
+    }
+    // ws: t [l] | up [beta][lP] | copy of the operand [2][l] | cxP [chunk][2][alpha] | delta [chunk][2][l]
+    const size_t chunk = hoist_chunk(c, l);
+    uint64_t *t = (uint64_t *)d_ws, *up = t + S, *copy = up + beta * lP * N, *cxP = copy + 2 * S, *delta = cxP + chunk * 2 * a * N;
+    const uint64_t *ct = d_ct;
+    if (on_top) {
+        CUDA_TRY(cudaMemcpyAsync(copy, d_ct, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
+        ct = copy;
+    }
+    int rc = modup_impl(c, l, ct + S, up, t, false, s);  // ModUp(c1) once (src/evaluate.cu:2013-2014)
+    if (rc) return rc;
+    // c0_out = perm(c0) + ModDown(cx0); c1_out = ModDown(cx1). The digits are permuted AFTER ModUp (src/evaluate.cu:2041-2045):
+    // the inner product reads them, c0 and the limbs a digit holds itself through the permutation. The steps go through each
+    // kernel in chunks, one launch for all steps of a chunk (eight steps at N = 2^15, 12 limbs: 504 us one after another).
+    for (size_t i0 = 0; i0 < n_steps; i0 += chunk) {
+        const uint32_t n = (uint32_t)std::min(chunk, n_steps - i0);
+        IpArgs ia = ip_args(c, l, up, ct + S, cxP, nullptr);
+        ia.fused = 1, ia.ct_acc = 0, ia.c0 = ct, ia.steps = n, ia.each = 1, ia.p_bs = (uint32_t)(2 * a);
+        EpiSubFromTab epi{};
+        for (uint32_t i = 0; i < n; i++) ia.perm[i] = perms[i0 + i], ia.ct_tab[i] = epi.tab[i] = d_outs[i0 + i];
+        rc = run_inner_prod(c, ia, ksk + i0 * n_evk, n_evk, n, n, s);
         if (rc) return rc;
-        // c0_out = perm(c0) + ModDown(cx0); c1_out = ModDown(cx1). The digits are permuted AFTER ModUp
-        // (src/evaluate.cu:2041-2045): the inner product reads them through the permutation, `pup` only serves as delta
-        CUDA_TRY(cudaMemcpyAsync(d_outs[i], pc0, S * 8, cudaMemcpyDeviceToDevice, s));
-        CUDA_TRY(cudaMemsetAsync(d_outs[i] + S, 0, S * 8, s));
-        rc = ks_tail_fused(c, l, up, nullptr, ksk + i * n_evk, n_evk, d_outs[i], cx, pup, s, perms[i]);
+        rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
+        if (rc) return rc;
+        if (c->bconv_tc && !c->tc_simple) {
+            const TcBatch tb{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l), 0};
+            rc = run_bconv_tc(c, false, cxP, delta, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, &tb);
+            if (rc) return rc;
+        } else {
+            for (uint32_t i = 0; i < n; i++) {
+                rc = run_bconv(c, false, cxP + i * 2 * a * N, delta + i * 2 * S, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a,
+                               (uint32_t)l, true, s, &pl.tc_dnf);
+                if (rc) return rc;
+            }
+        }
+        rc = run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, epi, s, 0, 0, 0, BatchDims{n, 0, (uint32_t)(2 * l), 0, (uint32_t)(2 * l)});
         if (rc) return rc;
     }
     return B2_OK;
 }
 
-// hoisting_inplace (src/evaluate.cu:1732-1927): the SUM of n_steps rotations from one ModUp and one ModDown pair.
+// hoisting_inplace (src/evaluate.cu:1732-1927): the SUM of n_steps rotations from one ModUp and one ModDown pair. The inner
+// products of the steps are summed inside one launch, before any reduction.
 extern "C" int b2_hoisting_sum(b2_ctx *c, size_t l, const uint64_t *d_ct, const uint32_t *elts, size_t n_steps, const uint64_t *const *ksk,
                                size_t n_evk, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
     CHECK_CTX(c);
@@ -2270,39 +1904,39 @@ extern "C" int b2_hoisting_sum(b2_ctx *c, size_t l, const uint64_t *d_ct, const 
     if (ws_bytes < b2_workspace_bytes(c, B2_OP_HOIST, l)) return fail(B2_EWS, "hoisting_sum: workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t N = c->N, a = c->size_P, lP = l + a, beta = c->plan[l].beta, S = l * N;
-    const LevelPlan &pl = c->plan[l];
     std::vector<const uint32_t *> perms(n_steps);
     for (size_t i = 0; i < n_steps; i++) {
         int rc = galois_lookup(c, elts[i], &perms[i]);
         if (rc) return rc;
     }
-    // ws: t [l] | up [beta][lP] | pup [beta][lP] | accP [2][alpha] + delta [2][l] (the 2*lP limbs of cx) | pc0 [l]
-    uint64_t *t = (uint64_t *)d_ws, *up = t + S, *pup = up + beta * lP * N /* unused: the digits are read through the permutation */, *accP = pup + beta * lP * N, *delta = accP + 2 * a * N,
-             *pc0 = accP + 2 * lP * N;
-    int rc = modup_impl(c, l, d_ct + S, up, t, true, s);
+    // ws: t [l] | up [beta][lP] | copy of the operand [2][l] | accP [2][alpha] | delta [2][l]
+    uint64_t *t = (uint64_t *)d_ws, *up = t + S, *copy = up + beta * lP * N, *accP = copy + 2 * S, *delta = accP + 2 * a * N;
+    const uint64_t *ct = d_ct;
+    if (overlap(d_out, d_ct, 2 * S)) {
+        CUDA_TRY(cudaMemcpyAsync(copy, d_ct, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
+        ct = copy;
+    }
+    int rc = modup_impl(c, l, ct + S, up, t, false, s);
     if (rc) return rc;
-    for (size_t i = 0; i < n_steps; i++) {
-        rc = gather_impl(c, perms[i], d_ct, i == 0 ? d_out : pc0, l, s);
-        if (rc) return rc;
-        if (i == 0) CUDA_TRY(cudaMemsetAsync(d_out + S, 0, S * 8, s));
-        else if ((rc = b2_poly_op(c, 0, l, d_out, pc0, d_out, stream))) return rc;
-        rc = inner_prod_impl(c, l, up, nullptr, ksk + i * n_evk, n_evk, accP, d_out, true, s, nullptr, i > 0, 1, nullptr, perms[i]);
+    const size_t chunk = std::max<size_t>(1, std::min<size_t>(IP_MAX_STEPS, IP_MAX_EVK / beta));
+    for (size_t i0 = 0; i0 < n_steps; i0 += chunk) {
+        const uint32_t n = (uint32_t)std::min(chunk, n_steps - i0);
+        IpArgs ia = ip_args(c, l, up, ct + S, accP, d_out);
+        ia.fused = 1, ia.ct_acc = ia.acc_p = i0 > 0, ia.c0 = ct, ia.steps = n;
+        for (uint32_t i = 0; i < n; i++) ia.perm[i] = perms[i0 + i];
+        rc = run_inner_prod(c, ia, ksk + i0 * n_evk, n_evk, n, 1, s);
         if (rc) return rc;
     }
-    rc = run_inv(c, accP, accP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
-    if (rc) return rc;
-    rc = run_bconv(c, false, accP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
-    if (rc) return rc;
-    return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_out}, s);
+    return ks_moddown(c, l, accP, delta, d_out, s);
 }
 
 extern "C" int b2_bsgs_mac(b2_ctx *c, size_t l, size_t M, const uint64_t *const *pts, const uint64_t *const *babies, uint64_t *d_out, void *stream) {
     CHECK_CTX(c);
     CHECK_LEVEL(c, l);
     if (!pts || !babies || !d_out || M == 0) return fail(B2_EINVAL, "bsgs_mac: bad argument");
-    const size_t n = l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "bsgs_mac");
-    launch_k(bsgs_mac_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, pts, babies, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)M);
+    launch_k(bsgs_mac_kernel<1>, dim3((unsigned)(c->N / 256), (unsigned)l), 256, 0, (cudaStream_t)stream, pts, babies, nullptr, d_out, c->d_mod, (uint32_t)c->N,
+             (uint32_t)l, (uint32_t)M, 1u);
     LAUNCH_CHECK("bsgs_mac_kernel");
     return B2_OK;
 }
@@ -2312,11 +1946,11 @@ extern "C" int b2_bsgs_mac_multi(b2_ctx *c, size_t l, size_t M, size_t n_giants,
     CHECK_CTX(c);
     CHECK_LEVEL(c, l);
     if (!pts || !babies || !outs || M == 0 || n_giants < 1 || n_giants > 4) return fail(B2_EINVAL, "bsgs_mac_multi: bad argument (1 to 4 giants)");
-    const size_t n = l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "bsgs_mac");
-    launch_k(bsgs_mac_multi_kernel<4>, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, pts, babies, outs, c->d_mod, (uint32_t)c->N, (uint32_t)l,
-                                                                                            (uint32_t)M, (uint32_t)n_giants);
-    LAUNCH_CHECK("bsgs_mac_multi_kernel");
+    auto k = n_giants == 1 ? bsgs_mac_kernel<1> : n_giants == 2 ? bsgs_mac_kernel<2> : n_giants == 3 ? bsgs_mac_kernel<3> : bsgs_mac_kernel<4>;
+    launch_k(k, dim3((unsigned)(c->N / 256), (unsigned)l), 256, 0, (cudaStream_t)stream, pts, babies, outs, nullptr, c->d_mod, (uint32_t)c->N, (uint32_t)l,
+             (uint32_t)M, (uint32_t)n_giants);
+    LAUNCH_CHECK("bsgs_mac_kernel");
     return B2_OK;
 }
 
@@ -2326,11 +1960,10 @@ extern "C" int b2_expand_signed(b2_ctx *c, size_t first_prime, size_t n_limbs, c
     if (!d_signed || !d_out) return fail(B2_EINVAL, "expand_signed: null pointer");
     if (n_limbs < 1 || first_prime + n_limbs > c->size_QP) return fail(B2_EINVAL, "expand_signed: limb range outside the modulus chain");
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t n = n_limbs * c->N;
     {
         LaunchScope ls(c, s, "expand_signed");
-        launch_k(expand_signed_kernel, (unsigned)((n + 255) / 256), 256, 0, s, d_signed, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
-                                                                        (uint32_t)first_prime);
+        LAUNCH_V(expand_signed_kernel, aligned32(d_signed) && aligned32(d_out), (unsigned)n_limbs, 1, s, d_signed, d_out, c->d_mod, (uint32_t)c->N,
+                 (uint32_t)n_limbs, (uint32_t)first_prime);
         LAUNCH_CHECK("expand_signed_kernel");
     }
     if (!to_ntt) return B2_OK;
@@ -2423,11 +2056,11 @@ extern "C" int b2_expand_single_chain_batch(b2_ctx *c, size_t l, size_t M, const
     CHECK_LEVEL(c, l);
     if (!d_signed || !d_out || M == 0) return fail(B2_EINVAL, "expand_single_chain_batch: bad argument");
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t n = M * l * c->N;
     {
         LaunchScope ls(c, s, "expand_signed");
-        launch_k(expand_signed_batch_kernel, (unsigned)((n + 255) / 256), 256, 0, s, d_signed, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)M);
-        LAUNCH_CHECK("expand_signed_batch_kernel");
+        LAUNCH_V(expand_signed_kernel, aligned32(d_signed) && aligned32(d_out), (unsigned)l, (unsigned)M, s, d_signed, d_out, c->d_mod, (uint32_t)c->N,
+                 (uint32_t)l, 0u);
+        LAUNCH_CHECK("expand_signed_kernel");
     }
     return run_fwd(c, d_out, d_out, nullptr, (uint32_t)(M * l), 0, EpiStore{}, s, (uint32_t)l);
 }
@@ -2435,10 +2068,9 @@ extern "C" int b2_expand_single_chain_batch(b2_ctx *c, size_t l, size_t M, const
 extern "C" int b2_poly_op(b2_ctx *c, int op, size_t n_limbs, const uint64_t *d_a, const uint64_t *d_b, uint64_t *d_out, void *stream) {
     CHECK_CTX(c);
     if (op < 0 || op > 3 || !d_a || !d_out || (op != 3 && !d_b) || n_limbs < 1 || n_limbs > c->size_QP) return fail(B2_EINVAL, "poly_op: bad argument");
-    const size_t n = n_limbs * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_op");
-    launch_k(poly_op_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
-                                                                                   (uint32_t)n_limbs, 0);
+    const bool wide = aligned32(d_a) && aligned32(d_out) && (op == 3 || aligned32(d_b));
+    LAUNCH_V(poly_op_kernel, wide, (unsigned)n_limbs, 1, (cudaStream_t)stream, op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs, 0);
     LAUNCH_CHECK("poly_op_kernel");
     return B2_OK;
 }
@@ -2447,10 +2079,9 @@ extern "C" int b2_ct_op(b2_ctx *c, int op, size_t l, size_t n_poly, const uint64
     CHECK_CTX(c);
     if (op < 0 || op > 3 || !d_a || !d_out || (op != 3 && !d_b) || l < 1 || l > c->size_QP || n_poly < 1 || n_poly > 3)
         return fail(B2_EINVAL, "ct_op: bad argument");
-    const size_t n = n_poly * l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_op");
-    launch_k(poly_op_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(n_poly * l),
-                                                                                   (uint32_t)l, op == 2);
+    const bool wide = aligned32(d_a) && aligned32(d_out) && (op == 3 || aligned32(d_b));
+    LAUNCH_V(poly_op_kernel, wide, (unsigned)(n_poly * l), 1, (cudaStream_t)stream, op, d_a, d_b, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, op == 2 ? 1 : 0);
     LAUNCH_CHECK("poly_op_kernel");
     return B2_OK;
 }
@@ -2464,10 +2095,9 @@ extern "C" int b2_poly_scalar(b2_ctx *c, int op, size_t n_limbs, const uint64_t 
         if (h_scalars[i] >= c->q[i]) return fail(B2_EINVAL, "poly_scalar: scalar not reduced");
         tab.v[i] = h_scalars[i];
     }
-    const size_t n = n_limbs * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_scalar");
-    launch_k(poly_scalar_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, op, d_a, tab, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)n_limbs,
-                                                                                       (uint32_t)n_limbs);
+    LAUNCH_V(poly_scalar_kernel, aligned32(d_a) && aligned32(d_out), (unsigned)n_limbs, 1, (cudaStream_t)stream, op, d_a, tab, d_out, c->d_mod, (uint32_t)c->N,
+             (uint32_t)n_limbs);
     LAUNCH_CHECK("poly_scalar_kernel");
     return B2_OK;
 }
@@ -2480,10 +2110,9 @@ extern "C" int b2_ct_scalar(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *
         if (h_scalars[i] >= c->q[i]) return fail(B2_EINVAL, "ct_scalar: scalar not reduced");
         tab.v[i] = h_scalars[i];
     }
-    const size_t n = n_poly * l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "poly_scalar");
-    launch_k(poly_scalar_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, 1, d_a, tab, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)(n_poly * l),
-                                                                                       (uint32_t)l);
+    LAUNCH_V(poly_scalar_kernel, aligned32(d_a) && aligned32(d_out), (unsigned)(n_poly * l), 1, (cudaStream_t)stream, 1, d_a, tab, d_out, c->d_mod,
+             (uint32_t)c->N, (uint32_t)l);
     LAUNCH_CHECK("poly_scalar_kernel");
     return B2_OK;
 }
@@ -2509,10 +2138,9 @@ extern "C" int b2_ct_lincomb(b2_ctx *c, size_t l, size_t n_poly, size_t n_terms,
         if (h_const[i] >= c->q[i]) return fail(B2_EINVAL, "ct_lincomb: constant not reduced");
         a.c[i] = h_const[i];
     }
-    const size_t n = n_poly * l * c->N;
     LaunchScope ls(c, (cudaStream_t)stream, "lincomb");
-    launch_k(lincomb_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, a, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l, (uint32_t)n_poly,
-                                                                                   (uint32_t)n_terms);
+    launch_k(lincomb_kernel, dim3((unsigned)(c->N / 256), (unsigned)(n_poly * l)), 256, 0, (cudaStream_t)stream, a, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l,
+             (uint32_t)n_terms);
     LAUNCH_CHECK("lincomb_kernel");
     return B2_OK;
 }

@@ -24,7 +24,8 @@
 namespace b2 {
 
 struct Mod {
-    uint64_t q, r0, r1, pad;  // r = floor(2^128 / q)
+    uint64_t q, r0, r1;  // r = floor(2^128 / q)
+    uint64_t mu;         // floor(2^(62 + n) / q), n = bit length of q
 };
 
 // One job = one limb transform: where the limb lives and which prime's tables it uses.
@@ -59,6 +60,7 @@ struct NttArgs {
     // lives at slot s * (lm1 + 1) + b * bs of the buffer. Zero-initialised fields mean one set, slots as they are.
     // Batch-major buffers [b][slots] use lm1 = 0, bs = slots per set; limb-major ones [slot][b] use lm1 = batch - 1, bs = 1.
     uint32_t src_lm1, src_bs, dst_lm1, dst_bs;
+    const uint32_t *perm;  // inverse row pass: the input is read through a Galois element's permutation (a rotation's c1)
 };
 
 // The sets of a batched launch are the slow grid dimension. With the sets fastest (the CTAs of all sets on one tile next to
@@ -174,6 +176,18 @@ struct EpiSubFrom {
             st256(o_ + o + 4 * i, sub_mod(r.u[i].a, x[4 * i], q), sub_mod(r.u[i].b, x[4 * i + 1], q), sub_mod(r.u[i].c, x[4 * i + 2], q),
                   sub_mod(r.u[i].d, x[4 * i + 3], q));
     }
+};
+
+// the same with a buffer per set of the batch (hoisted rotations: every result is a ciphertext of its own)
+constexpr int EPI_TAB_MAX = 16;
+struct EpiSubFromTab : EpiSubFrom {
+    uint64_t *tab[EPI_TAB_MAX];
+    bool aligned() const {
+        for (auto p : tab)
+            if (!aligned32(p)) return false;
+        return true;
+    }
+    __device__ __forceinline__ void init(const NttArgs &a, const Job &job, size_t N) { o_ = tab[set_idx(a)] + (size_t)job.w * N; }
 };
 
 template <int LOG_T, int RC>
@@ -605,6 +619,10 @@ struct MacArgs {
     // P limb i of polynomial k of set b lands at limb slot i * cxp_i + k * cxp_k + b * cxp_bs of cxp: [set][2][alpha] is
     // (1, alpha, 2 alpha), the limb-major exchange buffer [alpha][2][sets] is (2 sets, sets, 1)
     uint32_t cxp_i, cxp_k;
+    // a rotation: `own` and, added to polynomial 0, c0 [l][N] are read through perm; ct_set: ct is overwritten, not added to
+    const uint32_t *perm;
+    const uint64_t *c0;
+    uint32_t ct_set;
 };
 
 __device__ __forceinline__ u64x4 ld256_cs(const uint64_t *p) {  // streaming: the key is read once
@@ -714,7 +732,14 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
             cp_async_commit();
         }
         T y[E];
-        if (d == own_d) {
+        if (d == own_d && m.perm) {
+            const uint64_t *src = m.own + ((size_t)bset * m.own_bs + t) * N;
+#pragma unroll
+            for (int i = 0; i < E; i += 4) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(m.perm + o + i);
+                y[i] = A::from_u64(src[v.x], k), y[i + 1] = A::from_u64(src[v.y], k), y[i + 2] = A::from_u64(src[v.z], k), y[i + 3] = A::from_u64(src[v.w], k);
+            }
+        } else if (d == own_d) {
 #pragma unroll
             for (int i = 0; i < E; i += 4) {
                 const u64x4 v = ld256(m.own + ((size_t)bset * m.own_bs + t) * N + o + i);
@@ -756,7 +781,6 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
         uint64_t *c0 = m.ct + ((size_t)bset * m.ct_bs + t) * N + o, *c1 = c0 + (size_t)m.l * N;
 #pragma unroll
         for (int i = 0; i < E; i += 4) {
-            const u64x4 u = ld256(c0 + i), v = ld256(c1 + i);
             uint64_t r[4], s[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -764,8 +788,18 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
                 s[j] = Acc::finish(acc1[i + j], pi, k, mc);
                 if (FP) r[j] = mul_shoup(r[j], pi, q), s[j] = mul_shoup(s[j], pi, q);
             }
-            st256(c0 + i, add_mod(u.a, r[0], q), add_mod(u.b, r[1], q), add_mod(u.c, r[2], q), add_mod(u.d, r[3], q));
-            st256(c1 + i, add_mod(v.a, s[0], q), add_mod(v.b, s[1], q), add_mod(v.c, s[2], q), add_mod(v.d, s[3], q));
+            if (m.c0) {
+                const uint64_t *src = m.c0 + (size_t)t * N;
+                const uint4 v = *reinterpret_cast<const uint4 *>(m.perm + o + i);
+                r[0] = add_mod(r[0], src[v.x], q), r[1] = add_mod(r[1], src[v.y], q), r[2] = add_mod(r[2], src[v.z], q), r[3] = add_mod(r[3], src[v.w], q);
+            }
+            if (!m.ct_set) {
+                const u64x4 u = ld256(c0 + i), v = ld256(c1 + i);
+                r[0] = add_mod(u.a, r[0], q), r[1] = add_mod(u.b, r[1], q), r[2] = add_mod(u.c, r[2], q), r[3] = add_mod(u.d, r[3], q);
+                s[0] = add_mod(v.a, s[0], q), s[1] = add_mod(v.b, s[1], q), s[2] = add_mod(v.c, s[2], q), s[3] = add_mod(v.d, s[3], q);
+            }
+            st256(c0 + i, r[0], r[1], r[2], r[3]);
+            st256(c1 + i, s[0], s[1], s[2], s[3]);
         }
     } else {
         // a P limb: kept (or, acc_p, added to what is there) in the compact buffer [2][alpha][N] for the ModDown that
@@ -848,6 +882,15 @@ __device__ __forceinline__ void inv_body(const NttArgs &a, uint64_t *sm, const J
             for (int i = 0; i < EA; i++) {
                 const uint64_t v = p[(size_t)i * estride];
                 x[i] = FIRST ? A::from_u64(v, k) : A::from_raw(v);
+            }
+        } else if (FIRST && a.perm) {
+            // an aligned run of EA values comes from an aligned run of EA values: whole sectors are used
+            const uint32_t *pm = a.perm + base + (size_t)c * cstride + (size_t)ehi * EA;
+#pragma unroll
+            for (int i = 0; i < EA; i += 4) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(pm + i);
+                x[i] = A::from_u64(src[v.x], k), x[i + 1] = A::from_u64(src[v.y], k);
+                x[i + 2] = A::from_u64(src[v.z], k), x[i + 3] = A::from_u64(src[v.w], k);
             }
         } else {
 #pragma unroll

@@ -62,3 +62,73 @@ def test_prime_classes_at_their_upper_edges(log_n):
             d = dev(x)
             check(call(ctx._h, d.data_ptr(), len(primes), 0, torch.cuda.current_stream().cuda_stream))
             assert np.array_equal(host(d), want)
+
+
+@pytest.mark.parametrize("log_n,bits,special,l,n_steps", [
+    (12, [60, 40, 50, 45, 60], 1, 3, 19),                  # more steps than one launch takes, one limb per digit
+    (13, [60, 40, 36, 50, 40, 60, 59], 2, 5, 3),           # ragged last digit, every prime class
+    (16, [60, 40, 40, 60, 60], 2, 3, 5),                   # chunks bounded by the L2
+])
+def test_hoisted_rotations_equal_the_oracle(log_n, bits, special, l, n_steps):
+    """one result per step, their sum, and a result on top of its operand"""
+    N = 1 << log_n
+    steps = list(range(1, n_steps + 1))
+    elts = [ph.get_elt_from_step(s, N) for s in steps]
+    ctx, o = make_ctx(N, bits, special, elts)
+    keys = [o.synth_key(o.beta(l), 6, 100 + 40 * i) for i in range(n_steps)]
+    glk = ph.galois_key.from_keys([ph.relin_key.from_numpy(ctx, k) for k in keys])
+    ct_h = o.synth_ct(l, 6, 1)
+    chain = o.size_Q - l + 1
+    ct = ph.ciphertext.from_numpy(ctx, ct_h, chain)
+    for got, want in zip(ph.hoist_rotations(ctx, ct, glk, steps), o.hoist_rotations(l, ct_h, elts, keys)):
+        assert np.array_equal(got.numpy(), want)
+    assert np.array_equal(ph.hoisting(ctx, ct, glk, steps).numpy(), o.hoisting_sum(l, ct_h, elts, keys))
+    from pyPhantom import _native
+    from pyPhantom._native import LIB, check
+    s, tab = torch.cuda.current_stream().cuda_stream, glk.relin_keys[0].pointer_table()
+    want = o.apply_galois(l, elts[0], keys[0], ct_h)
+    for out in (ctx.empty(2, l), dev(ct_h)):
+        src = out if out.data_ptr() != ct.data.data_ptr() and np.array_equal(host(out), ct_h) else ct.data
+        ws, nb = ctx.workspace(_native.OP_ROTATE, l)
+        check(LIB.b2_apply_galois(ctx._h, l, elts[0], src.data_ptr(), tab.ctypes.data, len(tab), out.data_ptr(), ws.data_ptr(), nb, s))
+        assert np.array_equal(host(out), want)
+    out = dev(ct_h)
+    ws, nb = ctx.workspace(_native.OP_HOIST, l)
+    ptr = np.array([out.data_ptr()], dtype=np.uint64)
+    e0 = np.array(elts[:1], dtype=np.uint32)
+    check(LIB.b2_hoist_rotations(ctx._h, l, out.data_ptr(), e0.ctypes.data, 1, tab.ctypes.data, len(tab), ptr.ctypes.data, ws.data_ptr(), nb, s))
+    assert np.array_equal(host(out), o.hoist_rotations(l, ct_h, elts[:1], keys[:1])[0])
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("M", [1, 3, 64, 131])
+def test_giant_steps_on_every_prime_class(M):
+    """the sums of M products at the edges of their loops (groups of four, tables of 64, sums that have to be folded), operands
+    at q - 1 so that every term is as large as it gets"""
+    from oracle_lib import Oracle
+    from pyPhantom._native import LIB, check
+    N = 4096
+    primes = [_largest_prime(1 << b, 2 * N) for b in (61, 60, 50, 41, 30)] + [_largest_prime((1 << 58) + 1, 2 * N)]
+    parms = ph.params(ph.scheme_type.ckks)
+    parms.set_poly_modulus_degree(N)
+    parms.set_coeff_modulus(primes)
+    parms.set_special_modulus_size(1)
+    ctx, o, l = ph.context(parms), Oracle(N, primes, 1), 5
+    q = np.array(primes[:l], dtype=np.uint64)[:, None]
+    pts = [o.fill(1, o.primes[:l], 2, 10 + i)[0] for i in range(M)]
+    bab = [o.synth_ct(l, 2, 500 + i) for i in range(M)]
+    for i in range(M):
+        pts[i][:, : N // 2] = q - np.uint64(1)
+        bab[i][:, :, : N // 2] = q - np.uint64(1)
+    want = o.bsgs_mac(l, pts, bab)
+    dp, db = [dev(p) for p in pts], [dev(b) for b in bab]
+    table = lambda ts: torch.tensor([t.data_ptr() for t in ts], dtype=torch.int64, device="cuda")
+    s, tp, tb = torch.cuda.current_stream().cuda_stream, table(dp), table(db)
+    out = ctx.empty(2, l)
+    check(LIB.b2_bsgs_mac(ctx._h, l, M, tp.data_ptr(), tb.data_ptr(), out.data_ptr(), s))
+    assert np.array_equal(host(out), want)
+    for n in (2, 3, 4):
+        outs = [ctx.empty(2, l) for _ in range(n)]
+        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, n, torch.cat([tp] * n).data_ptr(), tb.data_ptr(), table(outs).data_ptr(), s))
+        for t in outs:
+            assert np.array_equal(host(t), want)
