@@ -129,6 +129,7 @@ def test_giant_steps_on_every_prime_class(M):
     assert np.array_equal(host(out), want)
     for n in (2, 3, 4):
         outs = [ctx.empty(2, l) for _ in range(n)]
-        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, n, torch.cat([tp] * n).data_ptr(), tb.data_ptr(), table(outs).data_ptr(), s))
+        tabs = torch.cat([tp] * n), table(outs)
+        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, n, tabs[0].data_ptr(), tb.data_ptr(), tabs[1].data_ptr(), s))
         for t in outs:
             assert np.array_equal(host(t), want)
