@@ -191,6 +191,18 @@ int b2_apply_galois(b2_ctx *ctx, size_t size_Ql, uint32_t galois_elt, const uint
                     const uint64_t *const *ksk, size_t n_evk, uint64_t *d_out, void *d_ws,
                     size_t ws_bytes, void *stream);
 
+/* No counterpart in the reference, which makes one call per ciphertext (src/bsgs.cu:194-359):
+ *   b2_apply_galois_batch: `batch` ciphertexts rotated by one element, every kernel one launch over the batch; set b at
+ *                          b * ct_stride / b * out_stride limbs, results distinct from the operands; workspace
+ *                          b2_keyswitch_batch_workspace_bytes;
+ *   b2_rotate_add:         d_acc += the rotated d_ct (distinct buffers; workspace B2_OP_KEYSWITCH). */
+int b2_apply_galois_batch(b2_ctx *ctx, size_t size_Ql, uint32_t galois_elt, size_t batch, const uint64_t *d_ct,
+                          size_t ct_stride, const uint64_t *const *ksk, size_t n_evk, uint64_t *d_out,
+                          size_t out_stride, void *d_ws, size_t ws_bytes, void *stream);
+int b2_rotate_add(b2_ctx *ctx, size_t size_Ql, uint32_t galois_elt, const uint64_t *d_ct,
+                  const uint64_t *const *ksk, size_t n_evk, uint64_t *d_acc, void *d_ws, size_t ws_bytes,
+                  void *stream);
+
 /* replaces hoisting_inplace (src/evaluate.cu:1732-1927): d_out [2][size_Ql][N] = the SUM over the n_steps Galois
  * elements of the rotated d_ct, from one ModUp of c1 and one ModDown per polynomial (ksk and workspace as for
  * b2_hoist_rotations; d_out must not alias d_ct) */
@@ -239,6 +251,11 @@ int b2_expand_single_chain(b2_ctx *ctx, size_t size_Ql, const int64_t *d_signed,
  * d_signed int64[M][N] -> d_out [M][size_Ql][N] in NTT form, two launches for the expansion and two for all transforms */
 int b2_expand_single_chain_batch(b2_ctx *ctx, size_t size_Ql, size_t M, const int64_t *d_signed, uint64_t *d_out,
                                  void *stream);
+
+/* the same from M separate vectors (a HOST array of pointers the device can read: pinned host memory or device memory,
+ * 16-byte aligned), coefficient form: d_out [M][size_Ql][N]; b2_ntt_forward_batch transforms M polynomials of size_Ql limbs */
+int b2_expand_gather(b2_ctx *ctx, size_t size_Ql, size_t M, const int64_t *const *srcs, uint64_t *d_out, void *stream);
+int b2_ntt_forward_batch(b2_ctx *ctx, uint64_t *d_data, size_t size_Ql, size_t M, void *stream);
 
 /* the same over any limb range [first_prime, first_prime + n_limbs), optionally left in coefficient
  * form: what the samplers and the encoder of the reference do per limb when they reduce a small

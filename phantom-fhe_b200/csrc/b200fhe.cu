@@ -1259,6 +1259,7 @@ struct KsRot {
     const uint32_t *perm = nullptr;
     const uint64_t *c0 = nullptr;
     bool ct_set = false;
+    uint32_t c0_bs = 0;  // batch stride of c0 in limbs
 };
 
 static IpArgs ip_args(const b2_ctx *c, size_t l, const uint64_t *digits, const uint64_t *own, uint64_t *out, uint64_t *ct) {
@@ -1295,7 +1296,7 @@ static int inner_prod_impl(b2_ctx *c, size_t l, const uint64_t *digits, const ui
     a.fused = fused, a.acc_p = acc_p;
     if (range) a.q0 = range->x, a.nq = range->y, a.p0 = range->z, a.np = range->w;
     if (ipb) a.dig_bs = ipb->dig_bs, a.own_bs = ipb->own_bs, a.ct_bs = ipb->ct_bs, a.p_mul_i = ipb->p_mul_i, a.p_mul_k = ipb->p_mul_k, a.p_lm1 = ipb->p_lm1, a.p_bs = ipb->p_bs;
-    a.perm[0] = rot.perm, a.c0 = rot.c0, a.ct_acc = !rot.ct_set;
+    a.perm[0] = rot.perm, a.c0 = rot.c0, a.c0_bs = rot.c0_bs, a.ct_acc = !rot.ct_set;
     return run_inner_prod(c, a, evk, n_evk, 1, batch, s);
 }
 
@@ -1433,7 +1434,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             m.interleave = c->mac_interleave ? 1 : 0;
             m.dig_bs = per, m.own_bs = kb.c2_bs, m.ct_bs = kb.ct_bs, m.cxp_bs = a2;
             m.p_off = 0, m.cxp_i = 1, m.cxp_k = (uint32_t)c->size_P;
-            m.perm = kb.rot.perm, m.c0 = kb.rot.c0, m.ct_set = kb.rot.ct_set;
+            m.perm = kb.rot.perm, m.c0 = kb.rot.c0, m.c0_bs = kb.rot.c0_bs, m.ct_set = kb.rot.ct_set;
             const uint32_t n_limbs = (uint32_t)l - m.first_limb + m.p_first;
             LaunchScope ls(c, s, "ntt_fwd_rows_mac");
             static_assert(Cfg::R_STRIDED == Cfg::R_CONTIG, "the fused pass wants equal stage groups");
@@ -1485,7 +1486,7 @@ extern "C" size_t b2_keyswitch_batch_workspace_bytes(const b2_ctx *c, size_t l, 
 // puts the sets that share a key tile next to one another in the grid, so all but the first find it in L2. Elsewhere the
 // key switches run one after another on the same stream. Workspace: t [batch][l] | up [batch][beta][l+alpha] | cxP [batch][2][alpha].
 static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_t *d_c2, size_t c2_stride, const uint64_t *const *evk, size_t n_evk,
-                                  uint64_t *d_ct, size_t ct_stride, void *d_ws, cudaStream_t s) {
+                                  uint64_t *d_ct, size_t ct_stride, void *d_ws, cudaStream_t s, const KsRot &rot = KsRot{}) {
     const LevelPlan &pl = c->plan[l];
     const size_t N = c->N, a = c->size_P, lP = l + a, beta = pl.beta;
     const uint32_t B = (uint32_t)batch, per = (uint32_t)(beta * lP);
@@ -1493,14 +1494,16 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     bool done = false;
     int rc = B2_OK;
     if (batch > 1) {
-        rc = modup_inner_fused(c, l, d_c2, evk, n_evk, d_ct, cxP, t, up, false, s, &done, KsBatch{B, (uint32_t)c2_stride, (uint32_t)ct_stride, KsRot{}});
+        rc = modup_inner_fused(c, l, d_c2, evk, n_evk, d_ct, cxP, t, up, false, s, &done, KsBatch{B, (uint32_t)c2_stride, (uint32_t)ct_stride, rot});
         if (rc) return rc;
     }
     if (!done) {
         // one at a time, each in its own block of the workspace
         const size_t one = l + beta * lP + 2 * a;
         for (size_t b = 0; b < batch; b++) {
-            rc = keyswitch_impl(c, l, d_c2 + b * c2_stride * N, evk, n_evk, d_ct + b * ct_stride * N, (uint64_t *)d_ws + b * one * N, s);
+            KsRot r = rot;
+            if (r.c0) r.c0 += b * rot.c0_bs * N;
+            rc = keyswitch_impl(c, l, d_c2 + b * c2_stride * N, evk, n_evk, d_ct + b * ct_stride * N, (uint64_t *)d_ws + b * one * N, s, r);
             if (rc) return rc;
         }
         return B2_OK;
@@ -1801,6 +1804,38 @@ extern "C" int b2_apply_galois(b2_ctx *c, size_t l, uint32_t elt, const uint64_t
     return keyswitch_impl(c, l, ct + S, ksk, n_evk, d_out, ws, s, KsRot{perm, ct, true});
 }
 
+// d_acc += the rotated d_ct (a Horner step of a BSGS product: one addition less to launch and to stream). Distinct buffers.
+extern "C" int b2_rotate_add(b2_ctx *c, size_t l, uint32_t elt, const uint64_t *d_ct, const uint64_t *const *ksk, size_t n_evk, uint64_t *d_acc,
+                             void *d_ws, size_t ws_bytes, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!d_ct || !ksk || !d_acc || !d_ws) return fail(B2_EINVAL, "rotate_add: null pointer");
+    if (overlap(d_acc, d_ct, 2 * l * c->N)) return fail(B2_EINVAL, "rotate_add: needs distinct operand and accumulator");
+    if (ws_bytes < b2_workspace_bytes(c, B2_OP_KEYSWITCH, l)) return fail(B2_EWS, "rotate_add: workspace too small");
+    const uint32_t *perm;
+    int rc = galois_lookup(c, elt, &perm);
+    if (rc) return rc;
+    return keyswitch_impl(c, l, d_ct + l * c->N, ksk, n_evk, d_acc, (uint64_t *)d_ws, (cudaStream_t)stream, KsRot{perm, d_ct, false});
+}
+
+// `batch` ciphertexts rotated by one Galois element, every kernel one launch over the batch (see b2_keyswitch_batch)
+extern "C" int b2_apply_galois_batch(b2_ctx *c, size_t l, uint32_t elt, size_t batch, const uint64_t *d_ct, size_t ct_stride, const uint64_t *const *ksk,
+                                     size_t n_evk, uint64_t *d_out, size_t out_stride, void *d_ws, size_t ws_bytes, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!d_ct || !ksk || !d_out || !d_ws || batch < 1 || batch > 65535) return fail(B2_EINVAL, "apply_galois_batch: bad argument");
+    if (ct_stride < 2 * l || out_stride < 2 * l || ct_stride > 0xFFFFFFFFull || out_stride > 0xFFFFFFFFull)
+        return fail(B2_EINVAL, "apply_galois_batch: a set's stride is smaller than the set");
+    if (d_out < d_ct + batch * ct_stride * c->N && d_ct < d_out + batch * out_stride * c->N)
+        return fail(B2_EINVAL, "apply_galois_batch: needs distinct operands and results");
+    if (ws_bytes < b2_keyswitch_batch_workspace_bytes(c, l, batch)) return fail(B2_EWS, "apply_galois_batch: workspace too small");
+    const uint32_t *perm;
+    int rc = galois_lookup(c, elt, &perm);
+    if (rc) return rc;
+    return keyswitch_batch_impl(c, l, batch, d_ct + l * c->N, ct_stride, ksk, n_evk, d_out, out_stride, d_ws, (cudaStream_t)stream,
+                                KsRot{perm, d_ct, true, (uint32_t)ct_stride});
+}
+
 // Rotations whose results are summed share one ModDown: each call adds perm(c0) + (inner product) * P^-1 on the Q limbs
 // of d_acc and the P limbs of the inner product to d_accP; b2_keyswitch_finish converts the P limbs once.
 extern "C" int b2_apply_galois_accumulate(b2_ctx *c, size_t l, uint32_t elt, const uint64_t *d_ct, const uint64_t *const *ksk, size_t n_evk,
@@ -2063,6 +2098,31 @@ extern "C" int b2_expand_single_chain_batch(b2_ctx *c, size_t l, size_t M, const
         LAUNCH_CHECK("expand_signed_kernel");
     }
     return run_fwd(c, d_out, d_out, nullptr, (uint32_t)(M * l), 0, EpiStore{}, s, (uint32_t)l);
+}
+
+extern "C" int b2_expand_gather(b2_ctx *c, size_t l, size_t M, const int64_t *const *srcs, uint64_t *d_out, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!srcs || !d_out || M == 0) return fail(B2_EINVAL, "expand_gather: bad argument");
+    for (size_t m0 = 0; m0 < M; m0 += GATHER_MAX) {
+        const size_t n = std::min<size_t>(GATHER_MAX, M - m0);
+        GatherPtrs g{};
+        for (size_t i = 0; i < n; i++) {
+            if (!srcs[m0 + i] || ((uintptr_t)srcs[m0 + i] & 15)) return fail(B2_EINVAL, "expand_gather: vectors must be there and 16-byte aligned");
+            g.p[i] = srcs[m0 + i];
+        }
+        LaunchScope ls(c, (cudaStream_t)stream, "expand_signed");
+        launch_k(expand_gather_kernel, GATHER_CTAS, 256, 0, (cudaStream_t)stream, g, d_out + m0 * l * c->N, c->d_mod, (uint32_t)c->logN, (uint32_t)l, (uint32_t)n);
+        LAUNCH_CHECK("expand_gather_kernel");
+    }
+    return B2_OK;
+}
+
+extern "C" int b2_ntt_forward_batch(b2_ctx *c, uint64_t *d, size_t l, size_t M, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!d || M == 0) return fail(B2_EINVAL, "ntt_forward_batch: bad argument");
+    return run_fwd(c, d, d, nullptr, (uint32_t)(M * l), 0, EpiStore{}, (cudaStream_t)stream, (uint32_t)l);
 }
 
 extern "C" int b2_poly_op(b2_ctx *c, int op, size_t n_limbs, const uint64_t *d_a, const uint64_t *d_b, uint64_t *d_out, void *stream) {

@@ -423,6 +423,32 @@ __global__ void __launch_bounds__(256) expand_signed_kernel(const int64_t *__res
     stv<V>(dst + ((size_t)blockIdx.z * l + blockIdx.y) * N + i, x);
 }
 
+// The same from M separate vectors that the device can read where they are (pinned host memory): every coefficient crosses
+// the link once and becomes its l residues in registers. A launch of GATHER_CTAS CTAs keeps a few hundred kilobytes of reads
+// in flight, which is what the link takes, and leaves the SMs to the kernels of other streams. (256 copies of 128 KB took 6.4
+// us each, a quarter of the link's rate, plus a host call each.)
+constexpr int GATHER_MAX = 128, GATHER_CTAS = 96;
+struct GatherPtrs {
+    const int64_t *p[GATHER_MAX];
+};
+__global__ void __launch_bounds__(256) expand_gather_kernel(const __grid_constant__ GatherPtrs src, uint64_t *__restrict__ dst, const Mod *mod, uint32_t logN,
+                                                            uint32_t l, uint32_t M) {
+    pdl_enter();
+    const uint32_t per = 1u << (logN - 1);  // pairs of coefficients in a vector
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < M * per; i += gridDim.x * 256) {
+        const uint32_t m = i >> (logN - 1), k = 2 * (i & (per - 1));
+        const longlong2 c = *reinterpret_cast<const longlong2 *>(src.p[m] + k);
+        const uint64_t ax = c.x >= 0 ? (uint64_t)c.x : (uint64_t)0 - (uint64_t)c.x, ay = c.y >= 0 ? (uint64_t)c.y : (uint64_t)0 - (uint64_t)c.y;
+        uint64_t *d = dst + (((size_t)m * l) << logN) + k;
+        for (uint32_t j = 0; j < l; j++) {
+            const Mod md = mod[j];
+            const uint64_t rx = barrett64(ax, md.q, md.r1), ry = barrett64(ay, md.q, md.r1);
+            *reinterpret_cast<ulonglong2 *>(d + ((size_t)j << logN)) =
+                make_ulonglong2(c.x >= 0 || rx == 0 ? rx : md.q - rx, c.y >= 0 || ry == 0 ? ry : md.q - ry);
+        }
+    }
+}
+
 // ---- key-switch inner product (src/eval_key_switch.cu:175-230) ---------------------------------------------------------------
 // For logical limb t (physical prime pp):  acc[k][t][n] = sum_d digits[d][t][n] * evk[d][k][pp][n],  k = 0, 1.
 // Pure streaming: two coefficients per thread, 16-byte loads, three digits' loads issued before the first multiply.
@@ -443,6 +469,7 @@ struct IpArgs {
     // blockIdx.z = set of a batch with one key: its digits, own, ct start z * dig_bs / own_bs / ct_bs limbs further, and P limb
     // i of polynomial k lands at slot (i * p_mul_i + k * p_mul_k) * (p_lm1 + 1) + z * p_bs of the P-limb buffer
     uint32_t dig_bs, own_bs, ct_bs, p_mul_i, p_mul_k, p_lm1, p_bs;
+    uint32_t c0_bs;  // a batch of rotations: c0 of set z starts z * c0_bs limbs further
     // hoisted rotations: steps > 0. Step s reads digits and own through perm[s] and has the key evk[s * beta ..]. each = 1: one
     // set per step, written to ct_tab[z] (P limbs as above); each = 0: the steps are summed.
     // A rotation whose c1 was permuted before ModUp: steps = 0 and perm[0] set; own and c0 are read through it, digits are not.
@@ -477,7 +504,7 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
         const uint32_t pn = a.perm[s] ? a.perm[s][n] : 0;
         const bool pm = a.perm[s] != nullptr;
         if (a.c0 && t < a.l) {
-            const ulonglong2 c = ld_pair(a.c0 + (size_t)t * N, n, pn, pm);
+            const ulonglong2 c = ld_pair(a.c0 + ((size_t)z * a.c0_bs + t) * N, n, pn, pm);
             g0 = add_mod(g0, c.x, md.q), g1 = add_mod(g1, c.y, md.q);
         }
         for (uint32_t d0 = 0; d0 < a.beta; d0 += U) {

@@ -622,7 +622,7 @@ struct MacArgs {
     // a rotation: `own` and, added to polynomial 0, c0 [l][N] are read through perm; ct_set: ct is overwritten, not added to
     const uint32_t *perm;
     const uint64_t *c0;
-    uint32_t ct_set;
+    uint32_t ct_set, c0_bs;  // c0 of set b of a batch starts b * c0_bs limbs further
 };
 
 __device__ __forceinline__ u64x4 ld256_cs(const uint64_t *p) {  // streaming: the key is read once
@@ -789,7 +789,7 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
                 if (FP) r[j] = mul_shoup(r[j], pi, q), s[j] = mul_shoup(s[j], pi, q);
             }
             if (m.c0) {
-                const uint64_t *src = m.c0 + (size_t)t * N;
+                const uint64_t *src = m.c0 + ((size_t)bset * m.c0_bs + t) * N;
                 const uint4 v = *reinterpret_cast<const uint4 *>(m.perm + o + i);
                 r[0] = add_mod(r[0], src[v.x], q), r[1] = add_mod(r[1], src[v.y], q), r[2] = add_mod(r[2], src[v.z], q), r[3] = add_mod(r[3], src[v.w], q);
             }

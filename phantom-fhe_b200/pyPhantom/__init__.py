@@ -802,9 +802,21 @@ class single_chain_plaintext:
     def __init__(self, coeffs=None, scale=1.0):
         self.scale = float(scale)
         self.coeffs = None
+
         if coeffs is not None:
             t = torch.from_numpy(np.ascontiguousarray(coeffs, dtype=np.int64).copy())
             self.coeffs = t.pin_memory() if torch.cuda.is_available() else t
+
+    @property
+    def coeffs(self):
+        return self._coeffs
+
+    @coeffs.setter
+    def coeffs(self, t):
+        self._coeffs = t
+        # what the device reads in place: the address of a pinned (or device) vector, else 0
+        ok = t is not None and (t.is_cuda or t.is_pinned()) and t.is_contiguous() and t.dtype == torch.int64 and t.data_ptr() % 16 == 0
+        self._readable = t.data_ptr() if ok else 0
 
     def coeffs_bytes(self):
         return self.coeffs.numpy().tobytes()
@@ -952,68 +964,148 @@ def bsgs_required_steps(baby_steps):
 
 
 def compute_bsgs_babies(ctx, galois_key_, x, baby_steps):
-    """src/bsgs.cu:194-214: babies[b] = rotate(babies[b - msb(b)], msb(b)) - chained, not hoisted"""
+    """src/bsgs.cu:194-214: babies[b] = rotate(babies[b - msb(b)], msb(b)) - chained, not hoisted. The babies with one
+    leading bit are rotations of those below it by one step: a batch, every kernel one launch over it."""
     if baby_steps == 0:
         raise ValueError("compute_bsgs_babies: baby_steps must be > 0")
-    babies = [x]
-    for b in range(1, baby_steps):
-        bit = 1 << (b.bit_length() - 1)
-        babies.append(rotate(ctx, babies[b - bit], bit, galois_key_))
-    return babies
+    l, N = x._limbs, ctx.N
+    keys = []
+    bit = 1
+    while bit < baby_steps:
+        elt = get_elt_from_step(bit, N)
+        if elt not in ctx.galois_elts or x._size != 2:
+            keys = None
+            break
+        ksk = galois_key_.resolve(ctx.galois_elts.index(elt))
+        if ksk is None:
+            raise ValueError("Galois key not present (no owned key, no fallback)")
+        keys.append((bit, elt, _key_table(ctx, ksk, l)))
+        bit <<= 1
+    if keys is None:  # a step without a key of its own is a chain of rotations
+        babies = [x]
+        for b in range(1, baby_steps):
+            bit = 1 << (b.bit_length() - 1)
+            babies.append(rotate(ctx, babies[b - bit], bit, galois_key_))
+        return babies
+    buf = ctx.empty(baby_steps, 2, l)
+    buf[0].copy_(x.data)
+    st = _stream()
+    for bit, elt, tab in keys:
+        n = min(bit, baby_steps - bit)
+        ws = keyswitch_batch_workspace(ctx, l, n)
+        check(LIB.b2_apply_galois_batch(ctx._h, l, elt, n, buf.data_ptr(), 2 * l, tab.ctypes.data, len(tab), buf[bit].data_ptr(), 2 * l,
+                                        ws.data_ptr(), ws.numel() * 8, st))
+    return [x._like(buf[b]) for b in range(baby_steps)]
+
+
+def _pointer_table(first, stride_words, count, device):
+    """device array of pointers at a constant distance, made on the device (no copy from the host to wait for)"""
+    return torch.arange(count, dtype=torch.int64, device=device).mul_(8 * stride_words).add_(first)
+
+
+_GIANT_POOL_BYTES = 1 << 28  # expanded plaintexts of the giants that share a launch
 
 
 def bsgs_apply_giants_with_babies(ctx, galois_key_, babies, diags):
     """src/bsgs.cu:216-359: per giant expand M plaintexts and run the fused MAC; Horner
     acc = rotate(acc, M) + partial_g from the last giant down; one rescale; scale reset to x's."""
+    if len(babies) != diags.baby_steps:
+        raise ValueError("bsgs_apply_giants_with_babies: babies size != baby_steps")
+    return _bsgs_product(ctx, galois_key_, babies[0], babies, diags)
+
+
+def _bsgs_product(ctx, galois_key_, x, babies, diags):
+    """The product of the two drivers; `babies` None: they are computed here, while the first diagonals are on their way.
+
+    Three streams: one reads the diagonals out of pinned host memory and makes their residues, one transforms them and
+    multiplies (up to four giants per launch, every baby read once for them), and the caller's runs the chain of
+    rotations, each of which lands on top of the next partial sum. Bound by the reads (8 N bytes per diagonal) or by the
+    chain of G - 1 dependent key switches, whichever is longer."""
     M, G = diags.baby_steps, diags.giant_steps
     if M == 0 or G == 0 or M * G != diags.d_pad:
         raise ValueError("bsgs_apply_giants_with_babies: M*G must equal d_pad")
-    if len(babies) != M:
-        raise ValueError("bsgs_apply_giants_with_babies: babies size != baby_steps")
     if len(diags.diagonals) != diags.d_pad:
         raise ValueError("bsgs_apply_giants_with_babies: diagonals size mismatch")
-    x = babies[0]
-    l, N = x._limbs, ctx.N
-    # Two pools of M expanded plaintexts: while the multiply-accumulate and the rotation of one giant run on the
-    # caller's stream, the next giant's diagonals are copied in and expanded on a second stream.
+    l, N, dev = x._limbs, ctx.N, ctx.device
+    for scp in diags.diagonals:
+        if scp.coeffs.numel() != N:
+            raise ValueError("bsgs_apply_giants_with_babies: scp coeff length != N")
+    scale = x._scale * diags.diagonals[(G - 1) * M].scale
+    for g in range(G - 1):
+        if not _are_close(scale, x._scale * diags.diagonals[g * M].scale):
+            raise ValueError("scale mismatch")
+    elt, tab = get_elt_from_step(M, N) if G > 1 else 0, None
+    if elt in ctx.galois_elts:
+        ksk = galois_key_.resolve(ctx.galois_elts.index(elt))
+        if ksk is None:
+            raise ValueError("Galois key not present (no owned key, no fallback)")
+        tab = _key_table(ctx, ksk, l)
+    per = max(1, min(4, G, _GIANT_POOL_BYTES // (M * l * N * 8)))
+    groups = [list(range(max(0, hi - per), hi)) for hi in range(G, 0, -per)]
     main = torch.cuda.current_stream()
-    side = torch.cuda.Stream()
-    pools = [ctx.empty(M, l) for _ in range(2)]
-    stages = [torch.empty(M, N, dtype=torch.int64, device=ctx.device) for _ in range(2)]
-    pt_ptrs = [torch.tensor([p[b].data_ptr() for b in range(M)], dtype=torch.int64, device=ctx.device) for p in pools]
-    baby_ptrs = torch.tensor([c.data.data_ptr() for c in babies], dtype=torch.int64, device=ctx.device)
-    ready = [torch.cuda.Event() for _ in range(2)]
-    free = [torch.cuda.Event() for _ in range(2)]
-    side.wait_stream(main)
+    read, work = torch.cuda.Stream(), torch.cuda.Stream()
+    pools = [ctx.empty(per * M, l) for _ in range(2)]
+    read.wait_stream(main)
+    staged = []
+    expanded, consumed = [torch.cuda.Event() for _ in range(2)], [torch.cuda.Event() for _ in range(2)]
 
-    def prepare(g, slot, wait_free):
-        with torch.cuda.stream(side):
-            if wait_free:
-                side.wait_event(free[slot])
-            for b in range(M):
-                scp = diags.diagonals[g * M + b]
-                if scp.coeffs.numel() != N:
-                    raise ValueError("bsgs_apply_giants_with_babies: scp coeff length != N")
-                stages[slot][b].copy_(scp.coeffs, non_blocking=True)
-            check(LIB.b2_expand_single_chain_batch(ctx._h, l, M, stages[slot].data_ptr(), pools[slot].data_ptr(), side.cuda_stream))
-            ready[slot].record(side)
+    def fetch(i):
+        if i >= len(groups):
+            return
+        gs, slot = groups[i], i & 1
+        if i >= 2:
+            read.wait_event(consumed[slot])
+        scps = diags.diagonals[gs[0] * M: (gs[-1] + 1) * M]
+        ptrs = np.array([s._readable for s in scps], dtype=np.uint64)
+        if not ptrs.all():  # vectors the device cannot read in place are copied first
+            with torch.cuda.stream(read):
+                stage = torch.stack([s.coeffs.to(dev, non_blocking=True) for s in scps])
+            staged.append(stage)
+            ptrs = np.array([stage[k].data_ptr() for k in range(len(scps))], dtype=np.uint64)
+        check(LIB.b2_expand_gather(ctx._h, l, len(scps), ptrs.ctypes.data, pools[slot].data_ptr(), read.cuda_stream))
+        expanded[slot].record(read)
 
-    def partial(g, slot):
-        main.wait_event(ready[slot])
-        out = ctx.empty(2, l)
-        check(LIB.b2_bsgs_mac(ctx._h, l, M, pt_ptrs[slot].data_ptr(), baby_ptrs.data_ptr(), out.data_ptr(), _stream()))
-        free[slot].record(main)
-        return x._like(out, scale=x._scale * diags.diagonals[g * M].scale)
-
-    order = list(range(G - 1, -1, -1))
-    prepare(order[0], 0, False)
+    fetch(0)
+    fetch(1)
+    if babies is None:
+        babies = compute_bsgs_babies(ctx, galois_key_, x, M)
+    parts = ctx.empty(G, 2, l)
+    pt_tabs = [_pointer_table(p.data_ptr(), l * N, per * M, dev) for p in pools]
+    part_tab = _pointer_table(parts.data_ptr(), 2 * l * N, G, dev)
+    ptrs = [c.data.data_ptr() for c in babies]
+    step = ptrs[1] - ptrs[0] if M > 1 else 8
+    if step > 0 and all(p == ptrs[0] + i * step for i, p in enumerate(ptrs)):
+        baby_tab = _pointer_table(ptrs[0], step // 8, M, dev)
+    else:
+        baby_tab = torch.tensor(ptrs, dtype=torch.int64, device=dev)
+    work.wait_stream(main)
+    done = {}
+    for i, gs in enumerate(groups):
+        slot = i & 1
+        work.wait_event(expanded[slot])
+        check(LIB.b2_ntt_forward_batch(ctx._h, pools[slot].data_ptr(), l, len(gs) * M, work.cuda_stream))
+        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, len(gs), pt_tabs[slot].data_ptr(), baby_tab.data_ptr(),
+                                    part_tab.data_ptr() + 8 * gs[0], work.cuda_stream))
+        consumed[slot].record(work)
+        done[gs[-1]] = torch.cuda.Event()
+        done[gs[-1]].record(work)
+        fetch(i + 2)
+    ws, nbytes = ctx.workspace(_native.OP_KEYSWITCH, l)
+    st = main.cuda_stream
     acc = None
-    for i, g in enumerate(order):
-        if i + 1 < len(order):
-            prepare(order[i + 1], (i + 1) & 1, i >= 1)
-        part = partial(g, i & 1)
-        acc = part if acc is None else add(ctx, rotate(ctx, acc, M, galois_key_), part)
-    main.wait_stream(side)
+    for g in range(G - 1, -1, -1):
+        if g in done:
+            main.wait_event(done[g])
+        part = x._like(parts[g], scale=scale)
+        if acc is None:
+            acc = part
+        elif tab is not None:
+            check(LIB.b2_rotate_add(ctx._h, l, elt, acc.data.data_ptr(), tab.ctypes.data, len(tab), part.data.data_ptr(), ws.data_ptr(), nbytes, st))
+            acc = part
+        else:
+            acc = add(ctx, rotate(ctx, acc, M, galois_key_), part)
+    main.wait_stream(read)
+    main.wait_stream(work)
     acc = rescale_to_next(ctx, acc)
     acc.set_scale(x._scale)
     return acc
@@ -1021,7 +1113,9 @@ def bsgs_apply_giants_with_babies(ctx, galois_key_, babies, diags):
 
 def bsgs_matmul_preencoded(ctx, galois_key_, x, diags):
     """src/bsgs.cu:361-367"""
-    return bsgs_apply_giants_with_babies(ctx, galois_key_, compute_bsgs_babies(ctx, galois_key_, x, diags.baby_steps), diags)
+    if diags.baby_steps == 0:
+        raise ValueError("compute_bsgs_babies: baby_steps must be > 0")
+    return _bsgs_product(ctx, galois_key_, x, None, diags)
 
 
 def bsgs_matmul_preencoded_complex(ctx, galois_key_, x, diags):

@@ -53,6 +53,8 @@ SIGNATURES = {
     "b2_galois_permute": (_int, [_vp, _u32, _vp, _vp, _sz, _vp]),
     "b2_apply_galois": (_int, [_vp, _sz, _u32, _vp, _vp, _sz, _vp, _vp, _sz, _vp]),
     "b2_apply_galois_accumulate": (_int, [_vp, _sz, _u32, _vp, _vp, _sz, _vp, _vp, _int, _vp, _sz, _vp]),
+    "b2_apply_galois_batch": (_int, [_vp, _sz, _u32, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp]),
+    "b2_rotate_add": (_int, [_vp, _sz, _u32, _vp, _vp, _sz, _vp, _vp, _sz, _vp]),
     "b2_keyswitch_finish": (_int, [_vp, _sz, _vp, _vp, _vp, _sz, _vp]),
     "b2_hoist_rotations": (_int, [_vp, _sz, _vp, _vp, _sz, _vp, _sz, _vp, _vp, _sz, _vp]),
     "b2_hoisting_sum": (_int, [_vp, _sz, _vp, _vp, _sz, _vp, _sz, _vp, _vp, _sz, _vp]),
@@ -60,6 +62,8 @@ SIGNATURES = {
     "b2_bsgs_mac_multi": (_int, [_vp, _sz, _sz, _sz, _vp, _vp, _vp, _vp]),
     "b2_expand_single_chain": (_int, [_vp, _sz, _vp, _vp, _vp]),
     "b2_expand_single_chain_batch": (_int, [_vp, _sz, _sz, _vp, _vp, _vp]),
+    "b2_expand_gather": (_int, [_vp, _sz, _sz, _vp, _vp, _vp]),
+    "b2_ntt_forward_batch": (_int, [_vp, _vp, _sz, _sz, _vp]),
     "b2_expand_signed": (_int, [_vp, _sz, _sz, _vp, _vp, _int, _vp]),
     "b2_poly_op": (_int, [_vp, _int, _sz, _vp, _vp, _vp, _vp]),
     "b2_ct_op": (_int, [_vp, _int, _sz, _sz, _vp, _vp, _vp, _vp]),

@@ -133,3 +133,47 @@ def test_giant_steps_on_every_prime_class(M):
         check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, n, tabs[0].data_ptr(), tb.data_ptr(), tabs[1].data_ptr(), s))
         for t in outs:
             assert np.array_equal(host(t), want)
+
+
+@pytest.mark.parametrize("log_n,l,batch", [(12, 3, 3), (15, 4, 2), (16, 3, 2)])
+def test_batched_rotation_and_rotation_on_top_of_a_sum(log_n, l, batch):
+    """b2_apply_galois_batch with gaps between the sets, and b2_rotate_add, against the oracle's rotations"""
+    from pyPhantom import _native
+    from pyPhantom._native import LIB, check
+    N = 1 << log_n
+    elt = ph.get_elt_from_step(3, N)
+    ctx, o = make_ctx(N, [60, 40, 50, 40, 60, 60], 2, [elt])
+    key = o.synth_key(o.beta(l), 8, 10)
+    rk = ph.relin_key.from_numpy(ctx, key)
+    tab, s = rk.pointer_table(), torch.cuda.current_stream().cuda_stream
+    cts = [o.synth_ct(l, 8, 20 + i) for i in range(batch)]
+    src = torch.zeros(batch, 2 * l + 1, N, dtype=torch.int64, device="cuda")
+    for i, c in enumerate(cts):
+        src[i, : 2 * l] = dev(c).reshape(2 * l, N)
+    out = torch.zeros(batch, 2 * l + 2, N, dtype=torch.int64, device="cuda")
+    ws = ph.keyswitch_batch_workspace(ctx, l, batch)
+    check(LIB.b2_apply_galois_batch(ctx._h, l, elt, batch, src.data_ptr(), 2 * l + 1, tab.ctypes.data, len(tab), out.data_ptr(), 2 * l + 2,
+                                    ws.data_ptr(), ws.numel() * 8, s))
+    want = [o.apply_galois(l, elt, key, c) for c in cts]
+    for i in range(batch):
+        assert np.array_equal(host(out[i, : 2 * l]).reshape(2, l, N), want[i])
+    assert not out[:, 2 * l:].any()
+    acc = dev(cts[1])
+    w1, nb = ctx.workspace(_native.OP_KEYSWITCH, l)
+    check(LIB.b2_rotate_add(ctx._h, l, elt, dev(cts[0]).data_ptr(), tab.ctypes.data, len(tab), acc.data_ptr(), w1.data_ptr(), nb, s))
+    assert np.array_equal(host(acc), np.stack([o.add(cts[1][k], want[0][k]) for k in range(2)]))
+
+
+def test_product_with_diagonals_outside_pinned_memory():
+    """the matrix product reads pinned diagonals in place; pageable ones are copied first and give the same limbs"""
+    N, l, M, G = 4096, 3, 4, 5
+    ctx, o = make_ctx(N, [60, 40, 40, 60], 1, [ph.get_elt_from_step(s, N) for s in (1, 2, 4)])
+    glk = ph.galois_key.from_keys([ph.relin_key.from_numpy(ctx, o.synth_key(o.beta(l), 3, 10 + 20 * i)) for i in range(3)])
+    coeffs = [o.synth_signed(5, 70 + d) for d in range(M * G)]
+    x = ph.ciphertext.from_numpy(ctx, o.synth_ct(l, 3, 1), 1, 2.0 ** 40)
+    pinned = ph.bsgs_diagonals([ph.single_chain_plaintext(c, 2.0 ** 40) for c in coeffs], M * G, M, G)
+    plain = ph.bsgs_diagonals([ph.single_chain_plaintext(c, 2.0 ** 40) for c in coeffs], M * G, M, G)
+    for p in plain.diagonals:
+        p.coeffs = p.coeffs.clone()
+    assert not plain.diagonals[0].coeffs.is_pinned()
+    assert torch.equal(ph.bsgs_matmul_preencoded(ctx, glk, x, pinned).data, ph.bsgs_matmul_preencoded(ctx, glk, x, plain).data)
