@@ -137,6 +137,21 @@ int b2_decode_compose(b2_ctx *ctx, size_t size_Ql, const uint64_t *d_res, const 
 int b2_sample(b2_ctx *ctx, int kind, const uint8_t *key32, const uint8_t *nonce12, size_t first_prime, size_t n_limbs,
               void *d_out, void *stream);
 
+/* Encoding, symmetric encryption, decryption and decoding as one call each (src/ckks.cu:68-190, src/secretkey.cu:236-299,
+ * 883-919); the tables are those of b2_special_fft and b2_decode_compose.
+ *   b2_encode_coeffs:     d_vals (N/2 complex values, overwritten) -> d_coeffs int64 [N], each below 2^62 in magnitude
+ *   b2_encrypt_symmetric: d_out [2][l][N] = (m - (a s + e), a); a and e from the key and nonce (32 + 12 bytes) given for
+ *                         each; d_sk [l][N]; d_pt [l][N] or null; d_ws N words
+ *   b2_decrypt:           d_out [l][N] = c0 + c1 s
+ *   b2_decode_slots:      d_pt [l][N] -> d_out N/2 complex values; d_ws (l + 1) N words */
+int b2_encode_coeffs(b2_ctx *ctx, void *d_vals, const uint32_t *d_rot, const void *d_ksi, double scale,
+                     int64_t *d_coeffs, void *stream);
+int b2_encrypt_symmetric(b2_ctx *ctx, size_t l, const uint8_t *mask44, const uint8_t *error44, const uint64_t *d_sk,
+                         const uint64_t *d_pt, uint64_t *d_out, void *d_ws, void *stream);
+int b2_decrypt(b2_ctx *ctx, size_t l, const uint64_t *d_ct, const uint64_t *d_sk, uint64_t *d_out, void *stream);
+int b2_decode_slots(b2_ctx *ctx, size_t l, const uint64_t *d_pt, const uint64_t *d_tab, double inv_scale,
+                    const uint32_t *d_rot, const void *d_ksi, void *d_ws, void *d_out, void *stream);
+
 /* replaces bgv_ckks_multiply's tensor product (src/evaluate.cu:345-397, src/polymath.cu:463-540):
  * d_a, d_b [2][size_Ql][N] -> d_out [3][size_Ql][N] */
 int b2_tensor_mul(b2_ctx *ctx, size_t size_Ql, const uint64_t *d_a, const uint64_t *d_b,

@@ -22,6 +22,8 @@
 #include "encoder.cuh"
 #include "bconv_tc.cuh"
 #include "elementwise.cuh"
+#include "launch.cuh"
+#include "ntt_whole.cuh"
 
 using namespace b2;
 typedef unsigned __int128 u128_t;
@@ -196,6 +198,9 @@ struct LevelPlan {
     BconvGroup *grp_up = nullptr;  // beta
     uint2 *outs_up = nullptr;      // (slot, prime) list, beta groups concatenated
     uint64_t *mat_up = nullptr;
+    W2 *matw_up = nullptr;         // mat_up with Shoup words (conversion fused into whole transforms)
+    BcJob *bc_up = nullptr;        // per entry of jobs_up_ntt: where its conversion reads and its row of matw_up
+    BcJob *bc_dnf = nullptr;       // per entry of jobs_dnf_ntt, rows of d_matw_dn_pinv
     double *matd_up = nullptr;     // mat_up as 21-bit pieces of (entry * 2^64 mod p), [..][3]
     BconvGroup *grp_dn = nullptr;  // 2 (one per polynomial)
     uint2 *outs_dn = nullptr;      // l entries shared by both groups
@@ -218,6 +223,7 @@ struct b2_ctx {
     W2 *d_Pinv = nullptr;       // [size_QP] indexed by prime (valid for Q primes): P^-1 mod q_j
     W2 *d_macfin = nullptr;     // [size_QP] closing constant of the fused inner product's Montgomery sums: P^-1 * 2^64 mod q_j, 2^64 mod p_i
     uint64_t *d_mat_dn = nullptr;  // [size_Q][size_P]: (P/p_i) mod q_j
+    W2 *d_matw_dn_pinv = nullptr;  // d_mat_dn_pinv with Shoup words
     uint64_t *d_mat_dn_pinv = nullptr;  // the same times P^-1 mod q_j (fused key switch)
     double *d_matd_dn = nullptr, *d_matd_dn_pinv = nullptr;  // FP64 piece forms
     struct RedcMeta {
@@ -296,23 +302,6 @@ struct LaunchScope {
     }
 };
 
-// Every kernel of the library is launched with the programmatic-serialisation attribute and begins with pdl_enter()
-// (modarith.cuh): the next kernel's launch and block scheduling overlap the end of the previous one, and its CTAs wait until
-// that kernel has completed and its writes are visible. At small sizes a key switch is a chain of a dozen kernels of 2 to 5
-// us, where launch latency is a third of the time (one transform pair of 8 limbs at N = 2^14: 30.7 -> 22.1 us; a rotation at
-// N = 2^13: 74 -> 54). No kernel signals before it ends (griddepcontrol.launch_dependents): CTAs that are scheduled early
-// take SM slots from the running grid and bunch up on the SMs that empty first (signalled on entry, eight hoisted rotations
-// at N = 2^15 take 708 us; before the exchange of the transforms 597; never 599; without the attribute 670).
-template <class... P, class... A>
-static void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = s, cfg.attrs = &at, cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);  // LAUNCH_CHECK reads the error
-}
-
 template <typename T>
 static T *blob_take(char *&cur, size_t count) {
     uintptr_t p = (reinterpret_cast<uintptr_t>(cur) + 15) & ~uintptr_t(15);
@@ -362,6 +351,14 @@ static int tc_upload(const TcBuild &b, void **blob, std::initializer_list<std::p
     return B2_OK;
 }
 
+// bit i: prime s + i has 50 bits or more (its residues go through an FP64 conversion in two parts)
+static uint32_t wide_mask(const b2_ctx *c, size_t s, size_t e) {
+    uint32_t m = 0;
+    for (size_t i = s; i < e; i++)
+        if (c->q[i] >= b2::FP_LIMIT) m |= 1u << (i - s);
+    return m;
+}
+
 static int build_level(b2_ctx *c, size_t l) {
     const size_t N = c->N, alpha = c->size_P, sQ = c->size_Q;
     const size_t beta = (l + alpha - 1) / alpha, lP = l + alpha;
@@ -372,7 +369,7 @@ static int build_level(b2_ctx *c, size_t l) {
     const size_t mat_up_words = beta * lP * alpha;
     // host staging mirrors the device blob
     size_t bytes = 64 + sizeof(Job) * (l + 2 * n_up_ntt + 4 * alpha + 4 * l + 3 + 3 * l) + sizeof(W2) * (2 * l + c->size_QP) +
-                   sizeof(BconvGroup) * (beta + 4 + 3) + sizeof(uint2) * (n_up_ntt + l + l) + 8 * mat_up_words * 4 + 16 * 24;
+                   sizeof(BconvGroup) * (beta + 4 + 3) + sizeof(uint2) * (n_up_ntt + l + l) + 8 * mat_up_words * 6 + sizeof(BcJob) * (n_up_ntt + 2 * l) + 16 * 32;
     std::vector<char> host(bytes, 0);
     char *cur = host.data();
     auto *jobs_up_intt = blob_take<Job>(cur, l);
@@ -391,6 +388,9 @@ static int build_level(b2_ctx *c, size_t l) {
     auto *outs_up = blob_take<uint2>(cur, n_up_ntt);
     auto *mat_up = blob_take<uint64_t>(cur, mat_up_words);
     auto *matd_up = blob_take<double>(cur, mat_up_words * 3);
+    auto *matw_up = blob_take<W2>(cur, mat_up_words);
+    auto *bc_up = blob_take<BcJob>(cur, n_up_ntt);
+    auto *bc_dnf = blob_take<BcJob>(cur, 2 * l);
     auto *grp_dn = blob_take<BconvGroup>(cur, 2);
     auto *outs_dn = blob_take<uint2>(cur, l);
     const size_t used = cur - host.data();
@@ -418,8 +418,10 @@ static int build_level(b2_ctx *c, size_t l) {
             const uint32_t pp = phys_prime(c, l, t);
             jobs_up_ntt[up_i] = make_uint4((uint32_t)(d * lP + t), pp, 0, 0);
             outs_up[up_i] = make_uint2((uint32_t)t, pp);
+            bc_up[up_i] = BcJob{(uint32_t)s, (uint32_t)ni, (uint32_t)mat_off, wide_mask(c, s, e)};
             for (size_t i = s; i < e; i++) {
                 mat_up[mat_off] = punctured(c->q, s, e, i, c->q[pp]);
+                matw_up[mat_off] = h_w2(mat_up[mat_off], c->q[pp]);
                 h_pieces(mat_up[mat_off], c->q[pp], matd_up + 3 * mat_off);
                 mat_off++;
             }
@@ -448,7 +450,8 @@ static int build_level(b2_ctx *c, size_t l) {
         for (size_t i = 0; i < alpha; i++)
             jobs_dnf_intt[k * alpha + i] = make_uint4((uint32_t)(k * alpha + i), (uint32_t)(sQ + i), (uint32_t)i, (uint32_t)(k * alpha + i));
         for (size_t j = 0; j < l; j++)
-            jobs_dnf_ntt[k * l + j] = make_uint4((uint32_t)(k * l + j), (uint32_t)j, 0, (uint32_t)(k * l + j));
+            jobs_dnf_ntt[k * l + j] = make_uint4((uint32_t)(k * l + j), (uint32_t)j, 0, (uint32_t)(k * l + j)),
+            bc_dnf[k * l + j] = BcJob{(uint32_t)(k * alpha), (uint32_t)alpha, (uint32_t)(j * alpha), wide_mask(c, sQ, sQ + alpha)};
         grp_dnf[k] = BconvGroup{(uint32_t)(k * alpha), (uint32_t)alpha, 0, 0, (uint32_t)l, (uint32_t)(k * l), 0, p_pieces};
     }
     for (size_t j = 0; j < l; j++) outs_dn[j] = make_uint2((uint32_t)j, (uint32_t)j);
@@ -488,6 +491,9 @@ static int build_level(b2_ctx *c, size_t l) {
     pl.grp_up = (BconvGroup *)dev(grp_up);
     pl.outs_up = (uint2 *)dev(outs_up);
     pl.mat_up = (uint64_t *)dev(mat_up);
+    pl.matw_up = (W2 *)dev(matw_up);
+    pl.bc_up = (BcJob *)dev(bc_up);
+    pl.bc_dnf = (BcJob *)dev(bc_dnf);
     pl.matd_up = (double *)dev(matd_up);
     pl.grp_dn = (BconvGroup *)dev(grp_dn);
     pl.outs_dn = (uint2 *)dev(outs_dn);
@@ -538,6 +544,7 @@ extern "C" void b2_ctx_destroy(b2_ctx *c) {
     cudaFree(c->d_macfin);
     cudaFree(c->d_mat_dn);
     cudaFree(c->d_mat_dn_pinv);
+    cudaFree(c->d_matw_dn_pinv);
     cudaFree(c->d_matd_dn);
     cudaFree(c->d_matd_dn_pinv);
     cudaFree(c->d_redc);
@@ -709,6 +716,12 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
     }
     if (e == cudaSuccess) e = up((void **)&c->d_mat_dn, mat_dn.data(), 8 * sQ * sP);
     if (e == cudaSuccess) e = up((void **)&c->d_mat_dn_pinv, mat_dn_pinv.data(), 8 * sQ * sP);
+    {
+        std::vector<W2> mw(sQ * sP);
+        for (size_t j = 0; j < sQ; j++)
+            for (size_t i = 0; i < sP; i++) mw[j * sP + i] = h_w2(mat_dn_pinv[j * sP + i], c->q[j]);
+        if (e == cudaSuccess) e = up((void **)&c->d_matw_dn_pinv, mw.data(), sizeof(W2) * mw.size());
+    }
     if (e == cudaSuccess) e = up((void **)&c->d_matd_dn, matd_dn.data(), 8 * matd_dn.size());
     if (e == cudaSuccess) e = up((void **)&c->d_matd_dn_pinv, matd_dn_pinv.data(), 8 * matd_dn_pinv.size());
     if (e == cudaSuccess) e = up((void **)&c->d_redc, redc.data(), sizeof(b2_ctx::RedcMeta) * size_QP);
@@ -875,6 +888,20 @@ struct BatchDims {
     const uint32_t *perm = nullptr;  // inverse transforms: the input is read through this permutation
 };
 
+// Whether `limbs` transforms run as whole ones (ntt_whole.cuh says why the lines lie here)
+static bool use_whole(const b2_ctx *c, size_t limbs) { return c->logN == 12 && c->size_P <= 8 && limbs <= 1024; }
+static bool use_whole_plain(const b2_ctx *c, size_t limbs, const Job *jobs, uint32_t first_prime, uint32_t njobs, uint32_t period) {
+    if (c->logN == 12) return use_whole(c, limbs);
+    if ((c->logN != 13 && c->logN != 14) || jobs || limbs > 32) return false;
+    for (uint32_t p = first_prime; p < first_prime + (period ? std::min(period, njobs) : njobs); p++)
+        if (c->q[p] >= b2::FP_LIMIT) return false;
+    return true;
+}
+template <class Epi, int SRC> struct WholeHas : std::false_type {};
+template <> struct WholeHas<EpiStore, 0> : std::true_type {};
+template <> struct WholeHas<EpiSubMul<false>, 1> : std::true_type {};
+template <> struct WholeHas<EpiSubMul<false>, 2> : std::true_type {};
+
 template <class Epi, int SRC = 0>
 static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Job *jobs, uint32_t njobs, uint32_t first_prime,
                    const Epi &epi, cudaStream_t s, uint32_t period = 0, uint32_t src_div = 0, uint64_t src_q = 0, const BatchDims &bd = BatchDims{}) {
@@ -882,6 +909,14 @@ static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if (!aligned32(src) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
     NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, period, src_div, src_q, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
     if (SRC != 0 && src_div == 0) return fail(B2_EINVAL, "the on-the-fly source needs its divisor");
+    if constexpr (WholeHas<Epi, SRC>::value) {
+        if (SRC == 0 ? use_whole_plain(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, period) : use_whole(c, (size_t)njobs * bd.batch)) {
+            LaunchScope ls(c, s, "ntt_fwd_whole");
+            launch_fwd_whole<Epi, SRC>(a, epi, WholeArgs{}, njobs, bd.batch, s);
+            LAUNCH_CHECK("ntt_fwd_whole");
+            return B2_OK;
+        }
+    }
     switch (c->logN) {
         case 17: launch_fwd<8, 9, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
         case 16: launch_fwd<8, 8, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
@@ -900,6 +935,12 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
     NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, bd.perm};
+    if (use_whole_plain(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, 0)) {
+        LaunchScope ls(c, s, "ntt_inv_whole");
+        launch_inv_whole(a, njobs, bd.batch, s);
+        LAUNCH_CHECK("ntt_inv_whole");
+        return B2_OK;
+    }
     switch (c->logN) {
         case 17: launch_inv<8, 9>(c, a, njobs, s, bd.batch); break;
         case 16: launch_inv<8, 8>(c, a, njobs, s, bd.batch); break;
@@ -910,6 +951,18 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
         default: return fail(B2_ESIZE, "unsupported polynomial degree");
     }
     LAUNCH_CHECK("ntt_inv_pass");
+    return B2_OK;
+}
+
+// base conversion and forward transform in one launch: job j's limb is made from the input limbs bc[j] names
+template <class Epi>
+static int run_bconv_fwd(const b2_ctx *c, const uint64_t *in, uint64_t *dst, const Job *jobs, const BcJob *bc, const W2 *mat, uint32_t njobs, const Epi &epi,
+                         cudaStream_t s, const BatchDims &bd = BatchDims{}) {
+    if (!aligned32(in) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
+    NttArgs a{in, dst, jobs, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
+    LaunchScope ls(c, s, "bconv_ntt_whole");
+    launch_fwd_whole<Epi, 3>(a, epi, WholeArgs{bc, mat}, njobs, bd.batch, s);
+    LAUNCH_CHECK("bconv_ntt_whole");
     return B2_OK;
 }
 
@@ -1240,6 +1293,7 @@ static int modup_impl(b2_ctx *c, size_t l, const uint64_t *c2, uint64_t *out, ui
     bd.perm = perm;
     int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, bd);
     if (rc) return rc;
+    if (!copy_own && use_whole(c, pl.n_up_ntt)) return run_bconv_fwd(c, t, out, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s);
     rc = run_bconv(c, copy_own, t, out, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)(l + c->size_P), true, s, &pl.tc_up);
     if (rc) return rc;
     return run_fwd(c, out, out, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s);
@@ -1344,6 +1398,7 @@ static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint6
     const size_t a = c->size_P;
     int rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
     if (rc) return rc;
+    if (use_whole(c, 2 * l)) return run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{ct}, s);
     rc = run_bconv(c, false, cxP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
     if (rc) return rc;
     return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
@@ -1371,7 +1426,8 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     const bool wide = (c->mac_wide < 0 ? batched : c->mac_wide == 1) && beta <= B2_MAC_MAX_BETA;
     // single calls at 2^15 run the stored row pass and the stand-alone inner product: the split by prime class costs two
     // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853)
-    const bool mac = c->use_mac && (batched || c->logN == 16 || c->mac_wide == 1) && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
+    const bool whole = batched && use_whole(c, (size_t)pl.n_up_ntt * kb.batch);
+    const bool mac = !whole && c->use_mac && (batched || c->logN == 16 || c->mac_wide == 1) && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
     if (!mac && !batched) return B2_OK;
     if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
         return B2_OK;  // the caller falls back to one key switch at a time
@@ -1380,7 +1436,9 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         const uint32_t B = kb.batch, per = (uint32_t)(beta * lP), a2 = (uint32_t)(2 * c->size_P);
         int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, kb.c2_bs, 0, (uint32_t)l, kb.rot.perm});
         if (rc) return rc;
-        if (batched) {
+        if (whole) {
+            rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
+        } else if (batched) {
             const TcBatch tb{B, 0, (uint32_t)l, 0, per, c->tc_serial_ld ? 1u : 0u};
             rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, &tb);
         } else {
@@ -1390,7 +1448,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (!mac) {
             // rings whose row pass is not the 256-point one (and keys of more than B2_MAC_MAX_BETA digits): both passes
             // stored for every limb, then the stand-alone inner product, each one launch over the batch
-            rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            if (!whole) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
             rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib, kb.rot);
@@ -1511,6 +1569,9 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     // ModDown of the P limbs of both polynomials of every set; delta takes the front of each set's `up` block
     rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{B, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
     if (rc) return rc;
+    if (use_whole(c, 2 * l * batch))
+        return run_bconv_fwd(c, cxP, up, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{d_ct, (uint32_t)ct_stride}, s,
+                             BatchDims{B, 0, (uint32_t)(2 * a), 0, per});
     const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per, 0};
     rc = run_bconv_tc(c, false, cxP, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, &tb);
     if (rc) return rc;
@@ -1912,6 +1973,12 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
         if (rc) return rc;
         rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
         if (rc) return rc;
+        if (use_whole(c, 2 * l * n)) {
+            rc = run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), epi, s,
+                               BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l)});
+            if (rc) return rc;
+            continue;
+        }
         if (c->bconv_tc && !c->tc_simple) {
             const TcBatch tb{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l), 0};
             rc = run_bconv_tc(c, false, cxP, delta, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, &tb);
@@ -2005,6 +2072,19 @@ extern "C" int b2_expand_signed(b2_ctx *c, size_t first_prime, size_t n_limbs, c
     return run_fwd(c, d_out, d_out, nullptr, (uint32_t)n_limbs, (uint32_t)first_prime, EpiStore{}, s);
 }
 
+// passes of the encoder's transform: n = 2^logn values as 2^(logn / 2) columns' worth of rows (8 stages a pass at most)
+static void run_cfft_inverse(const b2_ctx *c, double2 *v, double2 *out, int64_t *coeffs, const uint32_t *rot, const double2 *ksi, double scale, cudaStream_t s) {
+    const uint32_t logn = (uint32_t)c->logN - 1, la = logn / 2, lb = logn - la, grid = 1u << (logn - CFFT_LOG_TILE);
+    launch_k(cfft_pass_kernel<true, true, false>, grid, 512, 0, s, v, v, nullptr, logn, la, rot, ksi, 1.0);
+    if (coeffs) launch_k(cfft_pass_kernel<true, false, true>, grid, 512, 0, s, v, nullptr, coeffs, logn, lb, rot, ksi, scale);
+    else launch_k(cfft_pass_kernel<true, false, false>, grid, 512, 0, s, v, out, nullptr, logn, lb, rot, ksi, scale);
+}
+static void run_cfft_forward(const b2_ctx *c, const double2 *v, double2 *out, const uint32_t *rot, const double2 *ksi, double scale, cudaStream_t s) {
+    const uint32_t logn = (uint32_t)c->logN - 1, la = logn / 2, lb = logn - la, grid = 1u << (logn - CFFT_LOG_TILE);
+    launch_k(cfft_pass_kernel<false, false, false>, grid, 512, 0, s, v, out, nullptr, logn, lb, rot, ksi, scale);
+    launch_k(cfft_pass_kernel<false, true, false>, grid, 512, 0, s, out, out, nullptr, logn, la, rot, ksi, 1.0);
+}
+
 // The encoder's transform (encoder.cuh): n = N/2 complex values, rot = 5^j mod 2N (uint32 [n]), ksi = exp(2 pi i k / 2N)
 // (double2 [2N + 1]). inverse = 1 (encode): d_vals (natural order, overwritten) -> d_out = the embedding's preimage times
 // `scale`; inverse = 0 (decode): d_vals -> d_out = slot values times `scale`. d_vals and d_out must not overlap.
@@ -2012,18 +2092,21 @@ extern "C" int b2_special_fft(b2_ctx *c, void *d_vals, void *d_out, const uint32
     CHECK_CTX(c);
     if (!d_vals || !d_out || !d_rot || !d_ksi || d_vals == d_out) return fail(B2_EINVAL, "special_fft: bad argument");
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t n = (uint32_t)(c->N / 2), M = (uint32_t)(2 * c->N), logn = (uint32_t)c->logN - 1;
     double2 *v = (double2 *)d_vals, *o = (double2 *)d_out;
     LaunchScope ls(c, s, "special_fft");
-    if (inverse) {
-        for (uint32_t len = n; len >= 2; len >>= 1)
-            launch_k(b2::cfft_stage_kernel, (n / 2 + 255) / 256, 256, 0, s, v, n, len, d_rot, (const double2 *)d_ksi, M, 1);
-        launch_k(b2::cfft_bitrev_kernel, (n + 255) / 256, 256, 0, s, o, v, n, logn, scale);
-    } else {
-        launch_k(b2::cfft_bitrev_kernel, (n + 255) / 256, 256, 0, s, o, v, n, logn, scale);
-        for (uint32_t len = 2; len <= n; len <<= 1)
-            launch_k(b2::cfft_stage_kernel, (n / 2 + 255) / 256, 256, 0, s, o, n, len, d_rot, (const double2 *)d_ksi, M, 0);
-    }
+    if (inverse) run_cfft_inverse(c, v, o, nullptr, d_rot, (const double2 *)d_ksi, scale, s);
+    else run_cfft_forward(c, v, o, d_rot, (const double2 *)d_ksi, scale, s);
+    LAUNCH_CHECK("special_fft kernels");
+    return B2_OK;
+}
+
+// Encoding down to the coefficients in one call: b2_special_fft (inverse) and b2_encode_round without the complex values
+// between them. d_vals: N/2 complex values, overwritten; every coefficient must stay below 2^62.
+extern "C" int b2_encode_coeffs(b2_ctx *c, void *d_vals, const uint32_t *d_rot, const void *d_ksi, double scale, int64_t *d_coeffs, void *stream) {
+    CHECK_CTX(c);
+    if (!d_vals || !d_rot || !d_ksi || !d_coeffs) return fail(B2_EINVAL, "encode_coeffs: null pointer");
+    LaunchScope ls(c, (cudaStream_t)stream, "special_fft");
+    run_cfft_inverse(c, (double2 *)d_vals, nullptr, d_coeffs, d_rot, (const double2 *)d_ksi, scale, (cudaStream_t)stream);
     LAUNCH_CHECK("special_fft kernels");
     return B2_OK;
 }
@@ -2077,6 +2160,57 @@ extern "C" int b2_sample(b2_ctx *c, int kind, const uint8_t *key32, const uint8_
     else
         launch_k(b2::sample_small_kernel, (unsigned)((blocks + 127) / 128), 128, 0, s, (int64_t *)d_out, k, kind, (uint32_t)blocks);
     LAUNCH_CHECK("sample kernel");
+    return B2_OK;
+}
+
+// (c0, c1) = (m - (a s + e), a) at l limbs in one call (src/secretkey.cu:236-299): a drawn from the first key and nonce (44
+// bytes), e from the second. d_sk: [l][N], NTT form; d_pt: [l][N] or null (an encryption of zero); d_ws: N words.
+extern "C" int b2_encrypt_symmetric(b2_ctx *c, size_t l, const uint8_t *mask44, const uint8_t *error44, const uint64_t *d_sk, const uint64_t *d_pt,
+                                    uint64_t *d_out, void *d_ws, void *stream) {
+    CHECK_CTX(c);
+    if (!mask44 || !error44 || !d_sk || !d_out || !d_ws) return fail(B2_EINVAL, "encrypt_symmetric: null pointer");
+    if (l < 1 || l > c->size_QP) return fail(B2_EINVAL, "encrypt_symmetric: limb range outside the modulus chain");
+    const size_t S = l * c->N;
+    int rc = b2_sample(c, 0, mask44, mask44 + 32, 0, l, d_out + S, stream);
+    if (rc) return rc;
+    rc = b2_sample(c, 1, error44, error44 + 32, 0, 1, d_ws, stream);
+    if (rc) return rc;
+    rc = b2_expand_signed(c, 0, l, (const int64_t *)d_ws, d_out, 1, stream);
+    if (rc) return rc;
+    LaunchScope ls(c, (cudaStream_t)stream, "mask");
+    LAUNCH_V(mask_kernel, aligned32(d_sk) && aligned32(d_pt) && aligned32(d_out), (unsigned)l, 1, (cudaStream_t)stream, d_pt, d_out + S, d_sk, d_out, c->d_mod,
+             (uint32_t)c->N, 1);
+    LAUNCH_CHECK("mask_kernel");
+    return B2_OK;
+}
+
+// m = c0 + c1 s of a two-polynomial ciphertext [2][l][N] (src/secretkey.cu:883-919)
+extern "C" int b2_decrypt(b2_ctx *c, size_t l, const uint64_t *d_ct, const uint64_t *d_sk, uint64_t *d_out, void *stream) {
+    CHECK_CTX(c);
+    if (!d_ct || !d_sk || !d_out || l < 1 || l > c->size_QP) return fail(B2_EINVAL, "decrypt: bad argument");
+    LaunchScope ls(c, (cudaStream_t)stream, "mask");
+    LAUNCH_V(mask_kernel, aligned32(d_ct) && aligned32(d_sk) && aligned32(d_out), (unsigned)l, 1, (cudaStream_t)stream, d_ct, d_ct + l * c->N, d_sk, d_out, c->d_mod,
+             (uint32_t)c->N, 0);
+    LAUNCH_CHECK("mask_kernel");
+    return B2_OK;
+}
+
+// Decoding in one call: inverse transform, CRT composition, forward transform over the rotation group. d_pt: [l][N], NTT form,
+// left as it is; d_tab as for b2_decode_compose; d_ws: (l + 1) N words; d_out: N/2 complex values.
+extern "C" int b2_decode_slots(b2_ctx *c, size_t l, const uint64_t *d_pt, const uint64_t *d_tab, double inv_scale, const uint32_t *d_rot, const void *d_ksi,
+                               void *d_ws, void *d_out, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!d_pt || !d_tab || !d_rot || !d_ksi || !d_ws || !d_out) return fail(B2_EINVAL, "decode_slots: null pointer");
+    uint64_t *t = (uint64_t *)d_ws;
+    double2 *m = (double2 *)(t + l * c->N);
+    int rc = run_inv(c, d_pt, t, nullptr, (uint32_t)l, 0, c->d_fin_plain, (cudaStream_t)stream);
+    if (rc) return rc;
+    rc = b2_decode_compose(c, l, t, d_tab, inv_scale, m, stream);
+    if (rc) return rc;
+    LaunchScope ls(c, (cudaStream_t)stream, "special_fft");
+    run_cfft_forward(c, m, (double2 *)d_out, d_rot, (const double2 *)d_ksi, 1.0, (cudaStream_t)stream);
+    LAUNCH_CHECK("special_fft kernels");
     return B2_OK;
 }
 

@@ -385,6 +385,32 @@ __global__ void __launch_bounds__(256) poly_scalar_kernel(int op, const uint64_t
     stv<V>(out + o, x);
 }
 
+// symmetric encryption (src/secretkey.cu:236-299): out0 holds the error e, out1 the mask a; out0 <- m - (a s + e)
+// (m null: an encryption of zero). encrypt = 0, decryption (src/secretkey.cu:883-919): out0 <- m + a s
+template <int V>
+__global__ void __launch_bounds__(256) mask_kernel(const uint64_t *m, const uint64_t *a, const uint64_t *s, uint64_t *out0, const Mod *mod, uint32_t N, int encrypt) {
+    pdl_enter();
+    const size_t o = (size_t)blockIdx.y * N + (blockIdx.x * 256 + threadIdx.x) * V;
+    const Mod md = mod[blockIdx.y];
+    uint64_t x[V], y[V], z[V];
+    ldv<V>(x, a + o), ldv<V>(y, s + o);
+    if (encrypt) {
+        ldv<V>(z, out0 + o);
+    }
+    mul_limb<V>(x, y, md);
+    if (m) ldv<V>(y, m + o);
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+        if (encrypt) {
+            x[j] = add_mod(x[j], z[j], md.q);
+            x[j] = m ? sub_mod(y[j], x[j], md.q) : (x[j] ? md.q - x[j] : 0);
+        } else {
+            x[j] = add_mod(x[j], y[j], md.q);
+        }
+    }
+    stv<V>(out0 + o, x);
+}
+
 // NTT-domain automorphism (src/galois.cu:11-18): dst[l][i] = src[l][perm[i]]. An aligned run of 2^k values comes from an
 // aligned run of 2^k values (the low bits of a bit-reversed index are the high bits of the exponent), so the four reads of a
 // thread fall into one sector.

@@ -231,7 +231,7 @@ struct ArithIntLazy {
         uint64_t q, nq;   // nq = -q mod 2^64
         uint32_t m, s;    // floor(2^(64 + s) / q), normalised to 32 bits
     };
-    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_PASS = 16, GS_PASS = 6;
+    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_PASS = 16, GS_PASS = 6, B_BCONV = RED;
     __device__ __forceinline__ static K make(const Mod &md, int) {
         const uint32_t s = __clz((uint32_t)md.r1);  // r1 = floor(2^64 / q), in [2^4, 2^14]
         return K{md.q, 0 - md.q, (uint32_t)((md.r1 << s) | (md.r0 >> (64 - s))), s};
@@ -285,6 +285,9 @@ struct ArithIntLazy {
     __device__ __forceinline__ static T group_end(T v, const K &k, int B) { return B > GS_PASS ? reduce(v, k) : v; }
     __device__ __forceinline__ static T pass_end(T v, const K &k, int B) { return group_end(v, k, B); }
     __device__ __forceinline__ static uint64_t canon_fwd(T v, const K &k) { return csub(reduce(v, k), k.q); }
+    // a base conversion of up to eight terms, each below 2 q (B_BCONV bounds the result of bc_end)
+    __device__ __forceinline__ static T bc_add(T x, uint64_t t, const K &) { return x + t; }
+    __device__ __forceinline__ static T bc_end(T x, const K &k) { return reduce(x, k); }
     __device__ __forceinline__ static uint64_t canon_inv(T v, const K &) { return v; }  // gs_last is canonical
 };
 
@@ -296,7 +299,7 @@ struct ArithInt {
     struct K {
         uint64_t q, q2;
     };
-    static constexpr int B_CANON = 0, B_PASS = 0, GS_PASS = 0;
+    static constexpr int B_CANON = 0, B_PASS = 0, GS_PASS = 0, B_BCONV = 0;
     __device__ __forceinline__ static K make(const Mod &md, int) { return K{md.q, 2 * md.q}; }
     __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &) { return ldg_w2(tw + idx); }
     __device__ __forceinline__ static Tw ldfin(const W2 *p, const K &) { return ldg_w2(p); }
@@ -318,6 +321,8 @@ struct ArithInt {
     __device__ __forceinline__ static T group_end(T v, const K &, int) { return v; }
     __device__ __forceinline__ static T pass_end(T v, const K &, int) { return v; }
     __device__ __forceinline__ static uint64_t canon_fwd(T v, const K &k) { return csub(csub(v, k.q2), k.q); }
+    __device__ __forceinline__ static T bc_add(T x, uint64_t t, const K &k) { return csub(x + t, k.q2); }
+    __device__ __forceinline__ static T bc_end(T x, const K &) { return x; }
     __device__ __forceinline__ static uint64_t canon_inv(T v, const K &) { return v; }
 };
 
@@ -336,7 +341,8 @@ struct ArithFp {
         double q, qinv;
     };
     static constexpr int FACTOR = 32, LIM = 128, RED = 9;
-    static constexpr int B_CANON = BIG ? 16 : 0, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0;
+    static constexpr int B_CANON = BIG ? 16 : 0, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0, B_BCONV = BIG ? RED : 0;
+    static constexpr bool IS_BIG = BIG;
     __host__ __device__ static constexpr int prod(int B) { return 9 + (B + 3) / 4; }
     // table entry i of an FP64 prime is one double (8 bytes); w / q is rebuilt as w * (1/q), whose
     // relative error of 2^-52 is inside the slack of the quotient estimate
@@ -410,6 +416,7 @@ struct ArithFp {
         return (uint64_t)__double_as_longlong(__dadd_rn(v, FP_2_52)) & 0x000FFFFFFFFFFFFFull;
     }
     __device__ __forceinline__ static uint64_t canon_fwd(T v, const K &k) { return to_canon(reduce(v, k), k); }
+    __device__ __forceinline__ static T bc_end(T x, const K &k) { return reduce(x, k); }
     __device__ __forceinline__ static uint64_t canon_inv(T v, const K &k) { return to_canon(v, k); }
 };
 

@@ -1,0 +1,39 @@
+// ntt_whole.cu - the instantiations and launchers of ntt_whole.cuh (a translation unit of its own: it compiles beside b200fhe.cu)
+#include "ntt_whole.cuh"
+#include "launch.cuh"
+
+namespace b2 {
+
+template <int LOGN, class Epi, int SRC>
+static void fwd(const NttArgs &a, const Epi &epi, const WholeArgs &w, uint32_t njobs, uint32_t batch, cudaStream_t s) {
+    launch_cl(1u << WholeCfg<LOGN>::LOG_CL, ntt_fwd_whole<LOGN, Epi, SRC>, dim3(njobs << WholeCfg<LOGN>::LOG_CL, batch), WholeCfg<LOGN>::THREADS, whole_smem<LOGN>(), s, a, epi, w);
+}
+template <int LOGN>
+static void inv(const NttArgs &a, uint32_t njobs, uint32_t batch, cudaStream_t s) {
+    launch_cl(1u << WholeCfg<LOGN>::LOG_CL, ntt_inv_whole<LOGN>, dim3(njobs << WholeCfg<LOGN>::LOG_CL, batch), WholeCfg<LOGN>::THREADS, whole_smem<LOGN>(), s, a);
+}
+
+void launch_inv_whole(const NttArgs &a, uint32_t njobs, uint32_t batch, cudaStream_t s) {
+    switch (a.logN) {
+        case 12: inv<12>(a, njobs, batch, s); break;
+        case 13: inv<13>(a, njobs, batch, s); break;
+        default: inv<14>(a, njobs, batch, s); break;
+    }
+}
+template <class Epi, int SRC>
+void launch_fwd_whole(const NttArgs &a, const Epi &epi, const WholeArgs &w, uint32_t njobs, uint32_t batch, cudaStream_t s) {
+    if constexpr (SRC == 0) {
+        if (a.logN == 13) return fwd<13, Epi, SRC>(a, epi, w, njobs, batch, s);
+        if (a.logN == 14) return fwd<14, Epi, SRC>(a, epi, w, njobs, batch, s);
+    }
+    fwd<12, Epi, SRC>(a, epi, w, njobs, batch, s);
+}
+
+template void launch_fwd_whole<EpiStore, 0>(const NttArgs &, const EpiStore &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiStore, 3>(const NttArgs &, const EpiStore &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubFrom, 3>(const NttArgs &, const EpiSubFrom &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubFromTab, 3>(const NttArgs &, const EpiSubFromTab &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, 1>(const NttArgs &, const EpiSubMul<false> &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, 2>(const NttArgs &, const EpiSubMul<false> &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+
+}  // namespace b2

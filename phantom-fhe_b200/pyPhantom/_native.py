@@ -43,6 +43,10 @@ SIGNATURES = {
     "b2_peer_free": (_int, [_vp]),
     "b2_peer_copy": (_int, [_vp, _vp, _sz, _vp]),
     "b2_sample": (_int, [_vp, _int, _vp, _vp, _sz, _sz, _vp, _vp]),
+    "b2_encode_coeffs": (_int, [_vp, _vp, _vp, _vp, ctypes.c_double, _vp, _vp]),
+    "b2_encrypt_symmetric": (_int, [_vp, _sz, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "b2_decrypt": (_int, [_vp, _sz, _vp, _vp, _vp, _vp]),
+    "b2_decode_slots": (_int, [_vp, _sz, _vp, _vp, ctypes.c_double, _vp, _vp, _vp, _vp, _vp]),
     "b2_tensor_mul": (_int, [_vp, _sz, _vp, _vp, _vp, _vp]),
     "b2_multiply_and_relin": (_int, [_vp, _sz, _vp, _vp, _vp, _sz, _vp, _vp, _sz, _vp]),
     "b2_rescale": (_int, [_vp, _sz, _sz, _vp, _vp, _vp, _sz, _vp]),

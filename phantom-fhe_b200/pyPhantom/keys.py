@@ -118,11 +118,6 @@ def _signed_draw(ctx, rng, kind, n_limbs, ntt=True):
     return out
 
 
-def _uniform(ctx, rng, n_limbs):
-    """[n_limbs][N] uniform residues (already a valid NTT-form polynomial)"""
-    return _device_draw(ctx, rng, 0, n_limbs, ctx.empty(n_limbs))
-
-
 def _error(ctx, rng, n_limbs):
     """centred binomial, 21 coin pairs: standard deviation sqrt(21/2) = 3.24 (include/prng.cuh:67-76)"""
     return _signed_draw(ctx, rng, 1, n_limbs)
@@ -193,14 +188,13 @@ class secret_key:
         self._set(ctx, c)
 
     # ---- encryption of zero under this secret: (-(a s + e), a) over the first n_limbs primes -------
-    def _encrypt_zero(self, ctx, n_limbs):
-        a = _uniform(ctx, self._rng_pub, n_limbs)
-        e = _error(ctx, self._rng, n_limbs)
-        c0 = ctx.empty(n_limbs)
-        _poly(ctx, 2, n_limbs, a, self.data[:n_limbs], c0)
-        _poly(ctx, 0, n_limbs, c0, e, c0)
-        _poly(ctx, 3, n_limbs, c0, None, c0)
-        return torch.stack([c0, a])
+    def _encrypt_zero(self, ctx, n_limbs, pt=None):
+        """with a plaintext [n_limbs][N] added: (m - (a s + e), a)"""
+        out = ctx.empty(2, n_limbs)
+        ws = torch.empty(ctx.N, dtype=torch.int64, device=ctx.device)
+        check(LIB.b2_encrypt_symmetric(ctx._h, n_limbs, self._rng_pub.bytes(44), self._rng.bytes(44), self.data.data_ptr(),
+                                       0 if pt is None else pt.data_ptr(), out.data_ptr(), ws.data_ptr(), _stream()))
+        return out
 
     def gen_publickey(self, ctx):
         from . import ciphertext
@@ -288,17 +282,21 @@ class secret_key:
         """(c0, c1) = (-(a s + e) + m, a) at the plaintext's level (src/secretkey.cu:236-299, 771-812)"""
         from . import ciphertext
         l = pt._limbs
-        data = self._encrypt_zero(ctx, l)
-        _poly(ctx, 0, l, data[0], pt.data, data[0])
         ct = ciphertext()
         ct._chain_index, ct._size, ct._N, ct._limbs, ct._scale = pt._chain_index, 2, ctx.N, l, pt._scale
-        ct.data = data
+        ct.data = self._encrypt_zero(ctx, l, pt.data)
         return ct
 
     def decrypt(self, ctx, ct):
         """m = c0 + c1 s (+ c2 s^2) on the first l limbs of the key-level secret (src/secretkey.cu:883-919)"""
         from . import plaintext
         l = ct._limbs
+        pt = plaintext()
+        pt._chain_index, pt._N, pt._limbs, pt._scale = ct._chain_index, ctx.N, l, ct._scale
+        if ct._size == 2 and ct.data.is_contiguous():
+            pt.data = ctx.empty(l)
+            check(LIB.b2_decrypt(ctx._h, l, ct.data.data_ptr(), self.data.data_ptr(), pt.data.data_ptr(), _stream()))
+            return pt
         s = self.data[:l]
         acc = ct.data[0].clone()
         t = ctx.empty(l)
@@ -310,8 +308,6 @@ class secret_key:
                 nxt = ctx.empty(l)
                 _poly(ctx, 2, l, sp.contiguous(), s, nxt)
                 sp = nxt
-        pt = plaintext()
-        pt._chain_index, pt._N, pt._limbs, pt._scale = ct._chain_index, ctx.N, l, ct._scale
         pt.data = acc
         return pt
 
