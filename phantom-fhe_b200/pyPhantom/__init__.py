@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _native
-from ._native import LIB, check
+from ._native import LIB, check, current_stream as _stream
 
 __version__ = "b200-dev"
 
@@ -115,10 +115,6 @@ def set_cuda_device(i):
 
 def get_cuda_device_count():
     return torch.cuda.device_count()
-
-
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
 
 
 # ---------------------------------------------------------------------------------------------

@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from . import _native, bootmath
-from ._native import LIB, check
+from ._native import LIB, check, current_stream as _stream
 
 C2S_LAYERS, EVAL_LEVELS, S2C_LAYERS = 3, 10, 2
 BOOT_LEVELS = C2S_LAYERS + EVAL_LEVELS + S2C_LAYERS
@@ -31,10 +31,6 @@ K_RANGE, DOUBLE_ANGLES, COS_DEGREE = 28, 3, 63
 SCALE_UP_MARGIN_BITS = 10  # the raised message stays below q0 / 2^10
 GIANT_LANES = 3            # streams the giant steps of a linear transform are dealt over
 FORK_LANES = 6             # extra streams shared by the two EvalRound tracks for their independent pieces
-
-
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _elt(step, N):

@@ -21,7 +21,7 @@ import struct
 import numpy as np
 import torch
 
-from ._native import LIB, check
+from ._native import LIB, check, current_stream as _stream
 
 
 class _CtrDrbg:
@@ -84,10 +84,6 @@ def _rng_pair(seed):
     return np.random.default_rng(a), np.random.default_rng(b)
 
 _SK_HDR = struct.Struct("<QQQ")  # sk_max_power, N, coeff_mod_size (include/secretkey.h:537-554)
-
-
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _poly(ctx, op, n_limbs, a, b, out):

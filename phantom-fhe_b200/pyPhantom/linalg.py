@@ -18,13 +18,9 @@ import numpy as np
 import torch
 
 from . import _native, get_elt_from_step, rescale_to_next
-from ._native import LIB, check
+from ._native import LIB, check, current_stream as _stream
 
 LANES = 3
-
-
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
 
 
 class resident_bsgs:

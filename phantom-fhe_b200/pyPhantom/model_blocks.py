@@ -21,16 +21,12 @@ import torch
 
 from . import (_native, add, bsgs_apply_giants_with_babies, compute_bsgs_babies, mod_switch_to, mod_switch_to_next,
                multiply_and_relin, multiply_plain, rescale_to_next, rotate, sub)
-from ._native import LIB, check
+from ._native import LIB, check, current_stream as _stream
 from .blocks import eval_chebyshev_series, eval_polynomial, inner_sum, schedule_chain_index
 
 MAX_LANES = 3          # side streams next to the caller's
 _LANES = {}            # device index -> list of side streams
 _FORKED = [False]      # forks do not nest: an inner fork runs in order on its lane
-
-
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _is_pow2(v):
