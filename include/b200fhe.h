@@ -115,6 +115,19 @@ int b2_multiply_relin_rescale_batch(b2_ctx *ctx, size_t size_Ql, size_t batch, c
                                     uint64_t *d_out, size_t out_stride, int rescale, void *d_ws, size_t ws_bytes,
                                     void *stream);
 
+/* No counterpart in the reference: independent products of an evaluation circuit in one call, every kernel one launch over
+ * them. Product p multiplies `sets` pairs, operands [sets][2][la[p]][N] and [sets][2][lb[p]][N] (la, lb >= size_Ql: the first
+ * size_Ql limbs count); doubled if dbl; relinearised; rescaled by rounding to nearest (b2_rescale_rounded).
+ * d_out [products][sets][2][size_Ql - 1][N]; d_a, d_b host arrays of device pointers; at most 16 products; workspace
+ * b2_multiply_relin_batch_workspace_bytes(products * sets). b2_rescale_rounded_batch: [sets][2][size_Ql][N] ->
+ * [sets][2][size_Ql - 1][N], workspace 2 * sets limbs. */
+int b2_multiply_relin_rescale_many(b2_ctx *ctx, size_t size_Ql, size_t products, size_t sets, const uint64_t *const *d_a,
+                                   const uint32_t *la, const uint64_t *const *d_b, const uint32_t *lb, int dbl,
+                                   const uint64_t *const *rlk, size_t n_evk, uint64_t *d_out, void *d_ws,
+                                   size_t ws_bytes, void *stream);
+int b2_rescale_rounded_batch(b2_ctx *ctx, size_t size_Ql, size_t sets, const uint64_t *d_in, uint64_t *d_out,
+                             void *d_ws, size_t ws_bytes, void *stream);
+
 /* replaces special_fft_backward / special_fft_forward with their bit reversals (src/fft.cu:90-346, src/ckks.cu:97-105, 176-183):
  * n = N/2 complex doubles; d_rot uint32 [n] = 5^j mod 2N, d_ksi complex double [2N + 1] = exp(2 pi i k / 2N).
  * inverse = 1 (encode): d_vals (overwritten) -> d_out = preimage of the embedding times scale; inverse = 0 (decode):
@@ -285,7 +298,8 @@ int b2_poly_op(b2_ctx *ctx, int op, size_t n_limbs, const uint64_t *d_a, const u
 
 /* b2_poly_op over a whole ciphertext [n_poly][size_Ql][N] in one launch (limb t of polynomial p on prime t).
  * op 0 add, 1 sub: d_b is a ciphertext of the same shape; op 2: d_b is ONE polynomial [size_Ql][N] (a
- * plaintext) multiplied into every polynomial (multiply_plain, src/evaluate.cu:1150-1200); op 3 negate. */
+ * plaintext) multiplied into every polynomial (multiply_plain, src/evaluate.cu:1150-1200); op 3 negate. n_poly above 3 (64 at most, here and in
+ * b2_ct_scalar and b2_ct_lincomb): a stack of two-polynomial ciphertexts. */
 int b2_ct_op(b2_ctx *ctx, int op, size_t size_Ql, size_t n_poly, const uint64_t *d_a, const uint64_t *d_b,
              uint64_t *d_out, void *stream);
 /* every polynomial of a ciphertext times the per-limb integer h_scalars[i] (see b2_poly_scalar, op 1) */

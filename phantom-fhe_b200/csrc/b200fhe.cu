@@ -1670,6 +1670,19 @@ extern "C" int b2_rescale_rounded(b2_ctx *c, size_t l, size_t n_poly, const uint
     return rescale_tail<2>(c, l, n_poly, r, d_in, d_out, s);
 }
 
+// The same for `sets` two-polynomial ciphertexts, set b at b * in_bs / out_bs limbs; r: 2 * sets limbs of scratch
+template <int MODE>
+static int rescale_sets(const b2_ctx *c, size_t l, uint32_t sets, const uint64_t *d_in, uint32_t in_bs, uint64_t *r, uint64_t *d_out, uint32_t out_bs,
+                        cudaStream_t s) {
+    const LevelPlan &pl = c->plan[l];
+    int rc = run_inv(c, d_in, r, pl.jobs_rs_intt, 2, 0, c->d_fin_plain, s, BatchDims{sets, 0, in_bs, 0, 2});
+    if (rc) return rc;
+    EpiSubMul<false> epi{d_in, d_out, pl.qlast_inv};
+    epi.m_bs = in_bs, epi.o_bs = out_bs;
+    return run_fwd<EpiSubMul<false>, MODE>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, (uint32_t)(l - 1), c->q[l - 1],
+                                           BatchDims{sets, 0, 2, 0, out_bs});
+}
+
 extern "C" size_t b2_multiply_relin_batch_workspace_bytes(const b2_ctx *c, size_t l, size_t batch) {
     if (!c || l < 1 || l > c->size_Q || batch < 1) return 0;
     return batch * (3 * l + 2) * limb_bytes(c) + b2_keyswitch_batch_workspace_bytes(c, l, batch);
@@ -1704,19 +1717,54 @@ extern "C" int b2_multiply_relin_rescale_batch(b2_ctx *c, size_t l, size_t batch
     }
     int rc = keyswitch_batch_impl(c, l, batch, prod + 2 * S, 3 * l, rlk, n_evk, prod, 3 * l, ws, s);
     if (rc) return rc;
-    if (!rescale) {
-        for (size_t b = 0; b < batch; b++)
-            CUDA_TRY(cudaMemcpyAsync(d_out + b * out_stride * N, prod + b * 3 * S, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
-        return B2_OK;
+    if (rescale) return rescale_sets<1>(c, l, B, prod, (uint32_t)(3 * l), r, d_out, (uint32_t)out_stride, s);
+    for (size_t b = 0; b < batch; b++) CUDA_TRY(cudaMemcpyAsync(d_out + b * out_stride * N, prod + b * 3 * S, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
+    return B2_OK;
+}
+
+// Products of an evaluation circuit that do not depend on one another, every kernel one launch over all of them: product p of
+// `sets` ciphertext pairs (operands [sets][2][la[p]][N] and [sets][2][lb[p]][N], of which the first l limbs count), doubled if
+// `dbl`, relinearised, and rescaled by rounding to nearest. d_out [products][sets][2][l - 1][N]. Workspace:
+// b2_multiply_relin_batch_workspace_bytes(l, products * sets).
+extern "C" int b2_multiply_relin_rescale_many(b2_ctx *c, size_t l, size_t products, size_t sets, const uint64_t *const *d_a, const uint32_t *la,
+                                              const uint64_t *const *d_b, const uint32_t *lb, int dbl, const uint64_t *const *rlk, size_t n_evk,
+                                              uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!d_a || !la || !d_b || !lb || !rlk || !d_out || !d_ws || products < 1 || products > TENSOR_MANY_MAX || sets < 1 || products * sets > 65535)
+        return fail(B2_EINVAL, "multiply_relin_rescale_many: bad argument (at most 16 products)");
+    if (l < 2) return fail(B2_EINVAL, "multiply_relin_rescale_many: no prime left to drop");
+    const size_t batch = products * sets;
+    if (ws_bytes < b2_multiply_relin_batch_workspace_bytes(c, l, batch)) return fail(B2_EWS, "multiply_relin_rescale_many: workspace too small");
+    if (!aligned32(d_out) || !aligned32(d_ws)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
+    TensorMany tm{};
+    tm.sets = (uint32_t)sets, tm.dbl = dbl ? 1u : 0u;
+    for (size_t p = 0; p < products; p++) {
+        if (!d_a[p] || !d_b[p] || la[p] < l || lb[p] < l || !aligned32(d_a[p]) || !aligned32(d_b[p]))
+            return fail(B2_EINVAL, "multiply_relin_rescale_many: an operand is missing, misaligned or below the level");
+        tm.a[p] = d_a[p], tm.b[p] = d_b[p], tm.la[p] = la[p], tm.lb[p] = lb[p];
     }
-    const LevelPlan &pl = c->plan[l];
-    // the dropped limb of both polynomials of every pair, then every remaining limb (in_j - NTT_j(r mod q_j)) * q_last^-1
-    rc = run_inv(c, prod, r, pl.jobs_rs_intt, 2, 0, c->d_fin_plain, s, BatchDims{B, 0, (uint32_t)(3 * l), 0, 2});
+    cudaStream_t s = (cudaStream_t)stream;
+    const size_t N = c->N, S = l * N;
+    uint64_t *prod = (uint64_t *)d_ws, *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
+    {
+        LaunchScope ls(c, s, "tensor_mul");
+        launch_k(tensor_many_kernel, dim3((unsigned)(N / 1024), (unsigned)l, (unsigned)batch), 256, 0, s, tm, prod, c->d_mod, (uint32_t)N, (uint32_t)l);
+        LAUNCH_CHECK("tensor_many_kernel");
+    }
+    int rc = keyswitch_batch_impl(c, l, batch, prod + 2 * S, 3 * l, rlk, n_evk, prod, 3 * l, ws, s);
     if (rc) return rc;
-    EpiSubMul<false> epi{prod, d_out, pl.qlast_inv};
-    epi.m_bs = (uint32_t)(3 * l), epi.o_bs = (uint32_t)out_stride;
-    return run_fwd<EpiSubMul<false>, 1>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, (uint32_t)(l - 1), c->q[l - 1],
-                                         BatchDims{B, 0, 2, 0, (uint32_t)out_stride});
+    return rescale_sets<2>(c, l, (uint32_t)batch, prod, (uint32_t)(3 * l), r, d_out, (uint32_t)(2 * (l - 1)), s);
+}
+
+// b2_rescale_rounded for `sets` ciphertexts [sets][2][l][N] -> [sets][2][l - 1][N]; workspace 2 * sets limbs
+extern "C" int b2_rescale_rounded_batch(b2_ctx *c, size_t l, size_t sets, const uint64_t *d_in, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!d_in || !d_out || !d_ws || sets < 1 || sets > 65535) return fail(B2_EINVAL, "rescale_rounded_batch: bad argument");
+    if (l < 2) return fail(B2_EINVAL, "rescale_rounded_batch: no prime left to drop");
+    if (ws_bytes < 2 * sets * limb_bytes(c)) return fail(B2_EWS, "rescale_rounded_batch: workspace too small");
+    return rescale_sets<2>(c, l, (uint32_t)sets, d_in, (uint32_t)(2 * l), (uint64_t *)d_ws, d_out, (uint32_t)(2 * (l - 1)), (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2269,9 +2317,12 @@ extern "C" int b2_poly_op(b2_ctx *c, int op, size_t n_limbs, const uint64_t *d_a
     return B2_OK;
 }
 
+// n_poly above three: a stack of two-polynomial ciphertexts of one level
+constexpr size_t STACK_MAX = 64;
+
 extern "C" int b2_ct_op(b2_ctx *c, int op, size_t l, size_t n_poly, const uint64_t *d_a, const uint64_t *d_b, uint64_t *d_out, void *stream) {
     CHECK_CTX(c);
-    if (op < 0 || op > 3 || !d_a || !d_out || (op != 3 && !d_b) || l < 1 || l > c->size_QP || n_poly < 1 || n_poly > 3)
+    if (op < 0 || op > 3 || !d_a || !d_out || (op != 3 && !d_b) || l < 1 || l > c->size_QP || n_poly < 1 || n_poly > STACK_MAX)
         return fail(B2_EINVAL, "ct_op: bad argument");
     LaunchScope ls(c, (cudaStream_t)stream, "poly_op");
     const bool wide = aligned32(d_a) && aligned32(d_out) && (op == 3 || aligned32(d_b));
@@ -2298,7 +2349,7 @@ extern "C" int b2_poly_scalar(b2_ctx *c, int op, size_t n_limbs, const uint64_t 
 
 extern "C" int b2_ct_scalar(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *d_a, const uint64_t *h_scalars, uint64_t *d_out, void *stream) {
     CHECK_CTX(c);
-    if (!d_a || !d_out || !h_scalars || l < 1 || l > c->size_QP || l > 64 || n_poly < 1 || n_poly > 3) return fail(B2_EINVAL, "ct_scalar: bad argument");
+    if (!d_a || !d_out || !h_scalars || l < 1 || l > c->size_QP || l > 64 || n_poly < 1 || n_poly > STACK_MAX) return fail(B2_EINVAL, "ct_scalar: bad argument");
     ScalarTab tab;
     for (size_t i = 0; i < l; i++) {
         if (h_scalars[i] >= c->q[i]) return fail(B2_EINVAL, "ct_scalar: scalar not reduced");
@@ -2314,7 +2365,7 @@ extern "C" int b2_ct_scalar(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *
 extern "C" int b2_ct_lincomb(b2_ctx *c, size_t l, size_t n_poly, size_t n_terms, const uint64_t *const *h_terms, const uint32_t *h_term_limbs,
                              const uint64_t *h_scalars, const uint64_t *h_const, uint64_t *d_out, void *stream) {
     CHECK_CTX(c);
-    if (!h_terms || !h_term_limbs || !h_scalars || !d_out || l < 1 || l > c->size_QP || l > B2_LINCOMB_MAX_LIMBS || n_poly < 1 || n_poly > 3 ||
+    if (!h_terms || !h_term_limbs || !h_scalars || !d_out || l < 1 || l > c->size_QP || l > B2_LINCOMB_MAX_LIMBS || n_poly < 1 || n_poly > STACK_MAX ||
         n_terms < 1 || n_terms > B2_LINCOMB_MAX_TERMS)
         return fail(B2_EINVAL, "ct_lincomb: bad argument (at most 8 terms and 32 limbs)");
     LincombArgs a;
@@ -2334,7 +2385,7 @@ extern "C" int b2_ct_lincomb(b2_ctx *c, size_t l, size_t n_poly, size_t n_terms,
     }
     LaunchScope ls(c, (cudaStream_t)stream, "lincomb");
     launch_k(lincomb_kernel, dim3((unsigned)(c->N / 256), (unsigned)(n_poly * l)), 256, 0, (cudaStream_t)stream, a, d_out, c->d_mod, (uint32_t)c->N, (uint32_t)l,
-             (uint32_t)n_terms);
+             (uint32_t)n_terms, n_poly > 3 ? 2u : (uint32_t)n_poly);
     LAUNCH_CHECK("lincomb_kernel");
     return B2_OK;
 }

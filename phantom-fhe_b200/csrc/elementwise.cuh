@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(256, 2) bsgs_mac_kernel(const uint64_t *const 
     with_sum(md.q, [&](auto s) { bsgs_mac_body<decltype(s), G>(pts, babies, outs, out, sp, md, (size_t)l * N, idx, M, n_g); });
 }
 
-// ---- weighted sum: out = sum_t x_t * s_t (+ c on polynomial 0) with per-limb integer weights, one reduction per value. The
-// terms may sit at higher levels than the output (more limbs per polynomial): lt[t] is term t's limb count.
+// ---- weighted sum: out = sum_t x_t * s_t (+ c on polynomial 0 of every ciphertext of `per` polynomials) with per-limb integer weights,
+// one reduction per value. The terms may sit at higher levels than the output (more limbs per polynomial): lt[t] is term t's limb count.
 #define B2_LINCOMB_MAX_TERMS 8
 #define B2_LINCOMB_MAX_LIMBS 32
 struct LincombArgs {
@@ -246,7 +246,7 @@ struct LincombArgs {
     uint64_t c[B2_LINCOMB_MAX_LIMBS];
 };
 template <class S>
-__device__ __forceinline__ void lincomb_body(const LincombArgs &a, uint64_t *out, const Mod &md, uint32_t N, uint32_t l, uint32_t n_terms) {
+__device__ __forceinline__ void lincomb_body(const LincombArgs &a, uint64_t *out, const Mod &md, uint32_t N, uint32_t l, uint32_t n_terms, uint32_t per) {
     const typename S::K k = S::make(md);
     const uint32_t limb = blockIdx.y % l, p = blockIdx.y / l, i = blockIdx.x * 256 + threadIdx.x;
     typename S::Acc acc;
@@ -260,13 +260,13 @@ __device__ __forceinline__ void lincomb_body(const LincombArgs &a, uint64_t *out
         if (t < (int)n_terms) S::mac(acc, S::ld_a(a.s[t][limb], k), S::ld_b(v[t], k), k);
     }
     const uint64_t r = S::finish(acc, k);
-    out[(size_t)blockIdx.y * N + i] = p == 0 ? add_mod(r, a.c[limb], md.q) : r;
+    out[(size_t)blockIdx.y * N + i] = p % per == 0 ? add_mod(r, a.c[limb], md.q) : r;
 }
 __global__ void __launch_bounds__(256) lincomb_kernel(const __grid_constant__ LincombArgs a, uint64_t *out, const Mod *mod, uint32_t N, uint32_t l,
-                                                     uint32_t n_terms) {
+                                                     uint32_t n_terms, uint32_t per) {
     pdl_enter();
     const Mod md = mod[blockIdx.y % l];
-    with_sum(md.q, [&](auto s) { lincomb_body<decltype(s)>(a, out, md, N, l, n_terms); });
+    with_sum(md.q, [&](auto s) { lincomb_body<decltype(s)>(a, out, md, N, l, n_terms, per); });
 }
 
 // ---- vector access: V = 4 words with 256-bit loads where every buffer is 32-byte aligned, else one word -------------------
@@ -285,21 +285,10 @@ __device__ __forceinline__ void stv(uint64_t *p, const uint64_t (&x)[V]) {
     else *p = x[0];
 }
 
-// HMult tensor product (src/polymath.cu:463-498): d0 = a0 b0, d1 = a0 b1 + a1 b0, d2 = a1 b1. d0, d1 go to out[0..2S), d2 to
-// out2[0..S): the relinearising caller keeps d2 in scratch and the rest in its result. blockIdx.z = pair of a batch, whose
-// operands, result and d2 start z * bs.x / .y / .z / .w limbs further. Streams seven limbs; FP64 products below 2^50
-// (24 limbs at N = 2^16: 27.1 us with 128-bit integer products on one word per thread).
+// (a0, a1) x (b0, b1): a0 <- a0 b0, b0 <- a0 b1 + a1 b0, a1 <- a1 b1
 template <int V>
-__global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *a, const uint64_t *b, uint64_t *out, uint64_t *out2, const Mod *mod, uint32_t N,
-                                                        uint32_t l, uint4 bs) {
-    pdl_enter();
-    const size_t o = (size_t)blockIdx.y * N + (blockIdx.x * 256 + threadIdx.x) * V, S = (size_t)l * N;
-    a += (size_t)blockIdx.z * bs.x * N + o, b += (size_t)blockIdx.z * bs.y * N + o, out += (size_t)blockIdx.z * bs.z * N + o,
-        out2 += (size_t)blockIdx.z * bs.w * N + o;
-    const Mod md = mod[blockIdx.y];
+__device__ __forceinline__ void tensor_values(uint64_t (&a0)[V], uint64_t (&a1)[V], uint64_t (&b0)[V], const uint64_t (&b1)[V], const Mod &md) {
     const uint64_t q = md.q;
-    uint64_t a0[V], a1[V], b0[V], b1[V];
-    ldv<V>(a0, a), ldv<V>(a1, a + S), ldv<V>(b0, b), ldv<V>(b1, b + S);
     if (q < FP_LIMIT) {
         using F = ArithFp<true>;
         const F::K k = F::make(md, 0);
@@ -319,7 +308,50 @@ __global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *a, cons
             a0[i] = d0, b0[i] = sub_mod(sub_mod(m, d0, q), d2, q), a1[i] = d2;
         }
     }
+}
+
+// HMult tensor product (src/polymath.cu:463-498): d0 = a0 b0, d1 = a0 b1 + a1 b0, d2 = a1 b1. d0, d1 go to out[0..2S), d2 to
+// out2[0..S): the relinearising caller keeps d2 in scratch and the rest in its result. blockIdx.z = pair of a batch, whose
+// operands, result and d2 start z * bs.x / .y / .z / .w limbs further. Streams seven limbs; FP64 products below 2^50
+// (24 limbs at N = 2^16: 27.1 us with 128-bit integer products on one word per thread).
+template <int V>
+__global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *a, const uint64_t *b, uint64_t *out, uint64_t *out2, const Mod *mod, uint32_t N,
+                                                        uint32_t l, uint4 bs) {
+    pdl_enter();
+    const size_t o = (size_t)blockIdx.y * N + (blockIdx.x * 256 + threadIdx.x) * V, S = (size_t)l * N;
+    a += (size_t)blockIdx.z * bs.x * N + o, b += (size_t)blockIdx.z * bs.y * N + o, out += (size_t)blockIdx.z * bs.z * N + o,
+        out2 += (size_t)blockIdx.z * bs.w * N + o;
+    const Mod md = mod[blockIdx.y];
+    uint64_t a0[V], a1[V], b0[V], b1[V];
+    ldv<V>(a0, a), ldv<V>(a1, a + S), ldv<V>(b0, b), ldv<V>(b1, b + S);
+    tensor_values<V>(a0, a1, b0, b1, md);
     stv<V>(out, a0), stv<V>(out + S, b0), stv<V>(out2, a1);
+}
+
+// The same for products whose operands lie apart and may sit at higher levels (more limbs per polynomial): blockIdx.z =
+// product p * sets + set, operand p at a[p] + set * 2 la[p] limbs. out [product][3][l][N]; dbl: the doubled product.
+constexpr int TENSOR_MANY_MAX = 16;
+struct TensorMany {
+    const uint64_t *a[TENSOR_MANY_MAX], *b[TENSOR_MANY_MAX];
+    uint32_t la[TENSOR_MANY_MAX], lb[TENSOR_MANY_MAX];
+    uint32_t sets, dbl;
+};
+__global__ void __launch_bounds__(256) tensor_many_kernel(const __grid_constant__ TensorMany t, uint64_t *out, const Mod *mod, uint32_t N, uint32_t l) {
+    pdl_enter();
+    constexpr int V = 4;
+    const uint32_t p = blockIdx.z / t.sets, set = blockIdx.z % t.sets;
+    const size_t o = (size_t)blockIdx.y * N + (blockIdx.x * 256 + threadIdx.x) * V, S = (size_t)l * N;
+    const uint64_t *a = t.a[p] + (size_t)set * 2 * t.la[p] * N + o, *b = t.b[p] + (size_t)set * 2 * t.lb[p] * N + o;
+    const Mod md = mod[blockIdx.y];
+    uint64_t d0[V], d1[V], d2[V], b1[V];
+    ldv<V>(d0, a), ldv<V>(d2, a + (size_t)t.la[p] * N), ldv<V>(d1, b), ldv<V>(b1, b + (size_t)t.lb[p] * N);
+    tensor_values<V>(d0, d2, d1, b1, md);
+    if (t.dbl) {
+#pragma unroll
+        for (int i = 0; i < V; i++) d0[i] = add_mod(d0[i], d0[i], md.q), d1[i] = add_mod(d1[i], d1[i], md.q), d2[i] = add_mod(d2[i], d2[i], md.q);
+    }
+    out += (size_t)blockIdx.z * 3 * S + o;
+    stv<V>(out, d0), stv<V>(out + S, d1), stv<V>(out + 2 * S, d2);
 }
 
 // x y mod q for V pairs, FP64 below 2^50
