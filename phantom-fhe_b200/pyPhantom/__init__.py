@@ -133,6 +133,7 @@ class context:
         self.device = torch.cuda.current_device()
         self.N = parms._N
         self.primes = np.array([m.value() for m in parms._coeff_modulus], dtype=np.uint64)
+        self.primes_signed = self.primes.view(np.int64)
         self.size_QP = len(self.primes)
         self.size_P = parms._special
         self.size_Q = self.size_QP - self.size_P

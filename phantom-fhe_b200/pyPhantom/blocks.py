@@ -1,6 +1,7 @@
 """Small host compositions over the evaluator that the reference binds next to it
 (python/src/binding.cu:522-531, 589-593; src/linear.cu, src/ps.cu): slot-block sums, replication and
 polynomial evaluation. They are calls into the same C ABI as everything else."""
+import functools
 import math
 
 import numpy as np
@@ -58,6 +59,19 @@ def eval_chebyshev_series(context, relin_key_, ct, cheb, out_chain_index):
     return out
 
 
+@functools.lru_cache(maxsize=32)
+def _monomials_to_chebyshev(n):
+    """[n][n]: column k holds x^k in the Chebyshev basis (x T_j = (T_(j+1) + T_|j-1|) / 2)"""
+    m = np.zeros((n, n))
+    m[0, 0] = 1.0
+    for k in range(1, n):
+        for j in range(k):
+            m[j + 1, k] += m[j, k - 1] * (1.0 if j == 0 else 0.5)
+            if j:
+                m[j - 1, k] += 0.5 * m[j, k - 1]
+    return m
+
+
 def eval_polynomial(context, encoder, relin_key_, ct, coeffs):
     """sum_k coeffs[k] x^k on every slot (src/ps.cu:131-200). The reference runs Paterson-Stockmeyer in the monomial
     basis with a chain of dependent powers; here the polynomial is rewritten in the Chebyshev basis (an exact change of
@@ -66,7 +80,5 @@ def eval_polynomial(context, encoder, relin_key_, ct, coeffs):
     c = np.asarray(coeffs, dtype=np.float64).ravel()
     if c.size < 2:
         raise ValueError("eval_polynomial: degree must be >= 1")
-    cheb = np.polynomial.chebyshev.poly2cheb(c)
-    if cheb.size < c.size:
-        cheb = np.concatenate([cheb, np.zeros(c.size - cheb.size)])
+    cheb = _monomials_to_chebyshev(c.size) @ c
     return eval_chebyshev_series(context, relin_key_, ct, cheb, schedule_chain_index(ct, c.size - 1))

@@ -30,7 +30,6 @@ BOOT_LEVELS = C2S_LAYERS + EVAL_LEVELS + S2C_LAYERS
 K_RANGE, DOUBLE_ANGLES, COS_DEGREE = 28, 3, 63
 SCALE_UP_MARGIN_BITS = 10  # the raised message stays below q0 / 2^10
 GIANT_LANES = 3            # streams the giant steps of a linear transform are dealt over
-FORK_LANES = 6             # extra streams shared by the two EvalRound tracks for their independent pieces
 
 
 def _elt(step, N):
@@ -59,45 +58,6 @@ class CtOps:
         self.counts = {"mul": 0, "rescale": 0} if counts is None else counts
         self.stream = _stream()  # the stream current when the ops object is made: one lookup, not one per call
         self.tab = rlk.pointer_table()
-        self.pool = []           # free streams that fork() may use
-        self.keep = []           # results that crossed streams during a graph capture (see fork)
-
-    def on_current_stream(self):
-        """the same arithmetic bound to whatever stream is current now (shares the counters and the lane pool)"""
-        o = CtOps(self.ctx, self.rlk, self.counts)
-        o.pool, o.keep = self.pool, self.keep
-        return o
-
-    def fork(self, thunks):
-        """independent pieces of work: all but the first go to free streams of the pool (if any are left), the first
-        runs here; everything joins before this returns. Each thunk gets the arithmetic bound to its stream."""
-        pool = self.pool
-        here = torch.cuda.current_stream()
-        capturing = torch.cuda.is_current_stream_capturing()
-        results, lanes = [None] * len(thunks), []
-        for i in range(1, len(thunks)):
-            if not pool:
-                break
-            lane = pool.pop()
-            lanes.append((i, lane))
-            lane.wait_stream(here)
-            with torch.cuda.stream(lane):
-                results[i] = thunks[i](self.on_current_stream())
-        for i, t in enumerate(thunks):
-            if results[i] is None:
-                results[i] = t(self)
-        for i, lane in lanes:
-            here.wait_stream(lane)
-            if hasattr(results[i], "data"):
-                if capturing:
-                    # record_stream does nothing for the allocator of a capture: once freed, this block could be
-                    # handed to the lane's next user - which may hang off another stream, unordered with the reads
-                    # that follow here. Keep it allocated until the whole pipeline has been issued.
-                    self.keep.append(results[i])
-                else:
-                    results[i].data.record_stream(here)
-            pool.append(lane)
-        return results
 
     def prime(self, level):
         return float(self.ctx.primes[level - 1])
@@ -135,12 +95,63 @@ class CtOps:
         if l < 2:
             raise ValueError("out of levels")
         out = ctx.empty(x._size, l - 1)
+        if x._size > 3:  # a stack of ciphertexts
+            ws = ctx.empty(x._size)
+            check(LIB.b2_rescale_rounded_batch(ctx._h, l, x._size // 2, x.data.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel() * 8, self.stream))
+            self.counts["rescale"] += 1
+            return x._like(out, chain_index=x._chain_index + 1, scale=x._scale / self.prime(l))
         ws, nbytes = ctx.workspace(_native.OP_RESCALE, l)
         check(LIB.b2_rescale_rounded(ctx._h, l, x._size, x.data.data_ptr(), out.data_ptr(), ws.data_ptr(), nbytes, self.stream))
         self.counts["rescale"] += 1
         return x._like(out, chain_index=x._chain_index + 1, scale=x._scale / self.prime(l))
 
+    def products(self, pairs, double=False):
+        """x * y (twice that, if `double`) relinearised and rescaled for every pair; the pairs are independent and may be
+        stacks of ciphertexts. Those of one level are one call: every kernel one launch over all of them."""
+        ctx, out = self.ctx, [None] * len(pairs)
+        by_level = {}
+        for i, (x, y) in enumerate(pairs):
+            by_level.setdefault(min(x._limbs, y._limbs), []).append(i)
+        tab = self.tab
+        for l, idx in by_level.items():
+            if l < 2:
+                raise ValueError("out of levels")
+            size = pairs[idx[0]][0]._size
+            for k in range(0, len(idx), 16):
+                part = idx[k: k + 16]
+                n, sets = len(part), size // 2
+                res = ctx.empty(n, size, l - 1)
+                nbytes = int(LIB.b2_multiply_relin_batch_workspace_bytes(ctx._h, l, n * sets))
+                ws = torch.empty(nbytes // 8, dtype=torch.int64, device=ctx.device)
+                ptrs = [np.array([pairs[i][j].data.data_ptr() for i in part], dtype=np.uint64) for j in (0, 1)]
+                limbs = [np.array([pairs[i][j]._limbs for i in part], dtype=np.uint32) for j in (0, 1)]
+                check(LIB.b2_multiply_relin_rescale_many(ctx._h, l, n, sets, ptrs[0].ctypes.data, limbs[0].ctypes.data, ptrs[1].ctypes.data,
+                                                         limbs[1].ctypes.data, 1 if double else 0, tab.ctypes.data, len(tab), res.data_ptr(),
+                                                         ws.data_ptr(), nbytes, self.stream))
+                for k2, i in enumerate(part):
+                    x, y = pairs[i]
+                    out[i] = x._like(res[k2], chain_index=ctx.size_Q - l + 2, scale=x._scale * y._scale / self.prime(l))
+                self.counts["mul"] += n
+                self.counts["rescale"] += n
+        return out
+
+    def rescaled_sums(self, sums, level):
+        """[(terms, c0, scale)] -> the weighted sums at `level`, each rescaled by one prime: one rescale for all of them"""
+        ctx, x0 = self.ctx, sums[0][0][0][0]
+        size, n = x0._size, len(sums)
+        if level > 32 or any(len(t) > 8 for t, _, _ in sums):
+            return [self.rescale(self.lincomb(t, c0, level, s)) for t, c0, s in sums]
+        buf, res = ctx.empty(n, size, level), ctx.empty(n, size, level - 1)
+        for k, (terms, c0, s) in enumerate(sums):
+            self._lincomb_into(terms, c0, level, s, buf[k])
+        ws = ctx.empty(n * size)
+        check(LIB.b2_rescale_rounded_batch(ctx._h, level, n * size // 2, buf.data_ptr(), res.data_ptr(), ws.data_ptr(), ws.numel() * 8, self.stream))
+        self.counts["rescale"] += n
+        return [x0._like(res[k], chain_index=ctx.size_Q - level + 2, scale=s / self.prime(level)) for k, (_, _, s) in enumerate(sums)]
+
     def _scalars(self, k, l):
+        if -(1 << 63) <= k < 1 << 63:
+            return np.mod(np.int64(k), self.ctx.primes_signed[:l]).astype(np.uint64)
         return np.array([k % int(q) for q in self.ctx.primes[:l]], dtype=np.uint64)
 
     def mul_const(self, x, c, const_scale):
@@ -159,20 +170,29 @@ class CtOps:
                 t = self.mul_const(self.drop(x, level), c, cs)
                 acc = t if acc is None else self.add(acc, t)
             return self.add_const(acc, c0)
+        x0 = terms[0][0]
+        out = self.ctx.empty(x0._size, level)
+        self._lincomb_into(terms, c0, level, scale, out)
+        return x0._like(out, chain_index=x0._chain_index + (x0._limbs - level), scale=scale)
+
+    def _lincomb_into(self, terms, c0, level, scale, out):
         ptrs = np.array([x.data.data_ptr() for x, _, _ in terms], dtype=np.uint64)
         limbs = np.array([x._limbs for x, _, _ in terms], dtype=np.uint32)
         sc = np.concatenate([self._scalars(int(round(c * cs)), level) for _, c, cs in terms])
         c0v = self._scalars(int(round(c0 * scale)), level)
-        x0 = terms[0][0]
-        out = self.ctx.empty(x0._size, level)
-        check(LIB.b2_ct_lincomb(self.ctx._h, level, x0._size, n, ptrs.ctypes.data, limbs.ctypes.data, sc.ctypes.data, c0v.ctypes.data,
-                                out.data_ptr(), self.stream))
-        return x0._like(out, chain_index=x0._chain_index + (x0._limbs - level), scale=scale)
+        check(LIB.b2_ct_lincomb(self.ctx._h, level, terms[0][0]._size, len(terms), ptrs.ctypes.data, limbs.ctypes.data, sc.ctypes.data,
+                                c0v.ctypes.data, out.data_ptr(), self.stream))
 
     def add_const(self, x, c):
-        sc = self._scalars(int(round(c * x._scale)), x._limbs)
+        l = x._limbs
+        if l <= 32:  # one launch: 1 * x + c
+            out = torch.empty_like(x.data)
+            self._lincomb_into([(x, 1.0, 1.0)], c, l, x._scale, out)
+            return x._like(out)
+        sc = self._scalars(int(round(c * x._scale)), l)
         out = x.data.clone()
-        check(LIB.b2_poly_scalar(self.ctx._h, 0, x._limbs, x.data[0].data_ptr(), sc.ctypes.data, out[0].data_ptr(), self.stream))
+        for p in range(0, x._size, 2 if x._size > 3 else x._size):
+            check(LIB.b2_poly_scalar(self.ctx._h, 0, l, x.data[p].data_ptr(), sc.ctypes.data, out[p].data_ptr(), self.stream))
         return x._like(out)
 
     def _lin(self, op, x, y):
@@ -235,15 +255,8 @@ class bootstrap_key:
         self.conj = None
         self.c2s, self.s2c = [], []
         self._streams = []
-        self._fork_streams = None
         self.use_graph = True   # replay a captured CUDA graph per (input limbs, input scale) after the first call
         self._graphs = {}
-
-    def fork_pool(self):
-        """streams for the independent sub-computations inside EvalRound (disjoint from side_streams)"""
-        if self._fork_streams is None:
-            self._fork_streams = [torch.cuda.Stream() for _ in range(FORK_LANES)]
-        return list(self._fork_streams)
 
     def side_streams(self, n):
         while len(self._streams) < n:
@@ -511,19 +524,10 @@ def slot_to_coeff(ctx, bk, lo, hi, ops):
 
 
 def _eval_round_pair(ops, bk, lo, hi):
-    """the real and the imaginary track are independent: the second one runs on a side stream, with its own
-    scratch (everything it allocates belongs to that stream), and joins before SlotToCoeff"""
-    main = torch.cuda.current_stream()
-    side = bk.side_streams(1)[0]
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        b = bootmath.eval_round(ops.on_current_stream(), hi, K_RANGE, DOUBLE_ANGLES, COS_DEGREE, bk.eval_scale)
-    a = bootmath.eval_round(ops, lo, K_RANGE, DOUBLE_ANGLES, COS_DEGREE, bk.eval_scale)
-    main.wait_stream(side)
-    if not torch.cuda.is_current_stream_capturing():
-        for t in (b.data, hi.data):
-            t.record_stream(main)
-    return a, b
+    """the real and the imaginary track take the same steps at the same levels and scales: they run as one stack of two
+    ciphertexts, every kernel one launch over both (as single ciphertexts on two streams the launches half filled the GPU)"""
+    both = bootmath.eval_round(ops, lo._like(torch.cat([lo.data, hi.data])), K_RANGE, DOUBLE_ANGLES, COS_DEGREE, bk.eval_scale)
+    return both._like(both.data[:2]), both._like(both.data[2:])
 
 
 def bootstrap(context, encoder, ct, bk, user_scale, split_scale_down=False, stats=None):
@@ -561,7 +565,6 @@ def bootstrap_eager(context, encoder, ct, bk, user_scale, split_scale_down=False
     if ct._size != 2 or not ct._is_ntt_form:
         raise ValueError("bootstrap wants a 2-polynomial ciphertext in NTT form")
     ops = CtOps(ctx, bk.relin)
-    ops.pool = bk.fork_pool()
     scale_in = ct._scale
     x = ct
     if bk.user_scale == 0.0 or abs(scale_in / bk.user_scale - 1.0) > 2.0 ** -20:

@@ -219,10 +219,11 @@ class ChebyshevEvaluator:
         self.ops, self.m, self.tight = ops, babies, tight
         self.T = {1: u}
         self.giants = None
+        self._matched = None
 
-    def match(self, x, level, scale, ops=None):
+    def match(self, x, level, scale):
         """bring x down to (level, scale): free if it is already there, else one integer multiply and rescale"""
-        ops = ops or self.ops
+        ops = self.ops
         if ops.level(x) == level:
             if abs(ops.scale(x) / scale - 1.0) > 2.0 ** -40:
                 raise ValueError("operand already at the target level with a different scale")
@@ -233,23 +234,24 @@ class ChebyshevEvaluator:
         x = ops.mul_const(x, 1.0, scale * ops.prime(level + 1) / ops.scale(x))
         return ops.rescale(x)
 
-    def _power(self, k, ops):
-        """T_k from T_ceil(k/2), T_floor(k/2), both already there: 2 T_a T_b - T_(a-b), a - b in {0, 1}"""
-        a, b = (k + 1) // 2, k // 2
-        xa, xb = self.T[a], self.T[b]
-        lvl = min(ops.level(xa), ops.level(xb))
-        prod = ops.mul(ops.drop(xa, lvl), ops.drop(xb, lvl))
-        prod = ops.rescale(ops.add(prod, prod))
-        if a == b:
-            return ops.add_const(prod, -1.0)
-        return ops.sub(prod, self.match(self.T[1], ops.level(prod), ops.scale(prod), ops))
+    def _products(self, pairs, double=False):
+        """rescaled products (doubled) of independent pairs: one call where the arithmetic has it"""
+        ops = self.ops
+        if hasattr(ops, "products"):
+            return ops.products(pairs, double)
+        out = []
+        for x, y in pairs:
+            lvl = min(ops.level(x), ops.level(y))
+            p = ops.mul(ops.drop(x, lvl), ops.drop(y, lvl))
+            out.append(ops.rescale(ops.add(p, p) if double else p))
+        return out
 
     def prepare(self, degree):
-        """T_2 .. T_(m-1) and the giants T_m, T_2m, ...: powers of equal depth ceil(log2 k) only need shallower ones,
-        so each depth is one fork (independent work the arithmetic may spread over streams)"""
+        """T_2 .. T_(m-1) and the giants T_m, T_2m, ...: T_k = 2 T_a T_b - T_(a-b) with a = ceil(k/2), b = floor(k/2), and
+        powers of equal depth ceil(log2 k) only need shallower ones, so each depth is one set of independent products"""
         if getattr(self, "giants", None) is not None:
             return
-        g, giants = self.m, []
+        ops, g, giants = self.ops, self.m, []
         while g < degree or (g == degree and not self.tight):
             giants.append(g)
             g *= 2
@@ -260,59 +262,95 @@ class ChebyshevEvaluator:
             by_depth.setdefault((k - 1).bit_length(), []).append(k)
         for depth in sorted(by_depth):
             ks = by_depth[depth]
-            outs = self.ops.fork([(lambda o, k=k: self._power(k, o)) for k in ks])
-            for k, v in zip(ks, outs):
-                self.T[k] = v
+            for k, p in zip(ks, self._products([(self.T[(k + 1) // 2], self.T[k // 2]) for k in ks], double=True)):
+                if k % 2 == 0:
+                    self.T[k] = ops.add_const(p, -1.0)
+                else:
+                    self.T[k] = ops.sub(p, self._matched_u(ops.level(p), ops.scale(p)))
         self.giants = giants
 
-    def _leaf(self, c, level, scale, ops):
-        up = level + 1
-        target = scale * ops.prime(up)
-        if hasattr(ops, "lincomb"):  # one fused launch where the arithmetic has it
-            terms = [(self.T[i], float(c[i]), target / ops.scale(self.T[i])) for i in range(1, len(c)) if c[i] != 0.0]
-            if terms:
-                return ops.rescale(ops.lincomb(terms, float(c[0]), up, target))
-        acc = None
-        for i in range(1, len(c)):
-            if c[i] == 0.0 and not (acc is None and i == len(c) - 1):
-                continue
-            x = ops.drop(self.T[i], up)
-            term = ops.mul_const(x, float(c[i]), target / ops.scale(x))
-            acc = term if acc is None else ops.add(acc, term)
-        if acc is None:  # a bare constant: carry it on 0 * T_1
-            x = ops.drop(self.T[1], up)
-            acc = ops.mul_const(x, 0.0, target / ops.scale(x))
-        acc = ops.add_const(acc, float(c[0]))
-        return ops.rescale(acc)
+    def _matched_u(self, level, scale):
+        """T_1 at (level, scale): the odd powers of one depth share it"""
+        key, cached = (level, scale), self._matched
+        if cached is None or cached[0] != key:
+            self._matched = (key, self.match(self.T[1], level, scale))
+        return self._matched[1]
 
-    def _eval(self, c, level, scale, ops=None):
-        ops = ops or self.ops
+    def _leaves(self, tasks):
+        """[(coefficients of degree < m, level, scale)] -> values; where the arithmetic has fused sums, the leaves of one
+        level share a rescale"""
+        ops, out, sums = self.ops, [None] * len(tasks), {}
+        for i, (c, level, scale) in enumerate(tasks):
+            up = level + 1
+            target = scale * ops.prime(up)
+            if hasattr(ops, "lincomb"):
+                terms = [(self.T[j], float(c[j]), target / ops.scale(self.T[j])) for j in range(1, len(c)) if c[j] != 0.0]
+                if terms:
+                    sums.setdefault(up, []).append((i, (terms, float(c[0]), target)))
+                    continue
+            acc = None
+            for j in range(1, len(c)):
+                if c[j] == 0.0 and not (acc is None and j == len(c) - 1):
+                    continue
+                x = ops.drop(self.T[j], up)
+                term = ops.mul_const(x, float(c[j]), target / ops.scale(x))
+                acc = term if acc is None else ops.add(acc, term)
+            if acc is None:  # a bare constant: carry it on 0 * T_1
+                x = ops.drop(self.T[1], up)
+                acc = ops.mul_const(x, 0.0, target / ops.scale(x))
+            out[i] = ops.rescale(ops.add_const(acc, float(c[0])))
+        for up, group in sums.items():
+            for (i, _), v in zip(group, ops.rescaled_sums([s for _, s in group], up)):
+                out[i] = v
+        return out
+
+    def _trim(self, c):
         c = np.asarray(c, dtype=np.float64)
         d = len(c) - 1
         while d > 0 and c[d] == 0.0:
             d -= 1
-        c = c[: d + 1]
-        if d < self.m or (self.tight and d == self.m):
-            return self._leaf(c, level, scale, ops)
-        g = max(x for x in self.giants if x <= d)
-        q, r = cheb_divide(c, g)
-        tg = ops.drop(self.T[g], level + 1)
-        q_scale = scale * ops.prime(level + 1) / ops.scale(tg)
-        # quotient and remainder are independent until the final sum
-        qv, rv = ops.fork([lambda o: self._eval(q, level + 1, q_scale, o), lambda o: self._eval(r, level, scale, o)])
-        prod = ops.rescale(ops.mul(qv, tg))
-        return ops.add(prod, rv)
+        return c[: d + 1], d
+
+    def _is_leaf(self, d):
+        return d < self.m or (self.tight and d == self.m)
+
+    def _eval_many(self, tasks):
+        """[(coefficients, level, scale)] -> values at (level, scale), all of them in step: the nodes of one depth of the
+        division tree are one set of leaves and one set of products. A remainder is evaluated a level higher than it is
+        needed where its depth allows, at the level of the quotient next to it, so that their products are one set."""
+        ops, out = self.ops, [None] * len(tasks)
+        leaves, nodes, children = [], [], []
+        for i, (c, level, scale) in enumerate(tasks):
+            c, d = self._trim(c)
+            if self._is_leaf(d):
+                leaves.append((i, (c, level, scale)))
+                continue
+            g = max(x for x in self.giants if x <= d)
+            q, r = cheb_divide(c, g)
+            tg = self.T[g]
+            up = level + 1
+            r_level = up if not self._is_leaf(self._trim(r)[1]) and ops.level(self.T[1]) - self._depth(r) >= up else level
+            nodes.append((i, tg, level))
+            children += [(q, up, scale * ops.prime(up) / ops.scale(tg)), (r, r_level, scale)]
+        if leaves:
+            for (i, _), v in zip(leaves, self._leaves([t for _, t in leaves])):
+                out[i] = v
+        if nodes:
+            vals = self._eval_many(children)
+            prods = self._products([(vals[2 * k], tg) for k, (_, tg, _) in enumerate(nodes)])
+            for k, (i, _, level) in enumerate(nodes):
+                out[i] = ops.add(prods[k], ops.drop(vals[2 * k + 1], level))
+        return out
+
+    def _eval(self, c, level, scale):
+        return self._eval_many([(c, level, scale)])[0]
 
     def _depth(self, c):
         """levels below T_1 that _eval needs for these coefficients (a dry run of its recursion)"""
         ops = self.ops
-        c = np.asarray(c, dtype=np.float64)
-        d = len(c) - 1
-        while d > 0 and c[d] == 0.0:
-            d -= 1
-        c = c[: d + 1]
+        c, d = self._trim(c)
         top = ops.level(self.T[1])
-        if d < self.m or (self.tight and d == self.m):
+        if self._is_leaf(d):
             return 1 + max([top - ops.level(self.T[i]) for i in range(1, d + 1) if c[i] != 0.0], default=0)
         g = max(x for x in self.giants if x <= d)
         q, r = cheb_divide(c, g)
@@ -346,8 +384,7 @@ def eval_round(ops, u, K, r, degree, out_scale, babies=8):
     D = ev._eval(coeffs, lvl_poly, s)
     for _ in range(r):
         a = a * a
-        sq = ops.mul(D, D)
-        D = ops.add_const(ops.rescale(ops.add(sq, sq)), -a)
+        D = ops.add_const(ev._products([(D, D)], double=True)[0], -a)
     Ku = ev.match(ops.with_scale(u, ops.scale(u) / K), ops.level(D), ops.scale(D))
     return ops.sub(Ku, D)
 
@@ -368,10 +405,6 @@ class FloatOps:
 
     def prime(self, level):
         return float(self.primes[level - 1])
-
-    def fork(self, thunks):
-        """independent pieces of work, each given the arithmetic to use: here simply one after the other"""
-        return [t(self) for t in thunks]
 
     def level(self, x):
         return x.level
