@@ -231,6 +231,14 @@ int b2_rotate_add(b2_ctx *ctx, size_t size_Ql, uint32_t galois_elt, const uint64
                   const uint64_t *const *ksk, size_t n_evk, uint64_t *d_acc, void *d_ws, size_t ws_bytes,
                   void *stream);
 
+/* d_acc [2][size_Ql][N] (+)= sum_i (ciphertext i rotated by elts[i]), ciphertext i at d_cts + i * ct_stride limbs, its key's
+ * digits at ksk[i * n_evk ..]; one ModDown for the sum (the reference rotates and adds per giant step,
+ * src/bootstrap.cu:1290-1340). first != 0 overwrites d_acc. */
+size_t b2_rotate_sum_workspace_bytes(const b2_ctx *ctx, size_t size_Ql, size_t n);
+int b2_rotate_sum(b2_ctx *ctx, size_t size_Ql, size_t n, const uint32_t *elts, const uint64_t *d_cts, size_t ct_stride,
+                  const uint64_t *const *ksk, size_t n_evk, uint64_t *d_acc, int first, void *d_ws, size_t ws_bytes,
+                  void *stream);
+
 /* replaces hoisting_inplace (src/evaluate.cu:1732-1927): d_out [2][size_Ql][N] = the SUM over the n_steps Galois
  * elements of the rotated d_ct, from one ModUp of c1 and one ModDown per polynomial (ksk and workspace as for
  * b2_hoist_rotations; d_out must not alias d_ct) */

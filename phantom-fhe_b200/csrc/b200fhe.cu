@@ -1927,6 +1927,79 @@ extern "C" int b2_rotate_add(b2_ctx *c, size_t l, uint32_t elt, const uint64_t *
     return keyswitch_impl(c, l, d_ct + l * c->N, ksk, n_evk, d_acc, (uint64_t *)d_ws, (cudaStream_t)stream, KsRot{perm, d_ct, false});
 }
 
+// d_acc (+)= the sum over i of ciphertext i ([2][l][N], ct_stride limbs apart) rotated by elts[i] with its own key, from one
+// ModDown: the giant steps of a BSGS linear transform. In chunks that fit the L2 the c1 are permuted, decomposed together and
+// their inner products summed inside one launch; overwrites d_acc if `first`. d_cts and d_acc distinct.
+// ws: accP [2][alpha] | per chunk entry c1 [l] | t [l] | up [beta][l + alpha]; ModDown reuses the chunk part.
+static size_t rotate_sum_chunk(const b2_ctx *c, size_t l, size_t n) {
+    const size_t beta = (l + c->size_P - 1) / c->size_P, one = (2 * l + beta * (l + c->size_P)) * limb_bytes(c);
+    const size_t fit = std::max<size_t>(2, (size_t(128) << 20) / one);
+    return std::max<size_t>(1, std::min({n, fit, (size_t)IP_MAX_STEPS, (size_t)GATHER_TAB_MAX, IP_MAX_EVK / beta}));
+}
+extern "C" size_t b2_rotate_sum_workspace_bytes(const b2_ctx *c, size_t l, size_t n) {
+    if (!c || l < 1 || l > c->size_Q || n < 1) return 0;
+    const size_t a = c->size_P, beta = (l + a - 1) / a;
+    return (2 * a + rotate_sum_chunk(c, l, n) * (2 * l + beta * (l + a))) * limb_bytes(c);
+}
+extern "C" int b2_rotate_sum(b2_ctx *c, size_t l, size_t n, const uint32_t *elts, const uint64_t *d_cts, size_t ct_stride, const uint64_t *const *ksk, size_t n_evk,
+                             uint64_t *d_acc, int first, void *d_ws, size_t ws_bytes, void *stream) {
+    CHECK_CTX(c);
+    CHECK_LEVEL(c, l);
+    if (!elts || !d_cts || !ksk || !d_acc || !d_ws || n < 1) return fail(B2_EINVAL, "rotate_sum: bad argument");
+    if (ct_stride < 2 * l || ct_stride > 0xFFFFFFFFull) return fail(B2_EINVAL, "rotate_sum: a ciphertext's stride is smaller than the ciphertext");
+    if (ws_bytes < b2_rotate_sum_workspace_bytes(c, l, n)) return fail(B2_EWS, "rotate_sum: workspace too small");
+    if (!aligned32(d_cts) || !aligned32(d_acc) || !aligned32(d_ws)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
+    const size_t N = c->N, a = c->size_P, lP = l + a, S = l * N;
+    if (d_acc < d_cts + n * ct_stride * N && d_cts < d_acc + 2 * S) return fail(B2_EINVAL, "rotate_sum: needs distinct operands and sum");
+    const LevelPlan &pl = c->plan[l];
+    const size_t beta = pl.beta, chunk = rotate_sum_chunk(c, l, n);
+    cudaStream_t s = (cudaStream_t)stream;
+    std::vector<const uint32_t *> perms(n);
+    for (size_t i = 0; i < n; i++) {
+        int rc = galois_lookup(c, elts[i], &perms[i]);
+        if (rc) return rc;
+    }
+    uint64_t *accP = (uint64_t *)d_ws, *c1 = accP + 2 * a * N, *t = c1 + chunk * S, *up = t + chunk * S;
+    for (size_t i0 = 0; i0 < n; i0 += chunk) {
+        const uint32_t B = (uint32_t)std::min(chunk, n - i0), per = (uint32_t)(beta * lP);
+        GatherTab tab{};
+        for (uint32_t i = 0; i < B; i++) tab.perm[i] = perms[i0 + i];
+        {
+            LaunchScope ls(c, s, "galois_gather");
+            launch_k(galois_gather_tab_kernel, dim3((unsigned)(N / 1024), (unsigned)l, B), 256, 0, s, d_cts + (i0 * ct_stride + l) * N, c1, tab, (uint32_t)N,
+                     (uint32_t)ct_stride);
+            LAUNCH_CHECK("galois_gather_tab_kernel");
+        }
+        int rc = run_inv(c, c1, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, (uint32_t)l, 0, (uint32_t)l});
+        if (rc) return rc;
+        if (use_whole(c, (size_t)pl.n_up_ntt * B)) {
+            rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
+            if (rc) return rc;
+        } else {
+            if (c->bconv_tc && !c->tc_simple) {
+                const TcBatch tb{B, 0, (uint32_t)l, 0, per, c->tc_serial_ld ? 1u : 0u};
+                rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, &tb);
+                if (rc) return rc;
+            } else {
+                for (uint32_t i = 0; i < B; i++) {
+                    rc = run_bconv(c, false, t + i * S, up + (size_t)i * per * N, nullptr, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)a,
+                                   (uint32_t)lP, true, s, &pl.tc_up);
+                    if (rc) return rc;
+                }
+            }
+            rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            if (rc) return rc;
+        }
+        IpArgs ia = ip_args(c, l, up, c1, accP, d_acc);
+        ia.fused = 1, ia.ct_acc = i0 > 0 || !first, ia.acc_p = i0 > 0, ia.c0 = d_cts + i0 * ct_stride * N, ia.steps = B;
+        ia.apart = 1, ia.dig_ss = per, ia.own_ss = (uint32_t)l, ia.c0_ss = (uint32_t)ct_stride;
+        for (uint32_t i = 0; i < B; i++) ia.perm[i] = perms[i0 + i];
+        rc = run_inner_prod(c, ia, ksk + i0 * n_evk, n_evk, B, 1, s);
+        if (rc) return rc;
+    }
+    return ks_moddown(c, l, accP, c1, d_acc, s);
+}
+
 // `batch` ciphertexts rotated by one Galois element, every kernel one launch over the batch (see b2_keyswitch_batch)
 extern "C" int b2_apply_galois_batch(b2_ctx *c, size_t l, uint32_t elt, size_t batch, const uint64_t *d_ct, size_t ct_stride, const uint64_t *const *ksk,
                                      size_t n_evk, uint64_t *d_out, size_t out_stride, void *d_ws, size_t ws_bytes, void *stream) {

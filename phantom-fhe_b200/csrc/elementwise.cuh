@@ -20,6 +20,14 @@ __device__ __forceinline__ uint64_t mul_mod(uint64_t x, uint64_t y, const Mod &m
     return csub(lo - __umul64hi(t, m.mu) * m.q, m.q);
 }
 
+// the same for a sum of up to four products, q below 2^60: t < 2^64, the estimate is short by two at most
+__device__ __forceinline__ uint64_t reduce_sum4(u128 x, const Mod &m) {
+    const int n = 64 - __clzll((long long)m.q);
+    const uint64_t t = (x.hi << (66 - n)) | (x.lo >> (n - 2));
+    const uint64_t r = x.lo - __umul64hi(t, m.mu) * m.q;
+    return csub(csub(r, 2 * m.q), m.q);
+}
+
 // ---- sums of products: how operands are held and summed, per prime class -------------------------------------------------
 //   A, B     an operand as the sum wants it (split, or with its quotient); Acc the running sum; FLUSH how many terms it takes
 //   flush    brings a full sum back to where it takes FLUSH terms again
@@ -87,8 +95,7 @@ struct SumFp {
     __device__ __forceinline__ static void flush(Acc &s, const K &k) { s = F::reduce(s, k); }
     __device__ __forceinline__ static uint64_t finish(const Acc &s, const K &k) { return F::canon_fwd(s, k); }
     __device__ __forceinline__ static uint64_t finish_mul(const Acc &s, W2 w, const K &k) {
-        const double wd = (double)w.w;
-        return F::to_canon(F::mulmod(F::reduce(s, k), A{wd, __dmul_rn(wd, k.qinv)}, k), k);
+        return F::to_canon(F::mulmod(F::reduce(s, k), ld_a(w.w, k), k), k);
     }
 };
 // Primes below 2^60: 30-bit halves, four wide multiply-adds per term straight into 64-bit sums (two terms a sum of the
@@ -132,6 +139,11 @@ struct SumInt30 {
         }
     }
     __device__ __forceinline__ static uint64_t finish(const Acc &s, const K &k) { return barrett128(total(s), k.q, k.r0, k.r1); }
+    __device__ __forceinline__ static uint64_t finish_mul(const Acc &s, W2 w, const K &k) { return mul_shoup(finish(s, k), w, k.q); }
+};
+// at most four terms: half the multiplications at the end
+struct SumInt30Short : SumInt30 {
+    __device__ __forceinline__ static uint64_t finish(const Acc &s, const K &k) { return reduce_sum4(total(s), k); }
     __device__ __forceinline__ static uint64_t finish_mul(const Acc &s, W2 w, const K &k) { return mul_shoup(finish(s, k), w, k.q); }
 };
 // Any prime up to 61 bits: 128-bit sums
@@ -462,6 +474,20 @@ __global__ void __launch_bounds__(256) galois_gather_kernel(const uint64_t *__re
     stv<V>(dst + (size_t)blockIdx.y * N + i, x);
 }
 
+// the same for several polynomials, each through a permutation of its own: blockIdx.z = polynomial, src_bs limbs apart
+constexpr int GATHER_TAB_MAX = 16;
+struct GatherTab {
+    const uint32_t *perm[GATHER_TAB_MAX];
+};
+__global__ void __launch_bounds__(256) galois_gather_tab_kernel(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, const __grid_constant__ GatherTab tab,
+                                                               uint32_t N, uint32_t src_bs) {
+    pdl_enter();
+    const uint32_t i = (blockIdx.x * 256 + threadIdx.x) * 4;
+    const uint64_t *s = src + ((size_t)blockIdx.z * src_bs + blockIdx.y) * N;
+    const uint4 p = *reinterpret_cast<const uint4 *>(tab.perm[blockIdx.z] + i);
+    st256(dst + ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * N + i, s[p.x], s[p.y], s[p.z], s[p.w]);
+}
+
 // Signed coefficient vectors -> their residues in each of l primes from first_prime on (src/bootstrap.cu:660-686,
 // light_pt_expand_per_tower_kernel): src [M][N] -> dst [M][l][N], blockIdx.z = vector
 template <int V>
@@ -532,6 +558,9 @@ struct IpArgs {
     // set per step, written to ct_tab[z] (P limbs as above); each = 0: the steps are summed.
     // A rotation whose c1 was permuted before ModUp: steps = 0 and perm[0] set; own and c0 are read through it, digits are not.
     uint32_t steps, each;
+    // steps that are summed and have ciphertexts of their own, c1 permuted before ModUp: step s reads digits and own s * dig_ss /
+    // own_ss limbs further, as they are, and c0 s * c0_ss limbs further through perm[s]
+    uint32_t apart, dig_ss, own_ss, c0_ss;
     const uint32_t *perm[IP_MAX_STEPS];
     uint64_t *ct_tab[IP_MAX_STEPS];
     const uint64_t *evk[IP_MAX_EVK];
@@ -555,14 +584,14 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
     const uint64_t *digits = a.digits + ((size_t)z * a.dig_bs + t) * N, *own = a.own ? a.own + ((size_t)z * a.own_bs + t) * N : nullptr;
     const uint32_t own_d = (own && t < a.l) ? t / (a.lP - a.l) : 0xFFFFFFFFu;
     const uint32_t s0 = a.each ? z : 0, n_s = a.steps && !a.each ? a.steps : 1;
-    const bool hoist = a.steps != 0;
+    const bool hoist = a.steps != 0 && !a.apart;
     uint64_t g0 = 0, g1 = 0;  // permuted c0
     int pending = 0;
-    for (uint32_t s = s0; s < s0 + n_s; s++) {
+    for (uint32_t s = s0; s < s0 + n_s; s++, digits += (size_t)a.dig_ss * N, own += (size_t)a.own_ss * N) {
         const uint32_t pn = a.perm[s] ? a.perm[s][n] : 0;
         const bool pm = a.perm[s] != nullptr;
         if (a.c0 && t < a.l) {
-            const ulonglong2 c = ld_pair(a.c0 + ((size_t)z * a.c0_bs + t) * N, n, pn, pm);
+            const ulonglong2 c = ld_pair(a.c0 + ((size_t)z * a.c0_bs + (size_t)s * a.c0_ss + t) * N, n, pn, pm);
             g0 = add_mod(g0, c.x, md.q), g1 = add_mod(g1, c.y, md.q);
         }
         for (uint32_t d0 = 0; d0 < a.beta; d0 += U) {
@@ -571,7 +600,7 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
             for (int i = 0; i < U; i++) {
                 x[i] = e0[i] = e1[i] = make_ulonglong2(0, 0);
                 if (d0 + i < a.beta) {
-                    x[i] = d0 + i == own_d ? ld_pair(own, n, pn, pm) : ld_pair(digits + (size_t)(d0 + i) * a.lP * N, n, pn, hoist);
+                    x[i] = d0 + i == own_d ? ld_pair(own, n, pn, pm && !a.apart) : ld_pair(digits + (size_t)(d0 + i) * a.lP * N, n, pn, hoist);
                     const uint64_t *e = a.evk[s * a.beta + d0 + i] + (size_t)pp * N + n;
                     e0[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(e));
                     e1[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(e + (size_t)lim * N));
@@ -634,7 +663,15 @@ __global__ void __launch_bounds__(256, 3) ks_inner_prod_kernel(const __grid_cons
     const uint32_t pp = t < a.l ? t : a.size_Q + (t - a.l);
     const uint32_t n = 2 * (blockIdx.x * 256 + threadIdx.x);
     const Mod md = a.mod[pp];
-    with_sum(md.q, [&](auto s) { ip_body<decltype(s)>(a, t, n, pp, md); });
+    // few terms (a digit per term, single rotations): FP64 products and one reduction cost less than pieces and their
+    // recombination - 78 FP64 instructions a coefficient against 102 and 85 of the integer pipe at three digits
+    if (a.beta <= 4 && (a.steps <= 1 || a.each)) {
+        if (md.q < FP_LIMIT) ip_body<SumFp>(a, t, n, pp, md);
+        else if (md.q < INT_LAZY_LIMIT) ip_body<SumInt30Short>(a, t, n, pp, md);
+        else ip_body<SumInt>(a, t, n, pp, md);
+    } else {
+        with_sum(md.q, [&](auto s) { ip_body<decltype(s)>(a, t, n, pp, md); });
+    }
 }
 
 }  // namespace b2

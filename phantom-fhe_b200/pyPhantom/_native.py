@@ -63,6 +63,8 @@ SIGNATURES = {
     "b2_apply_galois_accumulate": (_int, [_vp, _sz, _u32, _vp, _vp, _sz, _vp, _vp, _int, _vp, _sz, _vp]),
     "b2_apply_galois_batch": (_int, [_vp, _sz, _u32, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp]),
     "b2_rotate_add": (_int, [_vp, _sz, _u32, _vp, _vp, _sz, _vp, _vp, _sz, _vp]),
+    "b2_rotate_sum_workspace_bytes": (_sz, [_vp, _sz, _sz]),
+    "b2_rotate_sum": (_int, [_vp, _sz, _sz, _vp, _vp, _sz, _vp, _sz, _vp, _int, _vp, _sz, _vp]),
     "b2_keyswitch_finish": (_int, [_vp, _sz, _vp, _vp, _vp, _sz, _vp]),
     "b2_hoist_rotations": (_int, [_vp, _sz, _vp, _vp, _sz, _vp, _sz, _vp, _vp, _sz, _vp]),
     "b2_hoisting_sum": (_int, [_vp, _sz, _vp, _vp, _sz, _vp, _sz, _vp, _vp, _sz, _vp]),

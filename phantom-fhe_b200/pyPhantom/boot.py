@@ -29,7 +29,6 @@ C2S_LAYERS, EVAL_LEVELS, S2C_LAYERS = 3, 10, 2
 BOOT_LEVELS = C2S_LAYERS + EVAL_LEVELS + S2C_LAYERS
 K_RANGE, DOUBLE_ANGLES, COS_DEGREE = 28, 3, 63
 SCALE_UP_MARGIN_BITS = 10  # the raised message stays below q0 / 2^10
-GIANT_LANES = 3            # streams the giant steps of a linear transform are dealt over
 
 
 def _elt(step, N):
@@ -220,23 +219,27 @@ class _Layer:
         self.rescales = rescales  # primes the layer's plaintext scale spans: that many rescales end the transform
         self.baby_steps = [(b, (b * plan.unit) % plan.n) for b in plan.babies]
         chain_index = ctx.size_Q - limbs + 1
-        self.giants = []  # (rotation step, [baby position], device pointer table, plaintext tensors)
         pos = {b: i for i, (b, _) in enumerate(self.baby_steps)}
+        self.giants = []  # (rotation step, {baby position: plaintext}); the giant without rotation, if any, comes first
         for g in plan.giants:
-            pts, idx = [], []
-            for b, d in plan.terms[g]:
-                pts.append(encoder.encode_complex_vector(ctx, d * value_factor, self.scale, chain_index).data)
-                idx.append(pos[b])
-            tab = torch.tensor([p.data_ptr() for p in pts], dtype=torch.int64, device=ctx.device)
-            self.giants.append(((g * plan.n1 * plan.unit) % plan.n, idx, tab, pts))
-        # the baby rotations land in buffers owned by the layer, so the pointer tables of the fused
-        # multiply-accumulate are built once
-        self.baby_buf = ctx.empty(len(self.baby_steps), 2, limbs)
-        self.baby_tabs = [torch.tensor([self.baby_buf[i].data_ptr() for i in idx], dtype=torch.int64, device=ctx.device)
-                          for _, idx, _, _ in self.giants]
+            pts = {pos[b]: encoder.encode_complex_vector(ctx, d * value_factor, self.scale, chain_index).data for b, d in plan.terms[g]}
+            self.giants.append(((g * plan.n1 * plan.unit) % plan.n, pts))
+        self.giants.sort(key=lambda x: x[0] != 0)
+        # the baby rotations land in buffers owned by the layer, so the pointer tables of the fused multiply-accumulate (four
+        # giants a launch; null: that giant has no diagonal for that baby) are built once
+        n_b = len(self.baby_steps)
+        self.baby_buf = ctx.empty(n_b, 2, limbs)
+        self.baby_tab = torch.tensor([self.baby_buf[i].data_ptr() for i in range(n_b)], dtype=torch.int64, device=ctx.device)
+        self.groups = []
+        for g0 in range(0, len(self.giants), 4):
+            chunk = self.giants[g0: g0 + 4]
+            tab = [pts[i].data_ptr() if i in pts else 0 for _, pts in chunk for i in range(n_b)]
+            self.groups.append((g0, len(chunk), torch.tensor(tab, dtype=torch.int64, device=ctx.device)))
+        self.part_buf = ctx.empty(len(self.giants), 2, limbs)
+        self.part_tab = torch.tensor([self.part_buf[i].data_ptr() for i in range(len(self.giants))], dtype=torch.int64, device=ctx.device)
 
     def steps(self):
-        return [s for _, s in self.baby_steps if s] + [s for s, _, _, _ in self.giants if s]
+        return [s for _, s in self.baby_steps if s] + [s for s, _ in self.giants if s]
 
 
 class small_bootstrap_key:
@@ -254,14 +257,8 @@ class bootstrap_key:
         self.rot = {}     # slot rotation step -> switching key
         self.conj = None
         self.c2s, self.s2c = [], []
-        self._streams = []
         self.use_graph = True   # replay a captured CUDA graph per (input limbs, input scale) after the first call
         self._graphs = {}
-
-    def side_streams(self, n):
-        while len(self._streams) < n:
-            self._streams.append(torch.cuda.Stream())
-        return self._streams[:n]
         self.user_limbs = 0
         self.user_scale, self.up_bits, self.down_const, self.final_target = 0.0, 0, 0, 0.0
         self.eval_scale = 0.0
@@ -417,80 +414,38 @@ def mod_raise(ctx, bk, ct):
 
 
 def linear_transform(ctx, bk, ct, layer, ops):
-    """one BSGS layer: hoisted baby rotations, a fused multiply-accumulate per giant, giant rotations, one rescale
+    """one BSGS layer: hoisted baby rotations, a fused multiply-accumulate for the giants, their rotations summed, one rescale
     (src/bootstrap.cu:1201-1353 does the same with one key switch per baby)"""
     ct = ops.drop(ct, layer.limbs)
-    l, N = layer.limbs, ctx.N
+    l, N, st, n_evk = layer.limbs, ctx.N, ops.stream, ctx.beta(layer.limbs)
     steps = [(i, s) for i, (_, s) in enumerate(layer.baby_steps) if s]
     for i, (_, s) in enumerate(layer.baby_steps):
         if s == 0:
             layer.baby_buf[i].copy_(ct.data)
-    main = torch.cuda.current_stream()
-    lanes = [main] + bk.side_streams(GIANT_LANES - 1)
-    for st in lanes[1:]:
-        st.wait_stream(main)
+
+    def keys(rotations):
+        return (np.array([_elt(s, N) for s in rotations], dtype=np.uint32),
+                np.concatenate([bk.rot[s].pointer_table()[:n_evk] for s in rotations]).astype(np.uint64))
+
     if steps:
-        # the babies are independent too: each lane hoists its share (its own ModUp of c1 - cheaper than waiting
-        # for the other lanes' steps, since one lane alone leaves most of the GPU idle at these sizes)
-        n_evk = ctx.beta(l)
-        n_lanes = min(len(lanes), max(1, len(steps) // 2))
-        for k in range(n_lanes):
-            mine = steps[k::n_lanes]
-            with torch.cuda.stream(lanes[k]):
-                elts = np.array([_elt(s, N) for _, s in mine], dtype=np.uint32)
-                ksk = np.concatenate([bk.rot[s].pointer_table()[:n_evk] for _, s in mine]).astype(np.uint64)
-                outs = np.array([layer.baby_buf[i].data_ptr() for i, _ in mine], dtype=np.uint64)
-                ws, nbytes = ctx.workspace(_native.OP_HOIST, l)
-                check(LIB.b2_hoist_rotations(ctx._h, l, ct.data.data_ptr(), elts.ctypes.data, len(mine), ksk.ctypes.data, n_evk,
-                                             outs.ctypes.data, ws.data_ptr(), nbytes, _stream()))
-        for st in lanes[1:n_lanes]:   # every giant reads every baby: join, then fork again
-            main.wait_stream(st)
-        for st in lanes[1:]:
-            st.wait_stream(main)
-    # the giants are independent until the final sum: deal them round-robin over the key's streams
-    # Giants on one lane are summed anyway, so they share one ModDown: every rotation adds its Q limbs to the lane's
-    # ciphertext accumulator and its P limbs to accP, and b2_keyswitch_finish converts the P limbs once per lane.
-    capturing = torch.cuda.is_current_stream_capturing()
-    a = ctx.size_P
-    accs, plain = [None] * len(lanes), None
-    n_evk = ctx.beta(l)
-    for gi, ((step, idx, tab, _), btab) in enumerate(zip(layer.giants, layer.baby_tabs)):
-        k = gi % len(lanes)
-        with torch.cuda.stream(lanes[k]):
-            st = _stream()
-            part = ctx.empty(2, l)
-            check(LIB.b2_bsgs_mac(ctx._h, l, len(idx), tab.data_ptr(), btab.data_ptr(), part.data_ptr(), st))
-            if not step:
-                plain = (k, part)  # the giant without rotation
-                continue
-            first = accs[k] is None
-            if first:
-                accs[k] = (ctx.empty(2, l), ctx.empty(2, a), ctx.workspace(_native.OP_ROTATE, l))
-            acc, accP, (ws, nbytes) = accs[k]
-            ktab = bk.rot[step].pointer_table()
-            check(LIB.b2_apply_galois_accumulate(ctx._h, l, _elt(step, N), part.data_ptr(), ktab.ctypes.data, n_evk, acc.data_ptr(),
-                                                 accP.data_ptr(), 1 if first else 0, ws.data_ptr(), nbytes, st))
-    total = None
-    for k, lane in enumerate(lanes):
-        if accs[k] is None:
-            continue
-        acc, accP, (ws, nbytes) = accs[k]
-        with torch.cuda.stream(lane):
-            check(LIB.b2_keyswitch_finish(ctx._h, l, accP.data_ptr(), acc.data_ptr(), ws.data_ptr(), nbytes, _stream()))
-        if k:
-            main.wait_stream(lane)
-            if not capturing:
-                acc.record_stream(main)
-        piece = ct._like(acc, scale=ct._scale * layer.scale)
-        total = piece if total is None else ops.add(total, piece)
-    if plain is not None:
-        k, part = plain
-        if k:
-            main.wait_stream(lanes[k])
-            if not capturing:
-                part.record_stream(main)
-        piece = ct._like(part, scale=ct._scale * layer.scale)
-        total = piece if total is None else ops.add(total, piece)
+        elts, ksk = keys([s for _, s in steps])
+        outs = np.array([layer.baby_buf[i].data_ptr() for i, _ in steps], dtype=np.uint64)
+        ws, nbytes = ctx.workspace(_native.OP_HOIST, l)
+        check(LIB.b2_hoist_rotations(ctx._h, l, ct.data.data_ptr(), elts.ctypes.data, len(steps), ksk.ctypes.data, n_evk, outs.ctypes.data,
+                                     ws.data_ptr(), nbytes, st))
+    for g0, n, tab in layer.groups:
+        check(LIB.b2_bsgs_mac_multi(ctx._h, l, len(layer.baby_steps), n, tab.data_ptr(), layer.baby_tab.data_ptr(), layer.part_tab.data_ptr() + 8 * g0, st))
+    # the rotated giants are summed, decomposed together, with one ModDown, onto the giant without rotation
+    plain = 1 if layer.giants[0][0] == 0 else 0
+    turned = [s for s, _ in layer.giants[plain:]]
+    total = layer.part_buf[0] if plain else ctx.empty(2, l)
+    if turned:
+        elts, ksk = keys(turned)
+        nbytes = int(LIB.b2_rotate_sum_workspace_bytes(ctx._h, l, len(turned)))
+        ws = torch.empty(nbytes // 8, dtype=torch.int64, device=ctx.device)
+        check(LIB.b2_rotate_sum(ctx._h, l, len(turned), elts.ctypes.data, layer.part_buf[plain].data_ptr(), 2 * l, ksk.ctypes.data, n_evk,
+                                total.data_ptr(), 0 if plain else 1, ws.data_ptr(), nbytes, st))
+    total = ct._like(total, scale=ct._scale * layer.scale)
     for _ in range(layer.rescales):
         total = ops.rescale(total)
     return total
