@@ -535,7 +535,9 @@ __global__ void __launch_bounds__(256) expand_gather_kernel(const __grid_constan
 
 // ---- key-switch inner product (src/eval_key_switch.cu:175-230) ---------------------------------------------------------------
 // For logical limb t (physical prime pp):  acc[k][t][n] = sum_d digits[d][t][n] * evk[d][k][pp][n],  k = 0, 1.
-// Pure streaming: two coefficients per thread, 16-byte loads, three digits' loads issued before the first multiply.
+// Pure streaming: two coefficients per thread, 16-byte loads, two digits at a time so that four CTAs fit an SM (three digits and
+// three CTAs: eight hoisted rotations at N = 2^15 the same, 32 products at 2^14 724 against 707 us), the loads of the key before
+// those that wait for a permutation.
 constexpr int IP_MAX_STEPS = 16, IP_MAX_EVK = 256;
 struct IpArgs {
     const uint64_t *digits;
@@ -574,7 +576,7 @@ __device__ __forceinline__ ulonglong2 ld_pair(const uint64_t *p, uint32_t n, uin
 
 template <class S>
 __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n, uint32_t pp, const Mod &md) {
-    constexpr int U = 3;
+    constexpr int U = 2;
     const size_t N = (size_t)1 << a.logN;
     const uint32_t z = blockIdx.z, lim = a.size_QP;
     const typename S::K k = S::make(md);
@@ -588,23 +590,29 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
     uint64_t g0 = 0, g1 = 0;  // permuted c0
     int pending = 0;
     for (uint32_t s = s0; s < s0 + n_s; s++, digits += (size_t)a.dig_ss * N, own += (size_t)a.own_ss * N) {
-        const uint32_t pn = a.perm[s] ? a.perm[s][n] : 0;
         const bool pm = a.perm[s] != nullptr;
-        if (a.c0 && t < a.l) {
-            const ulonglong2 c = ld_pair(a.c0 + ((size_t)z * a.c0_bs + (size_t)s * a.c0_ss + t) * N, n, pn, pm);
-            g0 = add_mod(g0, c.x, md.q), g1 = add_mod(g1, c.y, md.q);
-        }
+        const uint32_t pn = pm ? a.perm[s][n] : 0;
         for (uint32_t d0 = 0; d0 < a.beta; d0 += U) {
+            // the key's loads go first: they do not wait for the permutation
             ulonglong2 x[U], e0[U], e1[U];
 #pragma unroll
             for (int i = 0; i < U; i++) {
-                x[i] = e0[i] = e1[i] = make_ulonglong2(0, 0);
+                e0[i] = e1[i] = make_ulonglong2(0, 0);
                 if (d0 + i < a.beta) {
-                    x[i] = d0 + i == own_d ? ld_pair(own, n, pn, pm && !a.apart) : ld_pair(digits + (size_t)(d0 + i) * a.lP * N, n, pn, hoist);
                     const uint64_t *e = a.evk[s * a.beta + d0 + i] + (size_t)pp * N + n;
                     e0[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(e));
                     e1[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(e + (size_t)lim * N));
                 }
+            }
+#pragma unroll
+            for (int i = 0; i < U; i++) {
+                x[i] = make_ulonglong2(0, 0);
+                if (d0 + i < a.beta)
+                    x[i] = d0 + i == own_d ? ld_pair(own, n, pn, pm && !a.apart) : ld_pair(digits + (size_t)(d0 + i) * a.lP * N, n, pn, hoist);
+            }
+            if (d0 == 0 && a.c0 && t < a.l) {
+                const ulonglong2 c = ld_pair(a.c0 + ((size_t)z * a.c0_bs + (size_t)s * a.c0_ss + t) * N, n, pn, pm);
+                g0 = add_mod(g0, c.x, md.q), g1 = add_mod(g1, c.y, md.q);
             }
             if (pending + U > S::FLUSH) {
 #pragma unroll
@@ -656,7 +664,7 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
     *reinterpret_cast<ulonglong2 *>(o1) = make_ulonglong2(r[2], r[3]);
 }
 
-__global__ void __launch_bounds__(256, 3) ks_inner_prod_kernel(const __grid_constant__ IpArgs a) {
+__global__ void __launch_bounds__(256, 4) ks_inner_prod_kernel(const __grid_constant__ IpArgs a) {
     pdl_enter();
     // the limbs of the special primes (the longer arithmetic) first
     const uint32_t y = blockIdx.y, t = y < a.np ? a.l + a.p0 + y : a.q0 + (y - a.np);
