@@ -177,3 +177,73 @@ def test_product_with_diagonals_outside_pinned_memory():
         p.coeffs = p.coeffs.clone()
     assert not plain.diagonals[0].coeffs.is_pinned()
     assert torch.equal(ph.bsgs_matmul_preencoded(ctx, glk, x, pinned).data, ph.bsgs_matmul_preencoded(ctx, glk, x, plain).data)
+
+
+@pytest.mark.parametrize("log_n,bits,special,l,n", [
+    (12, [60, 40, 50, 45, 60], 1, 3, 19),                  # more ciphertexts than one launch takes, the elements repeat
+    (14, [60, 40, 36, 50, 40, 60, 59], 2, 5, 3),
+    (15, [60, 40, 40, 60, 60], 2, 3, 1),
+])
+def test_sum_of_rotated_ciphertexts(log_n, bits, special, l, n):
+    """b2_rotate_sum, alone and on top of a sum, against the oracle's stages: inner products added, one ModDown"""
+    from pyPhantom._native import LIB, check
+    N, n_elt = 1 << log_n, 3
+    elts = [ph.get_elt_from_step(s, N) for s in range(1, n_elt + 1)]
+    ctx, o = make_ctx(N, bits, special, elts)
+    keys = [o.synth_key(o.beta(l), 8, 10 + 40 * i) for i in range(n_elt)]
+    rks = [ph.relin_key.from_numpy(ctx, k) for k in keys]
+    cts = [o.synth_ct(l, 8, 200 + i) for i in range(n)]
+    q = np.concatenate([o.primes[:l], o.primes[-special:]])[None, :, None]
+    add = lambda x, y, m: (x + y) % m                      # residues are below 2^61
+    cx, c0 = 0, 0
+    for i, ct in enumerate(cts):
+        turned = ct[:, :, o.galois_perm(elts[i % n_elt])]
+        cx = add(o.ks_inner_prod(l, o.modup(l, turned[1]), keys[i % n_elt]), cx, q)
+        c0 = add(turned[0], c0, q[0, :l])
+    want = np.stack([o.moddown(l, cx[k]) for k in range(2)])
+    want[0] = add(want[0], c0, q[0, :l])
+    src = torch.zeros(n, 2 * l + 1, N, dtype=torch.int64, device="cuda")
+    for i, c in enumerate(cts):
+        src[i, : 2 * l] = dev(c).reshape(2 * l, N)
+    tab = np.concatenate([rks[i % n_elt].pointer_table() for i in range(n)])
+    e = np.array([elts[i % n_elt] for i in range(n)], dtype=np.uint32)
+    nb = int(LIB.b2_rotate_sum_workspace_bytes(ctx._h, l, n))
+    ws, before = torch.empty(nb // 8, dtype=torch.int64, device="cuda"), o.synth_ct(l, 8, 900)
+    for first, sum_ in ((1, want), (0, add(want, before, q[:, :l]))):
+        acc = dev(before)
+        check(LIB.b2_rotate_sum(ctx._h, l, n, e.ctypes.data, src.data_ptr(), 2 * l + 1, tab.ctypes.data, len(tab) // n, acc.data_ptr(), first,
+                                ws.data_ptr(), nb, torch.cuda.current_stream().cuda_stream))
+        assert np.array_equal(host(acc), sum_)
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("log_n,products,sets,dbl", [(12, 16, 1, 0), (14, 3, 2, 1), (16, 1, 2, 1)])
+def test_independent_products_in_one_call(log_n, products, sets, dbl):
+    """b2_multiply_relin_rescale_many with operands above the level, and b2_rescale_rounded_batch"""
+    from pyPhantom._native import LIB, check
+    N, l = 1 << log_n, 3
+    ctx, o = make_ctx(N, [60, 40, 50, 40, 40, 60, 60], 2)
+    key = o.synth_key(o.beta(l), 9, 10)
+    tab, s = ph.relin_key.from_numpy(ctx, key).pointer_table(), torch.cuda.current_stream().cuda_stream
+    la, lb = [l + p % 3 for p in range(products)], [l + (p + 1) % 2 for p in range(products)]
+    a = [[o.synth_ct(la[p], 9, 50 + 8 * p + i) for i in range(sets)] for p in range(products)]
+    b = [[o.synth_ct(lb[p], 9, 250 + 8 * p + i) for i in range(sets)] for p in range(products)]
+    da, db = [dev(np.stack(x)) for x in a], [dev(np.stack(x)) for x in b]
+    pa, pb = (np.array([t.data_ptr() for t in d], dtype=np.uint64) for d in (da, db))
+    na, nb = np.array(la, dtype=np.uint32), np.array(lb, dtype=np.uint32)
+    n_ws = int(LIB.b2_multiply_relin_batch_workspace_bytes(ctx._h, l, products * sets))
+    ws = torch.empty(n_ws // 8, dtype=torch.int64, device="cuda")
+    out = torch.empty(products, sets, 2, l - 1, N, dtype=torch.int64, device="cuda")
+    check(LIB.b2_multiply_relin_rescale_many(ctx._h, l, products, sets, pa.ctypes.data, na.ctypes.data, pb.ctypes.data, nb.ctypes.data, dbl,
+                                             tab.ctypes.data, len(tab), out.data_ptr(), ws.data_ptr(), n_ws, s))
+    q, got = o.primes[:l][None, :, None], host(out)
+    for p in range(products):
+        for i in range(sets):
+            ab = o.multiply_and_relin(l, a[p][i][:, :l], b[p][i][:, :l], key)
+            assert np.array_equal(got[p, i], o.rescale_rounded(l, ab * np.uint64(2) % q if dbl else ab)), (p, i)
+    stack = np.stack([o.synth_ct(l, 9, 700 + i) for i in range(sets)])
+    res, d = torch.empty(sets, 2, l - 1, N, dtype=torch.int64, device="cuda"), dev(stack)
+    check(LIB.b2_rescale_rounded_batch(ctx._h, l, sets, d.data_ptr(), res.data_ptr(), ws.data_ptr(), n_ws, s))
+    for i in range(sets):
+        assert np.array_equal(host(res)[i], o.rescale_rounded(l, stack[i]))
+    assert ctx.device_status() == 0
