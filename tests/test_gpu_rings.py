@@ -224,7 +224,8 @@ def test_independent_products_in_one_call(log_n, products, sets, dbl):
     N, l = 1 << log_n, 3
     ctx, o = make_ctx(N, [60, 40, 50, 40, 40, 60, 60], 2)
     key = o.synth_key(o.beta(l), 9, 10)
-    tab, s = ph.relin_key.from_numpy(ctx, key).pointer_table(), torch.cuda.current_stream().cuda_stream
+    rk = ph.relin_key.from_numpy(ctx, key)
+    tab, s = rk.pointer_table(), torch.cuda.current_stream().cuda_stream
     la, lb = [l + p % 3 for p in range(products)], [l + (p + 1) % 2 for p in range(products)]
     a = [[o.synth_ct(la[p], 9, 50 + 8 * p + i) for i in range(sets)] for p in range(products)]
     b = [[o.synth_ct(lb[p], 9, 250 + 8 * p + i) for i in range(sets)] for p in range(products)]
@@ -239,8 +240,9 @@ def test_independent_products_in_one_call(log_n, products, sets, dbl):
     q, got = o.primes[:l][None, :, None], host(out)
     for p in range(products):
         for i in range(sets):
-            ab = o.multiply_and_relin(l, a[p][i][:, :l], b[p][i][:, :l], key)
-            assert np.array_equal(got[p, i], o.rescale_rounded(l, ab * np.uint64(2) % q if dbl else ab)), (p, i)
+            t = o.tensor_mul(l, a[p][i][:, :l], b[p][i][:, :l])
+            t = t * np.uint64(2) % q if dbl else t
+            assert np.array_equal(got[p, i], o.rescale_rounded(l, o.keyswitch(l, t[2], key, t[:2]))), (p, i)
     stack = np.stack([o.synth_ct(l, 9, 700 + i) for i in range(sets)])
     res, d = torch.empty(sets, 2, l - 1, N, dtype=torch.int64, device="cuda"), dev(stack)
     check(LIB.b2_rescale_rounded_batch(ctx._h, l, sets, d.data_ptr(), res.data_ptr(), ws.data_ptr(), n_ws, s))
