@@ -2355,20 +2355,20 @@ extern "C" int b2_expand_single_chain_batch(b2_ctx *c, size_t l, size_t M, const
     return run_fwd(c, d_out, d_out, nullptr, (uint32_t)(M * l), 0, EpiStore{}, s, (uint32_t)l);
 }
 
-extern "C" int b2_expand_gather(b2_ctx *c, size_t l, size_t M, const int64_t *const *srcs, uint64_t *d_out, void *stream) {
+extern "C" int b2_gather_vectors(b2_ctx *c, size_t M, const int64_t *const *srcs, int64_t *d_out, void *stream) {
     CHECK_CTX(c);
-    CHECK_LEVEL(c, l);
-    if (!srcs || !d_out || M == 0) return fail(B2_EINVAL, "expand_gather: bad argument");
+    if (!srcs || !d_out || M == 0) return fail(B2_EINVAL, "gather_vectors: bad argument");
+    if ((uintptr_t)d_out & 15) return fail(B2_EINVAL, "gather_vectors: the result must be 16-byte aligned");
     for (size_t m0 = 0; m0 < M; m0 += GATHER_MAX) {
         const size_t n = std::min<size_t>(GATHER_MAX, M - m0);
         GatherPtrs g{};
         for (size_t i = 0; i < n; i++) {
-            if (!srcs[m0 + i] || ((uintptr_t)srcs[m0 + i] & 15)) return fail(B2_EINVAL, "expand_gather: vectors must be there and 16-byte aligned");
-            g.p[i] = srcs[m0 + i];
+            if (!srcs[m0 + i] || ((uintptr_t)srcs[m0 + i] & 15)) return fail(B2_EINVAL, "gather_vectors: vectors must be there and 16-byte aligned");
+            g.p[i] = (const ulonglong2 *)srcs[m0 + i];
         }
-        LaunchScope ls(c, (cudaStream_t)stream, "expand_signed");
-        launch_k(expand_gather_kernel, GATHER_CTAS, 256, 0, (cudaStream_t)stream, g, d_out + m0 * l * c->N, c->d_mod, (uint32_t)c->logN, (uint32_t)l, (uint32_t)n);
-        LAUNCH_CHECK("expand_gather_kernel");
+        LaunchScope ls(c, (cudaStream_t)stream, "gather_vectors");
+        launch_k(gather_vectors_kernel, GATHER_CTAS, GATHER_THREADS, 0, (cudaStream_t)stream, g, (ulonglong2 *)(d_out + m0 * c->N), (uint32_t)c->logN, (uint32_t)n);
+        LAUNCH_CHECK("gather_vectors_kernel");
     }
     return B2_OK;
 }

@@ -507,28 +507,30 @@ __global__ void __launch_bounds__(256) expand_signed_kernel(const int64_t *__res
     stv<V>(dst + ((size_t)blockIdx.z * l + blockIdx.y) * N + i, x);
 }
 
-// The same from M separate vectors that the device can read where they are (pinned host memory): every coefficient crosses
-// the link once and becomes its l residues in registers. A launch of GATHER_CTAS CTAs keeps a few hundred kilobytes of reads
-// in flight, which is what the link takes, and leaves the SMs to the kernels of other streams. (256 copies of 128 KB took 6.4
+// M separate vectors that the device can read where they are (pinned host memory) -> one array. One CTA with as many loads in
+// flight as the link needs, 112 KB: reads over the link beyond that only queue, and everything else that the GPU loads queues
+// behind them. 8 MB take 167 us (50 GB/s) with 96 KB to 400 KB in flight on 2 to 96 CTAs, but a transform of 384 limbs of 2^14
+// beside them 35 + 42 us with 96 KB, 60 + 65 with 400 KB, 120 + 125 with 800 KB; alone 26 + 32. (256 copies of 128 KB took 6.4
 // us each, a quarter of the link's rate, plus a host call each.)
-constexpr int GATHER_MAX = 128, GATHER_CTAS = 96;
+constexpr int GATHER_MAX = 128, GATHER_U = 7, GATHER_CTAS = 1, GATHER_THREADS = 1024;
 struct GatherPtrs {
-    const int64_t *p[GATHER_MAX];
+    const ulonglong2 *p[GATHER_MAX];
 };
-__global__ void __launch_bounds__(256) expand_gather_kernel(const __grid_constant__ GatherPtrs src, uint64_t *__restrict__ dst, const Mod *mod, uint32_t logN,
-                                                            uint32_t l, uint32_t M) {
+__global__ void __launch_bounds__(GATHER_THREADS) gather_vectors_kernel(const __grid_constant__ GatherPtrs src, ulonglong2 *__restrict__ dst, uint32_t logN,
+                                                                       uint32_t M) {
     pdl_enter();
-    const uint32_t per = 1u << (logN - 1);  // pairs of coefficients in a vector
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < M * per; i += gridDim.x * 256) {
-        const uint32_t m = i >> (logN - 1), k = 2 * (i & (per - 1));
-        const longlong2 c = *reinterpret_cast<const longlong2 *>(src.p[m] + k);
-        const uint64_t ax = c.x >= 0 ? (uint64_t)c.x : (uint64_t)0 - (uint64_t)c.x, ay = c.y >= 0 ? (uint64_t)c.y : (uint64_t)0 - (uint64_t)c.y;
-        uint64_t *d = dst + (((size_t)m * l) << logN) + k;
-        for (uint32_t j = 0; j < l; j++) {
-            const Mod md = mod[j];
-            const uint64_t rx = barrett64(ax, md.q, md.r1), ry = barrett64(ay, md.q, md.r1);
-            *reinterpret_cast<ulonglong2 *>(d + ((size_t)j << logN)) =
-                make_ulonglong2(c.x >= 0 || rx == 0 ? rx : md.q - rx, c.y >= 0 || ry == 0 ? ry : md.q - ry);
+    const uint32_t log_per = logN - 1, total = M << log_per, mask = (1u << log_per) - 1;  // pairs; at least 2048 in a vector
+    for (uint32_t i = blockIdx.x * (GATHER_THREADS * GATHER_U) + threadIdx.x; i < total; i += gridDim.x * (GATHER_THREADS * GATHER_U)) {
+        ulonglong2 x[GATHER_U];
+#pragma unroll
+        for (int u = 0; u < GATHER_U; u++) {
+            const uint32_t k = i + u * GATHER_THREADS;
+            if (k < total) x[u] = __ldcs(src.p[k >> log_per] + (k & mask));
+        }
+#pragma unroll
+        for (int u = 0; u < GATHER_U; u++) {
+            const uint32_t k = i + u * GATHER_THREADS;
+            if (k < total) dst[k] = x[u];
         }
     }
 }

@@ -132,6 +132,8 @@ class context:
             raise RuntimeError("pyPhantom needs a CUDA device: there is no CPU path")
         self.device = torch.cuda.current_device()
         self.N = parms._N
+        # of the matrix products: one set, so that what they allocate on them is cached once
+        self.side_streams = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream(priority=-1), torch.cuda.Stream(priority=-1)
         self.primes = np.array([m.value() for m in parms._coeff_modulus], dtype=np.uint64)
         self.primes_signed = self.primes.view(np.int64)
         self.size_QP = len(self.primes)
@@ -814,6 +816,7 @@ class single_chain_plaintext:
         # what the device reads in place: the address of a pinned (or device) vector, else 0
         ok = t is not None and (t.is_cuda or t.is_pinned()) and t.is_contiguous() and t.dtype == torch.int64 and t.data_ptr() % 16 == 0
         self._readable = t.data_ptr() if ok else 0
+        self._numel = -1 if t is None else t.numel()
 
     def coeffs_bytes(self):
         return self.coeffs.numpy().tobytes()
@@ -997,10 +1000,10 @@ def compute_bsgs_babies(ctx, galois_key_, x, baby_steps):
 
 def _pointer_table(first, stride_words, count, device):
     """device array of pointers at a constant distance, made on the device (no copy from the host to wait for)"""
-    return torch.arange(count, dtype=torch.int64, device=device).mul_(8 * stride_words).add_(first)
+    return torch.arange(first, first + 8 * stride_words * count, 8 * stride_words, dtype=torch.int64, device=device)
 
 
-_GIANT_POOL_BYTES = 1 << 28  # expanded plaintexts of the giants that share a launch
+_GIANT_POOL_BYTES = 1 << 28  # expanded plaintexts of the giants that share a launch; diagonals read ahead
 
 
 def bsgs_apply_giants_with_babies(ctx, galois_key_, babies, diags):
@@ -1014,19 +1017,20 @@ def bsgs_apply_giants_with_babies(ctx, galois_key_, babies, diags):
 def _bsgs_product(ctx, galois_key_, x, babies, diags):
     """The product of the two drivers; `babies` None: they are computed here, while the first diagonals are on their way.
 
-    Three streams: one reads the diagonals out of pinned host memory and makes their residues, one transforms them and
-    multiplies (up to four giants per launch, every baby read once for them), and the caller's runs the chain of
-    rotations, each of which lands on top of the next partial sum. Bound by the reads (8 N bytes per diagonal) or by the
-    chain of G - 1 dependent key switches, whichever is longer."""
+    Four streams beside the caller's: one reads the diagonals out of pinned host memory, up to 256 MB ahead; one makes their
+    residues and transforms them; and two of a higher priority, whose kernels the next rotation waits for, multiply (up to
+    four giants per launch, every baby read once for them) and rotate: the babies, then the chain of giants, each of which
+    lands on top of the next partial sum. Bound by the reads (8 N bytes per diagonal) or by the chain of G - 1 dependent key
+    switches, whichever is longer. 256 diagonals at N = 2^14, 6 limbs, 16 babies: 2140 us with the first two on one stream, two
+    buffers and 384 KB of reads in flight, 1790 us so."""
     M, G = diags.baby_steps, diags.giant_steps
     if M == 0 or G == 0 or M * G != diags.d_pad:
         raise ValueError("bsgs_apply_giants_with_babies: M*G must equal d_pad")
     if len(diags.diagonals) != diags.d_pad:
         raise ValueError("bsgs_apply_giants_with_babies: diagonals size mismatch")
     l, N, dev = x._limbs, ctx.N, ctx.device
-    for scp in diags.diagonals:
-        if scp.coeffs.numel() != N:
-            raise ValueError("bsgs_apply_giants_with_babies: scp coeff length != N")
+    if any([scp._numel != N for scp in diags.diagonals]):
+        raise ValueError("bsgs_apply_giants_with_babies: scp coeff length != N")
     scale = x._scale * diags.diagonals[(G - 1) * M].scale
     for g in range(G - 1):
         if not _are_close(scale, x._scale * diags.diagonals[g * M].scale):
@@ -1040,59 +1044,79 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
     per = max(1, min(4, G, _GIANT_POOL_BYTES // (M * l * N * 8)))
     groups = [list(range(max(0, hi - per), hi)) for hi in range(G, 0, -per)]
     main = torch.cuda.current_stream()
-    read, work = torch.cuda.Stream(), torch.cuda.Stream()
-    pools = [ctx.empty(per * M, l) for _ in range(2)]
-    read.wait_stream(main)
-    staged = []
-    expanded, consumed = [torch.cuda.Event() for _ in range(2)], [torch.cuda.Event() for _ in range(2)]
+    read, transform, work, chain = ctx.side_streams
+    if tab is None:  # the chain is made of public operations on the caller's stream
+        chain = main
+    n_stages = max(2, min(len(groups), _GIANT_POOL_BYTES // (per * M * N * 8)))
+    n_pools = min(2, len(groups))
+    stage, stage_words = torch.empty(n_stages * per * M, N, dtype=torch.int64, device=dev), per * M * N
+    pool, pool_words = ctx.empty(n_pools * per * M, l), per * M * l * N
+    parts = ctx.empty(G, 2, l)
+    ws, nbytes = ctx.workspace(_native.OP_KEYSWITCH, l)
+    for side in (read, transform, work, chain):
+        side.wait_stream(main)
+    readable = np.array([scp._readable for scp in diags.diagonals], dtype=np.uint64)
+    arrived, transformed, consumed = ([torch.cuda.Event() for _ in groups] for _ in range(3))
 
     def fetch(i):
         if i >= len(groups):
             return
-        gs, slot = groups[i], i & 1
-        if i >= 2:
-            read.wait_event(consumed[slot])
-        scps = diags.diagonals[gs[0] * M: (gs[-1] + 1) * M]
-        ptrs = np.array([s._readable for s in scps], dtype=np.uint64)
-        if not ptrs.all():  # vectors the device cannot read in place are copied first
+        slot, which = i % n_stages, slice(groups[i][0] * M, (groups[i][-1] + 1) * M)
+        if i >= n_stages:
+            read.wait_event(transformed[i - n_stages])
+        ptrs = readable[which]
+        if ptrs.all():
+            check(LIB.b2_gather_vectors(ctx._h, len(ptrs), ptrs.ctypes.data, stage.data_ptr() + 8 * slot * stage_words, read.cuda_stream))
+        else:  # vectors the device cannot read in place are copied
             with torch.cuda.stream(read):
-                stage = torch.stack([s.coeffs.to(dev, non_blocking=True) for s in scps])
-            staged.append(stage)
-            ptrs = np.array([stage[k].data_ptr() for k in range(len(scps))], dtype=np.uint64)
-        check(LIB.b2_expand_gather(ctx._h, l, len(scps), ptrs.ctypes.data, pools[slot].data_ptr(), read.cuda_stream))
-        expanded[slot].record(read)
+                for k, scp in enumerate(diags.diagonals[which]):
+                    stage[slot * per * M + k].copy_(scp.coeffs, non_blocking=True)
+        arrived[i].record(read)
 
-    fetch(0)
-    fetch(1)
-    if babies is None:
-        babies = compute_bsgs_babies(ctx, galois_key_, x, M)
-    parts = ctx.empty(G, 2, l)
-    pt_tabs = [_pointer_table(p.data_ptr(), l * N, per * M, dev) for p in pools]
-    part_tab = _pointer_table(parts.data_ptr(), 2 * l * N, G, dev)
-    ptrs = [c.data.data_ptr() for c in babies]
-    step = ptrs[1] - ptrs[0] if M > 1 else 8
-    if step > 0 and all(p == ptrs[0] + i * step for i, p in enumerate(ptrs)):
-        baby_tab = _pointer_table(ptrs[0], step // 8, M, dev)
-    else:
-        baby_tab = torch.tensor(ptrs, dtype=torch.int64, device=dev)
-    work.wait_stream(main)
+    def expand(i):
+        if i >= len(groups):
+            return
+        if i >= n_pools:
+            transform.wait_event(consumed[i - n_pools])
+        transform.wait_event(arrived[i])
+        check(LIB.b2_expand_single_chain_batch(ctx._h, l, len(groups[i]) * M, stage.data_ptr() + 8 * (i % n_stages) * stage_words,
+                                               pool.data_ptr() + 8 * (i % n_pools) * pool_words, transform.cuda_stream))
+        transformed[i].record(transform)
+
+    fetch(0)  # on its way while the host launches the babies
+    with torch.cuda.stream(chain):
+        if babies is None:
+            babies = compute_bsgs_babies(ctx, galois_key_, x, M)
+        pt_tab = _pointer_table(pool.data_ptr(), l * N, n_pools * per * M, dev)
+        part_tab = _pointer_table(parts.data_ptr(), 2 * l * N, G, dev)
+        ptrs = [c.data.data_ptr() for c in babies]
+        step = ptrs[1] - ptrs[0] if M > 1 else 8
+        if step > 0 and all(p == ptrs[0] + i * step for i, p in enumerate(ptrs)):
+            baby_tab = _pointer_table(ptrs[0], step // 8, M, dev)
+        else:
+            baby_tab = torch.tensor(ptrs, dtype=torch.int64, device=dev)
+    ready = torch.cuda.Event()
+    ready.record(chain)
+    for i in range(1, n_stages):
+        fetch(i)
+    for i in range(n_pools):
+        expand(i)
+    work.wait_event(ready)
     done = {}
     for i, gs in enumerate(groups):
-        slot = i & 1
-        work.wait_event(expanded[slot])
-        check(LIB.b2_ntt_forward_batch(ctx._h, pools[slot].data_ptr(), l, len(gs) * M, work.cuda_stream))
-        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, len(gs), pt_tabs[slot].data_ptr(), baby_tab.data_ptr(),
+        slot = i % n_pools
+        work.wait_event(transformed[i])
+        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, len(gs), pt_tab.data_ptr() + 8 * slot * per * M, baby_tab.data_ptr(),
                                     part_tab.data_ptr() + 8 * gs[0], work.cuda_stream))
-        consumed[slot].record(work)
-        done[gs[-1]] = torch.cuda.Event()
-        done[gs[-1]].record(work)
-        fetch(i + 2)
-    ws, nbytes = ctx.workspace(_native.OP_KEYSWITCH, l)
-    st = main.cuda_stream
+        consumed[i].record(work)
+        done[gs[-1]] = consumed[i]
+        fetch(i + n_stages)
+        expand(i + n_pools)
+    st = chain.cuda_stream
     acc = None
     for g in range(G - 1, -1, -1):
         if g in done:
-            main.wait_event(done[g])
+            chain.wait_event(done[g])
         part = x._like(parts[g], scale=scale)
         if acc is None:
             acc = part
@@ -1101,8 +1125,7 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
             acc = part
         else:
             acc = add(ctx, rotate(ctx, acc, M, galois_key_), part)
-    main.wait_stream(read)
-    main.wait_stream(work)
+    main.wait_stream(chain)
     acc = rescale_to_next(ctx, acc)
     acc.set_scale(x._scale)
     return acc
