@@ -626,7 +626,7 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
         uint64_t r0 = (uint64_t)((rem << 64) / q);
         // floor(2^(62 + n) / q) for q of n bits: 62 + n <= 123, so the numerator fits
         const uint64_t mu = (uint64_t)(((u128_t)1 << (62 + 64 - __builtin_clzll(q))) / q);
-        mods[l] = Mod{q, r0, r1, mu};
+        mods[l] = Mod{q, r0, r1, mu, 1.0 / (double)q};
     }
     // ---- P-related constants (src/rns.cu:100-138, 192-194) ----
     const size_t sQ = c->size_Q, sP = size_P;

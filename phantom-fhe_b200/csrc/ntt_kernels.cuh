@@ -26,6 +26,7 @@ namespace b2 {
 struct Mod {
     uint64_t q, r0, r1;  // r = floor(2^128 / q)
     uint64_t mu;         // floor(2^(62 + n) / q), n = bit length of q
+    double qinv;         // 1 / q
 };
 
 // One job = one limb transform: where the limb lives and which prime's tables it uses.
@@ -88,6 +89,17 @@ __device__ __forceinline__ u64x4 ld256(const uint64_t *p) {
 }
 __device__ __forceinline__ void st256(uint64_t *p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
     asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+}
+
+// one table entry, or two at a 32-byte boundary
+template <int CNT>
+__device__ __forceinline__ void ld_pairs(W2 (&w)[CNT], const W2 *p) {
+    if constexpr (CNT == 1) {
+        w[0] = ldg_w2(p);
+    } else {
+        const u64x4 v = ld256(reinterpret_cast<const uint64_t *>(p));
+        w[0] = W2{v.a, v.b}, w[1] = W2{v.c, v.d};
+    }
 }
 
 // ---- epilogues of the last forward (row) pass ---------------------------------------------------
@@ -236,7 +248,10 @@ struct ArithIntLazy {
         const uint32_t s = __clz((uint32_t)md.r1);  // r1 = floor(2^64 / q), in [2^4, 2^14]
         return K{md.q, 0 - md.q, (uint32_t)((md.r1 << s) | (md.r0 >> (64 - s))), s};
     }
-    __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &) { return ldg_w2(tw + idx); }
+    using TwRaw = W2;
+    static constexpr int TW_RUN = 2;  // twiddles in 32 bytes
+    template <int CNT> __device__ __forceinline__ static void ldtws(TwRaw (&w)[CNT], const W2 *tw, size_t idx) { ld_pairs(w, tw + idx); }
+    __device__ __forceinline__ static Tw twiddle(TwRaw w, const K &) { return w; }
     __device__ __forceinline__ static Tw ldfin(const W2 *p, const K &) { return ldg_w2(p); }
     __device__ __forceinline__ static T from_u64(uint64_t v, const K &) { return v; }
     __device__ __forceinline__ static T from_raw(uint64_t v) { return v; }
@@ -301,7 +316,10 @@ struct ArithInt {
     };
     static constexpr int B_CANON = 0, B_PASS = 0, GS_PASS = 0, B_BCONV = 0;
     __device__ __forceinline__ static K make(const Mod &md, int) { return K{md.q, 2 * md.q}; }
-    __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &) { return ldg_w2(tw + idx); }
+    using TwRaw = W2;
+    static constexpr int TW_RUN = 2;  // twiddles in 32 bytes
+    template <int CNT> __device__ __forceinline__ static void ldtws(TwRaw (&w)[CNT], const W2 *tw, size_t idx) { ld_pairs(w, tw + idx); }
+    __device__ __forceinline__ static Tw twiddle(TwRaw w, const K &) { return w; }
     __device__ __forceinline__ static Tw ldfin(const W2 *p, const K &) { return ldg_w2(p); }
     __device__ __forceinline__ static T from_u64(uint64_t v, const K &) { return v; }
     __device__ __forceinline__ static T from_raw(uint64_t v) { return v; }
@@ -346,17 +364,28 @@ struct ArithFp {
     __host__ __device__ static constexpr int prod(int B) { return 9 + (B + 3) / 4; }
     // table entry i of an FP64 prime is one double (8 bytes); w / q is rebuilt as w * (1/q), whose
     // relative error of 2^-52 is inside the slack of the quotient estimate
-    __device__ __forceinline__ static Tw ldtw(const W2 *tw, size_t idx, const K &k) {
-        const double w = __ldg(reinterpret_cast<const double *>(tw) + idx);
-        return Tw{w, __dmul_rn(w, k.qinv)};
+    using TwRaw = double;
+    static constexpr int TW_RUN = 4;  // twiddles in 32 bytes
+    template <int CNT> __device__ __forceinline__ static void ldtws(TwRaw (&w)[CNT], const W2 *tw, size_t idx) {
+        const double *p = reinterpret_cast<const double *>(tw) + idx;
+        if constexpr (CNT == 1) {
+            w[0] = __ldg(p);
+        } else if constexpr (CNT == 2) {
+            const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+            w[0] = v.x, w[1] = v.y;
+        } else {
+            const u64x4 v = ld256(reinterpret_cast<const uint64_t *>(p));
+            w[0] = from_raw(v.a), w[1] = from_raw(v.b), w[2] = from_raw(v.c), w[3] = from_raw(v.d);
+        }
     }
+    __device__ __forceinline__ static Tw twiddle(TwRaw w, const K &k) { return Tw{w, __dmul_rn(w, k.qinv)}; }
     __device__ __forceinline__ static Tw ldfin(const W2 *p, const K &) {
         const W2 v = ldg_w2(p);
         return Tw{__longlong_as_double((long long)v.w), __longlong_as_double((long long)v.ws)};
     }
     __device__ __forceinline__ static K make(const Mod &md, int) {
         const double q = (double)md.q;
-        return K{q, 1.0 / q};
+        return K{q, md.qinv};
     }
     __device__ __forceinline__ static T from_u64(uint64_t v, const K &) {
         return __dsub_rn(__longlong_as_double((long long)(v | 0x4330000000000000ull)), FP_2_52);
@@ -431,18 +460,24 @@ __device__ __forceinline__ void with_arith(uint64_t q, F &&f) {
 
 // ---- stage runners: compile-time recursion keeps every register index a constant --------------
 // forward: E residues x[] bounded by B, local stages S..R-1 of this stage group; twiddle index
-// (P << (shift + S)) + (k0 << S) + g.
-template <class A, int S, int R, int E, int B>
+// (P << (shift + S)) + (k0 << S) + g. The 2^S twiddles of a stage are one aligned run, read 32 bytes at a time: in the row passes,
+// which read one per residue, the loads of single entries were a third of the LSU's work (with 1 / q from the table of primes
+// instead of a division in every thread: 32 products at 2^14 710 -> 691 us, eight hoisted rotations at 2^15 255 -> 248 us).
+// (MAX_RUN 1: one by one, for kernels without the registers for more)
+template <class A, int S, int R, int E, int B, int MAX_RUN = A::TW_RUN>
 __device__ __forceinline__ void ct_stages(typename A::T (&x)[E], const W2 *tw, size_t P, int shift, size_t k0, const typename A::K &k) {
     if constexpr (S < R) {
         constexpr int half = E >> (S + 1);
+        constexpr int RUN = (1 << S) < MAX_RUN ? (1 << S) : MAX_RUN;
+        typename A::TwRaw ws[RUN];
 #pragma unroll
         for (int g = 0; g < (1 << S); g++) {
-            const typename A::Tw w = A::ldtw(tw, (P << (shift + S)) + (k0 << S) + g, k);
+            if (g % RUN == 0) A::ldtws(ws, tw, (P << (shift + S)) + (k0 << S) + g);
+            const typename A::Tw w = A::twiddle(ws[g % RUN], k);
 #pragma unroll
             for (int j = 0; j < half; j++) A::template ct<B>(x[g * 2 * half + j], x[g * 2 * half + j + half], w, k);
         }
-        ct_stages<A, S + 1, R, E, A::ct_out(B)>(x, tw, P, shift, k0, k);
+        ct_stages<A, S + 1, R, E, A::ct_out(B), MAX_RUN>(x, tw, P, shift, k0, k);
     }
 }
 // bound after R forward stages
@@ -485,9 +520,12 @@ __device__ __forceinline__ void gs_stages(typename A::T (&x)[E], const W2 *tw, s
     if constexpr (U < R) {
         constexpr int gap = 1 << U;
         constexpr GsBounds<E> bd = gs_bounds<A, E>(B, U);
+        constexpr int RUN = (E >> (U + 1)) < A::TW_RUN ? (E >> (U + 1)) : A::TW_RUN;
+        typename A::TwRaw ws[RUN];
 #pragma unroll
         for (int g = 0; g < (E >> (U + 1)); g++) {
-            const typename A::Tw w = A::ldtw(tw, (size_t)(m0 >> U) * P + (k0 >> U) + g, k);
+            if (g % RUN == 0) A::ldtws(ws, tw, (size_t)(m0 >> U) * P + (k0 >> U) + g);
+            const typename A::Tw w = A::twiddle(ws[g % RUN], k);
 #pragma unroll
             for (int j = 0; j < gap; j++) {
                 const int i = g * 2 * gap + j;
@@ -756,13 +794,13 @@ __device__ __forceinline__ void mac_body(const NttArgs &a, const MacArgs &m, uin
             const uint64_t *src = a.src + ((size_t)bset * m.dig_bs + (size_t)d * m.lP + t) * N + base + (size_t)c * TT + e;
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = A::from_raw(src[i * E]);
-            ct_stages<A, 0, R, E, A::B_PASS>(y, tw, P, 0, 0, k);
+            ct_stages<A, 0, R, E, A::B_PASS, 1>(y, tw, P, 0, 0, k);
 #pragma unroll
             for (int i = 0; i < E; i++) sm[c * TPAD + pad_idx<LOG_T, R>(e + i * E)] = A::to_raw(y[i]);
             __syncthreads();
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = A::from_raw(sm[c * TPAD + pad_idx<LOG_T, R>(e * E + i)]);
-            ct_stages<A, 0, R, E, ct_bound<A>(A::B_PASS, R)>(y, tw, P, R, e, k);
+            ct_stages<A, 0, R, E, ct_bound<A>(A::B_PASS, R), 1>(y, tw, P, R, e, k);
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = Acc::operand(y[i], k);
         }
