@@ -2253,8 +2253,9 @@ extern "C" int b2_decode_compose(b2_ctx *c, size_t l, const uint64_t *d_res, con
     if (!d_res || !d_tab || !d_out) return fail(B2_EINVAL, "decode_compose: null pointer");
     if (l > (size_t)b2::B2_CRT_MAX_LIMBS) return fail(B2_ESIZE, "decode_compose: more than 64 limbs");
     LaunchScope ls(c, (cudaStream_t)stream, "decode_compose");
-    launch_k(b2::decode_compose_kernel, (unsigned)((c->N + 127) / 128), 128, 0, (cudaStream_t)stream, d_res, d_tab, c->d_mod, (uint32_t)c->N, (uint32_t)l, inv_scale,
-                                                                                              (double2 *)d_out);
+    b2::with_crt_words(l, [&](auto kernel) {
+        launch_k(kernel, (unsigned)((c->N + 127) / 128), 128, l * (l + 3) * 8, (cudaStream_t)stream, d_res, d_tab, c->d_mod, (uint32_t)c->N, (uint32_t)l, inv_scale, (double2 *)d_out);
+    });
     LAUNCH_CHECK("decode_compose_kernel");
     return B2_OK;
 }

@@ -249,3 +249,28 @@ def test_independent_products_in_one_call(log_n, products, sets, dbl):
     for i in range(sets):
         assert np.array_equal(host(res)[i], o.rescale_rounded(l, stack[i]))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("l", [1, 8, 9, 16, 17, 24, 25, 32, 33, 48])
+def test_composition_at_the_edges_of_its_word_counts(l):
+    """b2_decode_compose where the kernel for one more group of eight words takes over: values at 0, Q / 2, Q and between, where
+    the quotient's estimate is one off"""
+    from pyPhantom._native import LIB, check
+    N = 4096
+    ctx, o = make_ctx(N, [60, 59] + [40] * 47, 1)
+    primes = [int(q) for q in o.primes[:l]]
+    Q = int(np.prod(primes, dtype=object))
+    rng = np.random.default_rng(l)
+    xs = [(k * Q // 16 + d) % Q for k in range(17) for d in (-2, -1, 0, 1, 2)]
+    xs += [int.from_bytes(rng.bytes(8 * l), "little") % Q for _ in range(200)] + [int(rng.integers(1 << 62)) % Q for _ in range(50)]
+    res = np.zeros((l, N), dtype=np.uint64)
+    for k, x in enumerate(xs):
+        res[:, k] = [x % q for q in primes]
+    d, out = dev(res), torch.empty(N // 2, dtype=torch.complex128, device="cuda")
+    check(LIB.b2_decode_compose(ctx._h, l, d.data_ptr(), ph.ckks_encoder(ctx)._crt_table(ctx, l).data_ptr(), 2.0 ** -30, out.data_ptr(),
+                                torch.cuda.current_stream().cuda_stream))
+    got = torch.view_as_real(out).cpu().numpy()[: len(xs), 0]
+    signed = [x - Q if x > Q // 2 else x for x in xs]
+    assert np.array_equal(np.sign(got), [(x > 0) - (x < 0) for x in signed])
+    small = [k for k, x in enumerate(signed) if abs(x) < 1 << 1000]  # the others are beyond a double
+    assert np.allclose(got[small], [float(signed[k]) * 2.0 ** -30 for k in small], rtol=4e-16, atol=0)
