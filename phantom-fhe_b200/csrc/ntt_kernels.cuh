@@ -234,8 +234,7 @@ constexpr double FP_2_52 = 4503599627370496.0;
 // Primes of [2^50, 2^60): residues run up to 16 q in a 64-bit word, bounds in units of q. The quotient of the Shoup product
 // leaves out the lowest of its four partial products (one low at most, so the product is below 3 q), and instead of a
 // conditional subtraction per butterfly (six ALU instructions on 64-bit words) a residue is brought below 2 q by a 32-bit
-// quotient estimate (four instructions) every fourth stage or so. Inverse passes over 60-bit primes, N = 2^16, on B200: see
-// launch_inv.
+// quotient estimate (four instructions) every fourth stage or so.
 struct ArithIntLazy {
     using T = uint64_t;
     using Tw = W2;
