@@ -1336,7 +1336,7 @@ static int run_inner_prod(const b2_ctx *c, IpArgs &a, const uint64_t *const *evk
         }
     if (a.nq + a.np == 0) return B2_OK;
     LaunchScope ls(c, s, "ks_inner_prod");
-    launch_k(ks_inner_prod_kernel, dim3((unsigned)(c->N / 512), a.nq + a.np, sets), 256, 0, s, a);
+    launch_k(ks_inner_prod_kernel, dim3((unsigned)(c->N / 256), a.nq + a.np, sets), 128, 0, s, a);
     LAUNCH_CHECK("ks_inner_prod_kernel");
     return B2_OK;
 }

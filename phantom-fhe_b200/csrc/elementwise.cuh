@@ -537,9 +537,10 @@ __global__ void __launch_bounds__(GATHER_THREADS) gather_vectors_kernel(const __
 
 // ---- key-switch inner product (src/eval_key_switch.cu:175-230) ---------------------------------------------------------------
 // For logical limb t (physical prime pp):  acc[k][t][n] = sum_d digits[d][t][n] * evk[d][k][pp][n],  k = 0, 1.
-// Pure streaming: two coefficients per thread, 16-byte loads, two digits at a time so that four CTAs fit an SM (three digits and
-// three CTAs: eight hoisted rotations at N = 2^15 the same, 32 products at 2^14 724 against 707 us), the loads of the key before
-// those that wait for a permutation.
+// Pure streaming: two coefficients per thread, 16-byte loads, two digits at a time so that 32 warps fit an SM (three digits and
+// 24: eight hoisted rotations at N = 2^15 the same, 32 products at 2^14 724 against 707 us), the loads of the key before
+// those that wait for a permutation. CTAs of 128 threads: with 256 the warps of an SM load and multiply more
+// in step (247.7 -> 245.3 us, 689 -> 684.6 us, a bootstrap 25.48 -> 25.37 ms).
 constexpr int IP_MAX_STEPS = 16, IP_MAX_EVK = 256;
 struct IpArgs {
     const uint64_t *digits;
@@ -666,12 +667,12 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
     *reinterpret_cast<ulonglong2 *>(o1) = make_ulonglong2(r[2], r[3]);
 }
 
-__global__ void __launch_bounds__(256, 4) ks_inner_prod_kernel(const __grid_constant__ IpArgs a) {
+__global__ void __launch_bounds__(128, 8) ks_inner_prod_kernel(const __grid_constant__ IpArgs a) {
     pdl_enter();
     // the limbs of the special primes (the longer arithmetic) first
     const uint32_t y = blockIdx.y, t = y < a.np ? a.l + a.p0 + y : a.q0 + (y - a.np);
     const uint32_t pp = t < a.l ? t : a.size_Q + (t - a.l);
-    const uint32_t n = 2 * (blockIdx.x * 256 + threadIdx.x);
+    const uint32_t n = 2 * (blockIdx.x * 128 + threadIdx.x);
     const Mod md = a.mod[pp];
     // few terms (a digit per term, single rotations): FP64 products and one reduction cost less than pieces and their
     // recombination - 78 FP64 instructions a coefficient against 102 and 85 of the integer pipe at three digits
