@@ -274,3 +274,33 @@ def test_composition_at_the_edges_of_its_word_counts(l):
     assert np.array_equal(np.sign(got), [(x > 0) - (x < 0) for x in signed])
     small = [k for k, x in enumerate(signed) if abs(x) < 1 << 1000]  # the others are beyond a double
     assert np.allclose(got[small], [float(signed[k]) * 2.0 ** -30 for k in small], rtol=4e-16, atol=0)
+
+
+@pytest.mark.parametrize("M", [1, 128, 129, 300])
+def test_vectors_gathered_from_host_memory(M):
+    """b2_gather_vectors at the edges of its table of pointers (128 a launch) and of its rounds of loads"""
+    from pyPhantom._native import LIB, check
+    N = 4096
+    ctx, o = make_ctx(N, [60, 40, 60], 1)
+    src = torch.from_numpy(np.random.default_rng(M).integers(-(1 << 62), 1 << 62, (M, N + 2))).pin_memory()
+    ptrs = np.array([src.data_ptr() + 8 * (N + 2) * m for m in range(M)], dtype=np.uint64)
+    out = torch.zeros(M + 1, N, dtype=torch.int64, device="cuda")
+    check(LIB.b2_gather_vectors(ctx._h, M, ptrs.ctypes.data, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(out[:M].cpu(), src[:, :N]) and not out[M].any()
+
+
+@pytest.mark.parametrize("pool_kb", [400, 800, 1 << 18])
+def test_matrix_product_when_the_buffers_come_round(monkeypatch, pool_kb):
+    """one, two and four giants a launch; fewer buffers than groups of giants, and enough for all of them"""
+    N, l, M, G = 4096, 3, 4, 9
+    ctx, o = make_ctx(N, [60, 40, 40, 60], 1, [ph.get_elt_from_step(s, N) for s in (1, 2, 4)])
+    keys = {s: o.synth_key(o.beta(l), 3, 10 + 20 * i) for i, s in enumerate((1, 2, 4))}
+    glk = ph.galois_key.from_keys([ph.relin_key.from_numpy(ctx, keys[s]) for s in (1, 2, 4)])
+    coeffs = [o.synth_signed(5, 70 + d) for d in range(M * G)]
+    x_h = o.synth_ct(l, 3, 1)
+    x = ph.ciphertext.from_numpy(ctx, x_h, 1, 2.0 ** 40)
+    diags = ph.bsgs_diagonals([ph.single_chain_plaintext(c, 2.0 ** 40) for c in coeffs], M * G, M, G)
+    monkeypatch.setattr(ph, "_GIANT_POOL_BYTES", pool_kb << 10)
+    want = o.bsgs_matmul(l, x_h, coeffs, M, G, keys)
+    for _ in range(2):
+        assert np.array_equal(ph.bsgs_matmul_preencoded(ctx, glk, x, diags).numpy(), want)
