@@ -13,9 +13,11 @@ and keys produced by either library load in the other.
 PyTorch is used only for device memory and streams; every computation is a call into the
 C ABI. There is no CPU path.
 """
+import collections
 import enum
 import io
 import struct
+import threading
 
 import numpy as np
 import torch
@@ -132,8 +134,7 @@ class context:
             raise RuntimeError("pyPhantom needs a CUDA device: there is no CPU path")
         self.device = torch.cuda.current_device()
         self.N = parms._N
-        # of the matrix products: one set, so that what they allocate on them is cached once
-        self.side_streams = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream(priority=-1), torch.cuda.Stream(priority=-1)
+        self._product_streams, self._product_lock = collections.OrderedDict(), threading.Lock()
         self.primes = np.array([m.value() for m in parms._coeff_modulus], dtype=np.uint64)
         self.primes_signed = self.primes.view(np.int64)
         self.size_QP = len(self.primes)
@@ -188,6 +189,21 @@ class context:
         st = _native.ctypes.c_uint32(0)
         check(LIB.b2_device_status(self._h, _native.ctypes.byref(st)))
         return int(st.value)
+
+    def product_streams(self):
+        """The four streams that a matrix product issued on torch's current stream works on (see _bsgs_product): a set of
+        its own for every caller's stream, so that products of several streams or threads do not wait for one another, and
+        the same set every time, so that what is allocated on it is cached once. At most 16 sets, the one longest unused
+        makes room (torch lends its streams out of a fixed pool: nothing is destroyed)."""
+        key = _stream()
+        with self._product_lock:
+            streams = self._product_streams.pop(key, None)
+            if streams is None:
+                while len(self._product_streams) >= 16:
+                    self._product_streams.popitem(last=False)
+                streams = tuple(torch.cuda.Stream(priority=p) for p in (0, 0, -1, -1))
+            self._product_streams[key] = streams
+        return streams
 
     def workspace(self, op, l):
         nbytes = int(LIB.b2_workspace_bytes(self._h, op, l))
@@ -1017,12 +1033,13 @@ def bsgs_apply_giants_with_babies(ctx, galois_key_, babies, diags):
 def _bsgs_product(ctx, galois_key_, x, babies, diags):
     """The product of the two drivers; `babies` None: they are computed here, while the first diagonals are on their way.
 
-    Four streams beside the caller's: one reads the diagonals out of pinned host memory, up to 256 MB ahead; one makes their
-    residues and transforms them; and two of a higher priority, whose kernels the next rotation waits for, multiply (up to
-    four giants per launch, every baby read once for them) and rotate: the babies, then the chain of giants, each of which
-    lands on top of the next partial sum. Bound by the reads (8 N bytes per diagonal) or by the chain of G - 1 dependent key
-    switches, whichever is longer. 256 diagonals at N = 2^14, 6 limbs, 16 babies: 2140 us with the first two on one stream, two
-    buffers and 384 KB of reads in flight, 1790 us so."""
+    Four streams beside the caller's, a set of its own for each of them (ctx.product_streams): one reads the diagonals out of
+    pinned host memory, up to 256 MB ahead; one makes their residues and transforms them; and two of a higher priority,
+    whose kernels the next rotation waits for, multiply (up to four giants per launch, every baby read once for them) and
+    rotate: the babies, then the chain of giants, each of which lands on top of the next partial sum. Bound by the reads
+    (8 N bytes per diagonal) or by the chain of G - 1 dependent key switches, whichever is longer. 256 diagonals at
+    N = 2^14, 6 limbs, 16 babies: 2140 us with the first two on one stream, two buffers and 384 KB of reads in flight,
+    1790 us so."""
     M, G = diags.baby_steps, diags.giant_steps
     if M == 0 or G == 0 or M * G != diags.d_pad:
         raise ValueError("bsgs_apply_giants_with_babies: M*G must equal d_pad")
@@ -1044,7 +1061,7 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
     per = max(1, min(4, G, _GIANT_POOL_BYTES // (M * l * N * 8)))
     groups = [list(range(max(0, hi - per), hi)) for hi in range(G, 0, -per)]
     main = torch.cuda.current_stream()
-    read, transform, work, chain = ctx.side_streams
+    read, transform, work, chain = ctx.product_streams()
     if tab is None:  # the chain is made of public operations on the caller's stream
         chain = main
     n_stages = max(2, min(len(groups), _GIANT_POOL_BYTES // (per * M * N * 8)))

@@ -304,3 +304,44 @@ def test_matrix_product_when_the_buffers_come_round(monkeypatch, pool_kb):
     want = o.bsgs_matmul(l, x_h, coeffs, M, G, keys)
     for _ in range(2):
         assert np.array_equal(ph.bsgs_matmul_preencoded(ctx, glk, x, diags).numpy(), want)
+
+
+def _matrix_product(M, G, missing=None):
+    """a context, its keys (the one of step `missing` left out), a ciphertext, the diagonals' coefficients and the oracle's product"""
+    N, l = 4096, 3
+    steps = ph.bsgs_required_steps(M)
+    ctx, o = make_ctx(N, [60, 40, 40, 60], 1, [ph.get_elt_from_step(s, N) for s in steps])
+    keys = {s: o.synth_key(o.beta(l), 3, 10 + 20 * i) for i, s in enumerate(steps)}
+    glk = ph.galois_key.from_keys([ph.relin_key() if s == missing else ph.relin_key.from_numpy(ctx, keys[s]) for s in steps])
+    coeffs = [o.synth_signed(5, 70 + d) for d in range(M * G)]
+    x_h = o.synth_ct(l, 3, 1)
+    want = o.bsgs_matmul(l, x_h, coeffs, M, G, keys) if missing is None else None
+    return ctx, glk, ph.ciphertext.from_numpy(ctx, x_h, 1, 2.0 ** 40), coeffs, want
+
+
+def _diagonals(coeffs, M):
+    return ph.bsgs_diagonals([ph.single_chain_plaintext(c, 2.0 ** 40) for c in coeffs], len(coeffs), M, len(coeffs) // M)
+
+
+def test_matrix_products_of_two_streams_do_not_wait_for_one_another():
+    """a product behind a stream that is busy for a while; one of another stream is done long before it"""
+    ctx, glk, x, coeffs, want = _matrix_product(4, 3)
+    diags, streams, got = _diagonals(coeffs, 4), [torch.cuda.Stream() for _ in range(2)], []
+    for s in streams:  # what the first calls on a stream set up is there
+        with torch.cuda.stream(s):
+            ph.bsgs_matmul_preencoded(ctx, glk, x, diags)
+    torch.cuda.synchronize()
+    for s, busy in zip(streams, (600_000_000, 0)):
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(busy)
+            got.append(ph.bsgs_matmul_preencoded(ctx, glk, x, diags))
+    streams[1].synchronize()
+    assert not streams[0].query()
+    torch.cuda.synchronize()
+    for c in got:
+        assert np.array_equal(c.numpy(), want)
+    sets = []
+    for s in streams + [streams[0]]:
+        with torch.cuda.stream(s):
+            sets.append([t.cuda_stream for t in ctx.product_streams()])
+    assert sets[0] == sets[2] and not set(sets[0]) & set(sets[1])
