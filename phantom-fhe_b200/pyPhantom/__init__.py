@@ -1100,48 +1100,54 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
                                                pool.data_ptr() + 8 * (i % n_pools) * pool_words, transform.cuda_stream))
         transformed[i].record(transform)
 
-    fetch(0)  # on its way while the host launches the babies
-    with torch.cuda.stream(chain):
-        if babies is None:
-            babies = compute_bsgs_babies(ctx, galois_key_, x, M)
-        pt_tab = _pointer_table(pool.data_ptr(), l * N, n_pools * per * M, dev)
-        part_tab = _pointer_table(parts.data_ptr(), 2 * l * N, G, dev)
-        ptrs = [c.data.data_ptr() for c in babies]
-        step = ptrs[1] - ptrs[0] if M > 1 else 8
-        if step > 0 and all(p == ptrs[0] + i * step for i, p in enumerate(ptrs)):
-            baby_tab = _pointer_table(ptrs[0], step // 8, M, dev)
-        else:
-            baby_tab = torch.tensor(ptrs, dtype=torch.int64, device=dev)
-    ready = torch.cuda.Event()
-    ready.record(chain)
-    for i in range(1, n_stages):
-        fetch(i)
-    for i in range(n_pools):
-        expand(i)
-    work.wait_event(ready)
-    done = {}
-    for i, gs in enumerate(groups):
-        slot = i % n_pools
-        work.wait_event(transformed[i])
-        check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, len(gs), pt_tab.data_ptr() + 8 * slot * per * M, baby_tab.data_ptr(),
-                                    part_tab.data_ptr() + 8 * gs[0], work.cuda_stream))
-        consumed[i].record(work)
-        done[gs[-1]] = consumed[i]
-        fetch(i + n_stages)
-        expand(i + n_pools)
-    st = chain.cuda_stream
-    acc = None
-    for g in range(G - 1, -1, -1):
-        if g in done:
-            chain.wait_event(done[g])
-        part = x._like(parts[g], scale=scale)
-        if acc is None:
-            acc = part
-        elif tab is not None:
-            check(LIB.b2_rotate_add(ctx._h, l, elt, acc.data.data_ptr(), tab.ctypes.data, len(tab), part.data.data_ptr(), ws.data_ptr(), nbytes, st))
-            acc = part
-        else:
-            acc = add(ctx, rotate(ctx, acc, M, galois_key_), part)
+    try:
+        fetch(0)  # on its way while the host launches the babies
+        with torch.cuda.stream(chain):
+            if babies is None:
+                babies = compute_bsgs_babies(ctx, galois_key_, x, M)
+            pt_tab = _pointer_table(pool.data_ptr(), l * N, n_pools * per * M, dev)
+            part_tab = _pointer_table(parts.data_ptr(), 2 * l * N, G, dev)
+            ptrs = [c.data.data_ptr() for c in babies]
+            step = ptrs[1] - ptrs[0] if M > 1 else 8
+            if step > 0 and all(p == ptrs[0] + i * step for i, p in enumerate(ptrs)):
+                baby_tab = _pointer_table(ptrs[0], step // 8, M, dev)
+            else:
+                baby_tab = torch.tensor(ptrs, dtype=torch.int64, device=dev)
+        ready = torch.cuda.Event()
+        ready.record(chain)
+        for i in range(1, n_stages):
+            fetch(i)
+        for i in range(n_pools):
+            expand(i)
+        work.wait_event(ready)
+        done = {}
+        for i, gs in enumerate(groups):
+            slot = i % n_pools
+            work.wait_event(transformed[i])
+            check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, len(gs), pt_tab.data_ptr() + 8 * slot * per * M, baby_tab.data_ptr(),
+                                        part_tab.data_ptr() + 8 * gs[0], work.cuda_stream))
+            consumed[i].record(work)
+            done[gs[-1]] = consumed[i]
+            fetch(i + n_stages)
+            expand(i + n_pools)
+        st = chain.cuda_stream
+        acc = None
+        for g in range(G - 1, -1, -1):
+            if g in done:
+                chain.wait_event(done[g])
+            part = x._like(parts[g], scale=scale)
+            if acc is None:
+                acc = part
+            elif tab is not None:
+                check(LIB.b2_rotate_add(ctx._h, l, elt, acc.data.data_ptr(), tab.ctypes.data, len(tab), part.data.data_ptr(), ws.data_ptr(), nbytes, st))
+                acc = part
+            else:
+                acc = add(ctx, rotate(ctx, acc, M, galois_key_), part)
+    except BaseException:
+        # a missing key, no memory: the buffers go back to the allocator now, and a kernel on a side stream may still use them
+        for side in (read, transform, work, chain):
+            main.wait_stream(side)
+        raise
     main.wait_stream(chain)
     acc = rescale_to_next(ctx, acc)
     acc.set_scale(x._scale)

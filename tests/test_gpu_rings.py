@@ -345,3 +345,19 @@ def test_matrix_products_of_two_streams_do_not_wait_for_one_another():
         with torch.cuda.stream(s):
             sets.append([t.cuda_stream for t in ctx.product_streams()])
     assert sets[0] == sets[2] and not set(sets[0]) & set(sets[1])
+
+
+def test_failed_matrix_product_leaves_no_stream_behind():
+    """a baby step without a key is noticed after the first diagonals are on their way: the caller's stream waits for the side
+    streams before the call's buffers can be used again"""
+    ctx, glk, x, coeffs, _ = _matrix_product(4, 3, missing=2)
+    diags = _diagonals(coeffs, 4)
+    torch.cuda.synchronize()
+    for side in ctx.product_streams()[:3]:
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000_000)
+        with pytest.raises(ValueError):
+            ph.bsgs_matmul_preencoded(ctx, glk, x, diags)
+        assert not torch.cuda.current_stream().query()
+        torch.cuda.synchronize()
+        assert torch.cuda.current_stream().query()
