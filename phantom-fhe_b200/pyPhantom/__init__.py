@@ -829,10 +829,20 @@ class single_chain_plaintext:
     @coeffs.setter
     def coeffs(self, t):
         self._coeffs = t
-        # what the device reads in place: the address of a pinned (or device) vector, else 0
-        ok = t is not None and (t.is_cuda or t.is_pinned()) and t.is_contiguous() and t.dtype == torch.int64 and t.data_ptr() % 16 == 0
-        self._readable = t.data_ptr() if ok else 0
-        self._numel = -1 if t is None else t.numel()
+        # where the device may read the vector in place: the address of a pinned one, else 0. It counts while the tensor is
+        # still there (readable_at); everything else is copied.
+        ok = t is not None and t.is_pinned() and t.is_contiguous() and t.dtype == torch.int64 and t.data_ptr() % 16 == 0
+        self._pinned_at = t.data_ptr() if ok else 0
+
+    def readable_at(self):
+        """the address at which a kernel of any stream may read the vector, 0 if it has to be copied"""
+        return self._pinned_at if self._coeffs.data_ptr() == self._pinned_at else 0
+
+    def __getstate__(self):
+        return {"scale": self.scale, "coeffs": self._coeffs}
+
+    def __setstate__(self, state):  # a copy's vector lies elsewhere, and is pinned or not
+        self.scale, self.coeffs = state["scale"], state["coeffs"]
 
     def coeffs_bytes(self):
         return self.coeffs.numpy().tobytes()
@@ -1046,7 +1056,8 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
     if len(diags.diagonals) != diags.d_pad:
         raise ValueError("bsgs_apply_giants_with_babies: diagonals size mismatch")
     l, N, dev = x._limbs, ctx.N, ctx.device
-    if any([scp._numel != N for scp in diags.diagonals]):
+    scps = list(diags.diagonals)
+    if {-1 if scp._coeffs is None else scp._coeffs.numel() for scp in scps} != {N}:
         raise ValueError("bsgs_apply_giants_with_babies: scp coeff length != N")
     scale = x._scale * diags.diagonals[(G - 1) * M].scale
     for g in range(G - 1):
@@ -1072,7 +1083,6 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
     ws, nbytes = ctx.workspace(_native.OP_KEYSWITCH, l)
     for side in (read, transform, work, chain):
         side.wait_stream(main)
-    readable = np.array([scp._readable for scp in diags.diagonals], dtype=np.uint64)
     arrived, transformed, consumed = ([torch.cuda.Event() for _ in groups] for _ in range(3))
 
     def fetch(i):
@@ -1081,12 +1091,12 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
         slot, which = i % n_stages, slice(groups[i][0] * M, (groups[i][-1] + 1) * M)
         if i >= n_stages:
             read.wait_event(transformed[i - n_stages])
-        ptrs = readable[which]
+        ptrs = np.array([scp.readable_at() for scp in scps[which]], dtype=np.uint64)
         if ptrs.all():
             check(LIB.b2_gather_vectors(ctx._h, len(ptrs), ptrs.ctypes.data, stage.data_ptr() + 8 * slot * stage_words, read.cuda_stream))
         else:  # vectors the device cannot read in place are copied
             with torch.cuda.stream(read):
-                for k, scp in enumerate(diags.diagonals[which]):
+                for k, scp in enumerate(scps[which]):
                     stage[slot * per * M + k].copy_(scp.coeffs, non_blocking=True)
         arrived[i].record(read)
 

@@ -361,3 +361,21 @@ def test_failed_matrix_product_leaves_no_stream_behind():
         assert not torch.cuda.current_stream().query()
         torch.cuda.synchronize()
         assert torch.cuda.current_stream().query()
+
+
+def test_diagonals_are_read_where_they_are_now():
+    """copies of pinned diagonals (their vectors are pageable), a vector that moved since it was set, and vectors in device memory"""
+    import copy
+    import pickle
+    ctx, glk, x, coeffs, want = _matrix_product(4, 3)
+    diags = _diagonals(coeffs, 4)
+    moved, on_device, mixed = _diagonals(coeffs, 4), _diagonals(coeffs, 4), _diagonals(coeffs, 4)
+    for scp in moved.diagonals:
+        scp.coeffs.data = scp.coeffs.clone()
+    for scp in on_device.diagonals:
+        scp.coeffs = scp.coeffs.cuda()
+    mixed.diagonals[5] = copy.deepcopy(mixed.diagonals[5])
+    for d in (diags, copy.copy(diags), copy.deepcopy(diags), pickle.loads(pickle.dumps(diags)), moved, on_device, mixed):
+        assert np.array_equal(ph.bsgs_matmul_preencoded(ctx, glk, x, d).numpy(), want)
+    assert diags.diagonals[0].readable_at() == diags.diagonals[0].coeffs.data_ptr()
+    assert not any(d.diagonals[0].readable_at() for d in (moved, on_device))
