@@ -817,7 +817,6 @@ class single_chain_plaintext:
     def __init__(self, coeffs=None, scale=1.0):
         self.scale = float(scale)
         self.coeffs = None
-
         if coeffs is not None:
             t = torch.from_numpy(np.ascontiguousarray(coeffs, dtype=np.int64).copy())
             self.coeffs = t.pin_memory() if torch.cuda.is_available() else t
@@ -828,6 +827,7 @@ class single_chain_plaintext:
 
     @coeffs.setter
     def coeffs(self, t):
+        self._reads_done()
         self._coeffs = t
         # where the device may read the vector in place: the address of a pinned one, else 0. It counts while the tensor is
         # still there (readable_at); everything else is copied.
@@ -837,6 +837,22 @@ class single_chain_plaintext:
     def readable_at(self):
         """the address at which a kernel of any stream may read the vector, 0 if it has to be copied"""
         return self._pinned_at if self._coeffs.data_ptr() == self._pinned_at else 0
+
+    # torch's pinned allocator knows of no kernel that reads a block: the vector is held until such reads are done
+    _reads = None  # {stream: event behind its last read}
+
+    def read_on(self, stream, event):
+        if self._reads is None:
+            self._reads = {}
+        self._reads[stream] = event
+
+    def _reads_done(self):
+        if self._reads:
+            for event in self._reads.values():
+                event.synchronize()
+            self._reads = None
+
+    __del__ = _reads_done
 
     def __getstate__(self):
         return {"scale": self.scale, "coeffs": self._coeffs}
@@ -1084,6 +1100,7 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
     for side in (read, transform, work, chain):
         side.wait_stream(main)
     arrived, transformed, consumed = ([torch.cuda.Event() for _ in groups] for _ in range(3))
+    read_done = torch.cuda.Event()
 
     def fetch(i):
         if i >= len(groups):
@@ -1158,6 +1175,11 @@ def _bsgs_product(ctx, galois_key_, x, babies, diags):
         for side in (read, transform, work, chain):
             main.wait_stream(side)
         raise
+    finally:
+        if not torch.cuda.is_current_stream_capturing():  # a graph's owner keeps what its replays read
+            read_done.record(read)
+            for scp in scps:
+                scp.read_on(read.cuda_stream, read_done)
     main.wait_stream(chain)
     acc = rescale_to_next(ctx, acc)
     acc.set_scale(x._scale)

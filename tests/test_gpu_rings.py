@@ -379,3 +379,41 @@ def test_diagonals_are_read_where_they_are_now():
         assert np.array_equal(ph.bsgs_matmul_preencoded(ctx, glk, x, d).numpy(), want)
     assert diags.diagonals[0].readable_at() == diags.diagonals[0].coeffs.data_ptr()
     assert not any(d.diagonals[0].readable_at() for d in (moved, on_device))
+
+
+@pytest.mark.parametrize("how", ["deleted", "replaced"])
+def test_diagonals_let_go_of_while_a_product_reads_them(how):
+    """the reads wait behind a busy stream; the vectors' memory is not handed out again before they are done"""
+    ctx, glk, x, coeffs, want = _matrix_product(4, 3)
+    diags = _diagonals(coeffs, 4)
+    ph.bsgs_matmul_preencoded(ctx, glk, x, diags)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(400_000_000)
+    got = ph.bsgs_matmul_preencoded(ctx, glk, x, diags)
+    assert not torch.cuda.current_stream().query()
+    if how == "deleted":
+        del diags
+    else:
+        for scp in diags.diagonals:
+            scp.coeffs = None
+    others = [torch.full((ctx.N,), 1 << 40, dtype=torch.int64).pin_memory() for _ in coeffs]
+    assert np.array_equal(got.numpy(), want) and len(others) == len(coeffs)
+
+
+def test_captured_matrix_product():
+    """replays of a captured product; its diagonals are let go of when the graph is"""
+    ctx, glk, x, coeffs, want = _matrix_product(4, 3)
+    diags = _diagonals(coeffs, 4)
+    ph.bsgs_matmul_preencoded(ctx, glk, x, diags)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ph.bsgs_matmul_preencoded(ctx, glk, x, diags)
+    for _ in range(2):
+        got.data.zero_()
+        graph.replay()
+        assert np.array_equal(got.numpy(), want)
+    torch.cuda.synchronize()
+    del graph
+    for scp in diags.diagonals:
+        scp.coeffs = None
