@@ -57,18 +57,16 @@ class resident_bsgs:
             tab = np.array([[self.pts[g * M + b].data_ptr() for b in range(M)] for g in chunk], dtype=np.int64)
             self.groups.append((len(chunk), torch.from_numpy(tab.ravel().copy()).to(ctx.device),
                                 torch.tensor([self.part_buf[g].data_ptr() for g in chunk], dtype=torch.int64, device=ctx.device)))
-        n_evk = ctx.beta(l)
-        self.baby_elts, self.baby_ksk = self._key_tables(range(1, M), n_evk)
-        self.giant_elts, self.giant_ksk = self._key_tables(range(M, M * G, M), n_evk)
+        self.baby_steps, self.giant_steps = range(1, M), range(M, M * G, M)
+        self.baby_elts, self.giant_elts = (np.array([self.keys[s][0] for s in steps], dtype=np.uint32) for steps in (self.baby_steps, self.giant_steps))
         self.baby_outs = np.array([self.baby_buf[b].data_ptr() for b in range(1, M)], dtype=np.uint64)
         torch.cuda.synchronize()
 
-    def _key_tables(self, steps, n_evk):
-        steps = list(steps)
-        if not steps:
-            return None, None
-        return (np.array([self.keys[s][0] for s in steps], dtype=np.uint32),
-                np.concatenate([self.keys[s][1].pointer_table()[:n_evk] for s in steps]).astype(np.uint64))
+    def _digits(self, steps, n_evk):
+        """the addresses of the first n_evk digits of every step's key, as they are at this call (a key may be loaded anew)"""
+        if any(self.keys[s][1].dnum() < n_evk for s in steps):
+            raise ValueError("key has fewer digits than this level needs")
+        return np.concatenate([self.keys[s][1].pointer_table()[:n_evk] for s in steps]).astype(np.uint64)
 
     def apply(self, x):
         ctx, l, N, M = self.ctx, self.l, self.ctx.N, self.M
@@ -78,7 +76,8 @@ class resident_bsgs:
         self.baby_buf[0].copy_(x.data)
         if M > 1:
             ws, nbytes = ctx.workspace(_native.OP_HOIST, l)
-            check(LIB.b2_hoist_rotations(ctx._h, l, x.data.data_ptr(), self.baby_elts.ctypes.data, M - 1, self.baby_ksk.ctypes.data, n_evk,
+            ksk = self._digits(self.baby_steps, n_evk)
+            check(LIB.b2_hoist_rotations(ctx._h, l, x.data.data_ptr(), self.baby_elts.ctypes.data, M - 1, ksk.ctypes.data, n_evk,
                                          self.baby_outs.ctypes.data, ws.data_ptr(), nbytes, st))
         for n, ptab, otab in self.groups:
             check(LIB.b2_bsgs_mac_multi(ctx._h, l, M, n, ptab.data_ptr(), self.baby_tab.data_ptr(), otab.data_ptr(), st))
@@ -87,7 +86,8 @@ class resident_bsgs:
             n = self.G - 1
             nbytes = int(LIB.b2_rotate_sum_workspace_bytes(ctx._h, l, n))
             ws = torch.empty(nbytes // 8, dtype=torch.int64, device=ctx.device)
-            check(LIB.b2_rotate_sum(ctx._h, l, n, self.giant_elts.ctypes.data, self.part_buf[1].data_ptr(), 2 * l, self.giant_ksk.ctypes.data, n_evk,
+            ksk = self._digits(self.giant_steps, n_evk)
+            check(LIB.b2_rotate_sum(ctx._h, l, n, self.giant_elts.ctypes.data, self.part_buf[1].data_ptr(), 2 * l, ksk.ctypes.data, n_evk,
                                     total.data_ptr(), 0, ws.data_ptr(), nbytes, st))
         out = rescale_to_next(ctx, x._like(total, scale=x._scale * self.pt_scale))
         out.set_scale(x._scale)

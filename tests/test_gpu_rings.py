@@ -417,3 +417,28 @@ def test_captured_matrix_product():
     del graph
     for scp in diags.diagonals:
         scp.coeffs = None
+
+
+def test_resident_product_with_keys_loaded_anew_or_cut():
+    """a plan uses the digits that its keys hold at the call: loaded anew from other bytes they give what a plan made from those
+    gives, and a key cut below the level's digits is refused"""
+    import io
+    from pyPhantom.linalg import resident_bsgs
+    N, l, M, G = 4096, 3, 2, 3
+    steps = [1, 2, 4]
+    ctx, o = make_ctx(N, [60, 40, 40, 60], 1, [ph.get_elt_from_step(s, N) for s in steps])
+    sets = [[ph.relin_key.from_numpy(ctx, o.synth_key(o.beta(l), seed, 10 + 20 * i)) for i in range(3)] for seed in (3, 4)]
+    x = ph.ciphertext.from_numpy(ctx, o.synth_ct(l, 3, 1), 1, 2.0 ** 40)
+    diags = _diagonals([o.synth_signed(5, 70 + d) for d in range(M * G)], M)
+    plan, other = (resident_bsgs(ctx, ph.galois_key.from_keys(keys), diags, 1) for keys in sets)
+    before, want = plan.apply(x).numpy(), other.apply(x).numpy()
+    assert not np.array_equal(before, want)
+    for key, new in zip(*sets):
+        buf = io.BytesIO()
+        new.save(buf)
+        buf.seek(0)
+        key.load(buf)
+    assert np.array_equal(plan.apply(x).numpy(), want)
+    sets[0][1].mod_drop_to_inplace(ctx, 2)
+    with pytest.raises(ValueError):
+        plan.apply(x)
