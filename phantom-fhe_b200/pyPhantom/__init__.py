@@ -137,6 +137,7 @@ class context:
         self._product_streams, self._product_lock = collections.OrderedDict(), threading.Lock()
         self.primes = np.array([m.value() for m in parms._coeff_modulus], dtype=np.uint64)
         self.primes_signed = self.primes.view(np.int64)
+        self.chain_bits = np.cumsum([0] + [int(q).bit_length() for q in self.primes]).tolist()  # of the first l primes
         self.size_QP = len(self.primes)
         self.size_P = parms._special
         self.size_Q = self.size_QP - self.size_P

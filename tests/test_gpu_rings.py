@@ -442,3 +442,20 @@ def test_resident_product_with_keys_loaded_anew_or_cut():
     sets[0][1].mod_drop_to_inplace(ctx, 2)
     with pytest.raises(ValueError):
         plan.apply(x)
+
+
+def test_encoder_checks_the_chain_it_encodes_for():
+    """an encoder belongs to a ring; the limits of what fits are those of the context given with the call, longer or shorter"""
+    N = 4096
+    ctxs = [make_ctx(N, bits, 1)[0] for bits in ([50, 30, 50], [60, 40, 40, 40, 60])]
+    values = np.linspace(-1.0, 1.0, N // 2)
+    for enc in (ph.ckks_encoder(c) for c in ctxs):
+        for ctx in ctxs:
+            same = ph.ckks_encoder(ctx).encode_double_vector(ctx, values, 2.0 ** 40)
+            assert torch.equal(enc.encode_double_vector(ctx, values, 2.0 ** 40).data, same.data)
+        with pytest.raises(ValueError):  # 80 bits of modulus
+            enc.encode_double_vector(ctxs[0], values, 2.0 ** 85)
+        with pytest.raises(ValueError):  # scale and value together
+            enc.encode_double_vector(ctxs[0], 1024.0 * values, 2.0 ** 71)
+        with pytest.raises(ValueError):  # 180 bits of modulus, but coefficients of more than 62
+            enc.encode_double_vector(ctxs[1], values, 2.0 ** 85)
