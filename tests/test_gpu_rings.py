@@ -459,3 +459,17 @@ def test_encoder_checks_the_chain_it_encodes_for():
             enc.encode_double_vector(ctxs[0], 1024.0 * values, 2.0 ** 71)
         with pytest.raises(ValueError):  # 180 bits of modulus, but coefficients of more than 62
             enc.encode_double_vector(ctxs[1], values, 2.0 ** 85)
+
+
+def test_decoding_of_limbs_that_lie_apart():
+    """a plaintext whose limbs are a strided view decodes as its compact copy does, and stays as it is"""
+    N = 4096
+    ctx, _ = make_ctx(N, [50, 40, 40, 50], 1)
+    enc = ph.ckks_encoder(ctx)
+    pt = enc.encode_double_vector(ctx, np.linspace(-1.0, 1.0, N // 2), 2.0 ** 40)
+    want, limbs = enc.decode_complex_vector(ctx, pt), pt.data
+    apart = torch.zeros(5, N, dtype=torch.int64, device="cuda")
+    apart[::2] = limbs
+    pt.data = apart[::2]
+    assert np.array_equal(enc.decode_complex_vector(ctx, pt), want)
+    assert torch.equal(apart[::2], limbs) and not apart[1::2].any()
