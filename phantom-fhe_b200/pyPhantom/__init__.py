@@ -1052,7 +1052,7 @@ _GIANT_POOL_BYTES = 1 << 28  # expanded plaintexts of the giants that share a la
 def bsgs_apply_giants_with_babies(ctx, galois_key_, babies, diags):
     """src/bsgs.cu:216-359: per giant expand M plaintexts and run the fused MAC; Horner
     acc = rotate(acc, M) + partial_g from the last giant down; one rescale; scale reset to x's."""
-    if len(babies) != diags.baby_steps:
+    if diags.baby_steps == 0 or len(babies) != diags.baby_steps:
         raise ValueError("bsgs_apply_giants_with_babies: babies size != baby_steps")
     return _bsgs_product(ctx, galois_key_, babies[0], babies, diags)
 

@@ -126,3 +126,10 @@ def test_batched_wrappers_check_their_arguments_before_any_device_call():
         ph.relinearize_batch(None, torch.zeros(2, 3, 3, 8, dtype=torch.int64).transpose(2, 3), None)
     with pytest.raises(ValueError, match="one shape"):
         ph.multiply_relin_rescale_batch(None, torch.zeros(2, 2, 3, 8, dtype=torch.int64), torch.zeros(2, 2, 4, 8, dtype=torch.int64), None)
+
+
+def test_matrix_product_without_babies_is_refused():
+    with pytest.raises(ValueError):
+        ph.bsgs_apply_giants_with_babies(None, None, [], ph.bsgs_diagonals([], 0, 0, 0))
+    with pytest.raises(ValueError):
+        ph.bsgs_matmul_preencoded(None, None, None, ph.bsgs_diagonals([], 0, 0, 0))
