@@ -120,9 +120,13 @@ def check(rc):
     raise RuntimeError(f"CUDA error {rc}: {msg}")
 
 
-_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+def _stream_lookup():
+    """torch's current stream on the current device, as the handle the C ABI takes. torch.cuda.current_stream() builds a Stream
+    object, 3 us in every call; the two functions under it are private to torch and may go, the public one stays."""
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
 
 
-def current_stream():
-    """handle of torch's current stream on the current device (torch.cuda.current_stream() builds a Stream object: 3 us)"""
-    return _raw_stream(_current_device())
+current_stream = _stream_lookup()

@@ -133,3 +133,12 @@ def test_matrix_product_without_babies_is_refused():
         ph.bsgs_apply_giants_with_babies(None, None, [], ph.bsgs_diagonals([], 0, 0, 0))
     with pytest.raises(ValueError):
         ph.bsgs_matmul_preencoded(None, None, None, ph.bsgs_diagonals([], 0, 0, 0))
+
+
+@pytest.mark.parametrize("gone", ["_cuda_getCurrentRawStream", "_cuda_getDevice"])
+def test_stream_lookup_without_torchs_private_functions(monkeypatch, gone):
+    """the package works with a torch that no longer has them: the handle then comes from the public stream object"""
+    import types
+    monkeypatch.delattr(torch._C, gone)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
+    assert _native._stream_lookup()() == 77
