@@ -2347,10 +2347,10 @@ extern "C" int b2_expand_single_chain_batch(b2_ctx *c, size_t l, size_t M, const
     CHECK_LEVEL(c, l);
     if (!d_signed || !d_out || M == 0) return fail(B2_EINVAL, "expand_single_chain_batch: bad argument");
     cudaStream_t s = (cudaStream_t)stream;
-    {
+    for (size_t m = 0; m < M; m += 65535) {  // the vectors are the grid's third dimension
         LaunchScope ls(c, s, "expand_signed");
-        LAUNCH_V(expand_signed_kernel, aligned32(d_signed) && aligned32(d_out), (unsigned)l, (unsigned)M, s, d_signed, d_out, c->d_mod, (uint32_t)c->N,
-                 (uint32_t)l, 0u);
+        LAUNCH_V(expand_signed_kernel, aligned32(d_signed) && aligned32(d_out), (unsigned)l, (unsigned)std::min<size_t>(M - m, 65535), s, d_signed + m * c->N,
+                 d_out + m * l * c->N, c->d_mod, (uint32_t)c->N, (uint32_t)l, 0u);
         LAUNCH_CHECK("expand_signed_kernel");
     }
     return run_fwd(c, d_out, d_out, nullptr, (uint32_t)(M * l), 0, EpiStore{}, s, (uint32_t)l);

@@ -473,3 +473,20 @@ def test_decoding_of_limbs_that_lie_apart():
     pt.data = apart[::2]
     assert np.array_equal(enc.decode_complex_vector(ctx, pt), want)
     assert torch.equal(apart[::2], limbs) and not apart[1::2].any()
+
+
+def test_more_vectors_than_a_grid_dimension_holds():
+    """b2_expand_single_chain_batch beyond 65535 vectors (4 GB): every one as b2_expand_single_chain makes it"""
+    from pyPhantom._native import LIB, check
+    N, M, K = 4096, 65537, 7
+    ctx, o = make_ctx(N, [40, 40, 60], 1)
+    s = torch.cuda.current_stream().cuda_stream
+    base = torch.from_numpy(np.stack([o.synth_signed(5, 70 + k) for k in range(K)])).cuda()
+    want = ctx.empty(K, 1)
+    for k in range(K):
+        check(LIB.b2_expand_single_chain(ctx._h, 1, base[k].data_ptr(), want[k].data_ptr(), s))
+    src, out = base.repeat(M // K + 1, 1)[:M].contiguous(), ctx.empty(M, 1)
+    check(LIB.b2_expand_single_chain_batch(ctx._h, 1, M, src.data_ptr(), out.data_ptr(), s))
+    for m in range(0, M, 8192 * K):
+        part = out[m: m + 8192 * K, 0]
+        assert torch.equal(part, want[:, 0].repeat(8192, 1)[: len(part)])
