@@ -1864,9 +1864,14 @@ extern "C" int b2_galois_prepare(b2_ctx *c, uint32_t elt) {
 }
 
 static int gather_impl(b2_ctx *c, const uint32_t *perm, const uint64_t *src, uint64_t *dst, size_t n_limbs, cudaStream_t s) {
-    LaunchScope ls(c, s, "galois_gather");
-    LAUNCH_V(galois_gather_kernel, aligned32(dst), (unsigned)n_limbs, 1, s, src, dst, perm, (uint32_t)c->N);
-    LAUNCH_CHECK("galois_gather_kernel");
+    size_t t = 0;
+    do {  // the limbs are the grid's second dimension
+        const size_t n = std::min<size_t>(n_limbs - t, 65535);
+        LaunchScope ls(c, s, "galois_gather");
+        LAUNCH_V(galois_gather_kernel, aligned32(dst), (unsigned)n, 1, s, src + t * c->N, dst + t * c->N, perm, (uint32_t)c->N);
+        LAUNCH_CHECK("galois_gather_kernel");
+        t += n;
+    } while (t < n_limbs);
     return B2_OK;
 }
 

@@ -490,3 +490,17 @@ def test_more_vectors_than_a_grid_dimension_holds():
     for m in range(0, M, 8192 * K):
         part = out[m: m + 8192 * K, 0]
         assert torch.equal(part, want[:, 0].repeat(8192, 1)[: len(part)])
+
+
+def test_more_limbs_than_a_grid_dimension_holds():
+    """b2_galois_permute beyond 65535 limbs (2 GB each way)"""
+    from pyPhantom._native import LIB, check
+    N, n = 4096, 65537
+    elt = ph.get_elt_from_step(3, N)
+    ctx, o = make_ctx(N, [40, 40, 60], 1, [elt])
+    src = torch.arange(n * N, dtype=torch.int64, device="cuda").reshape(n, N)
+    dst = torch.empty_like(src)
+    check(LIB.b2_galois_permute(ctx._h, elt, src.data_ptr(), dst.data_ptr(), n, torch.cuda.current_stream().cuda_stream))
+    perm = torch.from_numpy(o.galois_perm(elt).astype(np.int64)).cuda()
+    for t in range(0, n, 16384):
+        assert torch.equal(dst[t: t + 16384], src[t: t + 16384][:, perm])
