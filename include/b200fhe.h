@@ -289,9 +289,8 @@ int b2_expand_single_chain_batch(b2_ctx *ctx, size_t size_Ql, size_t M, const in
                                  void *stream);
 
 /* M separate vectors of N (a HOST array of pointers the device can read: pinned host memory or device memory, 16-byte aligned)
- * -> d_out int64[M][N], for b2_expand_single_chain_batch; b2_ntt_forward_batch transforms M polynomials of size_Ql limbs */
+ * -> d_out int64[M][N], for b2_expand_single_chain_batch */
 int b2_gather_vectors(b2_ctx *ctx, size_t M, const int64_t *const *srcs, int64_t *d_out, void *stream);
-int b2_ntt_forward_batch(b2_ctx *ctx, uint64_t *d_data, size_t size_Ql, size_t M, void *stream);
 
 /* the same over any limb range [first_prime, first_prime + n_limbs), optionally left in coefficient
  * form: what the samplers and the encoder of the reference do per limb when they reduce a small

@@ -828,24 +828,20 @@ static constexpr int pass_threads() {
     return (1 << ((COLS ? P::LOG_CC : P::LOG_C) + LOG_T)) >> (P::R_STRIDED > P::R_CONTIG ? P::R_STRIDED : P::R_CONTIG);
 }
 
-// grid of a two-pass transform kernel over `work` tiles and `batch` sets
-static dim3 pass_grid(NttArgs &, uint32_t work, uint32_t batch) { return dim3(work, batch); }
-
 template <int LOG_A, int LOG_B, class Epi, int SRC = 0>
 static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const Epi &epi, cudaStream_t s, uint32_t batch = 1) {
     using A = PassCfg<LOG_A>;
     using B = PassCfg<LOG_B>;
     const uint32_t N = 1u << a.logN;
     {
-        NttArgs a1 = a;
-        const dim3 grid = pass_grid(a1, njobs * (N >> (LOG_A + A::LOG_CC)), batch);
+        const dim3 grid(njobs * (N >> (LOG_A + A::LOG_CC)), batch);
         LaunchScope ls(c, s, "ntt_fwd_cols");
-        launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC>, grid, pass_threads<LOG_A, true>(), 0, s, a1, EpiStore{});
+        launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC>, grid, pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
     }
     NttArgs b = a;
     b.src = a.dst;  // second pass works in place on the first pass's output
     b.src_lm1 = a.dst_lm1, b.src_bs = a.dst_bs;
-    const dim3 grid = pass_grid(b, njobs * (N >> (LOG_B + B::LOG_C)), batch);
+    const dim3 grid(njobs * (N >> (LOG_B + B::LOG_C)), batch);
     LaunchScope ls(c, s, "ntt_fwd_rows");
     launch_k(ntt_fwd_pass<LOG_B, B::R_STRIDED, B::R_CONTIG, B::LOG_C, false, true, Epi>, grid, pass_threads<LOG_B>(), 0, s, b, epi);
 }
@@ -868,15 +864,14 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
     using B = PassCfg<LOG_B>;
     const uint32_t N = 1u << a.logN;
     {
-        NttArgs a1 = a;
-        const dim3 grid = pass_grid(a1, njobs * (N >> (LOG_B + B::LOG_C)), batch);
+        const dim3 grid(njobs * (N >> (LOG_B + B::LOG_C)), batch);
         LaunchScope ls(c, s, "ntt_inv_rows");
-        launch_k(ntt_inv_pass<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false>, grid, pass_threads<LOG_B>(), 0, s, a1);
+        launch_k(ntt_inv_pass<LOG_B, B::R_CONTIG, B::R_STRIDED, B::LOG_C, false, false>, grid, pass_threads<LOG_B>(), 0, s, a);
     }
     NttArgs b = a;
     b.src = a.dst;
     b.src_lm1 = a.dst_lm1, b.src_bs = a.dst_bs;
-    const dim3 grid = pass_grid(b, njobs * (N >> (LOG_A + A::LOG_CC)), batch);
+    const dim3 grid(njobs * (N >> (LOG_A + A::LOG_CC)), batch);
     LaunchScope ls(c, s, "ntt_inv_cols");
     launch_k(ntt_inv_pass<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_CC, true, true>, grid, pass_threads<LOG_A, true>(), 0, s, b);
 }
@@ -1467,7 +1462,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (!wide && pl.n_up_rows) {
             NttArgs b = a;
             b.jobs = pl.jobs_up_rows;
-            const dim3 grid = pass_grid(b, pl.n_up_rows * (uint32_t)(N >> (8 + Cfg::LOG_C)), B);
+            const dim3 grid(pl.n_up_rows * (uint32_t)(N >> (8 + Cfg::LOG_C)), B);
             LaunchScope ls(c, s, "ntt_fwd_rows");
             launch_k(ntt_fwd_pass<8, Cfg::R_STRIDED, Cfg::R_CONTIG, Cfg::LOG_C, false, true, EpiStore>, grid, pass_threads<8>(), 0, s, b, EpiStore{});
             LAUNCH_CHECK("ntt_fwd_pass");
@@ -2377,13 +2372,6 @@ extern "C" int b2_gather_vectors(b2_ctx *c, size_t M, const int64_t *const *srcs
         LAUNCH_CHECK("gather_vectors_kernel");
     }
     return B2_OK;
-}
-
-extern "C" int b2_ntt_forward_batch(b2_ctx *c, uint64_t *d, size_t l, size_t M, void *stream) {
-    CHECK_CTX(c);
-    CHECK_LEVEL(c, l);
-    if (!d || M == 0) return fail(B2_EINVAL, "ntt_forward_batch: bad argument");
-    return run_fwd(c, d, d, nullptr, (uint32_t)(M * l), 0, EpiStore{}, (cudaStream_t)stream, (uint32_t)l);
 }
 
 extern "C" int b2_poly_op(b2_ctx *c, int op, size_t n_limbs, const uint64_t *d_a, const uint64_t *d_b, uint64_t *d_out, void *stream) {

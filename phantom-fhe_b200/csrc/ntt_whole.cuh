@@ -154,15 +154,14 @@ __device__ __forceinline__ void whole_src(typename A::T (&x)[E], const NttArgs &
 template <class A, int LOGN, class Epi, int SRC>
 __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs &w, const Epi &epi, uint64_t *smem, const Job &job, uint32_t jobi, const Mod &md) {
     using Cfg = WholeCfg<LOGN>;
-    using T = typename A::T;
-    constexpr int CL = 1 << Cfg::LOG_CL, LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
+    constexpr int LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
     constexpr int N2 = 1 << Cfg::LOG_B, CC = 1 << LOG_CC;
     constexpr int B0 = SRC == 3 ? A::B_BCONV : A::B_CANON;
     constexpr size_t N = (size_t)1 << LOGN;
     uint64_t *slab = smem, *ex = smem + whole_slab<LOGN>();
     const typename A::K k = A::make(md, LOGN);
     const W2 *tw = a.tw + (size_t)job.y * N;
-    const uint32_t rank = CL > 1 ? cg::this_cluster().block_rank() : 0;
+    const uint32_t rank = cg::this_cluster().block_rank();
     BcJob bc{};
     if (SRC == 3) bc = w.bc[jobi];
     const uint64_t *src = a.src + src_slot(a, SRC == 3 ? bc.in_slot0 : SRC ? job.x / a.src_div : job.x) * N;
@@ -175,8 +174,7 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs
 #pragma unroll
             for (int i = 0; i < (int)(sizeof(x) / 8); i++) slab[(e0 + i) * CC + c] = A::to_raw(x[i]);
         });
-    if (CL > 1) cg::this_cluster().sync();
-    else __syncthreads();
+    cg::this_cluster().sync();
     Epi e = epi;
     e.init(a, job, N);
     const uint32_t row0 = rank << LOG_CR;
@@ -186,7 +184,7 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs
 #pragma unroll
             for (int i = 0; i < (int)(sizeof(x) / 8); i++) {
                 const int col = el + i * step;
-                const uint64_t *peer = CL > 1 ? cg::this_cluster().map_shared_rank(slab, col >> LOG_CC) : slab;
+                const uint64_t *peer = cg::this_cluster().map_shared_rank(slab, col >> LOG_CC);
                 x[i] = A::from_raw(peer[(row0 + c) * CC + (col & (CC - 1))]);
             }
         },
@@ -200,8 +198,7 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs
             for (int i = 0; i < E; i++) y[i] = A::canon_fwd(x[i], k);
             e.template finish<E>(regs, o, y, md.q);
         });
-    (void)sizeof(T);
-    if (CL > 1) cg::this_cluster().sync();  // nobody leaves while a peer may still read its slab
+    cg::this_cluster().sync();  // nobody leaves while a peer may still read its slab
 }
 
 template <int LOGN, class Epi, int SRC>
@@ -264,13 +261,13 @@ __device__ __forceinline__ void whole_inv_tile(uint64_t *sm, const W2 *tw, uint3
 template <class A, int LOGN>
 __device__ __forceinline__ void whole_inv_body(const NttArgs &a, uint64_t *smem, const Job &job, const Mod &md) {
     using Cfg = WholeCfg<LOGN>;
-    constexpr int CL = 1 << Cfg::LOG_CL, LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
+    constexpr int LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
     constexpr int N2 = 1 << Cfg::LOG_B, CC = 1 << LOG_CC, CR = 1 << LOG_CR;
     constexpr size_t N = (size_t)1 << LOGN;
     uint64_t *slab = smem, *ex = smem + whole_slab<LOGN>();
     const typename A::K k = A::make(md, LOGN);
     const W2 *tw = a.tw + (size_t)job.y * N;
-    const uint32_t rank = CL > 1 ? cg::this_cluster().block_rank() : 0, row0 = rank << LOG_CR;
+    const uint32_t rank = cg::this_cluster().block_rank(), row0 = rank << LOG_CR;
     const uint64_t *src = a.src + src_slot(a, job.x) * N;
     uint64_t *dst = a.dst + dst_slot(a, job.w) * N;
     whole_inv_tile<A, Cfg::LOG_B, Cfg::RB2, Cfg::RB1, LOG_CR, false, false, Cfg::THREADS, A::B_CANON>(
@@ -296,15 +293,14 @@ __device__ __forceinline__ void whole_inv_body(const NttArgs &a, uint64_t *smem,
 #pragma unroll
             for (int i = 0; i < (int)(sizeof(x) / 8); i++) slab[c * N2 + e + i * step] = A::to_raw(x[i]);
         });
-    if (CL > 1) cg::this_cluster().sync();
-    else __syncthreads();
+    cg::this_cluster().sync();
     whole_inv_tile<A, Cfg::LOG_A, Cfg::RA2, Cfg::RA1, LOG_CC, true, true, Cfg::THREADS, A::GS_PASS>(
         ex, tw, 1u, a.fin + 2 * (size_t)job.z, k,
         [&](int c, int e0, auto &x) {
 #pragma unroll
             for (int i = 0; i < (int)(sizeof(x) / 8); i++) {
                 const int row = e0 + i;
-                const uint64_t *peer = CL > 1 ? cg::this_cluster().map_shared_rank(slab, row >> LOG_CR) : slab;
+                const uint64_t *peer = cg::this_cluster().map_shared_rank(slab, row >> LOG_CR);
                 x[i] = A::from_raw(peer[(row & (CR - 1)) * N2 + rank * CC + c]);
             }
         },
@@ -312,7 +308,7 @@ __device__ __forceinline__ void whole_inv_body(const NttArgs &a, uint64_t *smem,
 #pragma unroll
             for (int i = 0; i < (int)(sizeof(x) / 8); i++) dst[(size_t)(e + i * step) * N2 + rank * CC + c] = A::canon_inv(x[i], k);
         });
-    if (CL > 1) cg::this_cluster().sync();
+    cg::this_cluster().sync();
 }
 
 template <int LOGN>
