@@ -883,14 +883,18 @@ struct BatchDims {
     const uint32_t *perm = nullptr;  // inverse transforms: the input is read through this permutation
 };
 
-// Whether `limbs` transforms run as whole ones (ntt_whole.cuh says why the lines lie here)
-static bool use_whole(const b2_ctx *c, size_t limbs) { return c->logN == 12 && c->size_P <= 8 && limbs <= 1024; }
-static bool use_whole_plain(const b2_ctx *c, size_t limbs, const Job *jobs, uint32_t first_prime, uint32_t njobs, uint32_t period) {
-    if (c->logN == 12) return use_whole(c, limbs);
+// Whether `limbs` transforms run as whole ones, and whether a base conversion of alpha input limbs (fewer in a ragged digit) is
+// made while they load (ntt_whole.cuh says why the lines lie here)
+static bool use_whole(const b2_ctx *c, size_t limbs, const Job *jobs, uint32_t first_prime, uint32_t njobs, uint32_t period) {
+    if (c->logN == 12) return limbs <= 192;
     if ((c->logN != 13 && c->logN != 14) || jobs || limbs > 32) return false;
     for (uint32_t p = first_prime; p < first_prime + (period ? std::min(period, njobs) : njobs); p++)
         if (c->q[p] >= b2::FP_LIMIT) return false;
     return true;
+}
+static bool use_whole_bconv(const b2_ctx *c, size_t limbs) {
+    static constexpr size_t LINE[9] = {0, SIZE_MAX, SIZE_MAX, SIZE_MAX, 768, 384, 144, 96, 96};  // by alpha
+    return c->logN == 12 && c->size_P <= 8 && limbs <= LINE[c->size_P];
 }
 template <class Epi, int SRC> struct WholeHas : std::false_type {};
 template <> struct WholeHas<EpiStore, 0> : std::true_type {};
@@ -905,7 +909,7 @@ static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, period, src_div, src_q, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
     if (SRC != 0 && src_div == 0) return fail(B2_EINVAL, "the on-the-fly source needs its divisor");
     if constexpr (WholeHas<Epi, SRC>::value) {
-        if (SRC == 0 ? use_whole_plain(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, period) : use_whole(c, (size_t)njobs * bd.batch)) {
+        if ((SRC == 0 || c->logN == 12) && use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, period)) {
             LaunchScope ls(c, s, "ntt_fwd_whole");
             launch_fwd_whole<Epi, SRC>(a, epi, WholeArgs{}, njobs, bd.batch, s);
             LAUNCH_CHECK("ntt_fwd_whole");
@@ -930,7 +934,7 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
     NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, bd.perm};
-    if (use_whole_plain(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, 0)) {
+    if (use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, 0)) {
         LaunchScope ls(c, s, "ntt_inv_whole");
         launch_inv_whole(a, njobs, bd.batch, s);
         LAUNCH_CHECK("ntt_inv_whole");
@@ -1288,7 +1292,7 @@ static int modup_impl(b2_ctx *c, size_t l, const uint64_t *c2, uint64_t *out, ui
     bd.perm = perm;
     int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, bd);
     if (rc) return rc;
-    if (!copy_own && use_whole(c, pl.n_up_ntt)) return run_bconv_fwd(c, t, out, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s);
+    if (!copy_own && use_whole_bconv(c, pl.n_up_ntt)) return run_bconv_fwd(c, t, out, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s);
     rc = run_bconv(c, copy_own, t, out, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)(l + c->size_P), true, s, &pl.tc_up);
     if (rc) return rc;
     return run_fwd(c, out, out, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s);
@@ -1393,7 +1397,7 @@ static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint6
     const size_t a = c->size_P;
     int rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
     if (rc) return rc;
-    if (use_whole(c, 2 * l)) return run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{ct}, s);
+    if (use_whole_bconv(c, 2 * l)) return run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{ct}, s);
     rc = run_bconv(c, false, cxP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
     if (rc) return rc;
     return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
@@ -1421,7 +1425,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     const bool wide = (c->mac_wide < 0 ? batched : c->mac_wide == 1) && beta <= B2_MAC_MAX_BETA;
     // single calls at 2^15 run the stored row pass and the stand-alone inner product: the split by prime class costs two
     // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853)
-    const bool whole = batched && use_whole(c, (size_t)pl.n_up_ntt * kb.batch);
+    const bool whole = batched && use_whole_bconv(c, (size_t)pl.n_up_ntt * kb.batch);
     const bool mac = !whole && c->use_mac && (batched || c->logN == 16 || c->mac_wide == 1) && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
     if (!mac && !batched) return B2_OK;
     if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
@@ -1564,7 +1568,7 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     // ModDown of the P limbs of both polynomials of every set; delta takes the front of each set's `up` block
     rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{B, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
     if (rc) return rc;
-    if (use_whole(c, 2 * l * batch))
+    if (use_whole_bconv(c, 2 * l * batch))
         return run_bconv_fwd(c, cxP, up, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{d_ct, (uint32_t)ct_stride}, s,
                              BatchDims{B, 0, (uint32_t)(2 * a), 0, per});
     const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per, 0};
@@ -1972,7 +1976,7 @@ extern "C" int b2_rotate_sum(b2_ctx *c, size_t l, size_t n, const uint32_t *elts
         }
         int rc = run_inv(c, c1, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, (uint32_t)l, 0, (uint32_t)l});
         if (rc) return rc;
-        if (use_whole(c, (size_t)pl.n_up_ntt * B)) {
+        if (use_whole_bconv(c, (size_t)pl.n_up_ntt * B)) {
             rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
             if (rc) return rc;
         } else {
@@ -2094,7 +2098,7 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
         if (rc) return rc;
         rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
         if (rc) return rc;
-        if (use_whole(c, 2 * l * n)) {
+        if (use_whole_bconv(c, 2 * l * n)) {
             rc = run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), epi, s,
                                BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l)});
             if (rc) return rc;

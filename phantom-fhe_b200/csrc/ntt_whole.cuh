@@ -7,13 +7,26 @@
 // inverse: the mirror image. What this removes is one launch, one trip through global memory and - with the conversion
 // fused - a second launch and trip: a key switch at 2^12 is five launches instead of eleven.
 //
-// When it pays (measured on B200, forward + inverse / product + rescale): at 2^12 always (15.6 -> 11.1 us whatever the limbs
-// and the primes, product 65 -> 48 us; level from about a thousand limbs on). At 2^13 and 2^14 for plain transforms of up to
-// 32 limbs on FP64 primes (15.7 -> 12.5 us); integer primes lose (a thread's 3200 instructions run alone on its scheduler, and
-// two launches spread them over twice the SMs: 15.8 -> 17.6 us), and so do key switches, whose special primes are integer
-// ones (a rotation at 2^13 44 -> 48 us). At 2^15 a limb would want sixteen CTAs; with eight everything loses. The loops over
-// a thread's register groups are not unrolled: the code a lone CTA streams through is fetched once per launch
-// (unrolled, the rotation took 57 us).
+// When it pays (B200, us on the device, the launches queued behind a busy stream so that the host does not count; two passes ->
+// whole):
+//   2^12, plain transforms and rescales, up to 192 limbs a launch: a 60-bit prime among eight, 8 limbs 5.1 -> 5.0, 96 6.7 -> 6.4,
+//     192 8.4 -> 8.1, 256 10.8 -> 11.3, 1024 28.8 -> 30.9; FP64 primes 192 7.9 -> 7.6, 256 9.2 -> 9.9, 1024 25.1 -> 28.0; 60-bit
+//     primes 192 12.3 -> 11.9, 256 15.2 -> 15.1, 512 24.9 -> 25.2. Above, every SM has CTAs enough for either form, and the whole
+//     one's rendezvous and its reads of the neighbours' slabs show.
+//   2^12, conversions: every output limb reads its alpha inputs again and multiplies in FP64 or 64-bit integers, where the tensor
+//     cores convert all outputs from one read: the larger alpha, the earlier that weighs more than the saved launch and
+//     trip. Whole relinearisations: alpha 1, 25 limbs 35.5 -> 28.4, 3200 411 -> 316; alpha 2, 32 35.0 -> 28.6, 4096 507 -> 466;
+//     alpha 3, 3456 502 -> 493; alpha 4, 512 79.0 -> 77.0, 1024 134.6 -> 135.9; alpha 5, 360 73.3 -> 72.0, 540 93.1 -> 95.5;
+//     alpha 6, 96 38.5 -> 35.3, 192 43.8 -> 44.5; alpha 7, 84 42.1 -> 40.3, 112 45.0 -> 46.9; alpha 8, 72 37.1 -> 35.6, 144
+//     42.4 -> 44.8, 576 91.5 -> 111.3.
+//   2^13 and 2^14, plain transforms on FP64 primes, up to 32 limbs. What they save is the host's second launch, which a program
+//     that issues transforms one by one waits for (forward, 8 limbs: 2^13 9.9 -> 7.6, 2^14 9.8 -> 7.4, whatever the limbs).
+//     On the device alone: 2^14, 8 limbs 6.4 -> 5.9, 16 5.9 -> 6.7, 32 7.7 -> 7.3, 60 11.4 -> 10.9; 2^13, 8 limbs 5.3 -> 5.8, 32
+//     5.7 -> 6.1, 60 7.2 -> 7.3 (a thread's stages run alone on its scheduler, and two launches spread them over twice the SMs).
+//     With a 60-bit prime among the limbs 2^13 takes 7.1 -> 8.1 on the device, 9.8 -> 8.1 with the host; 2^14 9.2 -> 8.2 and
+//     9.9 -> 8.3: there the line could go. Key switches (job lists) lose at 2^13 (a rotation 44 -> 48 us).
+// At 2^15 a limb would want sixteen CTAs; with eight everything loses. The loops over a thread's register groups are not
+// unrolled: the code a lone CTA streams through is fetched once per launch (unrolled, the rotation took 57 us).
 //
 // No flag and no spin: cluster.sync() is the only rendezvous, and every thread of every CTA reaches it.
 #pragma once

@@ -504,3 +504,73 @@ def test_more_limbs_than_a_grid_dimension_holds():
     perm = torch.from_numpy(o.galois_perm(elt).astype(np.int64)).cuda()
     for t in range(0, n, 16384):
         assert torch.equal(dst[t: t + 16384], src[t: t + 16384][:, perm])
+
+
+@pytest.mark.parametrize("log_n,bits,l", [(12, [60, 40, 50, 60], 3), (13, [40, 50, 36, 30, 60], 4), (14, [50, 40, 30, 45, 60], 4)])
+def test_batched_transforms_on_both_sides_of_the_whole_ones(log_n, bits, l):
+    """a stack of polynomials transformed in one launch: 192 limbs at 2^12 and 32 at 2^13 and 2^14 are the last that run as whole
+    transforms, one polynomial more as two passes"""
+    from pyPhantom._native import LIB, check
+    N, line = 1 << log_n, 192 if log_n == 12 else 32
+    ctx, o = make_ctx(N, bits, 1)
+    base = [o.synth_signed(5, 70 + k) for k in range(3)]
+    want = torch.stack([dev(o.expand_single_chain(l, b)) for b in base])
+    for M in (line // l, line // l + 1):
+        src, out = torch.from_numpy(np.stack([base[m % 3] for m in range(M)])).cuda(), ctx.empty(M, l)
+        check(LIB.b2_expand_single_chain_batch(ctx._h, l, M, src.data_ptr(), out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(out, want[torch.arange(M, device="cuda") % 3])
+
+
+@pytest.mark.parametrize("batch", [1, 6, 7, 12, 13, 25])
+def test_key_switches_on_both_sides_of_the_whole_conversions(batch):
+    """2^12 with eight special primes: ModUp's 8 limbs a set and ModDown's 16 are converted while they load up to 96 a launch,
+    the inverse transforms' 8 run whole up to 192; every set of a batch as it is alone, the first and last as the oracle has
+    them, and so for hoisted and for summed rotations"""
+    from pyPhantom._native import LIB, check
+    N, l, n_elt = 4096, 8, 2
+    elts = [ph.get_elt_from_step(s, N) for s in (1, 2)]
+    ctx, o = make_ctx(N, [60] + [40, 50, 36, 40, 45, 40, 40] + [60] * 7 + [59], 8, elts)
+    key = o.synth_key(o.beta(l), 4, 10)
+    a, b = ([o.synth_ct(l, 4, at + i) for i in range(batch)] for at in (20, 60))
+    da, db, rk = dev(np.stack(a)), dev(np.stack(b)), _key(ctx, key)
+    got = ph.multiply_relin_rescale_batch(ctx, da, db, rk)
+    for i in range(batch):
+        assert torch.equal(got[i], ph.multiply_relin_rescale_batch(ctx, da[i: i + 1], db[i: i + 1], rk)[0])
+    for i in {0, batch - 1}:
+        assert np.array_equal(host(got[i]), o.rescale(l, o.multiply_and_relin(l, a[i], b[i], key)))
+    keys = [o.synth_key(o.beta(l), 6, 100 + 40 * i) for i in range(n_elt)]
+    rks = [_key(ctx, k) for k in keys]
+    glk, ct = ph.galois_key.from_keys(rks), ph.ciphertext.from_numpy(ctx, a[0], 1)
+    steps = [1 + i % 2 for i in range(batch)]
+    want = o.hoist_rotations(l, a[0], elts, keys)
+    for i, c in enumerate(ph.hoist_rotations(ctx, ct, glk, steps)):
+        assert np.array_equal(c.numpy(), want[i % 2])
+    tab = np.concatenate([rks[i % 2].pointer_table() for i in range(batch)])
+    e, nb = np.array([elts[i % 2] for i in range(batch)], dtype=np.uint32), int(LIB.b2_rotate_sum_workspace_bytes(ctx._h, l, batch))
+    ws, acc = torch.empty(nb // 8, dtype=torch.int64, device="cuda"), ctx.empty(2, l)
+    check(LIB.b2_rotate_sum(ctx._h, l, batch, e.ctypes.data, da.data_ptr(), 2 * l, tab.ctypes.data, o.beta(l), acc.data_ptr(), 1, ws.data_ptr(), nb,
+                            torch.cuda.current_stream().cuda_stream))
+    q = np.concatenate([o.primes[:l], o.primes[-8:]])[None, :, None]
+    cx, c0 = 0, 0
+    for i in range(batch):
+        turned = a[i][:, :, o.galois_perm(elts[i % 2])]
+        cx = (o.ks_inner_prod(l, o.modup(l, turned[1]), keys[i % 2]) + cx) % q
+        c0 = (turned[0] + c0) % q[0, :l]
+    want = np.stack([o.moddown(l, cx[k]) for k in range(2)])
+    want[0] = (want[0] + c0) % q[0, :l]
+    assert np.array_equal(host(acc), want)
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("sets", [32, 33])
+def test_rescales_on_both_sides_of_the_whole_ones(sets):
+    """2^12: six limbs a ciphertext, whole up to 192 a launch"""
+    from pyPhantom._native import LIB, check
+    N, l = 4096, 4
+    ctx, o = make_ctx(N, [60, 40, 50, 45, 60], 1)
+    cts = [o.synth_ct(l, 9, 700 + i) for i in range(sets)]
+    d, res, ws = dev(np.stack(cts)), torch.empty(sets, 2, l - 1, N, dtype=torch.int64, device="cuda"), ctx.empty(2 * sets)
+    check(LIB.b2_rescale_rounded_batch(ctx._h, l, sets, d.data_ptr(), res.data_ptr(), ws.data_ptr(), ws.numel() * 8, torch.cuda.current_stream().cuda_stream))
+    got = host(res)
+    for i in range(sets):
+        assert np.array_equal(got[i], o.rescale_rounded(l, cts[i]))
