@@ -1403,10 +1403,10 @@ static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint6
     return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
 }
 
-// ModUp and inner product of the fused key switch. At N = 2^16 (batched calls: 2^15 too) the inner product of the FP64 limbs
-// runs inside the last forward pass when the level's Q limbs are FP64 primes behind a prefix of wide ones; batched calls in
-// the other rings store both passes and run the stand-alone inner product, every kernel one launch over the batch
-// (N = 2^14, 8 limbs, 2 special primes, 32 products and rescales: 3045 us one set after another, 822 us so).
+// ModUp and inner product of the fused key switch. At N = 2^16 (batched calls: 2^15 too, and where fused_rows_pay says so) the
+// inner product of the FP64 limbs runs inside the last forward pass when the level's Q limbs are FP64 primes behind a prefix
+// of wide ones; other batched calls store both passes and run the stand-alone inner product, every kernel one launch over
+// the batch (N = 2^14, 8 limbs, 2 special primes, 32 products and rescales: 3045 us one set after another, 822 us so).
 // *done tells whether it ran.
 // ct [2][l][N] += (inner product) * P^-1 on the Q limbs; cxP [2][alpha][N] = (acc_p: +=) the P limbs of the inner product.
 // A batch of key switches with one key, every kernel one launch over the batch: set b's input, ciphertext, and its scratch
@@ -1415,6 +1415,23 @@ struct KsBatch {
     uint32_t batch = 1, c2_bs = 0, ct_bs = 0;
     KsRot rot;
 };
+
+// Whether a batch is better off with the row pass that carries the inner product than with a stored row pass and the stand-alone
+// kernel. It saves the digits' write and read, more of them the more digits there are, but a lone digit is its own input and
+// nothing is saved; and its CTAs, three an SM and three times as long on the special primes, want several waves. B200, stored /
+// fused, us a batch (limbs, special primes; waves of the fused pass):
+//   1 digit   2^15 (8, 8) 16 sets 9.2 waves 462 / 475; 2^16 (8, 8) 8 sets 9.2 471 / 484, 16 sets 18 897 / 899
+//   2 digits  2^15 (16, 8) 4 sets 3.5 238 / 249, 8 sets 6.9 430 / 429, 16 sets 14 820 / 794; 2^16 (16, 8) 3 sets 5.2 342 / 349,
+//             6 sets 10 637 / 621; (8, 4) 16 sets 14 897 / 872
+//   3 digits  2^15 (12, 4) 2 sets 1.2 121 / 130, 6 sets 3.5 296 / 292; (6, 2) 8 sets 2.3 231 / 234, 16 sets 4.6 426 / 422;
+//             2^16 (24, 8) 2 sets 4.6 363 / 355, 16 sets 37 2560 / 2322
+//   4 to 6    2^15 (20, 5) 2 sets 1.8 188 / 185, 16 sets 14 1208 / 1105; (14, 3) 2 sets 1.2 166 / 171, 3 sets 1.8 224 / 215;
+//             (12, 2) 2 sets 1.0 161 / 174, 3 sets 1.5 217 / 210
+static bool fused_rows_pay(const b2_ctx *c, size_t l, size_t beta, size_t sets) {
+    using Cfg = PassCfg<8>;
+    const size_t ctas = sets * (l + c->size_P) * (c->N >> (8 + Cfg::LOG_C)), half_waves = beta >= 4 ? 3 : beta == 3 ? 6 : 14;
+    return beta > 1 && 2 * ctas >= half_waves * 3 * (size_t)c->sm_count;
+}
 
 static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint64_t *const *evk, size_t n_evk, uint64_t *ct, uint64_t *cxP,
                              uint64_t *t, uint64_t *up, bool acc_p, cudaStream_t s, bool *done, const KsBatch &kb = KsBatch{}) {
@@ -1426,7 +1443,9 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     // single calls at 2^15 run the stored row pass and the stand-alone inner product: the split by prime class costs two
     // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853)
     const bool whole = batched && use_whole_bconv(c, (size_t)pl.n_up_ntt * kb.batch);
-    const bool mac = !whole && c->use_mac && (batched || c->logN == 16 || c->mac_wide == 1) && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
+    // (a switch that says which limbs ride on the fused pass asks for it)
+    const bool pays = batched ? c->mac_wide >= 0 || fused_rows_pay(c, l, beta, kb.batch) : c->logN == 16 || c->mac_wide == 1;
+    const bool mac = !whole && c->use_mac && pays && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
     if (!mac && !batched) return B2_OK;
     if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
         return B2_OK;  // the caller falls back to one key switch at a time
@@ -1445,8 +1464,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         }
         if (rc) return rc;
         if (!mac) {
-            // rings whose row pass is not the 256-point one (and keys of more than B2_MAC_MAX_BETA digits): both passes
-            // stored for every limb, then the stand-alone inner product, each one launch over the batch
+            // both passes stored for every limb, then the stand-alone inner product, each one launch over the batch
             if (!whole) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};

@@ -574,3 +574,40 @@ def test_rescales_on_both_sides_of_the_whole_ones(sets):
     got = host(res)
     for i in range(sets):
         assert np.array_equal(got[i], o.rescale_rounded(l, cts[i]))
+
+
+@pytest.mark.parametrize("log_n", [13, 14])
+@pytest.mark.parametrize("first,n", [(1, 1), (1, 32), (1, 33), (0, 1), (0, 5), (30, 5)])
+def test_transforms_of_ranges_of_limbs(log_n, first, n):
+    """forward and inverse, on FP64 primes alone (whole transforms up to 32 limbs) and with a 60-bit one at either end"""
+    from pyPhantom._native import LIB, check
+    N = 1 << log_n
+    ctx, o = make_ctx(N, [60] + [40, 50, 36] * 11 + [60], 1)
+    x = o.fill(1, o.primes[first: first + n], 9, 50)[0]
+    for call, want in ((LIB.b2_ntt_forward, o.ntt_forward(x, first)), (LIB.b2_ntt_inverse, o.ntt_inverse(x, first))):
+        d = dev(x)
+        check(call(ctx._h, d.data_ptr(), n, first, torch.cuda.current_stream().cuda_stream))
+        assert np.array_equal(host(d), want)
+
+
+@pytest.mark.parametrize("log_n,special,l,below", [
+    (15, 2, 6, 10),   # three digits: three waves of the fused pass
+    (15, 1, 4, 8),    # four digits: one and a half
+    (15, 3, 6, 21),   # two digits: seven
+    (16, 2, 5, 5),    # a ragged third digit
+    (16, 2, 2, 6),    # one digit: never fused
+])
+def test_batches_on_both_sides_of_the_fused_row_pass(log_n, special, l, below):
+    """products with the last batch that stores the row pass on 148 SMs and the first that fuses it: every set as it is alone, the
+    last as the oracle has it"""
+    N = 1 << log_n
+    ctx, o = make_ctx(N, [60, 40, 50, 36, 40, 45][:l] + [60] * (special - 1) + [59], special)
+    key = o.synth_key(o.beta(l), 4, 10)
+    rk, a, b = _key(ctx, key), o.synth_ct(l, 4, 20), o.synth_ct(l, 4, 40)
+    da, db = (torch.stack([dev(x)] + [dev(o.synth_ct(l, 4, at + i)) for i in range(1, 3)]) for x, at in ((a, 60), (b, 80)))
+    one = torch.stack([ph.multiply_relin_rescale_batch(ctx, da[i: i + 1], db[i: i + 1], rk)[0] for i in range(3)])
+    assert np.array_equal(host(one[0]), o.rescale(l, o.multiply_and_relin(l, a, b, key)))
+    for batch in (below, below + 1):
+        pick = torch.arange(batch, device="cuda") % 3
+        assert torch.equal(ph.multiply_relin_rescale_batch(ctx, da[pick], db[pick], rk), one[pick])
+    assert ctx.device_status() == 0
