@@ -51,12 +51,14 @@ def test_emulated_ranks_reproduce_the_key_switch(world, l):
 
 
 @pytest.mark.parametrize("world,batch", [(1, 3), (2, 4), (3, 2), (8, 5)])
-@pytest.mark.parametrize("shape", ["n12", "n16"])
+@pytest.mark.parametrize("shape", ["n12", "n15", "n16"])
 def test_emulated_ranks_reproduce_a_batch_of_key_switches(world, batch, shape):
     """the batched phases (one launch per kernel over the whole batch, limb-major exchange buffers) with the ranks run one
     after another on shared buffers: every ciphertext of the batch must come out as the unsharded key switch gives it"""
     if shape == "n12":
         N, bits, special, levels = 4096, [55, 40, 41, 42, 43, 44, 45, 46, 58, 59, 60], 3, [8, 5]
+    elif shape == "n15":  # the fused row pass behind a 128-point column pass
+        N, bits, special, levels = 32768, [60, 40, 45, 50, 36, 60, 59], 2, [5, 2]
     else:
         N, bits, special, levels = 65536, [60] + [40] * 23 + [60] * 8, 8, [24]
         if world == 3:
