@@ -241,7 +241,7 @@ int b2_rotate_sum(b2_ctx *ctx, size_t size_Ql, size_t n, const uint32_t *elts, c
 
 /* replaces hoisting_inplace (src/evaluate.cu:1732-1927): d_out [2][size_Ql][N] = the SUM over the n_steps Galois
  * elements of the rotated d_ct, from one ModUp of c1 and one ModDown per polynomial (ksk and workspace as for
- * b2_hoist_rotations; d_out must not alias d_ct) */
+ * b2_hoist_rotations; d_out may overlap d_ct) */
 int b2_hoisting_sum(b2_ctx *ctx, size_t size_Ql, const uint64_t *d_ct, const uint32_t *elts, size_t n_steps,
                     const uint64_t *const *ksk, size_t n_evk, uint64_t *d_out, void *d_ws, size_t ws_bytes,
                     void *stream);
@@ -252,7 +252,8 @@ int b2_hoisting_sum(b2_ctx *ctx, size_t size_Ql, const uint64_t *d_ct, const uin
  *                               d_accP [2][size_P][N] (+)= P limbs of the same inner product;
  *                               first != 0 starts a new sum (both accumulators are overwritten);
  *   b2_keyswitch_finish:        d_acc -= NTT(BConv(INTT(d_accP)) * P^-1); d_accP is consumed.
- * One accumulate + finish equals b2_apply_galois bit for bit. Workspace: B2_OP_ROTATE bytes for accumulate,
+ * One accumulate + finish equals b2_apply_galois bit for bit; b2_rotate_sum does the whole sum in one call and is faster.
+ * For callers whose ciphertexts come one at a time. Workspace: B2_OP_ROTATE bytes for accumulate,
  * 2 * size_Ql limbs for finish. */
 int b2_apply_galois_accumulate(b2_ctx *ctx, size_t size_Ql, uint32_t galois_elt, const uint64_t *d_ct,
                                const uint64_t *const *ksk, size_t n_evk, uint64_t *d_acc, uint64_t *d_accP,

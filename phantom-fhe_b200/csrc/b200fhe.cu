@@ -243,13 +243,13 @@ struct b2_ctx {
     uint32_t *d_err = nullptr;     // device status word: set by a kernel whose bounded wait ran out
     std::vector<uint64_t> h_mat_dn, h_mat_dn_pinv;  // host copies of the ModDown matrices [size_Q][size_P]
     bool mac_interleave = false;   // B2_KS_FUSED_ORDER=1: consecutive CTAs of the fused pass walk limbs, not tiles (measured slower)
-    // The fused pass may also take the limbs on primes of 41 bits and more (q0 and P at the usual parameters): 10 launches
-    // instead of 12 and no stored digits at all. Measured on B200 at N = 2^16, l = 24: single calls lose 4 % of their
-    // four-stream throughput to it (the stand-alone inner product is memory-bound and hides behind other streams' transforms;
-    // fused, it is integer-multiply work) though a lone key switch gains 8 us; batched calls gain 1 %. So it is on for
-    // batched calls and off for single ones unless B2_KS_FUSED_WIDE = 0 | 1 says otherwise.
+    // The fused pass may also take the limbs on primes of 50 bits and more (q0 and P at the usual parameters): 10 launches
+    // instead of 12 and no stored digits at all. Batched calls do (1 % more per second at N = 2^16, l = 24), single calls do
+    // not: key switches per second over four streams / on one at those sizes 6398 / 4853 with the FP64 limbs on it, 5862 / 4841
+    // with all of them, 6088 / 4923 with none (the stand-alone inner product of the 60-bit limbs is memory-bound and hides
+    // behind other streams' transforms; fused, it is integer-multiply work). B2_KS_FUSED_WIDE = 0 | 1 says otherwise.
     int mac_wide = -1;
-    bool use_mac = false;          // N = 2^15, 2^16: ModUp's last forward pass carries the inner product (off with B2_KS_FUSED_IP=0)
+    bool use_mac = false;          // N = 2^15, 2^16: ModUp's last forward pass may carry the inner product (off with B2_KS_FUSED_IP=0)
     int sm_count = 148;
     // RNS-limb sharding of one ciphertext over `shard_world` GPUs: this rank's slice of every list
     int shard_rank = 0, shard_world = 1;
@@ -1441,7 +1441,8 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     const bool batched = kb.batch != 1;
     const bool wide = (c->mac_wide < 0 ? batched : c->mac_wide == 1) && beta <= B2_MAC_MAX_BETA;
     // single calls at 2^15 run the stored row pass and the stand-alone inner product: the split by prime class costs two
-    // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853)
+    // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853);
+    // those at 2^16 the FP64 limbs' fused pass (mac_wide has the figures)
     const bool whole = batched && use_whole_bconv(c, (size_t)pl.n_up_ntt * kb.batch);
     // (a switch that says which limbs ride on the fused pass asks for it)
     const bool pays = batched ? c->mac_wide >= 0 || fused_rows_pay(c, l, beta, kb.batch) : c->logN == 16 || c->mac_wide == 1;

@@ -1,7 +1,8 @@
 // modarith.cuh - 64-bit modular arithmetic for RNS limbs on sm_100a.
 //
-// All kernels keep residues as uint64 and use the primes' Shoup / Barrett constants. Inside a
-// transform values are kept lazily in [0,4q) (forward) or [0,2q) (inverse); every kernel's
+// Buffers hold residues as uint64 and the kernels use the primes' Shoup / Barrett constants. Inside
+// a transform values are kept lazily, within bounds that depend on the arithmetic of the prime
+// (the policies of ntt_kernels.cuh: 64-bit words up to 2, 4 or 16 q, or doubles); every kernel's
 // final store is canonical, i.e. in [0,q). That is the only property the reference's kernels
 // guarantee too (include/uintmodmath.cuh:96-136, 207-215; include/butterfly.cuh:17-71), so
 // outputs are bit-identical although the butterfly schedule differs.

@@ -16,7 +16,7 @@
 //       index = (P << s) + k'
 //   inverse, local stage with gap 2^u, pair group k':
 //       index = ((T >> (u + 1)) * P) + k'
-// Lazy ranges: forward keeps [0,4q), inverse keeps [0,2q); the last pass stores canonical values.
+// Lazy ranges are those of the prime's arithmetic policy (below); the last pass stores canonical values.
 #pragma once
 #include <type_traits>
 #include "modarith.cuh"
@@ -638,11 +638,13 @@ ntt_fwd_pass(NttArgs a, Epi epi) {
 }
 
 // ================================================================================================
-// Last forward (row) pass of ModUp fused with the key-switch inner product, for the limbs on FP64 primes.
+// Last forward (row) pass of ModUp fused with the key-switch inner product, for the limbs on FP64 primes (single calls) or
+// for all of them (batched calls).
 // A CTA owns one tile of one output limb t and walks the digits: the digit that holds limb t itself contributes the
 // NTT-form input as it is, every other digit's limb t is finished here (row pass of its column-pass output) and never
-// stored. Both polynomials of the key are multiplied in and accumulated in FP64 (|sum| < beta q), reduced once, and
-// ct[k][t] += sum_k * P^-1 as the stand-alone inner-product kernel does. Same residues as that kernel.
+// stored. Both polynomials of the key are multiplied in and summed - on FP64 primes in FP64 (|sum| < beta q), on the others
+// as Montgomery products in one word (MacAcc) -, reduced once, and ct[k][t] += sum_k * P^-1, or the P limb stored, as the
+// stand-alone inner-product kernel does. Same residues as that kernel.
 // ================================================================================================
 #define B2_MAC_MAX_BETA 8
 struct MacArgs {
@@ -668,12 +670,6 @@ struct MacArgs {
     const uint64_t *c0;
     uint32_t ct_set, c0_bs;  // c0 of set b of a batch starts b * c0_bs limbs further
 };
-
-__device__ __forceinline__ u64x4 ld256_cs(const uint64_t *p) {  // streaming: the key is read once
-    u64x4 v;
-    asm("ld.global.cs.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.a), "=l"(v.b), "=l"(v.c), "=l"(v.d) : "l"(p));
-    return v;
-}
 
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);

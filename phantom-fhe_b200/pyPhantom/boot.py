@@ -7,8 +7,8 @@ BSGS linear transforms, EvalRound on the real and imaginary halves, SlotToCoeff,
 subtraction  ct_raised - q0 * I  that leaves the message on the user levels. The linear transforms
 and the polynomial evaluation are this library's own arrangement (see bootmath.py):
 
-* the top three primes carry CoeffToSlot (three layers; they may be short primes, because EvalRound
-  is flat around the integers and does not pass CoeffToSlot's rounding errors on);
+* the top three primes carry CoeffToSlot (two layers on short primes, which EvalRound allows: it is
+  flat around the integers and passes on little of CoeffToSlot's rounding errors; else three);
 * the next ten carry EvalRound: a degree-63 Chebyshev cosine by Paterson-Stockmeyer (7 levels) and
   three double-angle steps;
 * the next two carry SlotToCoeff in two layers, whose last plaintext scale is chosen so that the
@@ -212,7 +212,8 @@ class CtOps:
 
 # ---- one layer of a linear transform, compiled to device plaintexts ----------------------------------------
 class _Layer:
-    """the LayerPlan of bootmath with every pre-rotated diagonal encoded at (limbs, scale) and resident in HBM"""
+    """the LayerPlan of bootmath with every pre-rotated diagonal encoded at (limbs, scale) and resident in HBM; its babies and
+    partial sums have buffers here, so one transform at a time"""
 
     def __init__(self, ctx, encoder, plan, limbs, scale, value_factor=1.0, rescales=1):
         self.limbs, self.scale, self.n = limbs, float(scale), plan.n
@@ -488,8 +489,9 @@ def _eval_round_pair(ops, bk, lo, hi):
 def bootstrap(context, encoder, ct, bk, user_scale, split_scale_down=False, stats=None):
     """python/src/binding.cu:329-336; src/bootstrap.cu:1702-1949: see bootstrap_eager for the pipeline. The
     sequence of launches depends only on the input's level and scale, so after one eager run (which also
-    warms every lazily built table) the whole pipeline is captured into a CUDA graph - its streams become
-    parallel branches - and later calls copy the input into the graph's buffer and replay it."""
+    warms every lazily built table) the whole pipeline is captured into a CUDA graph, and later calls
+    copy the input into the graph's buffer and replay it. The key's layers and the graph hold buffers: calls with one key
+    belong on one stream, or one waits for the other."""
     if not bk.use_graph or stats is not None or torch.cuda.is_current_stream_capturing():
         return bootstrap_eager(context, encoder, ct, bk, user_scale, split_scale_down, stats)
     key = (ct._limbs, ct._chain_index, ct._scale, ct._size, bool(split_scale_down), torch.cuda.current_device())

@@ -13,6 +13,8 @@ chain of dependent rotations. On a GPU with 180 GB of HBM the expanded diagonals
 
 It needs a Galois key for every baby step 1..M-1 and every giant step M, 2M, .. (G-1)M (the "64 + 64 keys" form);
 the result decrypts to the same product as the reference's driver but is not limb-identical to it (hoisted babies).
+Babies and partial sums live in buffers of the plan: two products of one plan belong on one stream, or the second waits for the
+first; concurrent ones take a plan each.
 """
 import numpy as np
 import torch
