@@ -202,7 +202,7 @@ class context:
             if streams is None:
                 while len(self._product_streams) >= 16:
                     self._product_streams.popitem(last=False)
-                streams = tuple(torch.cuda.Stream(priority=p) for p in (0, 0, -1, -1))
+                streams = tuple(torch.cuda.Stream(self.device, priority=p) for p in (0, 0, -1, -1))
             self._product_streams[key] = streams
         return streams
 

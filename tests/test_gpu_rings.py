@@ -344,6 +344,7 @@ def test_matrix_products_of_two_streams_do_not_wait_for_one_another():
     for s in streams + [streams[0]]:
         with torch.cuda.stream(s):
             sets.append([t.cuda_stream for t in ctx.product_streams()])
+            assert {t.device.index for t in ctx.product_streams()} == {ctx.device}
     assert sets[0] == sets[2] and not set(sets[0]) & set(sets[1])
 
 
