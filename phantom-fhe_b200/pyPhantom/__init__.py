@@ -858,8 +858,8 @@ class single_chain_plaintext:
     def __getstate__(self):
         return {"scale": self.scale, "coeffs": self._coeffs}
 
-    def __setstate__(self, state):  # a copy's vector lies elsewhere, and is pinned or not
-        self.scale, self.coeffs = state["scale"], state["coeffs"]
+    def __setstate__(self, state):  # a copy's vector lies elsewhere, and is pinned or not; files of other versions name it _coeffs
+        self.scale, self.coeffs = state["scale"], state["coeffs" if "coeffs" in state else "_coeffs"]
 
     def coeffs_bytes(self):
         return self.coeffs.numpy().tobytes()

@@ -142,3 +142,14 @@ def test_stream_lookup_without_torchs_private_functions(monkeypatch, gone):
     monkeypatch.delattr(torch._C, gone)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
     assert _native._stream_lookup()() == 77
+
+
+def test_single_chain_plaintexts_of_earlier_files_load():
+    """pickles hold the scale and the vector, under either name; an address written by an earlier version is not taken over"""
+    import copy
+    import pickle
+    scp = ph.single_chain_plaintext(np.arange(-8, 8), 2.0 ** 20)
+    old = ph.single_chain_plaintext.__new__(ph.single_chain_plaintext)
+    old.__setstate__({"scale": 2.0 ** 20, "_coeffs": scp.coeffs.clone(), "_readable": 4096, "_numel": 16})
+    for c in (old, copy.deepcopy(scp), pickle.loads(pickle.dumps(scp))):
+        assert c.get_scale() == 2.0 ** 20 and c.coeffs_bytes() == scp.coeffs_bytes() and c.readable_at() == 0
