@@ -134,6 +134,7 @@ class context:
             raise RuntimeError("pyPhantom needs a CUDA device: there is no CPU path")
         self.device = torch.cuda.current_device()
         self.N = parms._N
+        self._workspace_bytes = {}  # (operation, limbs) -> bytes
         self._product_streams, self._product_lock = collections.OrderedDict(), threading.Lock()
         self.primes = np.array([m.value() for m in parms._coeff_modulus], dtype=np.uint64)
         self.primes_signed = self.primes.view(np.int64)
@@ -207,7 +208,9 @@ class context:
         return streams
 
     def workspace(self, op, l):
-        nbytes = int(LIB.b2_workspace_bytes(self._h, op, l))
+        nbytes = self._workspace_bytes.get((op, l))
+        if nbytes is None:
+            nbytes = self._workspace_bytes[op, l] = int(LIB.b2_workspace_bytes(self._h, op, l))
         return torch.empty(max(nbytes // 8, 1), dtype=torch.int64, device=self.device), nbytes
 
     def table(self, which, prime_idx):
@@ -373,9 +376,12 @@ class relin_key:
         return k
 
     def pointer_table(self):
-        if self._ptrs is None or len(self._ptrs) != len(self.public_keys):
-            self._ptrs = np.array([pk.data.data_ptr() for pk in self.public_keys], dtype=np.uint64)
-        return self._ptrs
+        """the addresses of the digits, as the C ABI takes them; the array is kept while they are the same"""
+        now = [pk.data.data_ptr() for pk in self.public_keys]
+        kept = self._ptrs
+        if kept is None or kept[0] != now:
+            kept = self._ptrs = now, np.array(now, dtype=np.uint64)
+        return kept[1]
 
     def mod_drop_to_inplace(self, context, target_chain_index):
         """src/secretkey.cu:301-352: keep only the ceil(size_Ql / alpha) digits a key switch at `target_chain_index` (or any

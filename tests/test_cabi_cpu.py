@@ -153,3 +153,18 @@ def test_single_chain_plaintexts_of_earlier_files_load():
     old.__setstate__({"scale": 2.0 ** 20, "_coeffs": scp.coeffs.clone(), "_readable": 4096, "_numel": 16})
     for c in (old, copy.deepcopy(scp), pickle.loads(pickle.dumps(scp))):
         assert c.get_scale() == 2.0 ** 20 and c.coeffs_bytes() == scp.coeffs_bytes() and c.readable_at() == 0
+
+
+def test_pointer_table_follows_the_digits():
+    """a copied key, a digit put in another's place and one whose data moved: the table names the tensors the key holds"""
+    import copy
+    key = ph.relin_key()
+    for _ in range(3):
+        ct = ph.ciphertext()
+        ct.data = torch.zeros(2, 2, 8, dtype=torch.int64)
+        key.public_keys.append(ct)
+    assert key.pointer_table() is key.pointer_table()
+    for other in (key, copy.deepcopy(key)):
+        other.public_keys[1] = other.public_keys[1].clone()
+        other.public_keys[2].data = other.public_keys[2].data.clone()
+        assert other.pointer_table().tolist() == [pk.data.data_ptr() for pk in other.public_keys]
