@@ -847,15 +847,16 @@ static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const 
 }
 
 // the forward column pass alone, for the rings whose row pass has 256 points (2^15, 2^16)
-template <int LOG_A>
+template <int LOG_A, int SRC>
 static void launch_fwd_cols_n(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
     using A = PassCfg<LOG_A>;
     LaunchScope ls(c, s, "ntt_fwd_cols");
-    launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore>, dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
+    launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC>, dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
 }
+template <int SRC>
 static void launch_fwd_cols(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
-    if (a.logN == 16) launch_fwd_cols_n<8>(c, a, njobs, s, batch);
-    else launch_fwd_cols_n<7>(c, a, njobs, s, batch);
+    if (a.logN == 16) launch_fwd_cols_n<8, SRC>(c, a, njobs, s, batch);
+    else launch_fwd_cols_n<7, SRC>(c, a, njobs, s, batch);
 }
 
 template <int LOG_A, int LOG_B>
@@ -883,8 +884,7 @@ struct BatchDims {
     const uint32_t *perm = nullptr;  // inverse transforms: the input is read through this permutation
 };
 
-// Whether `limbs` transforms run as whole ones, and whether a base conversion of alpha input limbs (fewer in a ragged digit) is
-// made while they load (ntt_whole.cuh says why the lines lie here)
+// Whether `limbs` transforms run as whole ones (ntt_whole.cuh says why the lines lie here)
 static bool use_whole(const b2_ctx *c, size_t limbs, const Job *jobs, uint32_t first_prime, uint32_t njobs, uint32_t period) {
     if (c->logN == 12) return limbs <= 192;
     if ((c->logN != 13 && c->logN != 14) || jobs || limbs > 32) return false;
@@ -892,9 +892,27 @@ static bool use_whole(const b2_ctx *c, size_t limbs, const Job *jobs, uint32_t f
         if (c->q[p] >= b2::FP_LIMIT) return false;
     return true;
 }
-static bool use_whole_bconv(const b2_ctx *c, size_t limbs) {
-    static constexpr size_t LINE[9] = {0, SIZE_MAX, SIZE_MAX, SIZE_MAX, 768, 384, 144, 96, 96};  // by alpha
-    return c->logN == 12 && c->size_P <= 8 && limbs <= LINE[c->size_P];
+// Whether a base conversion of alpha input limbs (fewer in a ragged digit) is made while the `limbs` transforms behind it load
+// (2^12: whole transforms, lines as in ntt_whole.cuh)
+static bool convert_loading(const b2_ctx *c, size_t limbs) {
+    if (c->size_P > 8 || c->logN == 17) return false;
+    if (c->logN == 12) {
+        static constexpr size_t LINE[9] = {0, SIZE_MAX, SIZE_MAX, SIZE_MAX, 768, 384, 144, 96, 96};  // limbs, by alpha
+        return limbs <= LINE[c->size_P];
+    }
+    // Column passes of the other rings, 2048 residues a CTA; lines in CTAs, by alpha. Up to two input limbs the saved launch and
+    // trip are worth more at every size; with more, the limbs read and multiplied again for every output show sooner or later,
+    // at 2^13 later (three of the six column stages of a thread are behind it). B200, us, conversion kernel / in the column pass:
+    //   alpha 1: relinearisations 2^13, 6 limbs, 32 sets 240 / 207; 2^14, 8 limbs, 32 sets 678 / 609; 2^16, 4 limbs, 16 sets 524 / 470
+    //   alpha 2: rotations 2^13, 8 limbs 47.6 / 39.5; 2^14, 6 limbs 55.8 / 52.7; 2^16, 24 limbs 362 / 354; relinearisations 2^13,
+    //     128 sets 899 / 847; 2^14, 64 sets 928 / 908; 2^15, 32 sets 880 / 855; 2^16, 8 sets 480 / 470
+    //   alpha 3: rotations 2^13, 92 CTAs 44.9 / 37.8; 2^15, 1136 CTAs 97.8 / 93.6; 2^16, 384 CTAs 87.7 / 81.4; relinearisations 2^13,
+    //     1536 CTAs 108.7 / 105.8; 2^14, 1536 CTAs 118.7 / 119.5; 2^15, 9088 CTAs 444 / 453; 2^16, 3072 CTAs 208 / 215
+    //   alpha 4: 2^13, 144 CTAs 47.6 / 41.2, 576 CTAs 59.8 / 54.0, 1152 CTAs 101.3 / 101.5; 2^14, 128 CTAs 54.7 / 57.8; 2^16 97 / 104
+    //   alpha 5 to 8: 2^13, 80 CTAs 43.6 / 39.0, 320 CTAs 54.5 / 49.0, alpha 8 288 CTAs 53.0 / 51.0, 512 CTAs 74.9 / 85.0; 2^14, 160
+    //     CTAs 56.9 / 61.7; 2^15, 720 CTAs 89.3 / 93.6
+    static constexpr size_t LINE13[9] = {0, SIZE_MAX, SIZE_MAX, 1536, 1024, 320, 320, 288, 288}, LINE[9] = {0, SIZE_MAX, SIZE_MAX, 1152};
+    return limbs * (c->N / 2048) <= (c->logN == 13 ? LINE13 : LINE)[c->size_P];
 }
 template <class Epi, int SRC> struct WholeHas : std::false_type {};
 template <> struct WholeHas<EpiStore, 0> : std::true_type {};
@@ -911,7 +929,7 @@ static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     if constexpr (WholeHas<Epi, SRC>::value) {
         if ((SRC == 0 || c->logN == 12) && use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, period)) {
             LaunchScope ls(c, s, "ntt_fwd_whole");
-            launch_fwd_whole<Epi, SRC>(a, epi, WholeArgs{}, njobs, bd.batch, s);
+            launch_fwd_whole<Epi, SRC>(a, epi, njobs, bd.batch, s);
             LAUNCH_CHECK("ntt_fwd_whole");
             return B2_OK;
         }
@@ -953,15 +971,25 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     return B2_OK;
 }
 
-// base conversion and forward transform in one launch: job j's limb is made from the input limbs bc[j] names
+// base conversion made while the forward transform loads: job j's limb comes from the input limbs bc[j] names (2^12: one launch in
+// all, the other rings: in the column pass)
 template <class Epi>
 static int run_bconv_fwd(const b2_ctx *c, const uint64_t *in, uint64_t *dst, const Job *jobs, const BcJob *bc, const W2 *mat, uint32_t njobs, const Epi &epi,
                          cudaStream_t s, const BatchDims &bd = BatchDims{}) {
     if (!aligned32(in) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
     NttArgs a{in, dst, jobs, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
-    LaunchScope ls(c, s, "bconv_ntt_whole");
-    launch_fwd_whole<Epi, 3>(a, epi, WholeArgs{bc, mat}, njobs, bd.batch, s);
-    LAUNCH_CHECK("bconv_ntt_whole");
+    a.bc = bc, a.mat = mat;
+    switch (c->logN) {
+        case 16: launch_fwd<8, 8, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
+        case 15: launch_fwd<7, 8, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
+        case 14: launch_fwd<7, 7, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
+        case 13: launch_fwd<6, 7, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
+        default: {
+            LaunchScope ls(c, s, "bconv_ntt_whole");
+            launch_fwd_whole<Epi, 3>(a, epi, njobs, bd.batch, s);
+        }
+    }
+    LAUNCH_CHECK("bconv_ntt_fwd");
     return B2_OK;
 }
 
@@ -1292,7 +1320,7 @@ static int modup_impl(b2_ctx *c, size_t l, const uint64_t *c2, uint64_t *out, ui
     bd.perm = perm;
     int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, bd);
     if (rc) return rc;
-    if (!copy_own && use_whole_bconv(c, pl.n_up_ntt)) return run_bconv_fwd(c, t, out, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s);
+    if (!copy_own && convert_loading(c, pl.n_up_ntt)) return run_bconv_fwd(c, t, out, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s);
     rc = run_bconv(c, copy_own, t, out, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)(l + c->size_P), true, s, &pl.tc_up);
     if (rc) return rc;
     return run_fwd(c, out, out, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s);
@@ -1397,7 +1425,7 @@ static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint6
     const size_t a = c->size_P;
     int rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s);
     if (rc) return rc;
-    if (use_whole_bconv(c, 2 * l)) return run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{ct}, s);
+    if (convert_loading(c, 2 * l)) return run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{ct}, s);
     rc = run_bconv(c, false, cxP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
     if (rc) return rc;
     return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
@@ -1443,10 +1471,10 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     // single calls at 2^15 run the stored row pass and the stand-alone inner product: the split by prime class costs two
     // launches more, which a grid of that size does not win back (11 key switches of a polynomial: 2676 us against 2853);
     // those at 2^16 the FP64 limbs' fused pass (mac_wide has the figures)
-    const bool whole = batched && use_whole_bconv(c, (size_t)pl.n_up_ntt * kb.batch);
+    const bool loading = convert_loading(c, (size_t)pl.n_up_ntt * kb.batch);
     // (a switch that says which limbs ride on the fused pass asks for it)
     const bool pays = batched ? c->mac_wide >= 0 || fused_rows_pay(c, l, beta, kb.batch) : c->logN == 16 || c->mac_wide == 1;
-    const bool mac = !whole && c->use_mac && pays && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
+    const bool mac = c->use_mac && pays && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
     if (!mac && !batched) return B2_OK;
     if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
         return B2_OK;  // the caller falls back to one key switch at a time
@@ -1455,18 +1483,18 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         const uint32_t B = kb.batch, per = (uint32_t)(beta * lP), a2 = (uint32_t)(2 * c->size_P);
         int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, kb.c2_bs, 0, (uint32_t)l, kb.rot.perm});
         if (rc) return rc;
-        if (whole) {
+        if (loading && !mac) {
             rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
-        } else if (batched) {
+        } else if (!loading && batched) {
             const TcBatch tb{B, 0, (uint32_t)l, 0, per, c->tc_serial_ld ? 1u : 0u};
             rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, &tb);
-        } else {
+        } else if (!loading) {
             rc = run_bconv(c, false, t, up, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)lP, true, s, &pl.tc_up);
         }
         if (rc) return rc;
         if (!mac) {
             // both passes stored for every limb, then the stand-alone inner product, each one launch over the batch
-            if (!whole) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            if (!loading) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
             rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib, kb.rot);
@@ -1478,7 +1506,13 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         // product still handles (wide Q primes and P); for the FP64 limbs of Q it runs inside ntt_fwd_rows_mac
         NttArgs a{up, up, pl.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
         a.src_bs = a.dst_bs = batched ? per : 0;
-        launch_fwd_cols(c, a, pl.n_up_ntt, s, B);
+        if (loading) {
+            NttArgs b = a;
+            b.src = t, b.src_bs = batched ? (uint32_t)l : 0, b.bc = pl.bc_up, b.mat = pl.matw_up;
+            launch_fwd_cols<3>(c, b, pl.n_up_ntt, s, B);
+        } else {
+            launch_fwd_cols<0>(c, a, pl.n_up_ntt, s, B);
+        }
         LAUNCH_CHECK("ntt_fwd_pass");
         // the limbs on 60-bit primes (q0, P) either ride on the fused pass too (integer arithmetic) or, mac_wide off,
         // keep the stored row pass and the stand-alone inner product
@@ -1587,7 +1621,7 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     // ModDown of the P limbs of both polynomials of every set; delta takes the front of each set's `up` block
     rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{B, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
     if (rc) return rc;
-    if (use_whole_bconv(c, 2 * l * batch))
+    if (convert_loading(c, 2 * l * batch))
         return run_bconv_fwd(c, cxP, up, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{d_ct, (uint32_t)ct_stride}, s,
                              BatchDims{B, 0, (uint32_t)(2 * a), 0, per});
     const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per, 0};
@@ -1995,7 +2029,7 @@ extern "C" int b2_rotate_sum(b2_ctx *c, size_t l, size_t n, const uint32_t *elts
         }
         int rc = run_inv(c, c1, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, (uint32_t)l, 0, (uint32_t)l});
         if (rc) return rc;
-        if (use_whole_bconv(c, (size_t)pl.n_up_ntt * B)) {
+        if (convert_loading(c, (size_t)pl.n_up_ntt * B)) {
             rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
             if (rc) return rc;
         } else {
@@ -2117,7 +2151,7 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
         if (rc) return rc;
         rc = run_inv(c, cxP, cxP, pl.jobs_dnf_intt, (uint32_t)(2 * a), 0, c->d_fin_P, s, BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * a)});
         if (rc) return rc;
-        if (use_whole_bconv(c, 2 * l * n)) {
+        if (convert_loading(c, 2 * l * n)) {
             rc = run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), epi, s,
                                BatchDims{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l)});
             if (rc) return rc;
@@ -2839,7 +2873,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 NttArgs na{UP, UP, sp.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
                 na.src_bs = na.dst_bs = per;
                 if (sp.n_up_ntt) {
-                    launch_fwd_cols(c, na, sp.n_up_ntt, s, B);
+                    launch_fwd_cols<0>(c, na, sp.n_up_ntt, s, B);
                     LAUNCH_CHECK("ntt_fwd_pass");
                 }
                 MacArgs m{};

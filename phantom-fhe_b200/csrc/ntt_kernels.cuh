@@ -43,6 +43,11 @@ constexpr int ntt_min_blocks(int threads, int residues_per_thread = 16) {
     return (B2_NTT_RESIDENT_THREADS / (residues_per_thread > 16 ? 2 : 1)) / threads > 0 ? (B2_NTT_RESIDENT_THREADS / (residues_per_thread > 16 ? 2 : 1)) / threads : 1;
 }
 
+// One output limb of a base conversion: sum_i y_i[n] M_i mod p over `ni` input limbs from slot in_slot0 on; M_i at mat_off + i
+// as {M, floor(M 2^64 / p)}; bit i of `wide`: input limb i holds residues of a prime of 2^50 or more
+struct BcJob {
+    uint32_t in_slot0, ni, mat_off, wide;
+};
 struct NttArgs {
     const uint64_t *src;  // limb `slot` at src + slot * N
     uint64_t *dst;
@@ -62,6 +67,8 @@ struct NttArgs {
     // Batch-major buffers [b][slots] use lm1 = 0, bs = slots per set; limb-major ones [slot][b] use lm1 = batch - 1, bs = 1.
     uint32_t src_lm1, src_bs, dst_lm1, dst_bs;
     const uint32_t *perm;  // inverse row pass: the input is read through a Galois element's permutation (a rotation's c1)
+    const BcJob *bc;       // SRC = 3: one per job, the conversion that makes its limb, and the matrix entries
+    const W2 *mat;
 };
 
 // The sets of a batched launch are the slow grid dimension. With the sets fastest (the CTAs of all sets on one tile next to
@@ -535,17 +542,82 @@ __device__ __forceinline__ void gs_stages(typename A::T (&x)[E], const W2 *tw, s
     }
 }
 
+// term y M of a base conversion added to the running sums (B_BCONV bounds the result of load_src)
+template <bool BIG, int E>
+__device__ __forceinline__ void bc_term(double (&x)[E], const uint64_t (&y)[E], W2 m, bool wide, const typename ArithFp<BIG>::K &k) {
+    using F = ArithFp<BIG>;
+    const double w = (double)m.w;
+    const typename F::Tw t{w, __dmul_rn(w, k.qinv)};
+    if (!wide) {
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = __dadd_rn(x[i], F::mulmod(F::from_u64(y[i], k), t, k));
+        return;
+    }
+    // a residue of up to 61 bits in two parts: y = yl + 2^30 yh
+    const double w30 = F::mulmod(1073741824.0, t, k);
+    const typename F::Tw u{w30, __dmul_rn(w30, k.qinv)};
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+        const double l = F::from_u64(y[i] & 0x3FFFFFFFu, k), h = F::from_u64(y[i] >> 30, k);
+        x[i] = __dadd_rn(x[i], __dadd_rn(F::mulmod(l, t, k), F::mulmod(h, u, k)));
+    }
+}
+
+// E residues of a limb at positions n0, n0 + step, .. of what a forward transform reads. SRC: 0 = the words as they are, 1 = the
+// dropped limb's words reduced into the limb's prime, 2 = their centred representative (word - src_q when the word exceeds
+// src_q / 2) reduced: the remainder a rescale subtracts, floor or nearest; 3 = the base conversion of the limbs that bc names.
+template <class A, int SRC, int E>
+__device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a, const BcJob &bc, const uint64_t *src, size_t N, size_t n0,
+                                          size_t step, const Mod &md, const typename A::K &k) {
+    if constexpr (SRC != 3) {
+        const uint64_t half = SRC == 2 ? a.src_q >> 1 : 0, q_red = SRC == 2 ? barrett64(a.src_q, md.q, md.r1) : 0;
+#pragma unroll
+        for (int i = 0; i < E; i++) {
+            uint64_t v = src[n0 + i * step];
+            if (SRC) {
+                const uint64_t word = v;
+                v = barrett64(word, md.q, md.r1);
+                if (SRC == 2 && word > half) v = sub_mod(v, q_red, md.q);
+            }
+            x[i] = A::from_u64(v, k);
+        }
+    } else {
+        constexpr bool FP = std::is_same<typename A::T, double>::value;
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = 0;
+        const W2 *m = a.mat + bc.mat_off;
+        for (uint32_t j = 0; j < bc.ni; j++) {
+            uint64_t y[E];
+            const uint64_t *s = src + (size_t)j * (a.src_lm1 + 1) * N + n0;
+#pragma unroll
+            for (int i = 0; i < E; i++) y[i] = s[i * step];
+            const W2 c = ldg_w2(m + j);
+            if constexpr (FP) {
+                bc_term<A::IS_BIG, E>(x, y, c, (bc.wide >> j) & 1, k);
+                if (A::IS_BIG && j == 3) {
+#pragma unroll
+                    for (int i = 0; i < E; i++) x[i] = A::reduce(x[i], k);  // eight products at most between two reductions
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < E; i++) x[i] = A::bc_add(x[i], mul_shoup_lazy(y[i], c, md.q), k);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = A::bc_end(x[i], k);
+    }
+}
+
 // ================================================================================================
 // forward pass: R1 strided stages, exchange, R2 contiguous stages
 // FIRST: the input holds canonical residues (else the raw lazy values of the previous pass)
 // ================================================================================================
-// SRC (column pass only): 1 = the input word reduced into the limb's prime, 2 = its centred representative
-// (word - src_q when the word exceeds src_q / 2) reduced: the remainder a rescale subtracts, floor or nearest.
+// SRC (column pass only): where the input comes from, see load_src
 template <class A, int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, int SRC = 0>
-__device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint64_t *sm, const Job &job, const Mod &md, uint32_t tile) {
+__device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint64_t *sm, const Job &job, uint32_t jobi, const Mod &md, uint32_t tile) {
     using T = typename A::T;
     static_assert(SRC == 0 || COLS, "the on-the-fly source belongs to the column pass");
-    constexpr int B0 = COLS ? A::B_CANON : A::B_PASS, B1 = ct_bound<A>(B0, R1);
+    constexpr int B0 = SRC == 3 ? A::B_BCONV : COLS ? A::B_CANON : A::B_PASS, B1 = ct_bound<A>(B0, R1);
     static_assert(ct_bound<A>(B1, R2) <= A::B_PASS, "a forward pass stores residues within B_PASS");
     constexpr bool FIRST = COLS;
     constexpr int TT = 1 << LOG_T, E1 = 1 << R1, E2 = 1 << R2, C = 1 << LOG_C;
@@ -555,13 +627,14 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
     const size_t N = (size_t)1 << a.logN;
     const typename A::K k = A::make(md, (int)a.logN);
     const W2 *tw = a.tw + (size_t)job.y * N;
-    const uint64_t *src = a.src + src_slot(a, SRC ? job.x / a.src_div : job.x) * N;
+    BcJob bc{};
+    if (SRC == 3) bc = a.bc[jobi];
+    const uint64_t *src = a.src + src_slot(a, SRC == 3 ? bc.in_slot0 : SRC ? job.x / a.src_div : job.x) * N;
     const size_t estride = COLS ? (N >> LOG_T) : 1;
     const size_t cstride = COLS ? 1 : TT;
     const size_t base = COLS ? (size_t)tile * C : (size_t)tile * C * TT;
     const uint32_t n1 = (uint32_t)(N >> LOG_T);  // number of sub-transforms per limb
     const int tid = threadIdx.x;
-    const uint64_t src_half = SRC == 2 ? a.src_q >> 1 : 0, src_q_red = SRC == 2 ? barrett64(a.src_q, md.q, md.r1) : 0;
 
     // ---- stage group 1 ---------------------------------------------------------------------------
 #pragma unroll
@@ -571,16 +644,12 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
         const int elo = COLS ? (gid / C) : (gid % E2);
         const uint32_t P = COLS ? 1u : (n1 + tile * C + c);
         T x[E1];
-        const uint64_t *p = src + base + (size_t)c * cstride + (size_t)elo * estride;
+        const size_t n0 = base + (size_t)c * cstride + (size_t)elo * estride;
+        if (FIRST) {
+            load_src<A, SRC>(x, a, bc, src, N, n0, E2 * estride, md, k);
+        } else {
 #pragma unroll
-        for (int i = 0; i < E1; i++) {
-            uint64_t v = p[(size_t)i * E2 * estride];
-            if (SRC) {
-                const uint64_t word = v;
-                v = barrett64(word, md.q, md.r1);
-                if (SRC == 2 && word > src_half) v = sub_mod(v, src_q_red, md.q);
-            }
-            x[i] = FIRST ? A::from_u64(v, k) : A::from_raw(v);
+            for (int i = 0; i < E1; i++) x[i] = A::from_raw(src[n0 + (size_t)i * E2 * estride]);
         }
         ct_stages<A, 0, R1, E1, B0>(x, tw, P, 0, 0, k);
 #pragma unroll
@@ -634,7 +703,7 @@ ntt_fwd_pass(NttArgs a, Epi epi) {
     const uint32_t jobi = work_idx(a) / tiles, tile = work_idx(a) % tiles;
     const Job job = get_job(a, jobi);
     const Mod md = a.mod[job.y];
-    with_arith(md.q, [&](auto A) { fwd_body<decltype(A), LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, SRC>(a, epi, sm, job, md, tile); });
+    with_arith(md.q, [&](auto A) { fwd_body<decltype(A), LOG_T, R1, R2, LOG_C, COLS, LAST, Epi, SRC>(a, epi, sm, job, jobi, md, tile); });
 }
 
 // ================================================================================================

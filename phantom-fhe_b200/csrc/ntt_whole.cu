@@ -5,8 +5,8 @@
 namespace b2 {
 
 template <int LOGN, class Epi, int SRC>
-static void fwd(const NttArgs &a, const Epi &epi, const WholeArgs &w, uint32_t njobs, uint32_t batch, cudaStream_t s) {
-    launch_cl(1u << WholeCfg<LOGN>::LOG_CL, ntt_fwd_whole<LOGN, Epi, SRC>, dim3(njobs << WholeCfg<LOGN>::LOG_CL, batch), WholeCfg<LOGN>::THREADS, whole_smem<LOGN>(), s, a, epi, w);
+static void fwd(const NttArgs &a, const Epi &epi, uint32_t njobs, uint32_t batch, cudaStream_t s) {
+    launch_cl(1u << WholeCfg<LOGN>::LOG_CL, ntt_fwd_whole<LOGN, Epi, SRC>, dim3(njobs << WholeCfg<LOGN>::LOG_CL, batch), WholeCfg<LOGN>::THREADS, whole_smem<LOGN>(), s, a, epi);
 }
 template <int LOGN>
 static void inv(const NttArgs &a, uint32_t njobs, uint32_t batch, cudaStream_t s) {
@@ -21,19 +21,19 @@ void launch_inv_whole(const NttArgs &a, uint32_t njobs, uint32_t batch, cudaStre
     }
 }
 template <class Epi, int SRC>
-void launch_fwd_whole(const NttArgs &a, const Epi &epi, const WholeArgs &w, uint32_t njobs, uint32_t batch, cudaStream_t s) {
+void launch_fwd_whole(const NttArgs &a, const Epi &epi, uint32_t njobs, uint32_t batch, cudaStream_t s) {
     if constexpr (SRC == 0) {
-        if (a.logN == 13) return fwd<13, Epi, SRC>(a, epi, w, njobs, batch, s);
-        if (a.logN == 14) return fwd<14, Epi, SRC>(a, epi, w, njobs, batch, s);
+        if (a.logN == 13) return fwd<13, Epi, SRC>(a, epi, njobs, batch, s);
+        if (a.logN == 14) return fwd<14, Epi, SRC>(a, epi, njobs, batch, s);
     }
-    fwd<12, Epi, SRC>(a, epi, w, njobs, batch, s);
+    fwd<12, Epi, SRC>(a, epi, njobs, batch, s);
 }
 
-template void launch_fwd_whole<EpiStore, 0>(const NttArgs &, const EpiStore &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiStore, 3>(const NttArgs &, const EpiStore &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubFrom, 3>(const NttArgs &, const EpiSubFrom &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubFromTab, 3>(const NttArgs &, const EpiSubFromTab &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubMul<false>, 1>(const NttArgs &, const EpiSubMul<false> &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubMul<false>, 2>(const NttArgs &, const EpiSubMul<false> &, const WholeArgs &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiStore, 0>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiStore, 3>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubFrom, 3>(const NttArgs &, const EpiSubFrom &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubFromTab, 3>(const NttArgs &, const EpiSubFromTab &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, 1>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, 2>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
 
 }  // namespace b2

@@ -37,16 +37,6 @@
 namespace b2 {
 namespace cg = cooperative_groups;
 
-// One output limb of a base conversion: sum_i y_i[n] M_i mod p over `ni` input limbs from slot in_slot0 on; M_i at mat_off + i
-// as {M, floor(M 2^64 / p)}; bit i of `wide`: input limb i holds residues of a prime of 2^50 or more
-struct BcJob {
-    uint32_t in_slot0, ni, mat_off, wide;
-};
-struct WholeArgs {
-    const BcJob *bc;  // SRC = 3: one per job
-    const W2 *mat;
-};
-
 template <int LOGN> struct WholeCfg;
 //                                          column pass            row pass              log2 of CTAs per limb, threads
 template <> struct WholeCfg<12> { static constexpr int LOG_A = 6, RA1 = 3, RA2 = 3, LOG_B = 6, RB1 = 3, RB2 = 3, LOG_CL = 2, THREADS = 128; };
@@ -100,72 +90,8 @@ __device__ __forceinline__ void whole_fwd_tile(uint64_t *sm, const W2 *tw, uint3
     }
 }
 
-// term y M of a base conversion added to the running sums (B_BCONV of the result below: see whole_src)
-template <bool BIG, int E>
-__device__ __forceinline__ void bc_term(double (&x)[E], const uint64_t (&y)[E], W2 m, bool wide, const typename ArithFp<BIG>::K &k) {
-    using F = ArithFp<BIG>;
-    const double w = (double)m.w;
-    const typename F::Tw t{w, __dmul_rn(w, k.qinv)};
-    if (!wide) {
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = __dadd_rn(x[i], F::mulmod(F::from_u64(y[i], k), t, k));
-        return;
-    }
-    // a residue of up to 61 bits in two parts: y = yl + 2^30 yh
-    const double w30 = F::mulmod(1073741824.0, t, k);
-    const typename F::Tw u{w30, __dmul_rn(w30, k.qinv)};
-#pragma unroll
-    for (int i = 0; i < E; i++) {
-        const double l = F::from_u64(y[i] & 0x3FFFFFFFu, k), h = F::from_u64(y[i] >> 30, k);
-        x[i] = __dadd_rn(x[i], __dadd_rn(F::mulmod(l, t, k), F::mulmod(h, u, k)));
-    }
-}
-
-// E residues of limb `job` at positions n0, n0 + step, ..: read, reduced from the dropped limb (rescale) or converted
-template <class A, int SRC, int E>
-__device__ __forceinline__ void whole_src(typename A::T (&x)[E], const NttArgs &a, const WholeArgs &w, const BcJob &bc, const uint64_t *src, size_t N, size_t n0,
-                                          size_t step, const Mod &md, const typename A::K &k) {
-    if constexpr (SRC != 3) {
-        const uint64_t half = SRC == 2 ? a.src_q >> 1 : 0, q_red = SRC == 2 ? barrett64(a.src_q, md.q, md.r1) : 0;
-#pragma unroll
-        for (int i = 0; i < E; i++) {
-            uint64_t v = src[n0 + i * step];
-            if (SRC) {
-                const uint64_t word = v;
-                v = barrett64(word, md.q, md.r1);
-                if (SRC == 2 && word > half) v = sub_mod(v, q_red, md.q);
-            }
-            x[i] = A::from_u64(v, k);
-        }
-    } else {
-        constexpr bool FP = std::is_same<typename A::T, double>::value;
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = 0;
-        const W2 *m = w.mat + bc.mat_off;
-        for (uint32_t j = 0; j < bc.ni; j++) {
-            uint64_t y[E];
-            const uint64_t *s = src + (size_t)j * (a.src_lm1 + 1) * N + n0;
-#pragma unroll
-            for (int i = 0; i < E; i++) y[i] = s[i * step];
-            const W2 c = ldg_w2(m + j);
-            if constexpr (FP) {
-                bc_term<A::IS_BIG, E>(x, y, c, (bc.wide >> j) & 1, k);
-                if (A::IS_BIG && j == 3) {
-#pragma unroll
-                    for (int i = 0; i < E; i++) x[i] = A::reduce(x[i], k);  // eight products at most between two reductions
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < E; i++) x[i] = A::bc_add(x[i], mul_shoup_lazy(y[i], c, md.q), k);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < E; i++) x[i] = A::bc_end(x[i], k);
-    }
-}
-
 template <class A, int LOGN, class Epi, int SRC>
-__device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs &w, const Epi &epi, uint64_t *smem, const Job &job, uint32_t jobi, const Mod &md) {
+__device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const Epi &epi, uint64_t *smem, const Job &job, uint32_t jobi, const Mod &md) {
     using Cfg = WholeCfg<LOGN>;
     constexpr int LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
     constexpr int N2 = 1 << Cfg::LOG_B, CC = 1 << LOG_CC;
@@ -176,12 +102,12 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs
     const W2 *tw = a.tw + (size_t)job.y * N;
     const uint32_t rank = cg::this_cluster().block_rank();
     BcJob bc{};
-    if (SRC == 3) bc = w.bc[jobi];
+    if (SRC == 3) bc = a.bc[jobi];
     const uint64_t *src = a.src + src_slot(a, SRC == 3 ? bc.in_slot0 : SRC ? job.x / a.src_div : job.x) * N;
     whole_fwd_tile<A, Cfg::LOG_A, Cfg::RA1, Cfg::RA2, LOG_CC, true, Cfg::THREADS, B0>(
         ex, tw, 1u, k,
         [&](int c, int e, int step, auto &x) {
-            whole_src<A, SRC>(x, a, w, bc, src, N, (size_t)e * N2 + rank * CC + c, (size_t)step * N2, md, k);
+            load_src<A, SRC>(x, a, bc, src, N, (size_t)e * N2 + rank * CC + c, (size_t)step * N2, md, k);
         },
         [&](int c, int e0, auto &x) {
 #pragma unroll
@@ -215,13 +141,13 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const WholeArgs
 }
 
 template <int LOGN, class Epi, int SRC>
-__global__ void __launch_bounds__(WholeCfg<LOGN>::THREADS, 512 / WholeCfg<LOGN>::THREADS) ntt_fwd_whole(NttArgs a, const __grid_constant__ Epi epi, WholeArgs w) {
+__global__ void __launch_bounds__(WholeCfg<LOGN>::THREADS, 512 / WholeCfg<LOGN>::THREADS) ntt_fwd_whole(NttArgs a, const __grid_constant__ Epi epi) {
     pdl_enter();
     extern __shared__ __align__(16) uint64_t whole_sm[];
     const uint32_t jobi = blockIdx.x >> WholeCfg<LOGN>::LOG_CL;
     const Job job = get_job(a, jobi);
     const Mod md = a.mod[job.y];
-    with_arith(md.q, [&](auto A) { whole_fwd_body<decltype(A), LOGN, Epi, SRC>(a, w, epi, whole_sm, job, jobi, md); });
+    with_arith(md.q, [&](auto A) { whole_fwd_body<decltype(A), LOGN, Epi, SRC>(a, epi, whole_sm, job, jobi, md); });
 }
 
 // inverse tile: RA contiguous stages, exchange, RB strided stages; LAST: the transform's final stage with the scaling constants
@@ -338,6 +264,6 @@ static_assert(whole_smem<14>() <= 48 * 1024, "no opt-in to a larger shared memor
 // ---- launchers (ntt_whole.cu); they set no error state of their own: the caller reads cudaGetLastError -----------------------
 void launch_inv_whole(const NttArgs &a, uint32_t njobs, uint32_t batch, cudaStream_t s);
 template <class Epi, int SRC>
-void launch_fwd_whole(const NttArgs &a, const Epi &epi, const WholeArgs &w, uint32_t njobs, uint32_t batch, cudaStream_t s);
+void launch_fwd_whole(const NttArgs &a, const Epi &epi, uint32_t njobs, uint32_t batch, cudaStream_t s);
 
 }  // namespace b2

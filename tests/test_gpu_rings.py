@@ -612,3 +612,33 @@ def test_batches_on_both_sides_of_the_fused_row_pass(log_n, special, l, below):
         pick = torch.arange(batch, device="cuda") % 3
         assert torch.equal(ph.multiply_relin_rescale_batch(ctx, da[pick], db[pick], rk), one[pick])
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("log_n,bits,special,l,batch", [
+    (13, [60, 40, 50, 36, 45, 30, 60, 60, 60], 3, 6, 1),                          # every prime class, full digits
+    (13, [60, 40, 46, 36, 50, 45, 40, 60, 59, 60, 60, 60], 5, 7, 2),              # five input limbs, then two
+    (13, [60] + [40, 50] * 4 + [60] * 8, 8, 9, 2),                                # eight input limbs, then one
+    (13, [60, 40, 40, 40, 60], 1, 4, 1),                                          # one input limb
+    (14, [60, 40, 50, 36, 60, 60], 2, 3, 1),
+    (14, [60, 40, 50, 36, 60, 60], 2, 4, 3),
+    (14, [60, 40, 50, 36, 40, 60, 60, 60], 3, 5, 1),
+    (15, [60, 40, 50, 36, 60, 60], 2, 4, 1),
+    (15, [60, 40, 50, 36, 40, 60, 60], 2, 5, 12),                                 # behind it the row pass with the inner product
+    (16, [60, 40, 50, 36, 60, 60], 2, 4, 1),                                      # the same for the FP64 limbs of a single call
+    (16, [60, 40, 36, 60, 60], 2, 3, 4),
+])
+def test_conversion_in_the_column_pass_equals_the_oracle(log_n, bits, special, l, batch):
+    """key switches whose base conversions are made while the forward transforms load, ModUp and ModDown, single and batched"""
+    ctx, o = make_ctx(1 << log_n, bits, special)
+    key = o.synth_key(o.beta(l), 8, 10)
+    a, b = [o.synth_ct(l, 8, 20 + i) for i in range(batch)], [o.synth_ct(l, 8, 40 + i) for i in range(batch)]
+    rlk = _key(ctx, key)
+    if batch == 1:
+        ca, cb = (ph.ciphertext.from_numpy(ctx, v[0], ctx.size_Q - l + 1, 2.0 ** 40) for v in (a, b))
+        got = [host(ph.multiply_and_relin(ctx, ca, cb, rlk).data)]
+    else:
+        ext = dev(np.stack([o.tensor_mul(l, a[i], b[i]) for i in range(batch)]))
+        got = host(ph.relinearize_batch(ctx, ext, rlk))
+    for i in range(batch):
+        assert np.array_equal(got[i], o.multiply_and_relin(l, a[i], b[i], key)), f"set {i}"
+    assert ctx.device_status() == 0
