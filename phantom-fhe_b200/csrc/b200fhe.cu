@@ -168,12 +168,14 @@ struct BconvGroup {
     uint32_t in_pieces;      // 21-bit pieces needed to hold an input residue (2 below 2^42, else 3)
 };
 
-// One base conversion launch in tensor-core form: job list (grid.y), the groups and byte images they index
+// One base conversion launch in tensor-core form: job list, the groups and byte images they index (device form, bconv_tc.cuh)
 struct TcSet {
     const TcJob *jobs = nullptr;
     const TcGroup *groups = nullptr;
     const uint8_t *images = nullptr;
-    uint32_t n_jobs = 0, jobs_per_poly = 0, max_alloc = 32;
+    uint32_t n_jobs = 0, jobs_per_poly = 0;
+    uint32_t min_groups = 0, max_groups = 0, max_slices = 0;  // over the jobs: column groups, K slices
+    TcJob first[TC_JOBS_INLINE] = {};                         // the first jobs, for the launch's parameters
 };
 
 struct LevelPlan {
@@ -236,10 +238,6 @@ struct b2_ctx {
     bool bconv_fp = false;         // every digit satisfies sum(q_i) < 2^64 and alpha <= 8
     bool bconv_tc = false;         // base conversions on the tensor cores (alpha <= 8, primes above 2^16; off with B2_BCONV=fp|int)
     bool bconv_int = false;        // B2_BCONV=int: force the 128-bit integer kernel
-    int tc_wg = 4;                 // warpgroups per CTA of the tensor-core conversion (B2_BCONV_WG = 1, 2, 4)
-    bool tc_simple = false;        // B2_BCONV_TC_SIMPLE=1: one CTA per tile instead of the persistent pipelined kernel
-    bool tc_serial_ld = false;     // B2_BCONV_SERIAL_LD=1: the epilogue waits for every TMEM load before it reduces (no load in flight)
-    uint32_t tc_max_groups = 16;   // B2_BCONV_GROUPS: column groups per conversion job (8: at most 128 TMEM columns, four CTAs per SM)
     uint32_t *d_err = nullptr;     // device status word: set by a kernel whose bounded wait ran out
     std::vector<uint64_t> h_mat_dn, h_mat_dn_pinv;  // host copies of the ModDown matrices [size_Q][size_P]
     bool mac_interleave = false;   // B2_KS_FUSED_ORDER=1: consecutive CTAs of the fused pass walk limbs, not tiles (measured slower)
@@ -329,15 +327,25 @@ static inline void h_pieces(uint64_t m, uint64_t p, double *out3) {
 }
 static inline uint32_t h_npieces(uint64_t q) { return q < (1ull << 42) ? 2u : 3u; }
 
-// uploads what a TcBuild holds as one blob and points the sets' job lists (given as [first job, count) ranges) into it
+// uploads what a TcBuild holds, in device form, as one blob and points the sets' job lists (given as [first job, count) ranges)
+// into it
 static int tc_upload(const TcBuild &b, void **blob, std::initializer_list<std::pair<TcSet *, std::pair<uint32_t, uint32_t>>> sets) {
-    const size_t jb = (b.jobs.size() * sizeof(TcJob) + 255) & ~size_t(255), gb = (b.groups.size() * sizeof(TcGroup) + 255) & ~size_t(255);
-    const size_t total = jb + gb + b.images.size() + 256;
+    std::vector<TcJob> jobs = b.jobs;
+    std::vector<TcGroup> groups = b.groups;
+    std::vector<uint8_t> images;
+    for (size_t j = 0; j < jobs.size(); j++) {
+        jobs[j].img_off = (uint32_t)images.size();
+        tc_pair_image(b, b.jobs[j], images);
+    }
+    for (auto &g : groups)
+        for (auto &o : g.o) o.p = 0 - o.p;
+    const size_t jb = (jobs.size() * sizeof(TcJob) + 255) & ~size_t(255), gb = (groups.size() * sizeof(TcGroup) + 255) & ~size_t(255);
+    const size_t total = jb + gb + images.size() + 256;
     if (cudaMalloc(blob, total) != cudaSuccess) return fail(B2_ENOMEM, "cudaMalloc(tensor-core conversion plan) failed");
     char *base = (char *)*blob;
-    cudaError_t e = cudaMemcpy(base, b.jobs.data(), b.jobs.size() * sizeof(TcJob), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + jb, b.groups.data(), b.groups.size() * sizeof(TcGroup), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + jb + gb, b.images.data(), b.images.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpy(base, jobs.data(), jobs.size() * sizeof(TcJob), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(base + jb, groups.data(), groups.size() * sizeof(TcGroup), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(base + jb + gb, images.data(), images.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail((int)e, "cudaMemcpy(tensor-core conversion plan) failed");
     for (auto &s : sets) {
         TcSet *ts = s.first;
@@ -345,8 +353,14 @@ static int tc_upload(const TcBuild &b, void **blob, std::initializer_list<std::p
         ts->n_jobs = s.second.second;
         ts->groups = (const TcGroup *)(base + jb);
         ts->images = (const uint8_t *)(base + jb + gb);
-        ts->max_alloc = 32;
-        for (uint32_t j = 0; j < s.second.second; j++) ts->max_alloc = std::max(ts->max_alloc, b.jobs[s.second.first + j].alloc_cols);
+        ts->min_groups = ~0u;
+        for (uint32_t j = 0; j < s.second.second; j++) {
+            const TcJob &job = jobs[s.second.first + j];
+            if (j < TC_JOBS_INLINE) ts->first[j] = job;
+            ts->min_groups = std::min(ts->min_groups, job.n_groups);
+            ts->max_groups = std::max(ts->max_groups, job.n_groups);
+            ts->max_slices = std::max(ts->max_slices, (job.ni + 1) & ~1u);
+        }
     }
     return B2_OK;
 }
@@ -501,7 +515,6 @@ static int build_level(b2_ctx *c, size_t l) {
         // the same conversions as tensor-core jobs: ModUp digits, then ModDown of up to two polynomials with the plain
         // matrix (cx layout [2][lP]) and with the P^-1-carrying one (compact P limbs [2][alpha])
         TcBuild tb;
-        tb.max_groups = c->tc_max_groups;
         std::vector<TcSpecOut> outs;
         uint32_t n_up = 0, n_dn = 0, n_dnf = 0;
         for (size_t d = 0; d < beta; d++) {
@@ -739,15 +752,6 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
         for (size_t i = 0; i < size_QP; i++) tc_ok = tc_ok && c->q[i] > (1ull << 16);
         c->bconv_tc = tc_ok && bc == "tc";
         c->bconv_int = bc == "int";
-        const char *env_wg = getenv("B2_BCONV_WG");
-        c->tc_wg = env_wg ? atoi(env_wg) : 4;
-        if (c->tc_wg != 1 && c->tc_wg != 2 && c->tc_wg != 4) c->tc_wg = 4;
-        const char *env_sld = getenv("B2_BCONV_SERIAL_LD");
-        c->tc_serial_ld = env_sld && env_sld[0] == '1';
-        const char *env_groups = getenv("B2_BCONV_GROUPS");
-        if (env_groups && atoi(env_groups) >= 1 && atoi(env_groups) <= 16) c->tc_max_groups = (uint32_t)atoi(env_groups);
-        const char *env_simple = getenv("B2_BCONV_TC_SIMPLE");
-        c->tc_simple = env_simple && env_simple[0] == '1';
         if (cudaMalloc((void **)&c->d_err, 4) != cudaSuccess || cudaMemset(c->d_err, 0, 4) != cudaSuccess) {
             b2_ctx_destroy(c);
             return fail(B2_ENOMEM, "ctx_create: cudaMalloc(status word) failed");
@@ -763,16 +767,11 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
             }
         }
         if (c->bconv_tc) {
-            // per device: the conversion asks for more dynamic shared memory than it uses (see tc_smem_request)
-            cudaError_t ea = cudaFuncSetAttribute(bconv_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
-            if (ea == cudaSuccess) ea = cudaFuncSetAttribute(bconv_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
-            if (ea == cudaSuccess) ea = cudaFuncSetAttribute(bconv_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
-            if (ea == cudaSuccess) ea = cudaFuncSetAttribute(bconv_tc_persist<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
-            if (ea == cudaSuccess) ea = cudaFuncSetAttribute(bconv_tc_persist<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
-            if (ea == cudaSuccess) ea = cudaFuncSetAttribute(bconv_tc_persist<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
+            // per device: the conversion's rings and images are above the 48 KB default
+            cudaError_t ea = cudaFuncSetAttribute(bconv_tc_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX_REQUEST);
             if (ea != cudaSuccess) {
                 b2_ctx_destroy(c);
-                return fail((int)ea, std::string("ctx_create: cudaFuncSetAttribute(bconv_tc_kernel): ") + cudaGetErrorString(ea));
+                return fail((int)ea, std::string("ctx_create: cudaFuncSetAttribute(bconv_tc_pairs): ") + cudaGetErrorString(ea));
             }
         }
     }
@@ -1192,48 +1191,45 @@ struct IpBatch {
         else launch_k(kernel<1>, dim3((unsigned)(c->N / 256), gy, gz), 256, 0, s, __VA_ARGS__);              \
     } while (0)
 
-// Shared memory a conversion CTA asks for: what it uses, or enough that no more CTAs fit on an SM (228 KB) than its
-// 512 TMEM columns can serve, whichever is larger - so tcgen05.alloc finds its columns free and never waits.
-static uint32_t tc_smem_request(uint32_t alloc_cols, uint32_t used) {
-    const uint32_t fit = 512 / alloc_cols;
-    return std::max(used, TC_SM_SMEM / (fit + 1));
-}
+// strides of a batch of conversions: see TcArgs
+struct TcBatch {
+    uint32_t batch = 1, in_lm1 = 0, in_bs = 0, out_lm1 = 0, out_bs = 0;
+};
 
 // n_jobs: how many of the set's jobs to run (ModDown of one polynomial runs the first half)
 static int run_bconv_tc(const b2_ctx *c, bool copy, const uint64_t *in, uint64_t *out, const uint64_t *copy_src, const TcSet &tc, uint32_t n_jobs,
-                        cudaStream_t s, const TcBatch *tbp = nullptr) {
-    const uint32_t N = (uint32_t)c->N;
+                        cudaStream_t s, const TcBatch &tb = TcBatch{}) {
     if (n_jobs == 0) return B2_OK;
     if (copy && !copy_src) return fail(B2_EINVAL, "base conversion: missing copy source");
-    TcBatch tb = tbp ? *tbp : TcBatch{1, 0, 0, 0, 0, 0};
-    tb.serial_ld = c->tc_serial_ld ? 1u : 0u;
-    if (tb.batch != 1 && (copy || c->tc_simple)) return fail(B2_EINVAL, "a batched base conversion runs on the persistent kernel, without the own-limb copy");
+    if (tb.batch != 1 && copy) return fail(B2_EINVAL, "a batched base conversion runs without the own-limb copy");
+    if (!aligned32(in) || !aligned32(out)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
+    TcArgs a{};
+    a.in = in, a.out = out, a.copy_src = copy ? copy_src : nullptr;  // a null source: the jobs' copy slots are ignored
+    a.jobs = tc.jobs, a.groups = tc.groups, a.images = tc.images, a.err = c->d_err;
+    a.N = (uint32_t)c->N;
+    std::copy_n(tc.first, TC_JOBS_INLINE, a.job);
+    a.batch = tb.batch, a.in_lm1 = tb.in_lm1, a.in_bs = tb.in_bs, a.out_lm1 = tb.out_lm1, a.out_bs = tb.out_bs;
+    // Two CTAs an SM (their 256 TMEM columns each). Fewer items than that are split by column groups, as long as the longest
+    // CTA has less to do for it (a tile's way in and out counts for two groups).
+    const uint32_t ctas = 2 * (uint32_t)c->sm_count, items = n_jobs * tb.batch * (a.N / TC_TILE);
+    uint32_t best = ~0u;
+    for (uint32_t p = 1; p <= tc.min_groups && (p == 1 || items * (p - 1) < ctas); p++) {
+        const uint32_t cost = ((items * p + ctas - 1) / ctas) * ((tc.max_groups + p - 1) / p + 2);
+        if (cost < best) best = cost, a.parts = p;
+    }
+    a.stage_bytes = tc.max_slices * TC_SLICE;
+    a.b_bytes = (tc.max_groups + a.parts - 1) / a.parts * 512 * tc.max_slices;
+    a.part_recs = (tc.max_groups + a.parts - 1) / a.parts;
+    const uint32_t grid = std::min(items * a.parts, ctas);
+    a.items = items * a.parts / grid, a.more = items * a.parts % grid;
+    // a CTA's run of items touches at most this many parts
+    const uint32_t span = (n_jobs * a.parts + grid - 1) / grid + 1;
+    const uint32_t rest = TC_CTRL_BYTES + a.b_bytes + span * a.part_recs * (uint32_t)sizeof(TcGroup);
+    // what it uses, or enough that a third CTA, for which there are no TMEM columns, does not fit beside two
+    const uint32_t smem = std::max(rest + TC_STAGES * a.stage_bytes, TC_SM_SMEM / 3);
     LaunchScope ls(c, s, "bconv");
-    // without the copy the jobs' copy slots are ignored by handing the kernel a null source
-    const uint64_t *cs = copy ? copy_src : nullptr;
-    if (c->tc_simple) {
-        const dim3 grid(N / 128, n_jobs);
-        const uint32_t smem = tc_smem_request(tc.max_alloc, TC_SMEM_BYTES);
-        switch (c->tc_wg) {
-            case 1: launch_k(bconv_tc_kernel<1>, grid, 128, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
-            case 4: launch_k(bconv_tc_kernel<4>, grid, 512, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
-            default: launch_k(bconv_tc_kernel<2>, grid, 256, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, c->d_err); break;
-        }
-        LAUNCH_CHECK("bconv_tc_kernel");
-        return B2_OK;
-    }
-    // persistent CTAs: as many as stay resident (TMEM columns, threads), each walking its share of the (job, tile) items
-    const uint32_t threads = 128u * (uint32_t)c->tc_wg;
-    const uint32_t fit = std::min(512u / tc.max_alloc, 2048u / threads);
-    const uint32_t total = n_jobs * (N / 128) * tb.batch;
-    const uint32_t grid = std::min(total, fit * (uint32_t)c->sm_count);
-    const uint32_t smem = tc_smem_request(tc.max_alloc, TCP_SMEM_BYTES);
-    switch (c->tc_wg) {
-        case 1: launch_k(bconv_tc_persist<1>, grid, 128, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
-        case 2: launch_k(bconv_tc_persist<2>, grid, 256, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
-        default: launch_k(bconv_tc_persist<4>, grid, 512, smem, s, in, out, cs, tc.jobs, tc.groups, tc.images, N, n_jobs, tc.max_alloc, c->d_err, tb); break;
-    }
-    LAUNCH_CHECK("bconv_tc_persist");
+    launch_k(bconv_tc_pairs, grid, TC_THREADS, smem, s, a);
+    LAUNCH_CHECK("bconv_tc_pairs");
     return B2_OK;
 }
 
@@ -1476,7 +1472,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
     const bool pays = batched ? c->mac_wide >= 0 || fused_rows_pay(c, l, beta, kb.batch) : c->logN == 16 || c->mac_wide == 1;
     const bool mac = c->use_mac && pays && (pl.mac_ok || wide) && n_evk >= beta && aligned32(c2) && aligned32(ct) && aligned32(up) && aligned32(cxP);
     if (!mac && !batched) return B2_OK;
-    if (batched && (!c->bconv_tc || c->tc_simple || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
+    if (batched && (!c->bconv_tc || !pl.tc_up.jobs || !pl.tc_dnf.jobs))
         return B2_OK;  // the caller falls back to one key switch at a time
     {
         using Cfg = PassCfg<8>;
@@ -1486,8 +1482,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (loading && !mac) {
             rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
         } else if (!loading && batched) {
-            const TcBatch tb{B, 0, (uint32_t)l, 0, per, c->tc_serial_ld ? 1u : 0u};
-            rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, &tb);
+            rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, TcBatch{B, 0, (uint32_t)l, 0, per});
         } else if (!loading) {
             rc = run_bconv(c, false, t, up, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)lP, true, s, &pl.tc_up);
         }
@@ -1624,8 +1619,8 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     if (convert_loading(c, 2 * l * batch))
         return run_bconv_fwd(c, cxP, up, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{d_ct, (uint32_t)ct_stride}, s,
                              BatchDims{B, 0, (uint32_t)(2 * a), 0, per});
-    const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per, 0};
-    rc = run_bconv_tc(c, false, cxP, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, &tb);
+    const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per};
+    rc = run_bconv_tc(c, false, cxP, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, tb);
     if (rc) return rc;
     return run_fwd(c, up, up, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_ct, (uint32_t)ct_stride}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
 }
@@ -2033,9 +2028,9 @@ extern "C" int b2_rotate_sum(b2_ctx *c, size_t l, size_t n, const uint32_t *elts
             rc = run_bconv_fwd(c, t, up, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s, BatchDims{B, 0, (uint32_t)l, 0, per});
             if (rc) return rc;
         } else {
-            if (c->bconv_tc && !c->tc_simple) {
-                const TcBatch tb{B, 0, (uint32_t)l, 0, per, c->tc_serial_ld ? 1u : 0u};
-                rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, &tb);
+            if (c->bconv_tc) {
+                const TcBatch tb{B, 0, (uint32_t)l, 0, per};
+                rc = run_bconv_tc(c, false, t, up, nullptr, pl.tc_up, pl.tc_up.n_jobs, s, tb);
                 if (rc) return rc;
             } else {
                 for (uint32_t i = 0; i < B; i++) {
@@ -2157,9 +2152,9 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
             if (rc) return rc;
             continue;
         }
-        if (c->bconv_tc && !c->tc_simple) {
-            const TcBatch tb{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l), 0};
-            rc = run_bconv_tc(c, false, cxP, delta, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, &tb);
+        if (c->bconv_tc) {
+            const TcBatch tb{n, 0, (uint32_t)(2 * a), 0, (uint32_t)(2 * l)};
+            rc = run_bconv_tc(c, false, cxP, delta, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, tb);
             if (rc) return rc;
         } else {
             for (uint32_t i = 0; i < n; i++) {
@@ -2682,7 +2677,6 @@ static int build_shard_level(b2_ctx *c, size_t l) {
     if (c->bconv_tc) {
         // tensor-core jobs over the rank's outputs (a rank may own no output of a digit, or no Q limb at all)
         TcBuild tb;
-        tb.max_groups = c->tc_max_groups;
         std::vector<TcSpecOut> outs;
         uint32_t n_up = 0, n_dn = 0, n_dn_b = 0;
         for (size_t d = 0; d < beta; d++) {
@@ -2847,7 +2841,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
     if (c->shard.empty()) return fail(B2_EINVAL, "shard_keyswitch_phase_batch: call b2_ctx_set_shard first");
     if (!d_c2 || !evk || !d_ct || !d_ws || batch < 1 || batch > 65535) return fail(B2_EINVAL, "shard_keyswitch_phase_batch: bad argument");
     if (ws_bytes < b2_shard_batch_workspace_bytes(c, l, batch)) return fail(B2_EWS, "shard_keyswitch_phase_batch: workspace too small");
-    if (!c->bconv_tc || c->tc_simple) return fail(B2_EINVAL, "shard_keyswitch_phase_batch: needs the persistent tensor-core base conversion");
+    if (!c->bconv_tc) return fail(B2_EINVAL, "shard_keyswitch_phase_batch: needs the tensor-core base conversion");
     cudaStream_t s = (cudaStream_t)stream;
     const LevelPlan &pl = c->plan[l];
     const b2_ctx::ShardPlan &sp = c->shard[l];
@@ -2859,9 +2853,9 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
         case 0:
             return run_inv(c, d_c2, T, pl.jobs_up_intt + sp.q0, sp.nq, 0, pl.fin_up, s, BatchDims{B, 0, (uint32_t)l, B - 1, 1});
         case 1: {
-            const TcBatch tb{B, B - 1, 1, 0, per, 0};
+            const TcBatch tb{B, B - 1, 1, 0, per};
             if (sp.tc_up.jobs) {
-                rc = run_bconv_tc(c, false, T, UP, nullptr, sp.tc_up, sp.tc_up.n_jobs, s, &tb);
+                rc = run_bconv_tc(c, false, T, UP, nullptr, sp.tc_up, sp.tc_up.n_jobs, s, tb);
                 if (rc) return rc;
             }
             const bool fused = c->use_mac && beta <= B2_MAC_MAX_BETA && n_evk >= beta && (sp.nq + sp.np) > 0;
@@ -2903,8 +2897,8 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
         }
         case 2: {
             if (sp.nq == 0) return B2_OK;
-            const TcBatch tb{B, B - 1, 1, 0, per, 0};
-            rc = run_bconv_tc(c, false, CXP, UP, nullptr, sp.tc_dn_b, sp.tc_dn_b.n_jobs, s, &tb);
+            const TcBatch tb{B, B - 1, 1, 0, per};
+            rc = run_bconv_tc(c, false, CXP, UP, nullptr, sp.tc_dn_b, sp.tc_dn_b.n_jobs, s, tb);
             if (rc) return rc;
             return run_fwd(c, UP, UP, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct, (uint32_t)(2 * l)}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
         }

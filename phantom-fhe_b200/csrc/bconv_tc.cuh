@@ -1,14 +1,28 @@
 // bconv_tc.cuh - fast base conversion on the sm_100a tensor cores (tcgen05.mma kind::i8, accumulators in TMEM).
 // The formulation, the data structures and the host-side planning are in bconv_tc_plan.h.
 //
-// CTA = 128 coefficients (M = 128: TMEM lane = coefficient) x one job. The threads put the tile's input limbs into
-// shared memory as the rows of A (the raw 8 bytes of each residue) and copy the job's ready-made B image next to it;
-// one thread issues two MMAs (K = 2 x 32, N = 16 * groups <= 256) and commits them to an mbarrier; every warp then
-// reads its 32 TMEM lanes (tcgen05.ld 32x32b: one coefficient per thread, 16 columns = one output group at a time),
-// reduces and stores 8-byte words that are contiguous across the warp. 128 * WG threads: warp w reads lanes
-// 32 (w % 4) .. +31 and warpgroup w / 4 takes every WG-th column group.
-// No multicast, no cluster; the only wait (MMA completion) is bounded and reports through a status word instead of
-// spinning forever; TMEM is released on every path.
+// A tile is 256 coefficients of one job: 128 rows of two coefficients, so that an input limb's share of the tile is 2 KB of
+// consecutive memory AND, as it lies there, one 16-byte K slice of all rows of A. One cp.async.bulk per limb brings it in, no
+// thread touches it, and a thread of the epilogue (TMEM lane = row) holds both coefficients of an output: one record, one
+// address and one 16-byte store for the two. The price is a B whose blocks for the other coefficient of a row are zero, twice
+// the multiplications, on a unit that has them to spare.
+//
+// Fourteen warps a CTA, two CTAs an SM, each walking a run of consecutive items (job part, set, tile): warp 13 loads (a ring of
+// A tiles, the part's B image when the part changes), warp 12 issues the MMAs of three column groups at a time into one of two
+// 96-column accumulators, warps 0 to 11 (TMEM lanes 32 (w % 4) .. +31, a group each) reduce and store the other. Groups a
+// buffer, ModUp and ModDown of sixteen key switches of 24 limbs and 8 special primes at 2^16, us a key switch: two 18.6, three
+// 17.1, four 17.8 (spills). Four warps' worth of epilogue an SM sub-partition is what hides a warp's chain of TMEM load,
+// reduction and store: with eight warps taking two groups each in turn, and the records read from global memory, 21.8.
+// Two A tiles in flight: three or four are no faster, and their shared memory keeps the CTAs of other streams' kernels off the
+// SM, and this kernel's CTAs off an SM that those have not left (four streams of key switches 7420 a second with two, 6700
+// with four).
+// The form before (a coefficient a row, rows filled by cp.async of eight bytes, a barrier pair per tile of 128 coefficients)
+// took 73 warp instructions an output and 25.0 us; the bytes alone take 12.9 at the copy rate. A launch that gives a CTA one
+// tile takes 0.5 us longer than it did then: a bulk copy arrives a microsecond after its issue, where cp.async takes a third
+// of that, but the code that filled the first tile so cost more than it saved (the instructions of a kernel that runs for
+// three microseconds are fetched as they are executed).
+// No multicast, no cluster; every wait is bounded and reports through a status word instead of spinning forever; copies and
+// MMAs in flight are waited for and TMEM is released on every path.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -18,19 +32,23 @@
 
 namespace b2 {
 
-constexpr uint32_t TC_SMEM_A = 128 * 64;            // one tile of A
-constexpr uint32_t TC_SMEM_B = 256 * 64;            // largest B image
-constexpr uint32_t TC_SMEM_CTRL = TC_SMEM_A + TC_SMEM_B;
-constexpr uint32_t TC_SMEM_BYTES = TC_SMEM_CTRL + 32;
-constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;        // polls of the MMA barrier before giving up
+constexpr uint32_t TC_TILE = 256;                   // coefficients of a tile
+constexpr uint32_t TC_SLICE = TC_TILE * 8;          // bytes of one input limb's share of it: one K slice of A
+constexpr uint32_t TC_STAGES = 2;                   // A tiles in flight
+constexpr uint32_t TC_CHUNK = 3;                    // column groups of one accumulator buffer: one per warp of a TMEM quadrant
+constexpr uint32_t TC_ACC_COLS = 32 * TC_CHUNK, TC_TMEM_COLS = 256, TC_BUFS = TC_TMEM_COLS / TC_ACC_COLS;
+constexpr uint32_t TC_EPI_WARPS = 4 * TC_CHUNK, TC_THREADS = 32 * (TC_EPI_WARPS + 2);
+constexpr uint32_t TC_CTRL_BYTES = 256;             // barriers and the like
+constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;        // polls of a barrier before giving up
 constexpr uint32_t TC_SM_SMEM = 233472;             // shared memory of one SM (228 KB)
-constexpr uint32_t TC_SMEM_MAX_REQUEST = TC_SM_SMEM / 2;
+constexpr uint32_t TC_SMEM_MAX_REQUEST = TC_SM_SMEM / 2 - 1024;  // two CTAs an SM, a kilobyte each for the system
 
 __device__ __forceinline__ uint32_t tc_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// shared-memory matrix descriptor: K-major, no swizzle, LBO = 128 B, SBO = 512 B, descriptor version 1 (sm_100)
-__device__ __forceinline__ uint64_t tc_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(512u >> 4) << 32) | ((uint64_t)1 << 46);
+// shared-memory matrix descriptor: K-major, no swizzle; lbo = bytes between K-adjacent core matrices, 128 bytes between groups
+// of eight rows; descriptor version 1 (sm_100)
+__device__ __forceinline__ uint64_t tc_desc(uint32_t smem_addr, uint32_t lbo) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | ((uint64_t)1 << 46);
 }
 
 __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -43,66 +61,68 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint6
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_bar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void tc_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tc_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// bytes and both addresses multiples of 16
+__device__ __forceinline__ void tc_bulk(uint32_t smem_dst, const void *gsrc, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst), "l"(gsrc), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// waits for the phase of the given parity to end, at most TC_WAIT_LIMIT polls and not after another wait of the CTA gave up
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile uint32_t *gave_up) {
+    for (uint32_t it = 0; it < TC_WAIT_LIMIT; it++) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t"
+            ".reg .pred P1;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P1;\n\t"
+            "}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (*gave_up) return false;
+    }
+    *gave_up = 1u;
+    return false;
+}
 
-// 16 consecutive accumulator columns of this thread's TMEM lane; the wait is part of the same statement so
-// that no use of the registers can be scheduled ahead of it
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&c)[16]) {
+// 32 consecutive accumulator columns of this thread's TMEM lane, and the wait as a statement that owns the registers: a
+// group's planes can be on their way while the previous group is reduced
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&c)[32]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]), "=r"(c[8]), "=r"(c[9]),
-          "=r"(c[10]), "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15])
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]), "=r"(c[8]), "=r"(c[9]), "=r"(c[10]),
+          "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15]), "=r"(c[16]), "=r"(c[17]), "=r"(c[18]), "=r"(c[19]), "=r"(c[20]),
+          "=r"(c[21]), "=r"(c[22]), "=r"(c[23]), "=r"(c[24]), "=r"(c[25]), "=r"(c[26]), "=r"(c[27]), "=r"(c[28]), "=r"(c[29]), "=r"(c[30]), "=r"(c[31])
         : "r"(taddr)
         : "memory");
 }
-
-// the same load without the wait, and the wait as a statement that owns the registers: a group's planes can be on their way
-// while the previous group is reduced
-__device__ __forceinline__ void tc_ld16_nowait(uint32_t taddr, uint32_t (&c)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]), "=r"(c[8]), "=r"(c[9]),
-          "=r"(c[10]), "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld(uint32_t (&c)[16]) {
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&c)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c[4]), "+r"(c[5]), "+r"(c[6]), "+r"(c[7]), "+r"(c[8]), "+r"(c[9]),
-                   "+r"(c[10]), "+r"(c[11]), "+r"(c[12]), "+r"(c[13]), "+r"(c[14]), "+r"(c[15])
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c[4]), "+r"(c[5]), "+r"(c[6]), "+r"(c[7]), "+r"(c[8]), "+r"(c[9]), "+r"(c[10]),
+                   "+r"(c[11]), "+r"(c[12]), "+r"(c[13]), "+r"(c[14]), "+r"(c[15]), "+r"(c[16]), "+r"(c[17]), "+r"(c[18]), "+r"(c[19]), "+r"(c[20]),
+                   "+r"(c[21]), "+r"(c[22]), "+r"(c[23]), "+r"(c[24]), "+r"(c[25]), "+r"(c[26]), "+r"(c[27]), "+r"(c[28]), "+r"(c[29]), "+r"(c[30]), "+r"(c[31])
                  :
                  : "memory");
 }
 
+// One residue below 2 p from its planes: paired with shift-adds, joined by one (7 and 8 planes: two) wide multiply-adds, the
+// quotient estimate one high multiply, v + qhat (2^64 - p) one wide multiply-add and one narrow one. tc_reduce
+// (bconv_tc_plan.h) without its last subtraction, which the forward transform that follows does not need (B_IN).
+// r: {2^64 - p as two words, mu, slot}
 template <int NB>
-__device__ __forceinline__ void tc_group_outputs(const uint32_t (&c)[16], const TcGroup *g, uint32_t n_valid, uint64_t *__restrict__ out, size_t N,
-                                                 uint32_t n) {
-    constexpr int OPG = 16 / NB;
-#pragma unroll
-    for (int o = 0; o < OPG; o++) {
-        if (o < (int)n_valid) {
-            const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(&g->o[o]));
-            const uint64_t p = (uint64_t)raw.x | ((uint64_t)raw.y << 32);
-            out[(size_t)raw.w * N + n] = tc_reduce<NB>(&c[o * NB], p, raw.z);
-        }
-    }
-}
-
-
-// ---- lean epilogue of the persistent kernel ------------------------------------------------------------------------
-// One output as the epilogue wants it, 16 bytes in shared memory (one LDS.128): prime, reciprocal, and the output
-// limb's first element (slot * N); 0xFFFFFFFF marks a slot of a group that holds no output (p = 1 keeps its
-// arithmetic harmless), so the group is processed without a branch per output and only the store is predicated.
-struct TcOutS {
-    uint32_t p_lo, p_hi, mu, off;
-};
-
-// One output, written so that it costs about twenty instructions: the planes are paired with shift-adds, joined by one
-// (two for 7 and 8 planes) wide multiply-add, the quotient estimate is one high multiply, and the two subtractions, the
-// choice between r and r - p (sign of the difference: r < 2p < 2^62) and the predicated store are spelled out in PTX so
-// that no branch and no 64-bit compare is generated. Same value as tc_reduce / tc_reduce_dev (bconv_tc_plan.h).
-template <int NB, bool ALWAYS = false>
-__device__ __forceinline__ void tc_output(const uint32_t *c, const uint4 m, uint64_t *__restrict__ out_n) {
+__device__ __forceinline__ uint2 tc_residue(const uint32_t *c, const uint4 r) {
     constexpr int SH = 8 * NB - 17;
     const uint32_t x0 = c[0] + (c[1] << 8), x1 = c[2] + (c[3] << 8);
     uint32_t vl, vh, vq;  // V mod 2^64 as two words; V >> SH
@@ -118,372 +138,224 @@ __device__ __forceinline__ void tc_output(const uint32_t *c, const uint4 m, uint
         vl = (uint32_t)a, vh = (uint32_t)mid;
         vq = __funnelshift_r((uint32_t)mid, (uint32_t)(mid >> 32), SH - 32);
     }
-    const uint32_t qhat = __umulhi(vq, m.z);
-    const uint64_t qp = (uint64_t)qhat * m.x;
-    const uint32_t ql = (uint32_t)qp, qh = (uint32_t)(qp >> 32) + qhat * m.y;
-    uint32_t rl, rh;
-    // plain asm (no volatile): independent outputs of a group may be interleaved by the scheduler
-    asm("{\n\t"
-        ".reg .u32 tl, th;\n\t"
-        ".reg .pred pn;\n\t"
-        "sub.cc.u32 %0, %2, %4;\n\t"
-        "subc.u32 %1, %3, %5;\n\t"
-        "sub.cc.u32 tl, %0, %6;\n\t"
-        "subc.u32 th, %1, %7;\n\t"
-        "setp.lt.s32 pn, th, 0;\n\t"
-        "selp.u32 %0, %0, tl, pn;\n\t"
-        "selp.u32 %1, %1, th, pn;\n\t"
-        "}\n"
-        : "=&r"(rl), "=&r"(rh)
-        : "r"(vl), "r"(vh), "r"(ql), "r"(qh), "r"(m.x), "r"(m.y));
-    if constexpr (ALWAYS) {
-        asm volatile("st.global.v2.u32 [%0], {%1, %2};" ::"l"(out_n + m.w), "r"(rl), "r"(rh) : "memory");
-    } else {
-        asm volatile(
-            "{\n\t"
-            ".reg .pred pv;\n\t"
-            "setp.ne.u32 pv, %3, 0xFFFFFFFF;\n\t"
-            "@pv st.global.v2.u32 [%0], {%1, %2};\n\t"
-            "}\n" ::"l"(out_n + m.w),
-            "r"(rl), "r"(rh), "r"(m.w)
-            : "memory");
-    }
+    const uint32_t qhat = __umulhi(vq, r.z);
+    const uint64_t t = (uint64_t)qhat * r.x + (((uint64_t)vh << 32) | vl);
+    return make_uint2((uint32_t)t, (uint32_t)(t >> 32) + qhat * r.y);
 }
 
-// NV = number of outputs the group holds (0: not known at compile time, every slot is processed and the store of an empty
-// one is predicated off)
-template <int NB, int NV = 0>
-__device__ __forceinline__ void tc_group_lean(const uint32_t (&c)[16], uint32_t mo_smem, uint64_t *__restrict__ out_n) {
-    constexpr int OPG = NV ? NV : 16 / NB;
+// the NV outputs of a group, two coefficients each
+template <int NB, int NV>
+__device__ __forceinline__ void tc_group(const uint32_t (&c)[32], const TcGroup *g, uint32_t slot_words, uint64_t *__restrict__ out_n) {
 #pragma unroll
-    for (int o = 0; o < OPG; o++) {
-        uint4 m;
-        // the records do not change while a job's tiles are reduced: the load may move freely
-        asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(m.x), "=r"(m.y), "=r"(m.z), "=r"(m.w) : "r"(mo_smem + 16 * o));
-        tc_output<NB, NV != 0>(&c[o * NB], m, out_n);
+    for (int o = 0; o < NV; o++) {
+        const uint4 r = *reinterpret_cast<const uint4 *>(&g->o[o]);
+        const uint2 e = tc_residue<NB>(c + 2 * NB * o, r), f = tc_residue<NB>(c + 2 * NB * o + NB, r);
+        asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(out_n + r.w * slot_words), "r"(e.x), "r"(e.y), "r"(f.x), "r"(f.y) : "memory");
+    }
+}
+__device__ __forceinline__ void tc_group_any(const uint32_t (&c)[32], uint2 hdr, const TcGroup *g, uint32_t slot_words, uint64_t *__restrict__ out_n) {
+    switch (hdr.x * 8 + hdr.y) {  // (bytes per output, outputs in the group): no slot is processed in vain
+        case 4 * 8 + 1: tc_group<4, 1>(c, g, slot_words, out_n); break;
+        case 4 * 8 + 2: tc_group<4, 2>(c, g, slot_words, out_n); break;
+        case 4 * 8 + 3: tc_group<4, 3>(c, g, slot_words, out_n); break;
+        case 4 * 8 + 4: tc_group<4, 4>(c, g, slot_words, out_n); break;
+        case 5 * 8 + 1: tc_group<5, 1>(c, g, slot_words, out_n); break;
+        case 5 * 8 + 2: tc_group<5, 2>(c, g, slot_words, out_n); break;
+        case 5 * 8 + 3: tc_group<5, 3>(c, g, slot_words, out_n); break;
+        case 6 * 8 + 1: tc_group<6, 1>(c, g, slot_words, out_n); break;
+        case 6 * 8 + 2: tc_group<6, 2>(c, g, slot_words, out_n); break;
+        case 7 * 8 + 1: tc_group<7, 1>(c, g, slot_words, out_n); break;
+        case 7 * 8 + 2: tc_group<7, 2>(c, g, slot_words, out_n); break;
+        case 8 * 8 + 1: tc_group<8, 1>(c, g, slot_words, out_n); break;
+        case 8 * 8 + 2: tc_group<8, 2>(c, g, slot_words, out_n); break;
+        default: break;  // an empty group: the planner makes none
     }
 }
 
-// grid = (N / 128, jobs); dynamic shared memory >= TC_SMEM_BYTES (the launcher asks for more, so that the CTAs
-// resident on one SM can never want more than its 512 TMEM columns and the allocation never has to wait)
-template <int WG>
-__global__ void __launch_bounds__(128 * WG) bconv_tc_kernel(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
-                                                            const uint64_t *__restrict__ copy_src, const TcJob *__restrict__ jobs,
-                                                            const TcGroup *__restrict__ groups, const uint8_t *__restrict__ images, uint32_t N,
-                                                            uint32_t *err) {
-    pdl_enter();
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
-    uint8_t *sA = tc_smem, *sB = tc_smem + TC_SMEM_A;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tc_smem + TC_SMEM_CTRL);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tc_smem + TC_SMEM_CTRL + 8);
-    const TcJob job = jobs[blockIdx.y];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t n0 = blockIdx.x * 128;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"(job.alloc_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    // B: the ready-made byte image of this job
-    {
-        const int4 *src = reinterpret_cast<const int4 *>(images + job.img_off);
-        int4 *dst = reinterpret_cast<int4 *>(sB);
-        for (uint32_t i = tid; i < job.n_groups * 64; i += 128 * WG) dst[i] = __ldg(src + i);
-    }
-    // A: row = coefficient, the 8 bytes of input limb i at k = 8 i .. 8 i + 7 (two limbs per 16-byte store)
-    {
-        const uint32_t r = tid & 127, part = tid >> 7;
-        constexpr int PAIRS = 4 / WG;
-        const bool copy = copy_src != nullptr && job.copy_dst_slot0 != 0xFFFFFFFFu;
-#pragma unroll
-        for (int pp = 0; pp < PAIRS; pp++) {
-            const uint32_t i = 2 * (part * PAIRS + pp);
-            uint64_t v[2] = {0, 0};
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                if (i + h < job.ni) {
-                    const size_t off = (size_t)(job.in_slot0 + i + h) * N + n0 + r;
-                    v[h] = in[off];
-                    if (copy) out[(size_t)(job.copy_dst_slot0 + i + h) * N + n0 + r] = copy_src[off];
-                }
-            }
-            *reinterpret_cast<ulonglong2 *>(sA + (r >> 3) * 512 + (i >> 1) * 128 + (r & 7) * 16) = make_ulonglong2(v[0], v[1]);
-        }
-    }
-    // generic-proxy writes of A and B become visible to the tensor core's (async-proxy) reads
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-    if (tid == 0) {
-        const uint64_t adesc = tc_desc(tc_smem_u32(sA)), bdesc = tc_desc(tc_smem_u32(sB));
-        // D s32, A and B u8, both K-major, N = 16 * groups, M = 128
-        const uint32_t idesc = (2u << 4) | (((16u * job.n_groups) >> 3) << 17) | ((128u >> 4) << 24);
-        tc_mma_i8(tmem, adesc, bdesc, idesc, 0u);
-        tc_mma_i8(tmem, adesc + (256u >> 4), bdesc + (256u >> 4), idesc, 1u);  // k = 32..63: two core matrices further
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem_u32(bar)) : "memory");
-    }
-    // bounded wait for the accumulators
-    uint32_t done = 0;
-    for (uint32_t it = 0; it < TC_WAIT_LIMIT && !done; it++) {
-        asm volatile(
-            "{\n\t"
-            ".reg .pred P1;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P1;\n\t"
-            "}\n"
-            : "=r"(done)
-            : "r"(tc_smem_u32(bar)), "r"(0u)
-            : "memory");
-    }
-    const bool ok = __all_sync(0xFFFFFFFFu, done != 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-        const uint32_t wq = warp & 3, wg = warp >> 2;
-        const uint32_t n = n0 + wq * 32 + lane;
-        const uint32_t lane_base = tmem + ((wq * 32u) << 16);
-        for (uint32_t g = wg; g < job.n_groups; g += WG) {
-            uint32_t c[16];
-            tc_ld16(lane_base + g * 16, c);
-            const TcGroup *G = groups + job.grp_off + g;
-            const uint2 hdr = __ldg(reinterpret_cast<const uint2 *>(G));
-            switch (hdr.x) {
-                case 4: tc_group_outputs<4>(c, G, hdr.y, out, N, n); break;
-                case 5: tc_group_outputs<5>(c, G, hdr.y, out, N, n); break;
-                case 6: tc_group_outputs<6>(c, G, hdr.y, out, N, n); break;
-                case 7: tc_group_outputs<7>(c, G, hdr.y, out, N, n); break;
-                default: tc_group_outputs<8>(c, G, hdr.y, out, N, n); break;
-            }
-        }
-    } else if (lane == 0) {
-        atomicExch(err, 1u);  // the MMA never signalled: outputs of this tile are not written
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(job.alloc_cols) : "memory");
-}
-
-
-// ================================================================================================
-// Persistent form: a CTA stays on its SM and walks over work items (job, tile), job-major, with stride gridDim.x.
-// The job's B image and group table stay in shared memory until the job changes; the next item's A tile is fetched
-// with cp.async into the second A buffer while the current tile's accumulators are reduced and stored, so global
-// latency, the MMA and the epilogue overlap inside one CTA (and across the CTAs sharing the SM). TMEM is allocated
-// once per CTA. One mbarrier, used with alternating phase parity, signals each tile's MMA pair.
-// ================================================================================================
-constexpr uint32_t TCP_SMEM_A0 = 0, TCP_SMEM_A1 = TC_SMEM_A, TCP_SMEM_B = 2 * TC_SMEM_A, TCP_SMEM_GRP = TCP_SMEM_B + TC_SMEM_B;
-constexpr uint32_t TCP_SMEM_CTRL = TCP_SMEM_GRP + 16 * 4 * 16 + 64;  // 16 groups x 4 output records, then one byte count per group
-constexpr uint32_t TCP_SMEM_BYTES = TCP_SMEM_CTRL + 32;
-
-__device__ __forceinline__ void tc_cp_async8(uint32_t smem_dst, const void *gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_dst), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void tc_cp_async16(uint32_t smem_dst, const void *gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
-}
-
-// the rows of A for tile `tile` of `job`: 8 bytes per (coefficient, input limb), zeros for limbs the job does not have
-// A batch of conversions in one launch: set b reads input limb slot s at s * (in_lm1 + 1) + b * in_bs and writes output limb
-// slot s at s * (out_lm1 + 1) + b * out_bs (batch-major and limb-major buffers as for the transforms, ntt_kernels.cuh)
-struct TcBatch {
+constexpr uint32_t TC_JOBS_INLINE = 8;
+struct TcArgs {
+    const uint64_t *in;
+    uint64_t *out;
+    const uint64_t *copy_src;  // optional (one set): the digit's own limbs go from here to the jobs' copy slots
+    const TcJob *jobs;         // the first TC_JOBS_INLINE of them in job[] as well: a load from memory less before the first copy
+    const TcGroup *groups;     // device form: o[].p holds 2^64 - p
+    const uint8_t *images;     // device form: tc_pair_image
+    uint32_t *err;
+    uint32_t N;
+    uint32_t items, more;      // a CTA works on `items` (job part, set, tile)s, the first `more` CTAs on one more
+    uint32_t parts;            // a job's groups are dealt over this many parts, items of their own
+    uint32_t stage_bytes, b_bytes;
+    uint32_t part_recs;        // most groups of a part: the output records of a CTA's parts lie that far apart
+    // A batch of conversions in one launch: set b reads input limb slot s at s * (in_lm1 + 1) + b * in_bs and writes output
+    // limb slot s at s * (out_lm1 + 1) + b * out_bs (batch-major and limb-major buffers as for the transforms, ntt_kernels.cuh)
     uint32_t batch, in_lm1, in_bs, out_lm1, out_bs;
-    uint32_t serial_ld;  // 1: wait for every TMEM load before reducing it (no second register set in flight)
+    TcJob job[TC_JOBS_INLINE];
 };
+__device__ __forceinline__ TcJob tc_job(const TcArgs &a, uint32_t j) { return j < TC_JOBS_INLINE ? a.job[j] : a.jobs[j]; }
 
-template <int WG>
-__device__ __forceinline__ void tcp_fetch_a(uint8_t *sA, const uint64_t *__restrict__ in, const TcJob &job, uint32_t N, uint32_t tile, uint32_t b,
-                                            const TcBatch &tb) {
-    const uint32_t tid = threadIdx.x, r = tid & 127, part = tid >> 7;
-    constexpr int LIMBS = 8 / WG;
-#pragma unroll
-    for (int j = 0; j < LIMBS; j++) {
-        const uint32_t i = part * LIMBS + j;
-        uint8_t *dst = sA + (r >> 3) * 512 + (i >> 1) * 128 + (r & 7) * 16 + (i & 1) * 8;
-        if (i < job.ni) {
-            const size_t slot = (size_t)(job.in_slot0 + i * (job.in_stride1 + 1)) * (tb.in_lm1 + 1) + (size_t)b * tb.in_bs;
-            tc_cp_async8(tc_smem_u32(dst), in + slot * N + (size_t)tile * 128 + r);
-        } else {
-            *reinterpret_cast<uint64_t *>(dst) = 0;
-        }
-    }
+// part `part` of a job: groups [g0, g1)
+__device__ __forceinline__ void tc_part(const TcJob &job, uint32_t part, uint32_t parts, uint32_t &g0, uint32_t &g1) {
+    g0 = job.n_groups * part / parts, g1 = job.n_groups * (part + 1) / parts;
 }
 
-template <int WG>
-__global__ void __launch_bounds__(128 * WG, 8 / WG) bconv_tc_persist(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
-                                                             const uint64_t *__restrict__ copy_src, const TcJob *__restrict__ jobs,
-                                                             const TcGroup *__restrict__ groups, const uint8_t *__restrict__ images, uint32_t N,
-                                                             uint32_t n_jobs, uint32_t alloc_cols, uint32_t *err, const TcBatch tb) {
-    pdl_enter();
+__global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_constant__ TcArgs a) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
-    uint8_t *sB = tc_smem + TCP_SMEM_B;
-    TcOutS *sOut = reinterpret_cast<TcOutS *>(tc_smem + TCP_SMEM_GRP);              // [16][4]
-    uint32_t *sNb = reinterpret_cast<uint32_t *>(tc_smem + TCP_SMEM_GRP + 16 * 4 * 16);  // [16]
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tc_smem + TCP_SMEM_CTRL);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tc_smem + TCP_SMEM_CTRL + 8);
-    constexpr uint32_t THREADS = 128 * WG;
+    const uint32_t sA = tc_smem_u32(tc_smem), sB = sA + TC_STAGES * a.stage_bytes;
+    uint8_t *ctrl = tc_smem + TC_STAGES * a.stage_bytes + a.b_bytes;
+    const uint32_t bar = tc_smem_u32(ctrl);
+    const uint32_t full_a = bar, empty_a = bar + 32, full_t = bar + 64, empty_t = bar + 96, full_b = bar + 128, drained = bar + 136;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ctrl + 144);
+    volatile uint32_t *gave_up = reinterpret_cast<volatile uint32_t *>(ctrl + 148);
+    static_assert(TC_STAGES <= 4 && TC_BUFS <= 4, "four barriers of a kind");
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // items: job-major, then set of the batch, then tile (N is a power of two)
-    const uint32_t tiles = N >> 7, tile_mask = tiles - 1, log_tiles = 31 - __clz(tiles), per_job = tb.batch << log_tiles, total = n_jobs * per_job;
+    const uint32_t log_tiles = 31 - __clz(a.N / TC_TILE), per_part = a.batch << log_tiles, tile_mask = (1u << log_tiles) - 1;
+    // consecutive items: a CTA changes its part as seldom as can be
+    const uint32_t v0 = blockIdx.x * a.items + min(blockIdx.x, a.more), v1 = v0 + a.items + (blockIdx.x < a.more);
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"(alloc_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    uint32_t item = blockIdx.x, cur = 0, phase = 0, loaded_job = 0xFFFFFFFFu;
-    bool ok = true;
+    TcGroup *recs = reinterpret_cast<TcGroup *>(ctrl + TC_CTRL_BYTES);
+    const uint32_t first_part = v0 / per_part;
+
+    // ---- loads: one warp, a lane a copy. The first item's are under way before the CTA meets for the first time ---------------
+    uint32_t cur = 0xFFFFFFFFu, n_b = 0;
     TcJob job{};
-    if (item < total) {
-        job = jobs[item / per_job];
-        tcp_fetch_a<WG>(tc_smem + TCP_SMEM_A0, in, job, N, item & tile_mask, (item % per_job) >> log_tiles, tb);
+    auto load_item = [&](uint32_t v, uint32_t k) {
+        const uint32_t pi = v / per_part, st = k % TC_STAGES;
+        if (pi != cur) {
+            // the part's columns of the job's B image; the MMAs that read the old one are done when the last item's are
+            if (k && !__all_sync(0xFFFFFFFFu, tc_wait(empty_a + 8 * ((k - 1) % TC_STAGES), ((k - 1) / TC_STAGES) & 1, gave_up))) return false;
+            job = tc_job(a, pi / a.parts);
+            uint32_t g0, g1;
+            tc_part(job, pi % a.parts, a.parts, g0, g1);
+            const uint32_t slices = (job.ni + 1) & ~1u, row = job.n_groups * 512, part_row = (g1 - g0) * 512;
+            if (lane == 0) tc_expect(full_b, slices * part_row);
+            __syncwarp();
+            if (lane < slices) tc_bulk(sB + lane * part_row, a.images + job.img_off + g0 * 512 + lane * row, part_row, full_b);
+            cur = pi, n_b++;
+        }
+        if (k == 0) pdl_enter();  // all above is the plan's
+        if (k >= TC_STAGES && !__all_sync(0xFFFFFFFFu, tc_wait(empty_a + 8 * st, (k / TC_STAGES - 1) & 1, gave_up))) return false;
+        const uint32_t tile = v & tile_mask, set = (v - pi * per_part) >> log_tiles;
+        if (lane == 0) tc_expect(full_a + 8 * st, job.ni * TC_SLICE);
+        __syncwarp();
+        if (lane < job.ni) {
+            const size_t slot = (size_t)(job.in_slot0 + lane * (job.in_stride1 + 1)) * (a.in_lm1 + 1) + (size_t)set * a.in_bs;
+            tc_bulk(sA + st * a.stage_bytes + lane * TC_SLICE, a.in + slot * a.N + (size_t)tile * TC_TILE, TC_SLICE, full_a + 8 * st);
+        }
+        return true;
+    };
+    if (warp == TC_EPI_WARPS + 1) {
+        // barriers 0 .. 17 as laid out above; those of empty_t take an arrival from every warp of the epilogue
+        if (lane < 18) tc_bar_init(bar + 8 * lane, lane >= 12 && lane < 16 ? TC_EPI_WARPS : 1);
+        if (lane == 0) *gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        load_item(v0, 0);
+    } else if (warp == TC_EPI_WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"(TC_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+        // the output records of every part the CTA will work on
+        for (uint32_t pi = first_part + warp; pi <= (v1 - 1) / per_part; pi += TC_EPI_WARPS) {
+            const TcJob j = tc_job(a, pi / a.parts);
+            uint32_t g0, g1;
+            tc_part(j, pi % a.parts, a.parts, g0, g1);
+            const uint4 *src = reinterpret_cast<const uint4 *>(a.groups + j.grp_off + g0);
+            uint4 *dst = reinterpret_cast<uint4 *>(recs + (pi - first_part) * a.part_recs);
+            for (uint32_t i = lane; i < (g1 - g0) * (sizeof(TcGroup) / 16); i += 32) dst[i] = __ldg(src + i);
+        }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const uint32_t wq = warp & 3, wg = warp >> 2;
-    const uint32_t lane_base = tmem + ((wq * 32u) << 16);
 
-    while (item < total && ok) {
-        const uint32_t jb = item / per_job, tile = item & tile_mask, bset = (item - jb * per_job) >> log_tiles;
-        if (jb != loaded_job) {
-            // a new job: its B image and group table (the MMA that read the old image has completed: every thread
-            // waited for it before the previous epilogue, and the barrier at the end of that iteration has passed)
-            job = jobs[jb];
-            const uint8_t *img = images + job.img_off;
-            for (uint32_t i = tid; i < job.n_groups * 64; i += THREADS) tc_cp_async16(tc_smem_u32(sB + 16 * i), img + 16 * i);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            // output records in the epilogue's form (nobody reads the old ones any more: see above)
-            if (tid < job.n_groups * 4) {
-                const TcGroup *G = groups + job.grp_off + (tid >> 2);
-                const uint32_t o = tid & 3;
-                const uint2 hdr = __ldg(reinterpret_cast<const uint2 *>(G));
-                TcOutS rec{1u, 0u, 0u, 0xFFFFFFFFu};
-                if (o < hdr.y) {
-                    const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(&G->o[o]));
-                    rec = TcOutS{raw.x, raw.y, raw.z, raw.w * (tb.out_lm1 + 1) * N};
+    if (warp == TC_EPI_WARPS + 1) {
+        uint32_t k = 1;
+        for (uint32_t v = v0 + 1; v < v1; v++, k++)
+            if (!load_item(v, k)) break;
+        // nothing may be in flight when the CTA ends
+        for (uint32_t i = k > TC_STAGES ? k - TC_STAGES : 0; i < k; i++) tc_wait(full_a + 8 * (i % TC_STAGES), (i / TC_STAGES) & 1, gave_up);
+        tc_wait(full_b, (n_b - 1) & 1, gave_up);
+    } else if (warp == TC_EPI_WARPS) {
+        // ---- MMAs -------------------------------------------------------------------------------------------------
+        if (lane == 0) {
+            uint32_t n_t = 0, k = 0, cols = 0, steps = 0;
+            bool ok = true;
+            for (uint32_t v = v0; v < v1 && ok; v++, k++) {
+                const uint32_t pi = v / per_part, st = k % TC_STAGES;
+                if (pi != cur) {
+                    job = tc_job(a, pi / a.parts);
+                    uint32_t g0, g1;
+                    tc_part(job, pi % a.parts, a.parts, g0, g1);
+                    cols = (g1 - g0) * 32, steps = (job.ni + 1) / 2;
+                    if (!(ok = tc_wait(full_b, n_b & 1, gave_up))) break;
+                    cur = pi, n_b++;
                 }
-                sOut[tid] = rec;
-                if (o == 0) sNb[tid >> 2] = hdr.x * 8 + hdr.y;  // bytes per output, outputs in the group
+                if (!(ok = tc_wait(full_a + 8 * st, (k / TC_STAGES) & 1, gave_up))) break;
+                const uint64_t adesc = tc_desc(sA + st * a.stage_bytes, TC_SLICE);
+                for (uint32_t c0 = 0; c0 < cols; c0 += TC_ACC_COLS, n_t++) {
+                    const uint32_t buf = n_t % TC_BUFS, n = min(cols - c0, TC_ACC_COLS);
+                    if (n_t >= TC_BUFS && !(ok = tc_wait(empty_t + 8 * buf, (n_t / TC_BUFS - 1) & 1, gave_up))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t bdesc = tc_desc(sB + c0 * 16, cols * 16);
+                    // D s32, A and B u8, both K-major, M = 128, N = the columns of up to four groups
+                    const uint32_t idesc = (2u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+                    for (uint32_t s = 0; s < steps; s++)  // 32 bytes of K: two input limbs
+                        tc_mma_i8(tmem + buf * TC_ACC_COLS, adesc + s * (2 * TC_SLICE >> 4), bdesc + s * (2 * cols * 16 >> 4), idesc, s != 0);
+                    tc_commit(full_t + 8 * buf);
+                }
+                tc_commit(empty_a + 8 * st);
             }
-            loaded_job = jb;
+            tc_commit(drained);
+            tc_wait(drained, 0, gave_up);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        uint8_t *sA = tc_smem + (cur ? TCP_SMEM_A1 : TCP_SMEM_A0);
-        if (tid == 0) {
-            const uint64_t adesc = tc_desc(tc_smem_u32(sA)), bdesc = tc_desc(tc_smem_u32(sB));
-            const uint32_t idesc = (2u << 4) | (((16u * job.n_groups) >> 3) << 17) | ((128u >> 4) << 24);
-            tc_mma_i8(tmem, adesc, bdesc, idesc, 0u);
-            tc_mma_i8(tmem, adesc + (256u >> 4), bdesc + (256u >> 4), idesc, 1u);
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem_u32(bar)) : "memory");
-        }
-        // next item's rows of A into the other buffer (its last reader, the MMA of the previous iteration, is done)
-        const uint32_t next = item + gridDim.x;
-        if (next < total) {
-            const uint32_t njb = next / per_job, nb = (next - njb * per_job) >> log_tiles;
-            if (njb == jb) {
-                tcp_fetch_a<WG>(tc_smem + (cur ? TCP_SMEM_A0 : TCP_SMEM_A1), in, job, N, next & tile_mask, nb, tb);
-            } else {
-                const TcJob nj = jobs[njb];
-                tcp_fetch_a<WG>(tc_smem + (cur ? TCP_SMEM_A0 : TCP_SMEM_A1), in, nj, N, next & tile_mask, nb, tb);
+    } else {
+        // ---- reduction and stores -----------------------------------------------------------------------------------
+        pdl_enter();
+        const uint32_t lane_base = tmem + ((warp & 3) << 21), mine = warp >> 2, n_row = 2 * ((warp & 3) * 32 + lane);
+        const uint32_t slot_words = (a.out_lm1 + 1) * a.N;
+        uint32_t n_t = 0, k = 0, g0 = 0, g1 = 0;
+        bool ok = true;
+        for (uint32_t v = v0; v < v1 && ok; v++, k++) {
+            const uint32_t pi = v / per_part, tile = v & tile_mask, set = (v - pi * per_part) >> log_tiles;
+            if (pi != cur) {
+                job = tc_job(a, pi / a.parts);
+                tc_part(job, pi % a.parts, a.parts, g0, g1);
+                cur = pi;
+            }
+            if (a.copy_src != nullptr && g0 == 0 && job.copy_dst_slot0 != 0xFFFFFFFFu && tid < TC_TILE)
+                for (uint32_t i = 0; i < job.ni; i++)
+                    a.out[(size_t)(job.copy_dst_slot0 + i) * a.N + (size_t)tile * TC_TILE + tid] =
+                        a.copy_src[(size_t)(job.in_slot0 + i) * a.N + (size_t)tile * TC_TILE + tid];
+            uint64_t *out_n = a.out + (size_t)set * a.out_bs * a.N + (tile * TC_TILE + n_row);
+            // a last chunk that is not full is shared out evenly over the items
+            const uint32_t own = (mine + k) % TC_CHUNK;
+            for (uint32_t c0 = 0; c0 < g1 - g0; c0 += TC_CHUNK, n_t++) {
+                const uint32_t buf = n_t % TC_BUFS, g = c0 + own;
+                const bool work = g < g1 - g0;
+                const TcGroup *G = recs + (pi - first_part) * a.part_recs + (work ? g : 0);
+                const uint2 hdr = *reinterpret_cast<const uint2 *>(G);
+                ok = __all_sync(0xFFFFFFFFu, tc_wait(full_t + 8 * buf, (n_t / TC_BUFS) & 1, gave_up));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t c[32];
+                if (work) {
+                    tc_ld32(lane_base + buf * TC_ACC_COLS + own * 32, c);
+                    tc_wait_ld(c);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc_arrive(empty_t + 8 * buf);  // the planes are in registers
+                if (work) tc_group_any(c, hdr, G, slot_words, out_n);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        // ModUp: the digit's own limbs travel from the NTT-form input to the output buffer (single set only)
-        if (copy_src != nullptr && job.copy_dst_slot0 != 0xFFFFFFFFu) {
-            const uint32_t r = tid & 127, part = tid >> 7;
-            for (uint32_t i = part; i < job.ni; i += WG)
-                out[(size_t)(job.copy_dst_slot0 + i) * N + (size_t)tile * 128 + r] = copy_src[(size_t)(job.in_slot0 + i) * N + (size_t)tile * 128 + r];
-        }
-        // bounded wait for the accumulators
-        uint32_t done = 0;
-        for (uint32_t it = 0; it < TC_WAIT_LIMIT && !done; it++) {
-            asm volatile(
-                "{\n\t"
-                ".reg .pred P1;\n\t"
-                "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-                "selp.b32 %0, 1, 0, P1;\n\t"
-                "}\n"
-                : "=r"(done)
-                : "r"(tc_smem_u32(bar)), "r"(phase)
-                : "memory");
-        }
-        phase ^= 1u;
-        ok = __all_sync(0xFFFFFFFFu, done != 0);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok) {
-            uint64_t *out_n = out + (size_t)bset * tb.out_bs * N + (tile * 128 + wq * 32 + lane);
-            // (dealing single outputs instead of whole groups over the warpgroups evens the work but triples the TMEM loads:
-            // measured 56 against 37 us per key switch)
-            auto reduce_group = [&](const uint32_t (&c)[16], uint32_t g) {
-                const uint32_t mo = tc_smem_u32(sOut + 4 * g);
-                // one case per (bytes per output, outputs in the group): no slot is processed in vain and no store is predicated
-                switch (sNb[g]) {
-                    case 4 * 8 + 1: tc_group_lean<4, 1>(c, mo, out_n); break;
-                    case 4 * 8 + 2: tc_group_lean<4, 2>(c, mo, out_n); break;
-                    case 4 * 8 + 3: tc_group_lean<4, 3>(c, mo, out_n); break;
-                    case 4 * 8 + 4: tc_group_lean<4, 4>(c, mo, out_n); break;
-                    case 5 * 8 + 1: tc_group_lean<5, 1>(c, mo, out_n); break;
-                    case 5 * 8 + 2: tc_group_lean<5, 2>(c, mo, out_n); break;
-                    case 5 * 8 + 3: tc_group_lean<5, 3>(c, mo, out_n); break;
-                    case 6 * 8 + 1: tc_group_lean<6, 1>(c, mo, out_n); break;
-                    case 6 * 8 + 2: tc_group_lean<6, 2>(c, mo, out_n); break;
-                    case 7 * 8 + 1: tc_group_lean<7, 1>(c, mo, out_n); break;
-                    case 7 * 8 + 2: tc_group_lean<7, 2>(c, mo, out_n); break;
-                    case 8 * 8 + 1: tc_group_lean<8, 1>(c, mo, out_n); break;
-                    case 8 * 8 + 2: tc_group_lean<8, 2>(c, mo, out_n); break;
-                    default: break;  // an empty group: the planner makes none
-                }
-            };
-            // two register sets: the next group's planes travel from TMEM while this one is reduced
-            uint32_t ca[16], cb[16];
-            uint32_t g = wg;
-            if (tb.serial_ld) {
-                for (; g < job.n_groups; g += WG) {
-                    tc_ld16(lane_base + g * 16, ca);
-                    reduce_group(ca, g);
-                }
-            } else {
-                if (g < job.n_groups) tc_ld16_nowait(lane_base + g * 16, ca);
-                while (g < job.n_groups) {
-                    tc_wait_ld(ca);
-                    uint32_t gn = g + WG;
-                    if (gn < job.n_groups) tc_ld16_nowait(lane_base + gn * 16, cb);
-                    reduce_group(ca, g);
-                    g = gn;
-                    if (g >= job.n_groups) break;
-                    tc_wait_ld(cb);
-                    gn = g + WG;
-                    if (gn < job.n_groups) tc_ld16_nowait(lane_base + gn * 16, ca);
-                    reduce_group(cb, g);
-                    g = gn;
-                }
-            }
-        } else if (lane == 0) {
-            atomicExch(err, 1u);  // the MMA never signalled: this CTA stops, its remaining tiles are not written
-        }
-        // a CTA whose wait ran out must stop as a whole: make the outcome uniform over the CTA
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        ok = __syncthreads_and(ok);
-        cur ^= 1u;
-        item = next;
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(alloc_cols) : "memory");
+    if (tid == 0 && *gave_up) atomicExch(a.err, 1u);  // a barrier never completed: outputs from there on are not written
+    if (warp == TC_EPI_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
 }
 
 }  // namespace b2

@@ -20,6 +20,7 @@
 // a job (a digit of ModUp, a polynomial of ModDown) has at most 16 groups = 256 columns. A and B are laid out in
 // the canonical K-major no-swizzle form of the sm_100 shared-memory matrix descriptor (8-row x 16-byte core matrices):
 //     offset(row, k) = (row / 8) * 512 + (k / 16) * 128 + (row % 8) * 16 + k % 16.
+// This is the compact form; the kernel takes rows of two coefficients each (tc_pair_image).
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -185,5 +186,26 @@ struct TcBuild {
         return added;
     }
 };
+
+// A job's image as the kernel reads it. Its rows of A hold TWO coefficients: K slice i (16 bytes) is input limb i of both, and
+// the groups' 16 columns become 32, output o of a group in columns 2 nb o .. (first coefficient's nb bytes, then the second's),
+// zero in the half of every slice that belongs to the other coefficient. Slices (an even number: an MMA takes two) one after
+// another, in each the columns' 16 bytes. Appended to `out`.
+static inline void tc_pair_image(const TcBuild &b, const TcJob &job, std::vector<uint8_t> &out) {
+    const uint32_t slices = (job.ni + 1) & ~1u, cols = 32 * job.n_groups;
+    const size_t base = out.size();
+    out.resize(base + (size_t)slices * cols * 16, 0);
+    for (uint32_t g = 0; g < job.n_groups; g++) {
+        const TcGroup &G = b.groups[job.grp_off + g];
+        for (uint32_t w = 0; w < G.n_valid * G.nb; w++)  // column of the compact group: byte w % nb of output w / nb
+            for (uint32_t k = 0; k < 8 * job.ni; k++) {
+                const uint8_t v = b.images[job.img_off + tc_operand_offset(16 * g + w, k)];
+                for (uint32_t c = 0; c < 2; c++) {
+                    const uint32_t col = 32 * g + (w / G.nb) * 2 * G.nb + c * G.nb + w % G.nb;
+                    out[base + ((size_t)(k / 8) * cols + col) * 16 + 8 * c + k % 8] = v;
+                }
+            }
+    }
+}
 
 }  // namespace b2

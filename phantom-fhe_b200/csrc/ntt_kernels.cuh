@@ -231,7 +231,8 @@ __device__ __forceinline__ int pad_idx(int e) { return e + (e >> RC); }
 //   gs_sum / gs_prod   bounds of the two outputs of an inverse butterfly; gs(.., ba, bb) is that butterfly
 //   group_end          what is done to a residue that changes thread between two stage groups of a pass
 //   pass_end           what is done to a residue that is stored between the passes of an inverse transform
-//   B_CANON / B_PASS / GS_PASS   bounds of canonical input, of what a forward / an inverse pass stores
+//   B_CANON / B_IN / B_PASS / GS_PASS   bounds of canonical input, of a forward transform's input (canonical, or below 2 q as the
+//                       tensor-core conversion leaves it), of what a forward / an inverse pass stores
 constexpr uint64_t FP_SMALL_LIMIT = 1ull << 41;
 constexpr uint64_t FP_LIMIT = 1ull << 50;
 constexpr uint64_t INT_LAZY_LIMIT = 1ull << 60;
@@ -249,7 +250,7 @@ struct ArithIntLazy {
         uint64_t q, nq;   // nq = -q mod 2^64
         uint32_t m, s;    // floor(2^(64 + s) / q), normalised to 32 bits
     };
-    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_PASS = 16, GS_PASS = 6, B_BCONV = RED;
+    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_IN = 2, B_PASS = 16, GS_PASS = 6, B_BCONV = RED;
     __device__ __forceinline__ static K make(const Mod &md, int) {
         const uint32_t s = __clz((uint32_t)md.r1);  // r1 = floor(2^64 / q), in [2^4, 2^14]
         return K{md.q, 0 - md.q, (uint32_t)((md.r1 << s) | (md.r0 >> (64 - s))), s};
@@ -320,7 +321,7 @@ struct ArithInt {
     struct K {
         uint64_t q, q2;
     };
-    static constexpr int B_CANON = 0, B_PASS = 0, GS_PASS = 0, B_BCONV = 0;
+    static constexpr int B_CANON = 0, B_IN = 0, B_PASS = 0, GS_PASS = 0, B_BCONV = 0;
     __device__ __forceinline__ static K make(const Mod &md, int) { return K{md.q, 2 * md.q}; }
     using TwRaw = W2;
     static constexpr int TW_RUN = 2;  // twiddles in 32 bytes
@@ -365,7 +366,7 @@ struct ArithFp {
         double q, qinv;
     };
     static constexpr int FACTOR = 32, LIM = 128, RED = 9;
-    static constexpr int B_CANON = BIG ? 16 : 0, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0, B_BCONV = BIG ? RED : 0;
+    static constexpr int B_CANON = BIG ? 16 : 0, B_IN = 2 * B_CANON, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0, B_BCONV = BIG ? RED : 0;
     static constexpr bool IS_BIG = BIG;
     __host__ __device__ static constexpr int prod(int B) { return 9 + (B + 3) / 4; }
     // table entry i of an FP64 prime is one double (8 bytes); w / q is rebuilt as w * (1/q), whose
@@ -610,14 +611,14 @@ __device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a
 
 // ================================================================================================
 // forward pass: R1 strided stages, exchange, R2 contiguous stages
-// FIRST: the input holds canonical residues (else the raw lazy values of the previous pass)
+// FIRST: the input holds residues within B_IN as words (else the raw lazy values of the previous pass)
 // ================================================================================================
 // SRC (column pass only): where the input comes from, see load_src
 template <class A, int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, int SRC = 0>
 __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint64_t *sm, const Job &job, uint32_t jobi, const Mod &md, uint32_t tile) {
     using T = typename A::T;
     static_assert(SRC == 0 || COLS, "the on-the-fly source belongs to the column pass");
-    constexpr int B0 = SRC == 3 ? A::B_BCONV : COLS ? A::B_CANON : A::B_PASS, B1 = ct_bound<A>(B0, R1);
+    constexpr int B0 = SRC == 3 ? A::B_BCONV : COLS ? A::B_IN : A::B_PASS, B1 = ct_bound<A>(B0, R1);
     static_assert(ct_bound<A>(B1, R2) <= A::B_PASS, "a forward pass stores residues within B_PASS");
     constexpr bool FIRST = COLS;
     constexpr int TT = 1 << LOG_T, E1 = 1 << R1, E2 = 1 << R2, C = 1 << LOG_C;

@@ -95,7 +95,7 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const Epi &epi,
     using Cfg = WholeCfg<LOGN>;
     constexpr int LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
     constexpr int N2 = 1 << Cfg::LOG_B, CC = 1 << LOG_CC;
-    constexpr int B0 = SRC == 3 ? A::B_BCONV : A::B_CANON;
+    constexpr int B0 = SRC == 3 ? A::B_BCONV : A::B_IN;
     constexpr size_t N = (size_t)1 << LOGN;
     uint64_t *slab = smem, *ex = smem + whole_slab<LOGN>();
     const typename A::K k = A::make(md, LOGN);

@@ -642,3 +642,27 @@ def test_conversion_in_the_column_pass_equals_the_oracle(log_n, bits, special, l
     for i in range(batch):
         assert np.array_equal(got[i], o.multiply_and_relin(l, a[i], b[i], key)), f"set {i}"
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("log_n,special,l", [(12, 7, 8), (13, 1, 5), (14, 4, 9), (14, 5, 5), (15, 8, 17), (16, 6, 7), (17, 3, 4)])
+def test_pair_conversion_edges(log_n, special, l):
+    """the tensor-core conversion at odd numbers of input limbs, ragged digits and column groups that leave its items uneven:
+    ModUp (with the digits' own limbs copied) and a batch of key switches, every byte count of an output prime among them"""
+    from pyPhantom import _native
+    from pyPhantom._native import LIB, check
+    from gpu_helpers import stream
+    bits = ([60, 30, 40, 46, 50, 55, 36, 42] * 3)[:l] + [60] * special
+    ctx, o = make_ctx(1 << log_n, bits, special)
+    c2 = o.fill(1, o.primes[:l], 3, 7)[0]
+    up = ctx.empty(o.beta(l), l + special)
+    nb = LIB.b2_workspace_bytes(ctx._h, _native.OP_MODUP, l)
+    ws = torch.empty(nb // 8, dtype=torch.int64, device="cuda")
+    check(LIB.b2_modup(ctx._h, l, dev(c2).data_ptr(), up.data_ptr(), ws.data_ptr(), nb, stream()))
+    want = o.modup(l, c2)
+    assert np.array_equal(host(up).reshape(want.shape), want)
+    key = o.synth_key(o.beta(l), 3, 10)
+    sets = [o.fill(3, o.primes[:l], 3, 20 + i) for i in range(3)]
+    got = host(ph.relinearize_batch(ctx, dev(np.stack(sets)), _key(ctx, key)))
+    for i, s in enumerate(sets):
+        assert np.array_equal(got[i], o.keyswitch(l, s[2], key, s[:2])), f"set {i}"
+    assert ctx.device_status() == 0
