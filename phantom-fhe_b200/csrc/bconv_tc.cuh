@@ -199,6 +199,7 @@ __device__ __forceinline__ void tc_part(const TcJob &job, uint32_t part, uint32_
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_constant__ TcArgs a) {
+    pdl_enter();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     const uint32_t sA = tc_smem_u32(tc_smem), sB = sA + TC_STAGES * a.stage_bytes;
     uint8_t *ctrl = tc_smem + TC_STAGES * a.stage_bytes + a.b_bytes;
@@ -232,7 +233,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_con
             if (lane < slices) tc_bulk(sB + lane * part_row, a.images + job.img_off + g0 * 512 + lane * row, part_row, full_b);
             cur = pi, n_b++;
         }
-        if (k == 0) pdl_enter();  // all above is the plan's
         if (k >= TC_STAGES && !__all_sync(0xFFFFFFFFu, tc_wait(empty_a + 8 * st, (k / TC_STAGES - 1) & 1, gave_up))) return false;
         const uint32_t tile = v & tile_mask, set = (v - pi * per_part) >> log_tiles;
         if (lane == 0) tc_expect(full_a + 8 * st, job.ni * TC_SLICE);
@@ -312,7 +312,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_con
         }
     } else {
         // ---- reduction and stores -----------------------------------------------------------------------------------
-        pdl_enter();
         const uint32_t lane_base = tmem + ((warp & 3) << 21), mine = warp >> 2, n_row = 2 * ((warp & 3) * 32 + lane);
         const uint32_t slot_words = (a.out_lm1 + 1) * a.N;
         uint32_t n_t = 0, k = 0, g0 = 0, g1 = 0;
