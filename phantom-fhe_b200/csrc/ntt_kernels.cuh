@@ -89,7 +89,15 @@ __device__ __forceinline__ Job get_job(const NttArgs &a, uint32_t j) {
 struct u64x4 {
     uint64_t a, b, c, d;
 };
+// Volatile: a statement that is a function of its address to the compiler may be moved out of a loop and executed where the
+// condition around it does not hold (the fused row pass read past the end of its input for the P limbs so), or ahead of the
+// wait for the previous kernel. Tables of the context have neither problem: any index of theirs is there to be read.
 __device__ __forceinline__ u64x4 ld256(const uint64_t *p) {
+    u64x4 v;
+    asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.a), "=l"(v.b), "=l"(v.c), "=l"(v.d) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ u64x4 ld256_table(const uint64_t *p) {
     u64x4 v;
     asm("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.a), "=l"(v.b), "=l"(v.c), "=l"(v.d) : "l"(p));
     return v;
@@ -104,7 +112,7 @@ __device__ __forceinline__ void ld_pairs(W2 (&w)[CNT], const W2 *p) {
     if constexpr (CNT == 1) {
         w[0] = ldg_w2(p);
     } else {
-        const u64x4 v = ld256(reinterpret_cast<const uint64_t *>(p));
+        const u64x4 v = ld256_table(reinterpret_cast<const uint64_t *>(p));
         w[0] = W2{v.a, v.b}, w[1] = W2{v.c, v.d};
     }
 }
@@ -381,7 +389,7 @@ struct ArithFp {
             const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
             w[0] = v.x, w[1] = v.y;
         } else {
-            const u64x4 v = ld256(reinterpret_cast<const uint64_t *>(p));
+            const u64x4 v = ld256_table(reinterpret_cast<const uint64_t *>(p));
             w[0] = from_raw(v.a), w[1] = from_raw(v.b), w[2] = from_raw(v.c), w[3] = from_raw(v.d);
         }
     }
