@@ -193,6 +193,10 @@ struct LevelPlan {
     Job *jobs_dnf_intt = nullptr;  // fused key switch: P limbs live compactly in [2][alpha][N]
     Job *jobs_dnf_ntt = nullptr;   // 2*l, epilogue subtracts from the ciphertext
     BconvGroup *grp_dnf = nullptr; // 2
+    // ModDown and rescale in one on blocks [2][l] | [2][alpha] | [2] (moddown_rescale)
+    Job *jobs_drs_intt = nullptr;  // 2*alpha P limbs, then the dropped limb of both polynomials
+    Job *jobs_drs_ntt = nullptr;   // 2*(l-1)
+    BcJob *bc_drs = nullptr;
     Job *jobs_rs_intt = nullptr;   // 3 (one per polynomial)
     Job *jobs_rs_ntt = nullptr;    // 3*(l-1)
     W2 *fin_up = nullptr;          // [l][2]
@@ -221,6 +225,7 @@ struct b2_ctx {
     Mod *d_mod = nullptr;
     W2 *d_tw = nullptr, *d_itw = nullptr;
     W2 *d_fin_plain = nullptr;  // [size_QP][2] = {N^-1, itw[1]}
+    W2 *d_fin_drs = nullptr;    // d_fin_P, then d_fin_plain: inverse transforms of P limbs and others in one launch
     W2 *d_fin_P = nullptr;      // [size_P][2]  = the same times (P/p_i)^-1 mod p_i
     W2 *d_Pinv = nullptr;       // [size_QP] indexed by prime (valid for Q primes): P^-1 mod q_j
     W2 *d_macfin = nullptr;     // [size_QP] closing constant of the fused inner product's Montgomery sums: P^-1 * 2^64 mod q_j, 2^64 mod p_i
@@ -382,8 +387,8 @@ static int build_level(b2_ctx *c, size_t l) {
     const size_t n_up_ntt = beta * lP - l;
     const size_t mat_up_words = beta * lP * alpha;
     // host staging mirrors the device blob
-    size_t bytes = 64 + sizeof(Job) * (l + 2 * n_up_ntt + 4 * alpha + 4 * l + 3 + 3 * l) + sizeof(W2) * (2 * l + c->size_QP) +
-                   sizeof(BconvGroup) * (beta + 4 + 3) + sizeof(uint2) * (n_up_ntt + l + l) + 8 * mat_up_words * 6 + sizeof(BcJob) * (n_up_ntt + 2 * l) + 16 * 32;
+    size_t bytes = 64 + sizeof(Job) * (l + 2 * n_up_ntt + 6 * alpha + 6 * l + 5 + 3 * l) + sizeof(W2) * (2 * l + c->size_QP) +
+                   sizeof(BconvGroup) * (beta + 4 + 3) + sizeof(uint2) * (n_up_ntt + l + l) + 8 * mat_up_words * 6 + sizeof(BcJob) * (n_up_ntt + 4 * l) + 16 * 32;
     std::vector<char> host(bytes, 0);
     char *cur = host.data();
     auto *jobs_up_intt = blob_take<Job>(cur, l);
@@ -394,6 +399,8 @@ static int build_level(b2_ctx *c, size_t l) {
     auto *jobs_dnf_intt = blob_take<Job>(cur, 2 * alpha);
     auto *jobs_dnf_ntt = blob_take<Job>(cur, 2 * l);
     auto *grp_dnf = blob_take<BconvGroup>(cur, 2);
+    auto *jobs_drs_intt = blob_take<Job>(cur, 2 * alpha + 2);
+    auto *jobs_drs_ntt = blob_take<Job>(cur, 2 * l);
     auto *jobs_rs_intt = blob_take<Job>(cur, 3);
     auto *jobs_rs_ntt = blob_take<Job>(cur, 3 * l);
     auto *fin_up = blob_take<W2>(cur, 2 * l);
@@ -405,6 +412,7 @@ static int build_level(b2_ctx *c, size_t l) {
     auto *matw_up = blob_take<W2>(cur, mat_up_words);
     auto *bc_up = blob_take<BcJob>(cur, n_up_ntt);
     auto *bc_dnf = blob_take<BcJob>(cur, 2 * l);
+    auto *bc_drs = blob_take<BcJob>(cur, 2 * l);
     auto *grp_dn = blob_take<BconvGroup>(cur, 2);
     auto *outs_dn = blob_take<uint2>(cur, l);
     const size_t used = cur - host.data();
@@ -475,6 +483,18 @@ static int build_level(b2_ctx *c, size_t l) {
         for (size_t j = 0; j + 1 < l; j++) {
             qlast_inv[j] = h_w2(h_invmod(ql % c->q[j], c->q[j]), c->q[j]);
         }
+        for (size_t k = 0; k < 2; k++) {
+            for (size_t i = 0; i < alpha; i++) {
+                const uint32_t slot = (uint32_t)(2 * l + k * alpha + i);
+                jobs_drs_intt[k * alpha + i] = make_uint4(slot, (uint32_t)(sQ + i), (uint32_t)i, slot);
+            }
+            jobs_drs_intt[2 * alpha + k] = make_uint4((uint32_t)(k * l + l - 1), (uint32_t)(l - 1), (uint32_t)(alpha + l - 1), (uint32_t)(2 * l + 2 * alpha + k));
+            for (size_t j = 0; j + 1 < l; j++) {
+                const uint32_t slot = (uint32_t)(k * l + j);
+                jobs_drs_ntt[k * (l - 1) + j] = make_uint4(slot, (uint32_t)j, slot, (uint32_t)(k * (l - 1) + j));
+                bc_drs[k * (l - 1) + j] = bc_dnf[slot];
+            }
+        }
         for (size_t p = 0; p < 3; p++) {
             jobs_rs_intt[p] = make_uint4((uint32_t)(p * l + l - 1), (uint32_t)(l - 1), (uint32_t)(l - 1), (uint32_t)p);
             for (size_t j = 0; j + 1 < l; j++)
@@ -498,6 +518,9 @@ static int build_level(b2_ctx *c, size_t l) {
     pl.jobs_dnf_intt = (Job *)dev(jobs_dnf_intt);
     pl.jobs_dnf_ntt = (Job *)dev(jobs_dnf_ntt);
     pl.grp_dnf = (BconvGroup *)dev(grp_dnf);
+    pl.jobs_drs_intt = (Job *)dev(jobs_drs_intt);
+    pl.jobs_drs_ntt = (Job *)dev(jobs_drs_ntt);
+    pl.bc_drs = (BcJob *)dev(bc_drs);
     pl.jobs_rs_intt = (Job *)dev(jobs_rs_intt);
     pl.jobs_rs_ntt = (Job *)dev(jobs_rs_ntt);
     pl.fin_up = (W2 *)dev(fin_up);
@@ -553,6 +576,7 @@ extern "C" void b2_ctx_destroy(b2_ctx *c) {
     cudaFree(c->d_itw);
     cudaFree(c->d_fin_plain);
     cudaFree(c->d_fin_P);
+    cudaFree(c->d_fin_drs);
     cudaFree(c->d_Pinv);
     cudaFree(c->d_macfin);
     cudaFree(c->d_mat_dn);
@@ -716,6 +740,8 @@ extern "C" int b2_ctx_create(size_t N, const uint64_t *primes, size_t size_QP, s
             fp[2 * l + 1] = h_tw_enc(fin_plain[2 * l + 1].w, c->q[l]);
         }
         if (e == cudaSuccess) e = up((void **)&c->d_fin_plain, fp.data(), sizeof(W2) * 2 * size_QP);
+        fp.insert(fp.begin(), fin_P.begin(), fin_P.end());
+        if (e == cudaSuccess) e = up((void **)&c->d_fin_drs, fp.data(), sizeof(W2) * fp.size());
     }
     if (e == cudaSuccess) e = up((void **)&c->d_fin_P, fin_P.data(), sizeof(W2) * 2 * sP);
     if (e == cudaSuccess) e = up((void **)&c->d_Pinv, Pinv.data(), sizeof(W2) * size_QP);
@@ -876,7 +902,6 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
     launch_k(ntt_inv_pass<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_CC, true, true>, grid, pass_threads<LOG_A, true>(), 0, s, b);
 }
 
-// SRC != 0: the column pass makes limb job.x from slot job.x / src_div of src (words mod src_q) instead of reading it
 // A batched launch: `batch` polynomial sets, slot s of set b at s * (lm1 + 1) + b * bs of the source / destination
 struct BatchDims {
     uint32_t batch = 1, src_lm1 = 0, src_bs = 0, dst_lm1 = 0, dst_bs = 0;
@@ -915,16 +940,25 @@ static bool convert_loading(const b2_ctx *c, size_t limbs) {
 }
 template <class Epi, int SRC> struct WholeHas : std::false_type {};
 template <> struct WholeHas<EpiStore, 0> : std::true_type {};
-template <> struct WholeHas<EpiSubMul<false>, 1> : std::true_type {};
-template <> struct WholeHas<EpiSubMul<false>, 2> : std::true_type {};
+template <> struct WholeHas<EpiSubMul<false>, SRC_REM> : std::true_type {};
+template <> struct WholeHas<EpiSubMul<false>, SRC_REM | SRC_NEAR> : std::true_type {};
+
+// The remainders a rescale by prime q subtracts: see NttArgs::rem
+struct RemSrc {
+    const uint64_t *rem = nullptr;
+    uint32_t div = 1, bs = 0;
+    uint64_t q = 0;
+    bool rounded = false;
+    void put(NttArgs &a) const { a.rem = rem, a.rem_div = div, a.rem_bs = bs, a.rem_q = q, a.rem_half = rounded ? q >> 1 : ~0ull; }
+};
 
 template <class Epi, int SRC = 0>
 static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Job *jobs, uint32_t njobs, uint32_t first_prime,
-                   const Epi &epi, cudaStream_t s, uint32_t period = 0, uint32_t src_div = 0, uint64_t src_q = 0, const BatchDims &bd = BatchDims{}) {
+                   const Epi &epi, cudaStream_t s, uint32_t period = 0, const BatchDims &bd = BatchDims{}, const RemSrc &rem = RemSrc{}) {
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, period, src_div, src_q, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
-    if (SRC != 0 && src_div == 0) return fail(B2_EINVAL, "the on-the-fly source needs its divisor");
+    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, period, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
+    rem.put(a);
     if constexpr (WholeHas<Epi, SRC>::value) {
         if ((SRC == 0 || c->logN == 12) && use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, period)) {
             LaunchScope ls(c, s, "ntt_fwd_whole");
@@ -950,7 +984,7 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
                    const W2 *fin, cudaStream_t s, const BatchDims &bd = BatchDims{}) {
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, bd.perm};
+    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, bd.perm};
     if (use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, 0)) {
         LaunchScope ls(c, s, "ntt_inv_whole");
         launch_inv_whole(a, njobs, bd.batch, s);
@@ -970,22 +1004,23 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
     return B2_OK;
 }
 
-// base conversion made while the forward transform loads: job j's limb comes from the input limbs bc[j] names (2^12: one launch in
-// all, the other rings: in the column pass)
-template <class Epi>
+// base conversion made while the forward transform loads (plus, SRC = SRC_CONV | SRC_REM, a remainder): job j's limb comes from the
+// input limbs bc[j] names (2^12: one launch in all, the other rings: in the column pass)
+template <class Epi, int SRC = SRC_CONV>
 static int run_bconv_fwd(const b2_ctx *c, const uint64_t *in, uint64_t *dst, const Job *jobs, const BcJob *bc, const W2 *mat, uint32_t njobs, const Epi &epi,
-                         cudaStream_t s, const BatchDims &bd = BatchDims{}) {
+                         cudaStream_t s, const BatchDims &bd = BatchDims{}, const RemSrc &rem = RemSrc{}) {
     if (!aligned32(in) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{in, dst, jobs, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0, 0, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
+    NttArgs a{in, dst, jobs, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
     a.bc = bc, a.mat = mat;
+    rem.put(a);
     switch (c->logN) {
-        case 16: launch_fwd<8, 8, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
-        case 15: launch_fwd<7, 8, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
-        case 14: launch_fwd<7, 7, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
-        case 13: launch_fwd<6, 7, Epi, 3>(c, a, njobs, epi, s, bd.batch); break;
+        case 16: launch_fwd<8, 8, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
+        case 15: launch_fwd<7, 8, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
+        case 14: launch_fwd<7, 7, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
+        case 13: launch_fwd<6, 7, Epi, SRC>(c, a, njobs, epi, s, bd.batch); break;
         default: {
             LaunchScope ls(c, s, "bconv_ntt_whole");
-            launch_fwd_whole<Epi, 3>(a, epi, njobs, bd.batch, s);
+            launch_fwd_whole<Epi, SRC>(a, epi, njobs, bd.batch, s);
         }
     }
     LAUNCH_CHECK("bconv_ntt_fwd");
@@ -1438,6 +1473,7 @@ static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint6
 struct KsBatch {
     uint32_t batch = 1, c2_bs = 0, ct_bs = 0;
     KsRot rot;
+    uint32_t cxp_bs = 0;  // 0: 2 alpha
 };
 
 // Whether a batch is better off with the row pass that carries the inner product than with a stored row pass and the stand-alone
@@ -1476,7 +1512,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         return B2_OK;  // the caller falls back to one key switch at a time
     {
         using Cfg = PassCfg<8>;
-        const uint32_t B = kb.batch, per = (uint32_t)(beta * lP), a2 = (uint32_t)(2 * c->size_P);
+        const uint32_t B = kb.batch, per = (uint32_t)(beta * lP), a2 = kb.cxp_bs ? kb.cxp_bs : (uint32_t)(2 * c->size_P);
         int rc = run_inv(c, c2, t, pl.jobs_up_intt, (uint32_t)l, 0, pl.fin_up, s, BatchDims{B, 0, kb.c2_bs, 0, (uint32_t)l, kb.rot.perm});
         if (rc) return rc;
         if (loading && !mac) {
@@ -1489,7 +1525,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (rc) return rc;
         if (!mac) {
             // both passes stored for every limb, then the stand-alone inner product, each one launch over the batch
-            if (!loading) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            if (!loading) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
             rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib, kb.rot);
@@ -1504,7 +1540,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (loading) {
             NttArgs b = a;
             b.src = t, b.src_bs = batched ? (uint32_t)l : 0, b.bc = pl.bc_up, b.mat = pl.matw_up;
-            launch_fwd_cols<3>(c, b, pl.n_up_ntt, s, B);
+            launch_fwd_cols<SRC_CONV>(c, b, pl.n_up_ntt, s, B);
         } else {
             launch_fwd_cols<0>(c, a, pl.n_up_ntt, s, B);
         }
@@ -1622,7 +1658,7 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per};
     rc = run_bconv_tc(c, false, cxP, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, tb);
     if (rc) return rc;
-    return run_fwd(c, up, up, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_ct, (uint32_t)ct_stride}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+    return run_fwd(c, up, up, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_ct, (uint32_t)ct_stride}, s, 0, BatchDims{B, 0, per, 0, per});
 }
 
 extern "C" int b2_keyswitch_batch(b2_ctx *c, size_t l, size_t batch, const uint64_t *d_c2, size_t c2_stride, const uint64_t *const *evk, size_t n_evk,
@@ -1669,15 +1705,16 @@ extern "C" int b2_multiply_and_relin(b2_ctx *c, size_t l, const uint64_t *d_a, c
 }
 
 // Second half of a rescale. r [n_poly][N]: the dropped limb of every polynomial in coefficient form. Every remaining
-// limb j gets (in_j - NTT_j(rem mod q_j)) * q_last^-1 with rem = r (MODE 1, the reference's floor: src/rns.cu:1128-1183)
-// or its centred representative (MODE 2, round to nearest). The forward column pass reduces r into q_j as it loads, so
+// limb j gets (in_j - NTT_j(rem mod q_j)) * q_last^-1 with rem = r (the reference's floor: src/rns.cu:1128-1183)
+// or its centred representative (rounded: to nearest). The forward column pass reduces r into q_j as it loads, so
 // the (l-1) reduced copies are never written out.
-template <int MODE>
-static int rescale_tail(const b2_ctx *c, size_t l, size_t n_poly, const uint64_t *r, const uint64_t *d_in, uint64_t *d_out, cudaStream_t s) {
+static int rescale_tail(const b2_ctx *c, size_t l, size_t n_poly, const uint64_t *r, const uint64_t *d_in, uint64_t *d_out, bool rounded, cudaStream_t s) {
     const LevelPlan &pl = c->plan[l];
     EpiSubMul<false> epi{d_in, d_out, pl.qlast_inv};
     const uint32_t njobs = (uint32_t)(n_poly * (l - 1));
-    return run_fwd<EpiSubMul<false>, MODE>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, (uint32_t)(l - 1), c->q[l - 1]);
+    const RemSrc rem{r, (uint32_t)(l - 1), 0, c->q[l - 1], rounded};
+    if (rounded) return run_fwd<EpiSubMul<false>, SRC_REM | SRC_NEAR>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, BatchDims{}, rem);
+    return run_fwd<EpiSubMul<false>, SRC_REM>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, BatchDims{}, rem);
 }
 
 extern "C" int b2_rescale(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *d_in, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
@@ -1695,7 +1732,7 @@ extern "C" int b2_rescale(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *d_
         int rc = run_inv(c, d_in, r, pl.jobs_rs_intt, (uint32_t)n_poly, 0, c->d_fin_plain, s);
         if (rc) return rc;
     }
-    return rescale_tail<1>(c, l, n_poly, r, d_in, d_out, s);
+    return rescale_tail(c, l, n_poly, r, d_in, d_out, false, s);
 }
 
 extern "C" int b2_rescale_rounded(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *d_in, uint64_t *d_out, void *d_ws, size_t ws_bytes,
@@ -1714,20 +1751,76 @@ extern "C" int b2_rescale_rounded(b2_ctx *c, size_t l, size_t n_poly, const uint
         int rc = run_inv(c, d_in, r, pl.jobs_rs_intt, (uint32_t)n_poly, 0, c->d_fin_plain, s);
         if (rc) return rc;
     }
-    return rescale_tail<2>(c, l, n_poly, r, d_in, d_out, s);
+    return rescale_tail(c, l, n_poly, r, d_in, d_out, true, s);
 }
 
 // The same for `sets` two-polynomial ciphertexts, set b at b * in_bs / out_bs limbs; r: 2 * sets limbs of scratch
-template <int MODE>
 static int rescale_sets(const b2_ctx *c, size_t l, uint32_t sets, const uint64_t *d_in, uint32_t in_bs, uint64_t *r, uint64_t *d_out, uint32_t out_bs,
-                        cudaStream_t s) {
+                        bool rounded, cudaStream_t s) {
     const LevelPlan &pl = c->plan[l];
     int rc = run_inv(c, d_in, r, pl.jobs_rs_intt, 2, 0, c->d_fin_plain, s, BatchDims{sets, 0, in_bs, 0, 2});
     if (rc) return rc;
     EpiSubMul<false> epi{d_in, d_out, pl.qlast_inv};
     epi.m_bs = in_bs, epi.o_bs = out_bs;
-    return run_fwd<EpiSubMul<false>, MODE>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, (uint32_t)(l - 1), c->q[l - 1],
-                                           BatchDims{sets, 0, 2, 0, out_bs});
+    const BatchDims bd{sets, 0, 2, 0, out_bs};
+    const RemSrc rem{r, (uint32_t)(l - 1), 2, c->q[l - 1], rounded};
+    if (rounded) return run_fwd<EpiSubMul<false>, SRC_REM | SRC_NEAR>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, bd, rem);
+    return run_fwd<EpiSubMul<false>, SRC_REM>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, bd, rem);
+}
+
+// ModDown and rescale in one, for `sets` blocks of `bs` limbs each, [2][l] ciphertext | [2][alpha] P limbs | [2] scratch: the inner
+// product has left ct + acc * P^-1 in the ciphertext. Both steps subtract the transform of something they have in coefficient
+// form, so one transform of the sum does: with delta the converted P limbs and r the dropped limb after ModDown,
+//     r = INTT(ct_last) - delta_last,    out_j = (ct_j - NTT(delta_j + r mod q_j)) * q_last^-1,
+// the same limbs with 2 l transforms less (2^16, 24 limbs, alpha 8: 160 of 208) and as many trips of the ciphertext. B200, one
+// after another -> in one: 32 products at 2^14, 8 limbs 600 -> 535 us; a polynomial of degree 31 at 2^15 (eleven products, one to
+// four at a time) 1285 -> 1199 us; a bootstrap at 2^16 24.46 -> 23.52 ms.
+// up: scratch, 2 l limbs a set from set * up_bs on.
+static int moddown_rescale(const b2_ctx *c, size_t l, uint32_t sets, uint64_t *blk, uint32_t bs, uint64_t *up, uint32_t up_bs, uint64_t *d_out, uint32_t out_bs,
+                           bool rounded, cudaStream_t s) {
+    const LevelPlan &pl = c->plan[l];
+    const size_t N = c->N, a = c->size_P;
+    uint64_t *P = blk + 2 * l * N, *r = P + 2 * a * N;
+    int rc = run_inv(c, blk, blk, pl.jobs_drs_intt, (uint32_t)(2 * a + 2), 0, c->d_fin_drs, s, BatchDims{sets, 0, bs, 0, bs});
+    if (rc) return rc;
+    {
+        LaunchScope ls(c, s, "rescale_remainder");
+        launch_k(rescale_remainder_kernel, dim3((unsigned)(N / 1024), 2, sets), 256, 0, s, (const uint64_t *)P, r, c->d_matw_dn_pinv + (l - 1) * a, c->d_mod + (l - 1),
+                 (uint32_t)N, (uint32_t)a, bs);
+        LAUNCH_CHECK("rescale_remainder_kernel");
+    }
+    EpiSubMul<false> epi{blk, d_out, pl.qlast_inv};
+    epi.m_bs = bs, epi.o_bs = out_bs;
+    const uint32_t njobs = (uint32_t)(2 * (l - 1));
+    const RemSrc rem{r, (uint32_t)l, bs, c->q[l - 1], rounded};
+    if (convert_loading(c, (size_t)njobs * sets))
+        return run_bconv_fwd<EpiSubMul<false>, SRC_CONV | SRC_REM>(c, P, up, pl.jobs_drs_ntt, pl.bc_drs, c->d_matw_dn_pinv, njobs, epi, s,
+                                                                   BatchDims{sets, 0, bs, 0, up_bs}, rem);
+    rc = run_bconv_tc(c, false, P, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, TcBatch{sets, 0, bs, 0, up_bs});
+    if (rc) return rc;
+    return run_fwd<EpiSubMul<false>, SRC_WORDS | SRC_REM>(c, up, up, pl.jobs_drs_ntt, njobs, 0, epi, s, 0, BatchDims{sets, 0, up_bs, 0, up_bs}, rem);
+}
+
+// Key switch of `sets` products and the rescale behind it. Block layout and `up` as above, a block's last l limbs the third
+// polynomial; t: l limbs a set.
+static int keyswitch_rescale(b2_ctx *c, size_t l, uint32_t sets, uint64_t *blk, const uint64_t *const *evk, size_t n_evk, uint64_t *t, uint64_t *up, uint64_t *d_out,
+                             uint32_t out_bs, bool rounded, cudaStream_t s) {
+    const LevelPlan &pl = c->plan[l];
+    const size_t N = c->N, a = c->size_P;
+    const uint32_t bs = (uint32_t)(3 * l + 2 * a + 2), per = (uint32_t)(pl.beta * (l + a));
+    uint64_t *P = blk + 2 * l * N, *c2 = P + (2 * a + 2) * N;
+    bool done = false;
+    KsBatch kb;
+    kb.batch = sets, kb.c2_bs = kb.ct_bs = kb.cxp_bs = bs;
+    int rc = modup_inner_fused(c, l, c2, evk, n_evk, blk, P, t, up, false, s, &done, kb);
+    if (rc) return rc;
+    if (!done) {  // one set
+        rc = modup_impl(c, l, c2, up, t, false, s);
+        if (rc) return rc;
+        rc = inner_prod_impl(c, l, up, c2, evk, n_evk, P, blk, true, s);
+        if (rc) return rc;
+    }
+    return moddown_rescale(c, l, sets, blk, bs, up, per, d_out, out_bs, rounded, s);
 }
 
 extern "C" size_t b2_multiply_relin_batch_workspace_bytes(const b2_ctx *c, size_t l, size_t batch) {
@@ -1755,16 +1848,23 @@ extern "C" int b2_multiply_relin_rescale_batch(b2_ctx *c, size_t l, size_t batch
     cudaStream_t s = (cudaStream_t)stream;
     const size_t N = c->N, S = l * N;
     const uint32_t B = (uint32_t)batch;
-    uint64_t *prod = (uint64_t *)d_ws, *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
+    const bool merged = rescale && c->bconv_tc;
+    const size_t pl_limbs = merged ? 2 * c->size_P + 2 : 0, bs = 3 * l + pl_limbs;  // a product's block: d0, d1, (P limbs, scratch,) d2
+    uint64_t *prod = (uint64_t *)d_ws;
     {
         LaunchScope ls(c, s, "tensor_mul");
-        LAUNCH_V(tensor_mul_kernel, true, (unsigned)l, B, s, d_a, d_b, prod, prod + 2 * S, c->d_mod, (uint32_t)N, (uint32_t)l,
-                 make_uint4((uint32_t)a_stride, (uint32_t)b_stride, (uint32_t)(3 * l), (uint32_t)(3 * l)));
+        LAUNCH_V(tensor_mul_kernel, true, (unsigned)l, B, s, d_a, d_b, prod, prod + 2 * S + pl_limbs * N, c->d_mod, (uint32_t)N, (uint32_t)l,
+                 make_uint4((uint32_t)a_stride, (uint32_t)b_stride, (uint32_t)bs, (uint32_t)bs));
         LAUNCH_CHECK("tensor_mul_kernel");
     }
+    if (merged) {
+        uint64_t *t = prod + batch * bs * N;
+        return keyswitch_rescale(c, l, B, prod, rlk, n_evk, t, t + batch * S, d_out, (uint32_t)out_stride, false, s);
+    }
+    uint64_t *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
     int rc = keyswitch_batch_impl(c, l, batch, prod + 2 * S, 3 * l, rlk, n_evk, prod, 3 * l, ws, s);
     if (rc) return rc;
-    if (rescale) return rescale_sets<1>(c, l, B, prod, (uint32_t)(3 * l), r, d_out, (uint32_t)out_stride, s);
+    if (rescale) return rescale_sets(c, l, B, prod, (uint32_t)(3 * l), r, d_out, (uint32_t)out_stride, false, s);
     for (size_t b = 0; b < batch; b++) CUDA_TRY(cudaMemcpyAsync(d_out + b * out_stride * N, prod + b * 3 * S, 2 * S * 8, cudaMemcpyDeviceToDevice, s));
     return B2_OK;
 }
@@ -1793,15 +1893,22 @@ extern "C" int b2_multiply_relin_rescale_many(b2_ctx *c, size_t l, size_t produc
     }
     cudaStream_t s = (cudaStream_t)stream;
     const size_t N = c->N, S = l * N;
-    uint64_t *prod = (uint64_t *)d_ws, *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
+    const size_t pl_limbs = c->bconv_tc ? 2 * c->size_P + 2 : 0, bs = 3 * l + pl_limbs;  // as in the batch above
+    uint64_t *prod = (uint64_t *)d_ws;
+    tm.out_bs = (uint32_t)bs, tm.d2 = (uint32_t)(2 * l + pl_limbs);
     {
         LaunchScope ls(c, s, "tensor_mul");
         launch_k(tensor_many_kernel, dim3((unsigned)(N / 1024), (unsigned)l, (unsigned)batch), 256, 0, s, tm, prod, c->d_mod, (uint32_t)N, (uint32_t)l);
         LAUNCH_CHECK("tensor_many_kernel");
     }
+    if (c->bconv_tc) {
+        uint64_t *t = prod + batch * bs * N;
+        return keyswitch_rescale(c, l, (uint32_t)batch, prod, rlk, n_evk, t, t + batch * S, d_out, (uint32_t)(2 * (l - 1)), true, s);
+    }
+    uint64_t *r = prod + batch * 3 * S, *ws = r + batch * 2 * N;
     int rc = keyswitch_batch_impl(c, l, batch, prod + 2 * S, 3 * l, rlk, n_evk, prod, 3 * l, ws, s);
     if (rc) return rc;
-    return rescale_sets<2>(c, l, (uint32_t)batch, prod, (uint32_t)(3 * l), r, d_out, (uint32_t)(2 * (l - 1)), s);
+    return rescale_sets(c, l, (uint32_t)batch, prod, (uint32_t)(3 * l), r, d_out, (uint32_t)(2 * (l - 1)), true, s);
 }
 
 // b2_rescale_rounded for `sets` ciphertexts [sets][2][l][N] -> [sets][2][l - 1][N]; workspace 2 * sets limbs
@@ -1811,7 +1918,7 @@ extern "C" int b2_rescale_rounded_batch(b2_ctx *c, size_t l, size_t sets, const 
     if (!d_in || !d_out || !d_ws || sets < 1 || sets > 65535) return fail(B2_EINVAL, "rescale_rounded_batch: bad argument");
     if (l < 2) return fail(B2_EINVAL, "rescale_rounded_batch: no prime left to drop");
     if (ws_bytes < 2 * sets * limb_bytes(c)) return fail(B2_EWS, "rescale_rounded_batch: workspace too small");
-    return rescale_sets<2>(c, l, (uint32_t)sets, d_in, (uint32_t)(2 * l), (uint64_t *)d_ws, d_out, (uint32_t)(2 * (l - 1)), (cudaStream_t)stream);
+    return rescale_sets(c, l, (uint32_t)sets, d_in, (uint32_t)(2 * l), (uint64_t *)d_ws, d_out, (uint32_t)(2 * (l - 1)), true, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1866,7 +1973,7 @@ extern "C" int b2_rescale_static(b2_ctx *c, size_t l, size_t n_poly, const uint6
         rc = run_inv(c, d_in + (p * l + l - 1) * c->N, r + p * c->N, nullptr, 1, (uint32_t)(l - 1), c->d_fin_plain, s);
         if (rc) return rc;
     }
-    return rescale_tail<1>(c, l, n_poly, r, d_in, d_out, s);
+    return rescale_tail(c, l, n_poly, r, d_in, d_out, false, s);
 }
 
 extern "C" uint32_t b2_galois_elt_from_step(int step, size_t N) {
@@ -2039,7 +2146,7 @@ extern "C" int b2_rotate_sum(b2_ctx *c, size_t l, size_t n, const uint32_t *elts
                     if (rc) return rc;
                 }
             }
-            rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
         }
         IpArgs ia = ip_args(c, l, up, c1, accP, d_acc);
@@ -2163,7 +2270,7 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
                 if (rc) return rc;
             }
         }
-        rc = run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, epi, s, 0, 0, 0, BatchDims{n, 0, (uint32_t)(2 * l), 0, (uint32_t)(2 * l)});
+        rc = run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, epi, s, 0, BatchDims{n, 0, (uint32_t)(2 * l), 0, (uint32_t)(2 * l)});
         if (rc) return rc;
     }
     return B2_OK;
@@ -2886,7 +2993,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 launch_k(ntt_fwd_rows_mac<8, Cfg::R_CONTIG, Cfg::LOG_C>, dim3(B, (sp.nq + sp.np) * (uint32_t)(N >> (8 + Cfg::LOG_C))), pass_threads<8>(), mac_smem_bytes<8, Cfg::R_CONTIG, Cfg::LOG_C>(), s, na, m);
                 LAUNCH_CHECK("ntt_fwd_rows_mac");
             } else {
-                rc = run_fwd(c, UP, UP, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+                rc = run_fwd(c, UP, UP, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
                 if (rc) return rc;
                 const uint4 rg = make_uint4(sp.q0, sp.nq, sp.p0, sp.np);
                 const IpBatch ib{per, (uint32_t)l, (uint32_t)(2 * l), 2, 1, B - 1, 1};
@@ -2900,7 +3007,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
             const TcBatch tb{B, B - 1, 1, 0, per};
             rc = run_bconv_tc(c, false, CXP, UP, nullptr, sp.tc_dn_b, sp.tc_dn_b.n_jobs, s, tb);
             if (rc) return rc;
-            return run_fwd(c, UP, UP, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct, (uint32_t)(2 * l)}, s, 0, 0, 0, BatchDims{B, 0, per, 0, per});
+            return run_fwd(c, UP, UP, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct, (uint32_t)(2 * l)}, s, 0, BatchDims{B, 0, per, 0, per});
         }
         default:
             return fail(B2_EINVAL, "shard_keyswitch_phase_batch: phase must be 0, 1 or 2");

@@ -341,12 +341,13 @@ __global__ void __launch_bounds__(256) tensor_mul_kernel(const uint64_t *a, cons
 }
 
 // The same for products whose operands lie apart and may sit at higher levels (more limbs per polynomial): blockIdx.z =
-// product p * sets + set, operand p at a[p] + set * 2 la[p] limbs. out [product][3][l][N]; dbl: the doubled product.
+// product p * sets + set, operand p at a[p] + set * 2 la[p] limbs. dbl: the doubled product.
 constexpr int TENSOR_MANY_MAX = 16;
 struct TensorMany {
     const uint64_t *a[TENSOR_MANY_MAX], *b[TENSOR_MANY_MAX];
     uint32_t la[TENSOR_MANY_MAX], lb[TENSOR_MANY_MAX];
     uint32_t sets, dbl;
+    uint32_t out_bs, d2;  // a product's results lie out_bs limbs apart, its third polynomial d2 limbs behind the first
 };
 __global__ void __launch_bounds__(256) tensor_many_kernel(const __grid_constant__ TensorMany t, uint64_t *out, const Mod *mod, uint32_t N, uint32_t l) {
     pdl_enter();
@@ -362,8 +363,34 @@ __global__ void __launch_bounds__(256) tensor_many_kernel(const __grid_constant_
 #pragma unroll
         for (int i = 0; i < V; i++) d0[i] = add_mod(d0[i], d0[i], md.q), d1[i] = add_mod(d1[i], d1[i], md.q), d2[i] = add_mod(d2[i], d2[i], md.q);
     }
-    out += (size_t)blockIdx.z * 3 * S + o;
-    stv<V>(out, d0), stv<V>(out + S, d1), stv<V>(out + 2 * S, d2);
+    out += (size_t)blockIdx.z * t.out_bs * N + o;
+    stv<V>(out, d0), stv<V>(out + S, d1), stv<V>(out + (size_t)t.d2 * N, d2);
+}
+
+// The dropped limb of a rescale after ModDown, in coefficient form: r -= sum_i P_i M_i mod q over the alpha P limbs (M: the last
+// prime's row of the ModDown matrix). blockIdx.y = polynomial, blockIdx.z = set, bs limbs apart.
+__global__ void __launch_bounds__(256) rescale_remainder_kernel(const uint64_t *P, uint64_t *r, const W2 *m, const Mod *mod, uint32_t N, uint32_t alpha, uint32_t bs) {
+    pdl_enter();
+    constexpr int V = 4;
+    const Mod md = *mod;
+    const bool tight = md.q >= INT_LAZY_LIMIT;  // eight terms below 2 q could pass 2^64
+    const size_t o = (size_t)blockIdx.z * bs * N + (blockIdx.x * 256 + threadIdx.x) * V;
+    P += o + (size_t)blockIdx.y * alpha * N, r += o + (size_t)blockIdx.y * N;
+    uint64_t x[V], s[V] = {0, 0, 0, 0};
+    ldv<V>(x, r);
+    for (uint32_t i = 0; i < alpha; i++) {
+        const W2 w = ldg_w2(m + i);
+        uint64_t y[V];
+        ldv<V>(y, P + (size_t)i * N);
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            s[j] += mul_shoup_lazy(y[j], w, md.q);
+            if (tight) s[j] = csub(s[j], 2 * md.q);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < V; j++) x[j] = sub_mod(x[j], barrett64(s[j], md.q, md.r1), md.q);
+    stv<V>(r, x);
 }
 
 // x y mod q for V pairs, FP64 below 2^50

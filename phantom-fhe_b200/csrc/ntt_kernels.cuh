@@ -58,18 +58,23 @@ struct NttArgs {
     const Mod *mod;        // [size_QP]
     const W2 *fin;         // inverse only: [idx][2] = {scale of the x outputs, last-stage twiddle}
     uint32_t period;       // without a job list: limb j uses prime first_prime + j % period (0: + j), a batch of polynomials
-    // forward column pass with SRC != 0 (rescale): limb job.x is not read from its own slot but made on the fly from
-    // slot job.x / src_div of src, whose words are residues mod src_q, reduced into the limb's prime
-    uint32_t src_div;
-    uint64_t src_q;
     // A batch of polynomial sets in one launch (the two-pass kernels only): blockIdx.y = set b, and limb slot s of set b
     // lives at slot s * (lm1 + 1) + b * bs of the buffer. Zero-initialised fields mean one set, slots as they are.
     // Batch-major buffers [b][slots] use lm1 = 0, bs = slots per set; limb-major ones [slot][b] use lm1 = batch - 1, bs = 1.
     uint32_t src_lm1, src_bs, dst_lm1, dst_bs;
     const uint32_t *perm;  // inverse row pass: the input is read through a Galois element's permutation (a rotation's c1)
-    const BcJob *bc;       // SRC = 3: one per job, the conversion that makes its limb, and the matrix entries
+    const BcJob *bc;       // SRC_CONV: one per job, the conversion that makes its limb, and the matrix entries
     const W2 *mat;
+    // SRC_REM: the dropped limbs of a rescale, residues mod rem_q in coefficient form; limb job.x takes slot job.x / rem_div, set b's
+    // start b * rem_bs limbs further; words above rem_half stand for word - rem_q (rounding to nearest; all ones: floor)
+    const uint64_t *rem;
+    uint32_t rem_div, rem_bs;
+    uint64_t rem_q, rem_half;
 };
+// What a forward transform reads: the words as they are (0, or with a remainder SRC_WORDS | SRC_REM), the base conversion of other
+// limbs (SRC_CONV), the remainder that a rescale subtracts (SRC_REM: floor, SRC_REM | SRC_NEAR: nearest), or the sum of a remainder
+// (either) and one of the others
+enum { SRC_REM = 1, SRC_CONV = 2, SRC_WORDS = 4, SRC_NEAR = 8 };
 
 // The sets of a batched launch are the slow grid dimension. With the sets fastest (the CTAs of all sets on one tile next to
 // one another, sharing its twiddles in L2) the row passes ran as fast and the column passes 8 % slower on B200.
@@ -77,6 +82,11 @@ __device__ __forceinline__ uint32_t set_idx(const NttArgs &) { return blockIdx.y
 __device__ __forceinline__ uint32_t work_idx(const NttArgs &) { return blockIdx.x; }
 __device__ __forceinline__ size_t src_slot(const NttArgs &a, uint32_t slot) { return (size_t)slot * (a.src_lm1 + 1) + (size_t)set_idx(a) * a.src_bs; }
 __device__ __forceinline__ size_t dst_slot(const NttArgs &a, uint32_t slot) { return (size_t)slot * (a.dst_lm1 + 1) + (size_t)set_idx(a) * a.dst_bs; }
+
+template <int SRC>
+__device__ __forceinline__ const uint64_t *src_rem(const NttArgs &a, const Job &job, size_t N) {
+    return SRC & SRC_REM ? a.rem + ((size_t)(job.x / a.rem_div) + (size_t)set_idx(a) * a.rem_bs) * N : nullptr;
+}
 
 __device__ __forceinline__ Job get_job(const NttArgs &a, uint32_t j) {
     if (a.jobs) return a.jobs[j];
@@ -572,24 +582,26 @@ __device__ __forceinline__ void bc_term(double (&x)[E], const uint64_t (&y)[E], 
     }
 }
 
-// E residues of a limb at positions n0, n0 + step, .. of what a forward transform reads. SRC: 0 = the words as they are, 1 = the
-// dropped limb's words reduced into the limb's prime, 2 = their centred representative (word - src_q when the word exceeds
-// src_q / 2) reduced: the remainder a rescale subtracts, floor or nearest; 3 = the base conversion of the limbs that bc names.
+// E residues of a limb at positions n0, n0 + step, .. of the transform's source
 template <class A, int SRC, int E>
-__device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a, const BcJob &bc, const uint64_t *src, size_t N, size_t n0,
-                                          size_t step, const Mod &md, const typename A::K &k) {
-    if constexpr (SRC != 3) {
-        const uint64_t half = SRC == 2 ? a.src_q >> 1 : 0, q_red = SRC == 2 ? barrett64(a.src_q, md.q, md.r1) : 0;
+__device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a, const BcJob &bc, const uint64_t *src, const uint64_t *rem, size_t N, size_t n0,
+                                         size_t step, const Mod &md, const typename A::K &k) {
+    if constexpr (SRC & SRC_REM) {
+        if constexpr (SRC & SRC_CONV) load_src<A, SRC_CONV>(x, a, bc, src, nullptr, N, n0, step, md, k);
+        else if constexpr (SRC & SRC_WORDS) load_src<A, 0>(x, a, bc, src, nullptr, N, n0, step, md, k);
+        const uint64_t q_red = SRC == SRC_REM ? 0 : barrett64(a.rem_q, md.q, md.r1);
+        uint64_t v[E];
+#pragma unroll
+        for (int i = 0; i < E; i++) v[i] = rem[n0 + i * step];
 #pragma unroll
         for (int i = 0; i < E; i++) {
-            uint64_t v = src[n0 + i * step];
-            if (SRC) {
-                const uint64_t word = v;
-                v = barrett64(word, md.q, md.r1);
-                if (SRC == 2 && word > half) v = sub_mod(v, q_red, md.q);
-            }
-            x[i] = A::from_u64(v, k);
+            uint64_t r = barrett64(v[i], md.q, md.r1);
+            if (SRC != SRC_REM && v[i] > a.rem_half) r = sub_mod(r, q_red, md.q);
+            x[i] = SRC & (SRC_CONV | SRC_WORDS) ? x[i] + A::from_u64(r, k) : A::from_u64(r, k);
         }
+    } else if constexpr (SRC == 0) {
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = A::from_u64(src[n0 + i * step], k);
     } else {
         constexpr bool FP = std::is_same<typename A::T, double>::value;
 #pragma unroll
@@ -617,16 +629,22 @@ __device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a
     }
 }
 
+// bound of what load_src gives
+template <class A, int SRC>
+__host__ __device__ constexpr int src_bound() {
+    return (SRC & SRC_REM ? A::B_CANON : 0) + (SRC & SRC_CONV ? A::B_BCONV : (SRC & SRC_WORDS) || SRC == 0 ? A::B_IN : 0);
+}
+
 // ================================================================================================
 // forward pass: R1 strided stages, exchange, R2 contiguous stages
 // FIRST: the input holds residues within B_IN as words (else the raw lazy values of the previous pass)
 // ================================================================================================
-// SRC (column pass only): where the input comes from, see load_src
+// SRC (column pass only): where the input comes from
 template <class A, int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, int SRC = 0>
 __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint64_t *sm, const Job &job, uint32_t jobi, const Mod &md, uint32_t tile) {
     using T = typename A::T;
     static_assert(SRC == 0 || COLS, "the on-the-fly source belongs to the column pass");
-    constexpr int B0 = SRC == 3 ? A::B_BCONV : COLS ? A::B_IN : A::B_PASS, B1 = ct_bound<A>(B0, R1);
+    constexpr int B0 = COLS ? src_bound<A, SRC>() : A::B_PASS, B1 = ct_bound<A>(B0, R1);
     static_assert(ct_bound<A>(B1, R2) <= A::B_PASS, "a forward pass stores residues within B_PASS");
     constexpr bool FIRST = COLS;
     constexpr int TT = 1 << LOG_T, E1 = 1 << R1, E2 = 1 << R2, C = 1 << LOG_C;
@@ -637,8 +655,8 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
     const typename A::K k = A::make(md, (int)a.logN);
     const W2 *tw = a.tw + (size_t)job.y * N;
     BcJob bc{};
-    if (SRC == 3) bc = a.bc[jobi];
-    const uint64_t *src = a.src + src_slot(a, SRC == 3 ? bc.in_slot0 : SRC ? job.x / a.src_div : job.x) * N;
+    if (SRC & SRC_CONV) bc = a.bc[jobi];
+    const uint64_t *src = a.src + src_slot(a, SRC & SRC_CONV ? bc.in_slot0 : job.x) * N, *rem = src_rem<SRC>(a, job, N);
     const size_t estride = COLS ? (N >> LOG_T) : 1;
     const size_t cstride = COLS ? 1 : TT;
     const size_t base = COLS ? (size_t)tile * C : (size_t)tile * C * TT;
@@ -655,7 +673,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
         T x[E1];
         const size_t n0 = base + (size_t)c * cstride + (size_t)elo * estride;
         if (FIRST) {
-            load_src<A, SRC>(x, a, bc, src, N, n0, E2 * estride, md, k);
+            load_src<A, SRC>(x, a, bc, src, rem, N, n0, E2 * estride, md, k);
         } else {
 #pragma unroll
             for (int i = 0; i < E1; i++) x[i] = A::from_raw(src[n0 + (size_t)i * E2 * estride]);

@@ -30,10 +30,11 @@ void launch_fwd_whole(const NttArgs &a, const Epi &epi, uint32_t njobs, uint32_t
 }
 
 template void launch_fwd_whole<EpiStore, 0>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiStore, 3>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubFrom, 3>(const NttArgs &, const EpiSubFrom &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubFromTab, 3>(const NttArgs &, const EpiSubFromTab &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubMul<false>, 1>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
-template void launch_fwd_whole<EpiSubMul<false>, 2>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiStore, SRC_CONV>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubFrom, SRC_CONV>(const NttArgs &, const EpiSubFrom &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubFromTab, SRC_CONV>(const NttArgs &, const EpiSubFromTab &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, SRC_REM | SRC_NEAR>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, SRC_REM>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiSubMul<false>, SRC_CONV | SRC_REM>(const NttArgs &, const EpiSubMul<false> &, uint32_t, uint32_t, cudaStream_t);
 
 }  // namespace b2

@@ -95,19 +95,19 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const Epi &epi,
     using Cfg = WholeCfg<LOGN>;
     constexpr int LOG_CC = Cfg::LOG_B - Cfg::LOG_CL, LOG_CR = Cfg::LOG_A - Cfg::LOG_CL;
     constexpr int N2 = 1 << Cfg::LOG_B, CC = 1 << LOG_CC;
-    constexpr int B0 = SRC == 3 ? A::B_BCONV : A::B_IN;
+    constexpr int B0 = src_bound<A, SRC>();
     constexpr size_t N = (size_t)1 << LOGN;
     uint64_t *slab = smem, *ex = smem + whole_slab<LOGN>();
     const typename A::K k = A::make(md, LOGN);
     const W2 *tw = a.tw + (size_t)job.y * N;
     const uint32_t rank = cg::this_cluster().block_rank();
     BcJob bc{};
-    if (SRC == 3) bc = a.bc[jobi];
-    const uint64_t *src = a.src + src_slot(a, SRC == 3 ? bc.in_slot0 : SRC ? job.x / a.src_div : job.x) * N;
+    if (SRC & SRC_CONV) bc = a.bc[jobi];
+    const uint64_t *src = a.src + src_slot(a, SRC & SRC_CONV ? bc.in_slot0 : job.x) * N, *rem = src_rem<SRC>(a, job, N);
     whole_fwd_tile<A, Cfg::LOG_A, Cfg::RA1, Cfg::RA2, LOG_CC, true, Cfg::THREADS, B0>(
         ex, tw, 1u, k,
         [&](int c, int e, int step, auto &x) {
-            load_src<A, SRC>(x, a, bc, src, N, (size_t)e * N2 + rank * CC + c, (size_t)step * N2, md, k);
+            load_src<A, SRC>(x, a, bc, src, rem, N, (size_t)e * N2 + rank * CC + c, (size_t)step * N2, md, k);
         },
         [&](int c, int e0, auto &x) {
 #pragma unroll

@@ -666,3 +666,37 @@ def test_pair_conversion_edges(log_n, special, l):
     for i, s in enumerate(sets):
         assert np.array_equal(got[i], o.keyswitch(l, s[2], key, s[:2])), f"set {i}"
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("log_n,bits,special,l,batch", [
+    (12, [60, 40, 40, 30, 60], 1, 4, 1),                          # whole transforms; a short prime goes
+    (12, [60, 40, 50, 36, 60, 60, 60], 2, 4, 40),                 # more limbs than whole transforms take
+    (13, [60, 40, 40, 60, 60, 60], 2, 4, 1),                      # a 60-bit prime goes; converted in the column pass
+    (13, [60, 40, 46, 36, 50] + [60] * 5, 5, 5, 3),
+    (14, [60, 40, 36, 45, 40, 50] + [60] * 4, 4, 6, 1),           # converted on the tensor cores
+    (14, [60, 40, 36, 45, 40, 50] + [60] * 4, 4, 2, 2),           # one limb is left
+    (16, [60, 40, 36, 45, 40] + [60] * 3, 3, 5, 1),
+    (16, [60, 40, 36, 45, 40] + [60] * 4, 4, 5, 2),
+])
+def test_moddown_and_rescale_in_one_equal_the_oracle(log_n, bits, special, l, batch):
+    """products relinearised and rescaled by floor (b2_multiply_relin_rescale_batch) and to nearest (.._many), single and batched"""
+    from pyPhantom._native import LIB, check
+    from gpu_helpers import key_dev, stream
+    ctx, o = make_ctx(1 << log_n, bits, special)
+    key = o.synth_key(o.beta(l), 6, 10)
+    a, b = [o.synth_ct(l, 6, 20 + i) for i in range(batch)], [o.synth_ct(l, 6, 120 + i) for i in range(batch)]
+    da, db = dev(np.stack(a)), dev(np.stack(b))
+    got = host(ph.multiply_relin_rescale_batch(ctx, da, db, _key(ctx, key)))
+    kt, kp = key_dev(key)
+    nb = LIB.b2_multiply_relin_batch_workspace_bytes(ctx._h, l, batch)
+    ws, out = torch.empty(nb // 8, dtype=torch.int64, device="cuda"), ctx.empty(batch, 2, l - 1)
+    pa, pb = (np.array([t.data_ptr()], dtype=np.uint64) for t in (da, db))
+    ll = np.array([l], dtype=np.uint32)
+    check(LIB.b2_multiply_relin_rescale_many(ctx._h, l, 1, batch, pa.ctypes.data, ll.ctypes.data, pb.ctypes.data, ll.ctypes.data, 0, kp.ctypes.data, len(kp),
+                                             out.data_ptr(), ws.data_ptr(), nb, stream()))
+    near = host(out)
+    for i in range(min(batch, 3)):
+        prod = o.multiply_and_relin(l, a[i], b[i], key)
+        assert np.array_equal(got[i], o.rescale(l, prod)), f"floor, pair {i}"
+        assert np.array_equal(near[i], o.rescale_rounded(l, prod)), f"nearest, pair {i}"
+    assert ctx.device_status() == 0
