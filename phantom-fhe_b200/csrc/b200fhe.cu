@@ -861,7 +861,7 @@ static void launch_fwd(const b2_ctx *c, const NttArgs &a, uint32_t njobs, const 
     {
         const dim3 grid(njobs * (N >> (LOG_A + A::LOG_CC)), batch);
         LaunchScope ls(c, s, "ntt_fwd_cols");
-        launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC>, grid, pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
+        launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC, LOG_B>, grid, pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
     }
     NttArgs b = a;
     b.src = a.dst;  // second pass works in place on the first pass's output
@@ -876,7 +876,7 @@ template <int LOG_A, int SRC>
 static void launch_fwd_cols_n(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
     using A = PassCfg<LOG_A>;
     LaunchScope ls(c, s, "ntt_fwd_cols");
-    launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC>, dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
+    launch_k(ntt_fwd_pass<LOG_A, A::R_STRIDED, A::R_CONTIG, A::LOG_CC, true, false, EpiStore, SRC, 8>, dim3(njobs * ((1u << a.logN) >> (LOG_A + A::LOG_CC)), batch), pass_threads<LOG_A, true>(), 0, s, a, EpiStore{});
 }
 template <int SRC>
 static void launch_fwd_cols(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaStream_t s, uint32_t batch) {
@@ -899,7 +899,7 @@ static void launch_inv(const b2_ctx *c, const NttArgs &a, uint32_t njobs, cudaSt
     b.src_lm1 = a.dst_lm1, b.src_bs = a.dst_bs;
     const dim3 grid(njobs * (N >> (LOG_A + A::LOG_CC)), batch);
     LaunchScope ls(c, s, "ntt_inv_cols");
-    launch_k(ntt_inv_pass<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_CC, true, true>, grid, pass_threads<LOG_A, true>(), 0, s, b);
+    launch_k(ntt_inv_pass<LOG_A, A::R_CONTIG, A::R_STRIDED, A::LOG_CC, true, true, LOG_B>, grid, pass_threads<LOG_A, true>(), 0, s, b);
 }
 
 // A batched launch: `batch` polynomial sets, slot s of set b at s * (lm1 + 1) + b * bs of the source / destination
