@@ -128,7 +128,7 @@ __device__ __forceinline__ void ld_pairs(W2 (&w)[CNT], const W2 *p) {
 }
 
 // ---- epilogues of the last forward (row) pass ---------------------------------------------------
-// The row pass leaves every thread with E consecutive canonical residues starting at limb offset o.
+// The row pass leaves every thread with E canonical residues in runs of four, `step` apart, the first at limb offset o.
 // An epilogue first preloads whatever else it needs for those positions (before the butterflies, so
 // the loads are in flight while the ALUs work) and then finishes and stores them.
 __host__ __device__ inline bool aligned32(const void *p) { return ((uintptr_t)p & 31) == 0; }
@@ -138,10 +138,10 @@ struct EpiStore {
     bool aligned() const { return true; }  // dst is the transform's own output, checked by the launcher
     template <int E> struct Regs {};
     __device__ __forceinline__ void init(const NttArgs &a, const Job &job, size_t N) { dst = a.dst + dst_slot(a, job.x) * N; }
-    template <int E> __device__ __forceinline__ void preload(Regs<E> &, size_t) const {}
-    template <int E> __device__ __forceinline__ void finish(const Regs<E> &, size_t o, uint64_t (&x)[E], uint64_t) const {
+    template <int E> __device__ __forceinline__ void preload(Regs<E> &, size_t, int) const {}
+    template <int E> __device__ __forceinline__ void finish(const Regs<E> &, size_t o, int step, uint64_t (&x)[E], uint64_t) const {
 #pragma unroll
-        for (int i = 0; i < E; i += 4) st256(dst + o + i, x[i], x[i + 1], x[i + 2], x[i + 3]);
+        for (int i = 0; i < E / 4; i++) st256(dst + o + i * step, x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
     }
 };
 
@@ -167,14 +167,14 @@ struct EpiSubMul {
         o_ = out + ((size_t)job.w + (size_t)set_idx(a) * o_bs) * N;
         kk = k[job.y];
     }
-    template <int E> __device__ __forceinline__ void preload(Regs<E> &r, size_t o) const {
+    template <int E> __device__ __forceinline__ void preload(Regs<E> &r, size_t o, int step) const {
 #pragma unroll
         for (int i = 0; i < E / 4; i++) {
-            r.m[i] = ld256(m_ + o + 4 * i);
-            if (ACCUM) r.acc[i] = ld256(o_ + o + 4 * i);
+            r.m[i] = ld256(m_ + o + i * step);
+            if (ACCUM) r.acc[i] = ld256(o_ + o + i * step);
         }
     }
-    template <int E> __device__ __forceinline__ void finish(const Regs<E> &r, size_t o, uint64_t (&x)[E], uint64_t q) const {
+    template <int E> __device__ __forceinline__ void finish(const Regs<E> &r, size_t o, int step, uint64_t (&x)[E], uint64_t q) const {
 #pragma unroll
         for (int i = 0; i < E / 4; i++) {
             uint64_t r0 = mul_shoup(sub_mod(r.m[i].a, x[4 * i], q), kk, q);
@@ -187,7 +187,7 @@ struct EpiSubMul {
                 r2 = add_mod(r.acc[i].c, r2, q);
                 r3 = add_mod(r.acc[i].d, r3, q);
             }
-            st256(o_ + o + 4 * i, r0, r1, r2, r3);
+            st256(o_ + o + i * step, r0, r1, r2, r3);
         }
     }
 };
@@ -203,14 +203,14 @@ struct EpiSubFrom {
         u64x4 u[E / 4];
     };
     __device__ __forceinline__ void init(const NttArgs &a, const Job &job, size_t N) { o_ = out + ((size_t)job.w + (size_t)set_idx(a) * bs) * N; }
-    template <int E> __device__ __forceinline__ void preload(Regs<E> &r, size_t o) const {
+    template <int E> __device__ __forceinline__ void preload(Regs<E> &r, size_t o, int step) const {
 #pragma unroll
-        for (int i = 0; i < E / 4; i++) r.u[i] = ld256(o_ + o + 4 * i);
+        for (int i = 0; i < E / 4; i++) r.u[i] = ld256(o_ + o + i * step);
     }
-    template <int E> __device__ __forceinline__ void finish(const Regs<E> &r, size_t o, uint64_t (&x)[E], uint64_t q) const {
+    template <int E> __device__ __forceinline__ void finish(const Regs<E> &r, size_t o, int step, uint64_t (&x)[E], uint64_t q) const {
 #pragma unroll
         for (int i = 0; i < E / 4; i++)
-            st256(o_ + o + 4 * i, sub_mod(r.u[i].a, x[4 * i], q), sub_mod(r.u[i].b, x[4 * i + 1], q), sub_mod(r.u[i].c, x[4 * i + 2], q),
+            st256(o_ + o + i * step, sub_mod(r.u[i].a, x[4 * i], q), sub_mod(r.u[i].b, x[4 * i + 1], q), sub_mod(r.u[i].c, x[4 * i + 2], q),
                   sub_mod(r.u[i].d, x[4 * i + 3], q));
     }
 };
@@ -699,8 +699,14 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
         const int ehi = COLS ? (gid / C) : (gid % E1);
         const uint32_t P = COLS ? 1u : (n1 + tile * C + c);
         const size_t o = base + (size_t)c * cstride + (size_t)ehi * E2 * estride;
+        // What the last pass stores goes through the exchange buffer once more: a thread holds a run of E2 residues, but its accesses
+        // are to every E1-th run of four, so that those of a warp cover whole lines one after another. With the runs accessed as
+        // they are every lane of a 256-bit access falls into a line of its own, and the row pass that subtracts from the ciphertext
+        // stood at 84 % of the L1 (sixteen key switches of 24 limbs at 2^16: 15.1 -> 12.6 us a key switch; eight hoisted rotations at
+        // 2^15 219.7 -> 212.6 us in all).
+        const size_t o4 = base + (size_t)c * cstride + (size_t)ehi * 4;
         typename Epi::template Regs<E2> regs;
-        if (LAST) e.template preload<E2>(regs, o);
+        if (LAST) e.template preload<E2>(regs, o4, 4 * E1);
         T x[E2];
 #pragma unroll
         for (int i = 0; i < E2; i++) {
@@ -710,10 +716,14 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
         ct_stages<A, 0, R2, E2, B1>(x, tw, P, R1, ehi, k);
         if (LAST) {
             static_assert(!LAST || !COLS, "the last forward pass is the row pass");
+            static_assert(!LAST || (32 % E1 == 0 && EPT == E2), "the threads of a sub-transform are lanes of one warp");
             uint64_t y[E2];
 #pragma unroll
-            for (int i = 0; i < E2; i++) y[i] = A::canon_fwd(x[i], k);
-            e.template finish<E2>(regs, o, y, md.q);
+            for (int i = 0; i < E2; i++) sm[c * TPAD + pad_idx<LOG_T, R2>(ehi * E2 + i)] = A::canon_fwd(x[i], k);  // where this thread alone read
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < E2; i++) y[i] = sm[c * TPAD + pad_idx<LOG_T, R2>((i / 4 * E1 + ehi) * 4 + i % 4)];
+            e.template finish<E2>(regs, o4, 4 * E1, y, md.q);
         } else {
 #pragma unroll
             for (int i = 0; i < E2; i++) dst[o + (size_t)i * estride] = A::to_raw(x[i]);

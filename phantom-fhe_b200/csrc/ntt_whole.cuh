@@ -131,11 +131,11 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const Epi &epi,
             constexpr int E = (int)(sizeof(x) / 8);
             const size_t o = (size_t)(row0 + c) * N2 + e0;
             typename Epi::template Regs<E> regs;
-            e.template preload<E>(regs, o);
+            e.template preload<E>(regs, o, 4);
             uint64_t y[E];
 #pragma unroll
             for (int i = 0; i < E; i++) y[i] = A::canon_fwd(x[i], k);
-            e.template finish<E>(regs, o, y, md.q);
+            e.template finish<E>(regs, o, 4, y, md.q);
         });
     cg::this_cluster().sync();  // nobody leaves while a peer may still read its slab
 }
