@@ -224,8 +224,21 @@ struct EpiSubFromTab : EpiSubFrom {
             if (!aligned32(p)) return false;
         return true;
     }
-    __device__ __forceinline__ void init(const NttArgs &a, const Job &job, size_t N) { o_ = tab[set_idx(a)] + (size_t)job.w * N; }
 };
+
+// the epilogue of the job at hand; one with a table becomes the one without (the table stays in the kernel's parameters: indexed in a
+// copy, every thread wrote it to local memory)
+template <class Epi>
+__device__ __forceinline__ Epi live_epi(const Epi &epi, const NttArgs &a, const Job &job, size_t N) {
+    Epi e = epi;
+    e.init(a, job, N);
+    return e;
+}
+__device__ __forceinline__ EpiSubFrom live_epi(const EpiSubFromTab &epi, const NttArgs &a, const Job &job, size_t N) {
+    EpiSubFrom e{};
+    e.o_ = epi.tab[set_idx(a)] + (size_t)job.w * N;
+    return e;
+}
 
 template <int LOG_T, int RC>
 __device__ __forceinline__ int pad_idx(int e) { return e + (e >> RC); }
@@ -689,8 +702,10 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
     }
     __syncthreads();
     // ---- stage group 2 ---------------------------------------------------------------------------
-    Epi e = epi;
-    if (LAST) e.init(a, job, N);
+    const auto e = [&] {
+        if constexpr (LAST) return live_epi(epi, a, job, N);
+        else return epi;
+    }();
     uint64_t *dst = a.dst + dst_slot(a, job.x) * N;
 #pragma unroll
     for (int gi = 0; gi < EPT / E2; gi++) {
@@ -705,7 +720,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
         // stood at 84 % of the L1 (sixteen key switches of 24 limbs at 2^16: 15.1 -> 12.6 us a key switch; eight hoisted rotations at
         // 2^15 219.7 -> 212.6 us in all).
         const size_t o4 = base + (size_t)c * cstride + (size_t)ehi * 4;
-        typename Epi::template Regs<E2> regs;
+        typename std::remove_const_t<decltype(e)>::template Regs<E2> regs;
         if (LAST) e.template preload<E2>(regs, o4, 4 * E1);
         T x[E2];
 #pragma unroll
@@ -733,7 +748,7 @@ __device__ __forceinline__ void fwd_body(const NttArgs &a, const Epi &epi, uint6
 
 template <int LOG_T, int R1, int R2, int LOG_C, bool COLS, bool LAST, class Epi, int SRC = 0, int LOG_REST = -1>
 __global__ void __launch_bounds__((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2)), ntt_min_blocks((1 << (LOG_C + LOG_T)) / (1 << (R1 > R2 ? R1 : R2)), 1 << (R1 > R2 ? R1 : R2)))
-ntt_fwd_pass(NttArgs a, Epi epi) {
+ntt_fwd_pass(NttArgs a, const __grid_constant__ Epi epi) {
     pdl_enter();
     static_assert(R1 + R2 == LOG_T, "stage split");
     constexpr int TT = 1 << LOG_T, C = 1 << LOG_C;

@@ -114,8 +114,7 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const Epi &epi,
             for (int i = 0; i < (int)(sizeof(x) / 8); i++) slab[(e0 + i) * CC + c] = A::to_raw(x[i]);
         });
     cg::this_cluster().sync();
-    Epi e = epi;
-    e.init(a, job, N);
+    const auto e = live_epi(epi, a, job, N);
     const uint32_t row0 = rank << LOG_CR;
     whole_fwd_tile<A, Cfg::LOG_B, Cfg::RB1, Cfg::RB2, LOG_CR, false, Cfg::THREADS, A::B_PASS>(
         ex, tw, (uint32_t)(N >> Cfg::LOG_B) + row0, k,
@@ -130,7 +129,7 @@ __device__ __forceinline__ void whole_fwd_body(const NttArgs &a, const Epi &epi,
         [&](int c, int e0, auto &x) {
             constexpr int E = (int)(sizeof(x) / 8);
             const size_t o = (size_t)(row0 + c) * N2 + e0;
-            typename Epi::template Regs<E> regs;
+            typename std::remove_const_t<decltype(e)>::template Regs<E> regs;
             e.template preload<E>(regs, o, 4);
             uint64_t y[E];
 #pragma unroll
