@@ -1394,7 +1394,8 @@ static int run_inner_prod(const b2_ctx *c, IpArgs &a, const uint64_t *const *evk
         }
     if (a.nq + a.np == 0) return B2_OK;
     LaunchScope ls(c, s, "ks_inner_prod");
-    launch_k(ks_inner_prod_kernel, dim3((unsigned)(c->N / 256), a.nq + a.np, sets), 128, 0, s, a);
+    const bool few = a.beta <= 4 && (a.steps <= 1 || a.each);
+    launch_k(few ? ks_inner_prod_kernel<true> : ks_inner_prod_kernel<false>, dim3((unsigned)(c->N / 256), a.nq + a.np, sets), 128, 0, s, a);
     LAUNCH_CHECK("ks_inner_prod_kernel");
     return B2_OK;
 }

@@ -604,7 +604,8 @@ __device__ __forceinline__ ulonglong2 ld_pair(const uint64_t *p, uint32_t n, uin
     return permuted && (pn & 1u) ? make_ulonglong2(v.y, v.x) : v;
 }
 
-template <class S>
+// FEW: four terms at most in a sum, one step
+template <class S, bool FEW>
 __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n, uint32_t pp, const Mod &md) {
     constexpr int U = 2;
     const size_t N = (size_t)1 << a.logN;
@@ -615,7 +616,7 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
     for (int i = 0; i < 2; i++) S::zero(acc[i][0]), S::zero(acc[i][1]);
     const uint64_t *digits = a.digits + ((size_t)z * a.dig_bs + t) * N, *own = a.own ? a.own + ((size_t)z * a.own_bs + t) * N : nullptr;
     const uint32_t own_d = (own && t < a.l) ? t / (a.lP - a.l) : 0xFFFFFFFFu;
-    const uint32_t s0 = a.each ? z : 0, n_s = a.steps && !a.each ? a.steps : 1;
+    const uint32_t s0 = a.each ? z : 0, n_s = !FEW && a.steps && !a.each ? a.steps : 1;
     const bool hoist = a.steps != 0 && !a.apart;
     uint64_t g0 = 0, g1 = 0;  // permuted c0
     int pending = 0;
@@ -644,7 +645,7 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
                 const ulonglong2 c = ld_pair(a.c0 + ((size_t)z * a.c0_bs + (size_t)s * a.c0_ss + t) * N, n, pn, pm);
                 g0 = add_mod(g0, c.x, md.q), g1 = add_mod(g1, c.y, md.q);
             }
-            if (pending + U > S::FLUSH) {
+            if (!FEW && pending + U > S::FLUSH) {
 #pragma unroll
                 for (int i = 0; i < 2; i++) S::flush(acc[i][0], k), S::flush(acc[i][1], k);
                 pending = 0;
@@ -694,6 +695,11 @@ __device__ __forceinline__ void ip_body(const IpArgs &a, uint32_t t, uint32_t n,
     *reinterpret_cast<ulonglong2 *>(o1) = make_ulonglong2(r[2], r[3]);
 }
 
+// FEW (a digit per term, at most four, single rotations): FP64 products and one reduction cost less than pieces and their
+// recombination - 78 FP64 instructions a coefficient against 102 and 85 of the integer pipe at three digits. Kernels of their own:
+// in one, 132 bytes of spills at the 64 registers of eight CTAs an SM; apart 8 (few) and 92 (eight hoisted rotations at 2^15 209.0 ->
+// 204.0 us, a bootstrap at 2^16 22.81 -> 22.57 ms).
+template <bool FEW>
 __global__ void __launch_bounds__(128, 8) ks_inner_prod_kernel(const __grid_constant__ IpArgs a) {
     pdl_enter();
     // the limbs of the special primes (the longer arithmetic) first
@@ -701,14 +707,12 @@ __global__ void __launch_bounds__(128, 8) ks_inner_prod_kernel(const __grid_cons
     const uint32_t pp = t < a.l ? t : a.size_Q + (t - a.l);
     const uint32_t n = 2 * (blockIdx.x * 128 + threadIdx.x);
     const Mod md = a.mod[pp];
-    // few terms (a digit per term, single rotations): FP64 products and one reduction cost less than pieces and their
-    // recombination - 78 FP64 instructions a coefficient against 102 and 85 of the integer pipe at three digits
-    if (a.beta <= 4 && (a.steps <= 1 || a.each)) {
-        if (md.q < FP_LIMIT) ip_body<SumFp>(a, t, n, pp, md);
-        else if (md.q < INT_LAZY_LIMIT) ip_body<SumInt30Short>(a, t, n, pp, md);
-        else ip_body<SumInt>(a, t, n, pp, md);
+    if constexpr (FEW) {
+        if (md.q < FP_LIMIT) ip_body<SumFp, true>(a, t, n, pp, md);
+        else if (md.q < INT_LAZY_LIMIT) ip_body<SumInt30Short, true>(a, t, n, pp, md);
+        else ip_body<SumInt, true>(a, t, n, pp, md);
     } else {
-        with_sum(md.q, [&](auto s) { ip_body<decltype(s)>(a, t, n, pp, md); });
+        with_sum(md.q, [&](auto s) { ip_body<decltype(s), false>(a, t, n, pp, md); });
     }
 }
 
