@@ -1481,16 +1481,16 @@ struct KsBatch {
 // kernel. It saves the digits' write and read, more of them the more digits there are, but a lone digit is its own input and
 // nothing is saved; and its CTAs, three an SM and three times as long on the special primes, want several waves. B200, stored /
 // fused, us a batch (limbs, special primes; waves of the fused pass):
-//   1 digit   2^15 (8, 8) 16 sets 9.2 waves 462 / 475; 2^16 (8, 8) 8 sets 9.2 471 / 484, 16 sets 18 897 / 899
-//   2 digits  2^15 (16, 8) 4 sets 3.5 238 / 249, 8 sets 6.9 430 / 429, 16 sets 14 820 / 794; 2^16 (16, 8) 3 sets 5.2 342 / 349,
-//             6 sets 10 637 / 621; (8, 4) 16 sets 14 897 / 872
-//   3 digits  2^15 (12, 4) 2 sets 1.2 121 / 130, 6 sets 3.5 296 / 292; (6, 2) 8 sets 2.3 231 / 234, 16 sets 4.6 426 / 422;
-//             2^16 (24, 8) 2 sets 4.6 363 / 355, 16 sets 37 2560 / 2322
-//   4 to 6    2^15 (20, 5) 2 sets 1.8 188 / 185, 16 sets 14 1208 / 1105; (14, 3) 2 sets 1.2 166 / 171, 3 sets 1.8 224 / 215;
-//             (12, 2) 2 sets 1.0 161 / 174, 3 sets 1.5 217 / 210
+//   1 digit   2^15 (8, 8) 16 sets 9.2 waves 401 / 421
+//   2 digits  2^15 (16, 8) 4 sets 3.5 209 / 225, 8 sets 6.9 379 / 384, 16 sets 14 725 / 712; 2^16 (16, 8) 3 sets 5.2 303 / 315,
+//             6 sets 10 563 / 557; (8, 4) 16 sets 14 764 / 750
+//   3 digits  2^15 (12, 4) 2 sets 1.2 106 / 113, 6 sets 3.5 252 / 253; (6, 2) 8 sets 2.3 179 / 188, 16 sets 4.6 333 / 332;
+//             2^16 (24, 8) 2 sets 4.6 328 / 327, 16 sets 37 2256 / 2111
+//   4 to 6    2^15 (20, 5) 2 sets 1.8 166 / 165, 16 sets 14 1070 / 992; (14, 3) 2 sets 1.2 142 / 151, 3 sets 1.8 189 / 187;
+//             (12, 2) 2 sets 1.0 129 / 144, 3 sets 1.5 172 / 170
 static bool fused_rows_pay(const b2_ctx *c, size_t l, size_t beta, size_t sets) {
     using Cfg = PassCfg<8>;
-    const size_t ctas = sets * (l + c->size_P) * (c->N >> (8 + Cfg::LOG_C)), half_waves = beta >= 4 ? 3 : beta == 3 ? 6 : 14;
+    const size_t ctas = sets * (l + c->size_P) * (c->N >> (8 + Cfg::LOG_C)), half_waves = beta >= 4 ? 3 : beta == 3 ? 9 : 14;
     return beta > 1 && 2 * ctas >= half_waves * 3 * (size_t)c->sm_count;
 }
 
