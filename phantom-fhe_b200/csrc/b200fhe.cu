@@ -248,8 +248,8 @@ struct b2_ctx {
     bool mac_interleave = false;   // B2_KS_FUSED_ORDER=1: consecutive CTAs of the fused pass walk limbs, not tiles (measured slower)
     // The fused pass may also take the limbs on primes of 50 bits and more (q0 and P at the usual parameters): 10 launches
     // instead of 12 and no stored digits at all. Batched calls do (1 % more per second at N = 2^16, l = 24), single calls do
-    // not: key switches per second over four streams / on one at those sizes 6398 / 4853 with the FP64 limbs on it, 5862 / 4841
-    // with all of them, 6088 / 4923 with none (the stand-alone inner product of the 60-bit limbs is memory-bound and hides
+    // not: key switches per second over four streams / on one at those sizes 6832 / 5242 with the FP64 limbs on it, 6132 / 5273
+    // with all of them, 6639 / 5409 with none (the stand-alone inner product of the 60-bit limbs is memory-bound and hides
     // behind other streams' transforms; fused, it is integer-multiply work). B2_KS_FUSED_WIDE = 0 | 1 says otherwise.
     int mac_wide = -1;
     bool use_mac = false;          // N = 2^15, 2^16: ModUp's last forward pass may carry the inner product (off with B2_KS_FUSED_IP=0)
