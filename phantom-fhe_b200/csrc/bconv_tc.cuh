@@ -11,16 +11,16 @@
 // A tiles, the part's B image when the part changes), warp 12 issues the MMAs of three column groups at a time into one of two
 // 96-column accumulators, warps 0 to 11 (TMEM lanes 32 (w % 4) .. +31, a group each) reduce and store the other. Groups a
 // buffer, ModUp and ModDown of sixteen key switches of 24 limbs and 8 special primes at 2^16, us a key switch: two 18.6, three
-// 17.1, four 17.8 (spills). Four warps' worth of epilogue an SM sub-partition is what hides a warp's chain of TMEM load,
-// reduction and store: with eight warps taking two groups each in turn, and the records read from global memory, 21.8.
+// 17.1, four 17.8 (spills). Six warps of the epilogue on an SM sub-partition hide a warp's chain of TMEM load, reduction and store:
+// with four, of two groups each in turn, and the records read from global memory, 21.8.
 // Two A tiles in flight: three or four are no faster, and their shared memory keeps the CTAs of other streams' kernels off the
 // SM, and this kernel's CTAs off an SM that those have not left (four streams of key switches 7420 a second with two, 6700
 // with four).
 // The form before (a coefficient a row, rows filled by cp.async of eight bytes, a barrier pair per tile of 128 coefficients)
 // took 73 warp instructions an output and 25.0 us; the bytes alone take 12.9 at the copy rate. A launch that gives a CTA one
-// tile takes 0.5 us longer than it did then: a bulk copy arrives a microsecond after its issue, where cp.async takes a third
-// of that, but the code that filled the first tile so cost more than it saved (the instructions of a kernel that runs for
-// three microseconds are fetched as they are executed).
+// tile takes 0.5 us longer than it did then: a bulk copy arrives a microsecond after its issue. The first tile filled by all
+// threads was slower still (rotations at 2^14, 16 limbs, alpha 8 60.8 -> 64.2 us): the instructions of a kernel that runs for
+// three microseconds are fetched as they are executed.
 // No multicast, no cluster; every wait is bounded and reports through a status word instead of spinning forever; copies and
 // MMAs in flight are waited for and TMEM is released on every path.
 #pragma once
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_con
                     if (n_t >= TC_BUFS && !(ok = tc_wait(empty_t + 8 * buf, (n_t / TC_BUFS - 1) & 1, gave_up))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bdesc = tc_desc(sB + c0 * 16, cols * 16);
-                    // D s32, A and B u8, both K-major, M = 128, N = the columns of up to four groups
+                    // D s32, A and B u8, both K-major, M = 128, N = the columns of up to TC_CHUNK groups
                     const uint32_t idesc = (2u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
                     for (uint32_t s = 0; s < steps; s++)  // 32 bytes of K: two input limbs
                         tc_mma_i8(tmem + buf * TC_ACC_COLS, adesc + s * (2 * TC_SLICE >> 4), bdesc + s * (2 * cols * 16 >> 4), idesc, s != 0);

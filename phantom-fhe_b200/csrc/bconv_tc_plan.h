@@ -52,7 +52,7 @@ struct TcJob {
     uint32_t n_groups;         // column groups (<= 16)
     uint32_t img_off;          // byte offset of the B image (n_groups * 1024 bytes)
     uint32_t grp_off;          // first TcGroup of the job
-    uint32_t alloc_cols;       // TMEM columns to allocate: power of two >= max(32, 16 n_groups)
+    uint32_t alloc_cols;       // TMEM columns of the compact form: power of two >= max(32, 16 n_groups)
     uint32_t in_stride1;       // input limb i sits at slot in_slot0 + i * (in_stride1 + 1)
 };
 static_assert(sizeof(TcOut) == 16 && sizeof(TcGroup) == 80 && sizeof(TcJob) == 32, "device layouts");
@@ -123,7 +123,7 @@ struct TcBuild {
     std::vector<TcGroup> groups;
     std::vector<uint8_t> images;
     bool ok = true;
-    uint32_t max_groups = 16;  // column groups per job: 16 -> up to 256 TMEM columns (two CTAs per SM), 8 -> 128 (four)
+    uint32_t max_groups = 16;  // column groups per job
     // One conversion (a digit, a polynomial): outputs are packed, in order, into 16-column groups of equal byte count;
     // more than max_groups groups are dealt evenly over further jobs on the same inputs. Returns the number of jobs added.
     uint32_t add(uint32_t in_slot0, uint32_t ni, uint32_t copy_dst, const std::vector<TcSpecOut> &outs, uint32_t in_stride = 1) {
