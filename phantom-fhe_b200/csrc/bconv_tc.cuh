@@ -22,7 +22,7 @@
 // threads was slower still (rotations at 2^14, 16 limbs, alpha 8 60.8 -> 64.2 us): the instructions of a kernel that runs for
 // three microseconds are fetched as they are executed.
 // No multicast, no cluster; every wait is bounded and reports through a status word instead of spinning forever; copies and
-// MMAs in flight are waited for and TMEM is released on every path.
+// MMAs in flight are waited for, with a limit of their own when another wait has run out, and TMEM is released on every path.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -39,7 +39,6 @@ constexpr uint32_t TC_CHUNK = 3;                    // column groups of one accu
 constexpr uint32_t TC_ACC_COLS = 32 * TC_CHUNK, TC_TMEM_COLS = 256, TC_BUFS = TC_TMEM_COLS / TC_ACC_COLS;
 constexpr uint32_t TC_EPI_WARPS = 4 * TC_CHUNK, TC_THREADS = 32 * (TC_EPI_WARPS + 2);
 constexpr uint32_t TC_CTRL_BYTES = 256;             // barriers and the like
-constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;        // polls of a barrier before giving up
 constexpr uint32_t TC_SM_SMEM = 233472;             // shared memory of one SM (228 KB)
 constexpr uint32_t TC_SMEM_MAX_REQUEST = TC_SM_SMEM / 2 - 1024;  // two CTAs an SM, a kilobyte each for the system
 
@@ -76,24 +75,24 @@ __device__ __forceinline__ void tc_bulk(uint32_t smem_dst, const void *gsrc, uin
     asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst), "l"(gsrc), "r"(bytes), "r"(bar)
                  : "memory");
 }
-// waits for the phase of the given parity to end, at most TC_WAIT_LIMIT polls and not after another wait of the CTA gave up
+// waits for the phase of the given parity to end (tc_poll has the limits)
+template <bool DRAIN = false>
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile uint32_t *gave_up) {
-    for (uint32_t it = 0; it < TC_WAIT_LIMIT; it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t"
-            ".reg .pred P1;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P1;\n\t"
-            "}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (*gave_up) return false;
-    }
-    *gave_up = 1u;
-    return false;
+    return tc_poll(
+        [&] {
+            uint32_t done;
+            asm volatile(
+                "{\n\t"
+                ".reg .pred P1;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+                "selp.b32 %0, 1, 0, P1;\n\t"
+                "}\n"
+                : "=r"(done)
+                : "r"(bar), "r"(parity)
+                : "memory");
+            return done != 0;
+        },
+        gave_up, DRAIN);
 }
 
 // 32 consecutive accumulator columns of this thread's TMEM lane, and the wait as a statement that owns the registers: a
@@ -275,8 +274,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_con
         for (uint32_t v = v0 + 1; v < v1; v++, k++)
             if (!load_item(v, k)) break;
         // nothing may be in flight when the CTA ends
-        for (uint32_t i = k > TC_STAGES ? k - TC_STAGES : 0; i < k; i++) tc_wait(full_a + 8 * (i % TC_STAGES), (i / TC_STAGES) & 1, gave_up);
-        tc_wait(full_b, (n_b - 1) & 1, gave_up);
+        for (uint32_t i = k > TC_STAGES ? k - TC_STAGES : 0; i < k; i++) tc_wait<true>(full_a + 8 * (i % TC_STAGES), (i / TC_STAGES) & 1, gave_up);
+        tc_wait<true>(full_b, (n_b - 1) & 1, gave_up);
     } else if (warp == TC_EPI_WARPS) {
         // ---- MMAs -------------------------------------------------------------------------------------------------
         if (lane == 0) {
@@ -308,7 +307,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_con
                 tc_commit(empty_a + 8 * st);
             }
             tc_commit(drained);
-            tc_wait(drained, 0, gave_up);
+            tc_wait<true>(drained, 0, gave_up);
         }
     } else {
         // ---- reduction and stores -----------------------------------------------------------------------------------

@@ -110,6 +110,21 @@ B2_HD uint64_t tc_reduce_dev(const uint32_t *c, uint32_t p_lo, uint32_t p_hi, ui
     return (int64_t)t < 0 ? r : t;
 }
 
+// How long a warp polls a barrier: until its phase has ended, TC_WAIT_LIMIT polls at most, and ONE poll once another wait of the
+// CTA has run out, so that the CTA ends soon. `drain`: the waits before the CTA ends for what it has in flight itself. Whether
+// another wait gave up says nothing about them, and the hardware still writes to shared and tensor memory until they are over:
+// they take their own limit.
+constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;
+template <class Poll>
+B2_HD bool tc_poll(Poll &&poll, volatile uint32_t *gave_up, bool drain) {
+    for (uint32_t it = 0; it < TC_WAIT_LIMIT; it++) {
+        if (poll()) return true;
+        if (!drain && *gave_up) return false;
+    }
+    *gave_up = 1u;
+    return false;
+}
+
 struct TcSpecOut {
     uint32_t slot;        // absolute output limb
     uint64_t p;           // its prime
