@@ -940,6 +940,7 @@ static bool convert_loading(const b2_ctx *c, size_t limbs) {
 }
 template <class Epi, int SRC> struct WholeHas : std::false_type {};
 template <> struct WholeHas<EpiStore, 0> : std::true_type {};
+template <> struct WholeHas<EpiStore, SRC_WORDS> : std::true_type {};
 template <> struct WholeHas<EpiSubMul<false>, SRC_REM> : std::true_type {};
 template <> struct WholeHas<EpiSubMul<false>, SRC_REM | SRC_NEAR> : std::true_type {};
 
@@ -952,7 +953,8 @@ struct RemSrc {
     void put(NttArgs &a) const { a.rem = rem, a.rem_div = div, a.rem_bs = bs, a.rem_q = q, a.rem_half = rounded ? q >> 1 : ~0ull; }
 };
 
-template <class Epi, int SRC = 0>
+// SRC: SRC_WORDS behind a base conversion, 0 where the words are canonical
+template <int SRC = 0, class Epi>
 static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Job *jobs, uint32_t njobs, uint32_t first_prime,
                    const Epi &epi, cudaStream_t s, uint32_t period = 0, const BatchDims &bd = BatchDims{}, const RemSrc &rem = RemSrc{}) {
     if (njobs == 0) return B2_OK;
@@ -1354,7 +1356,7 @@ static int modup_impl(b2_ctx *c, size_t l, const uint64_t *c2, uint64_t *out, ui
     if (!copy_own && convert_loading(c, pl.n_up_ntt)) return run_bconv_fwd(c, t, out, pl.jobs_up_ntt, pl.bc_up, pl.matw_up, pl.n_up_ntt, EpiStore{}, s);
     rc = run_bconv(c, copy_own, t, out, c2, pl.grp_up, pl.beta, pl.outs_up, pl.mat_up, pl.matd_up, (uint32_t)c->size_P, (uint32_t)(l + c->size_P), true, s, &pl.tc_up);
     if (rc) return rc;
-    return run_fwd(c, out, out, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s);
+    return run_fwd<SRC_WORDS>(c, out, out, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s);
 }
 
 extern "C" int b2_modup(b2_ctx *c, size_t l, const uint64_t *d_c2, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
@@ -1434,10 +1436,10 @@ static int moddown_impl(b2_ctx *c, size_t l, size_t n_poly, uint64_t *cx, uint64
     if (rc) return rc;
     if (accum) {
         EpiSubMul<true> epi{cx, out, c->d_Pinv};
-        return run_fwd(c, delta, delta, pl.jobs_dn_ntt, (uint32_t)(n_poly * l), 0, epi, s);
+        return run_fwd<SRC_WORDS>(c, delta, delta, pl.jobs_dn_ntt, (uint32_t)(n_poly * l), 0, epi, s);
     }
     EpiSubMul<false> epi{cx, out, c->d_Pinv};
-    return run_fwd(c, delta, delta, pl.jobs_dn_ntt, (uint32_t)(n_poly * l), 0, epi, s);
+    return run_fwd<SRC_WORDS>(c, delta, delta, pl.jobs_dn_ntt, (uint32_t)(n_poly * l), 0, epi, s);
 }
 
 extern "C" int b2_moddown(b2_ctx *c, size_t l, size_t n_poly, uint64_t *d_cx, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
@@ -1460,7 +1462,7 @@ static int ks_moddown(b2_ctx *c, size_t l, uint64_t *cxP, uint64_t *delta, uint6
     if (convert_loading(c, 2 * l)) return run_bconv_fwd(c, cxP, delta, pl.jobs_dnf_ntt, pl.bc_dnf, c->d_matw_dn_pinv, (uint32_t)(2 * l), EpiSubFrom{ct}, s);
     rc = run_bconv(c, false, cxP, delta, nullptr, pl.grp_dnf, 2, pl.outs_dn, c->d_mat_dn_pinv, c->d_matd_dn_pinv, (uint32_t)a, (uint32_t)l, true, s, &pl.tc_dnf);
     if (rc) return rc;
-    return run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
+    return run_fwd<SRC_WORDS>(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{ct}, s);
 }
 
 // ModUp and inner product of the fused key switch. At N = 2^16 (batched calls: 2^15 too, and where fused_rows_pay says so) the
@@ -1526,7 +1528,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         if (rc) return rc;
         if (!mac) {
             // both passes stored for every limb, then the stand-alone inner product, each one launch over the batch
-            if (!loading) rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
+            if (!loading) rc = run_fwd<SRC_WORDS>(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
             const IpBatch ib{per, kb.c2_bs, kb.ct_bs, 1, (uint32_t)c->size_P, 0, a2};
             rc = inner_prod_impl(c, l, up, c2, evk, n_evk, cxP, ct, true, s, nullptr, acc_p, B, &ib, kb.rot);
@@ -1543,7 +1545,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
             b.src = t, b.src_bs = batched ? (uint32_t)l : 0, b.bc = pl.bc_up, b.mat = pl.matw_up;
             launch_fwd_cols<SRC_CONV>(c, b, pl.n_up_ntt, s, B);
         } else {
-            launch_fwd_cols<0>(c, a, pl.n_up_ntt, s, B);
+            launch_fwd_cols<SRC_WORDS>(c, a, pl.n_up_ntt, s, B);
         }
         LAUNCH_CHECK("ntt_fwd_pass");
         // the limbs on 60-bit primes (q0, P) either ride on the fused pass too (integer arithmetic) or, mac_wide off,
@@ -1659,7 +1661,7 @@ static int keyswitch_batch_impl(b2_ctx *c, size_t l, size_t batch, const uint64_
     const TcBatch tb{B, 0, (uint32_t)(2 * a), 0, per};
     rc = run_bconv_tc(c, false, cxP, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, tb);
     if (rc) return rc;
-    return run_fwd(c, up, up, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_ct, (uint32_t)ct_stride}, s, 0, BatchDims{B, 0, per, 0, per});
+    return run_fwd<SRC_WORDS>(c, up, up, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, EpiSubFrom{d_ct, (uint32_t)ct_stride}, s, 0, BatchDims{B, 0, per, 0, per});
 }
 
 extern "C" int b2_keyswitch_batch(b2_ctx *c, size_t l, size_t batch, const uint64_t *d_c2, size_t c2_stride, const uint64_t *const *evk, size_t n_evk,
@@ -1714,8 +1716,8 @@ static int rescale_tail(const b2_ctx *c, size_t l, size_t n_poly, const uint64_t
     EpiSubMul<false> epi{d_in, d_out, pl.qlast_inv};
     const uint32_t njobs = (uint32_t)(n_poly * (l - 1));
     const RemSrc rem{r, (uint32_t)(l - 1), 0, c->q[l - 1], rounded};
-    if (rounded) return run_fwd<EpiSubMul<false>, SRC_REM | SRC_NEAR>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, BatchDims{}, rem);
-    return run_fwd<EpiSubMul<false>, SRC_REM>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, BatchDims{}, rem);
+    if (rounded) return run_fwd<SRC_REM | SRC_NEAR>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, BatchDims{}, rem);
+    return run_fwd<SRC_REM>(c, r, d_out, pl.jobs_rs_ntt, njobs, 0, epi, s, 0, BatchDims{}, rem);
 }
 
 extern "C" int b2_rescale(b2_ctx *c, size_t l, size_t n_poly, const uint64_t *d_in, uint64_t *d_out, void *d_ws, size_t ws_bytes, void *stream) {
@@ -1765,8 +1767,8 @@ static int rescale_sets(const b2_ctx *c, size_t l, uint32_t sets, const uint64_t
     epi.m_bs = in_bs, epi.o_bs = out_bs;
     const BatchDims bd{sets, 0, 2, 0, out_bs};
     const RemSrc rem{r, (uint32_t)(l - 1), 2, c->q[l - 1], rounded};
-    if (rounded) return run_fwd<EpiSubMul<false>, SRC_REM | SRC_NEAR>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, bd, rem);
-    return run_fwd<EpiSubMul<false>, SRC_REM>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, bd, rem);
+    if (rounded) return run_fwd<SRC_REM | SRC_NEAR>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, bd, rem);
+    return run_fwd<SRC_REM>(c, r, d_out, pl.jobs_rs_ntt, (uint32_t)(2 * (l - 1)), 0, epi, s, 0, bd, rem);
 }
 
 // ModDown and rescale in one, for `sets` blocks of `bs` limbs each, [2][l] ciphertext | [2][alpha] P limbs | [2] scratch: the inner
@@ -1799,7 +1801,7 @@ static int moddown_rescale(const b2_ctx *c, size_t l, uint32_t sets, uint64_t *b
                                                                    BatchDims{sets, 0, bs, 0, up_bs}, rem);
     rc = run_bconv_tc(c, false, P, up, nullptr, pl.tc_dnf, pl.tc_dnf.n_jobs, s, TcBatch{sets, 0, bs, 0, up_bs});
     if (rc) return rc;
-    return run_fwd<EpiSubMul<false>, SRC_WORDS | SRC_REM>(c, up, up, pl.jobs_drs_ntt, njobs, 0, epi, s, 0, BatchDims{sets, 0, up_bs, 0, up_bs}, rem);
+    return run_fwd<SRC_WORDS | SRC_REM>(c, up, up, pl.jobs_drs_ntt, njobs, 0, epi, s, 0, BatchDims{sets, 0, up_bs, 0, up_bs}, rem);
 }
 
 // Key switch of `sets` products and the rescale behind it. Block layout and `up` as above, a block's last l limbs the third
@@ -2147,7 +2149,7 @@ extern "C" int b2_rotate_sum(b2_ctx *c, size_t l, size_t n, const uint32_t *elts
                     if (rc) return rc;
                 }
             }
-            rc = run_fwd(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
+            rc = run_fwd<SRC_WORDS>(c, up, up, pl.jobs_up_ntt, pl.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
             if (rc) return rc;
         }
         IpArgs ia = ip_args(c, l, up, c1, accP, d_acc);
@@ -2271,7 +2273,7 @@ extern "C" int b2_hoist_rotations(b2_ctx *c, size_t l, const uint64_t *d_ct, con
                 if (rc) return rc;
             }
         }
-        rc = run_fwd(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, epi, s, 0, BatchDims{n, 0, (uint32_t)(2 * l), 0, (uint32_t)(2 * l)});
+        rc = run_fwd<SRC_WORDS>(c, delta, delta, pl.jobs_dnf_ntt, (uint32_t)(2 * l), 0, epi, s, 0, BatchDims{n, 0, (uint32_t)(2 * l), 0, (uint32_t)(2 * l)});
         if (rc) return rc;
     }
     return B2_OK;
@@ -2865,7 +2867,7 @@ extern "C" int b2_shard_keyswitch_phase(b2_ctx *c, size_t l, int phase, const ui
         case 1: {
             rc = run_bconv(c, false, t, up, d_c2, sp.grp_up, (uint32_t)beta, sp.outs_up, sp.mat_up, sp.matd_up, (uint32_t)a, (uint32_t)lP, true, s, &sp.tc_up);
             if (rc) return rc;
-            rc = run_fwd(c, up, up, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s);
+            rc = run_fwd<SRC_WORDS>(c, up, up, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s);
             if (rc) return rc;
             const uint4 rg = make_uint4(sp.q0, sp.nq, sp.p0, sp.np);
             rc = inner_prod_impl(c, l, up, d_c2, evk, n_evk, cxP, d_ct, true, s, &rg);
@@ -2876,7 +2878,7 @@ extern "C" int b2_shard_keyswitch_phase(b2_ctx *c, size_t l, int phase, const ui
             if (sp.nq == 0) return B2_OK;
             rc = run_bconv(c, false, cxP, up, nullptr, sp.grp_dn, 2, sp.outs_dn, sp.mat_dn, sp.matd_dn, (uint32_t)a, (uint32_t)l, true, s, &sp.tc_dn);
             if (rc) return rc;
-            return run_fwd(c, up, up, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct}, s);
+            return run_fwd<SRC_WORDS>(c, up, up, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct}, s);
         default:
             return fail(B2_EINVAL, "shard_keyswitch_phase: phase must be 0, 1 or 2");
     }
@@ -2975,7 +2977,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 NttArgs na{UP, UP, sp.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
                 na.src_bs = na.dst_bs = per;
                 if (sp.n_up_ntt) {
-                    launch_fwd_cols<0>(c, na, sp.n_up_ntt, s, B);
+                    launch_fwd_cols<SRC_WORDS>(c, na, sp.n_up_ntt, s, B);
                     LAUNCH_CHECK("ntt_fwd_pass");
                 }
                 MacArgs m{};
@@ -2994,7 +2996,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 launch_k(ntt_fwd_rows_mac<8, Cfg::R_CONTIG, Cfg::LOG_C>, dim3(B, (sp.nq + sp.np) * (uint32_t)(N >> (8 + Cfg::LOG_C))), pass_threads<8>(), mac_smem_bytes<8, Cfg::R_CONTIG, Cfg::LOG_C>(), s, na, m);
                 LAUNCH_CHECK("ntt_fwd_rows_mac");
             } else {
-                rc = run_fwd(c, UP, UP, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
+                rc = run_fwd<SRC_WORDS>(c, UP, UP, sp.jobs_up_ntt, sp.n_up_ntt, 0, EpiStore{}, s, 0, BatchDims{B, 0, per, 0, per});
                 if (rc) return rc;
                 const uint4 rg = make_uint4(sp.q0, sp.nq, sp.p0, sp.np);
                 const IpBatch ib{per, (uint32_t)l, (uint32_t)(2 * l), 2, 1, B - 1, 1};
@@ -3008,7 +3010,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
             const TcBatch tb{B, B - 1, 1, 0, per};
             rc = run_bconv_tc(c, false, CXP, UP, nullptr, sp.tc_dn_b, sp.tc_dn_b.n_jobs, s, tb);
             if (rc) return rc;
-            return run_fwd(c, UP, UP, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct, (uint32_t)(2 * l)}, s, 0, BatchDims{B, 0, per, 0, per});
+            return run_fwd<SRC_WORDS>(c, UP, UP, sp.jobs_dn_ntt, 2 * sp.nq, 0, EpiSubFrom{d_ct, (uint32_t)(2 * l)}, s, 0, BatchDims{B, 0, per, 0, per});
         }
         default:
             return fail(B2_EINVAL, "shard_keyswitch_phase_batch: phase must be 0, 1 or 2");

@@ -118,7 +118,7 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t (&c)[32]) {
 
 // One residue below 2 p from its planes: paired with shift-adds, joined by one (7 and 8 planes: two) wide multiply-adds, the
 // quotient estimate one high multiply, v + qhat (2^64 - p) one wide multiply-add and one narrow one. tc_reduce
-// (bconv_tc_plan.h) without its last subtraction, which the forward transform that follows does not need (B_IN).
+// (bconv_tc_plan.h) without its last subtraction, which the forward transform that follows does not need (B_WORDS).
 // r: {2^64 - p as two words, mu, slot}
 template <int NB>
 __device__ __forceinline__ uint2 tc_residue(const uint32_t *c, const uint4 r) {

@@ -71,9 +71,9 @@ struct NttArgs {
     uint32_t rem_div, rem_bs;
     uint64_t rem_q, rem_half;
 };
-// What a forward transform reads: the words as they are (0, or with a remainder SRC_WORDS | SRC_REM), the base conversion of other
-// limbs (SRC_CONV), the remainder that a rescale subtracts (SRC_REM: floor, SRC_REM | SRC_NEAR: nearest), or the sum of a remainder
-// (either) and one of the others
+// What a forward transform reads: canonical words (0), words below 2 q as the base conversion leaves them (SRC_WORDS), the base
+// conversion of other limbs (SRC_CONV), the remainder that a rescale subtracts (SRC_REM: floor, SRC_REM | SRC_NEAR: nearest), or the
+// sum of a remainder (either) and one of the last two before it
 enum { SRC_REM = 1, SRC_CONV = 2, SRC_WORDS = 4, SRC_NEAR = 8 };
 
 // The sets of a batched launch are the slow grid dimension. With the sets fastest (the CTAs of all sets on one tile next to
@@ -262,8 +262,8 @@ __device__ __forceinline__ int pad_idx(int e) { return e + (e >> RC); }
 //   gs_sum / gs_prod   bounds of the two outputs of an inverse butterfly; gs(.., ba, bb) is that butterfly
 //   group_end          what is done to a residue that changes thread between two stage groups of a pass
 //   pass_end           what is done to a residue that is stored between the passes of an inverse transform
-//   B_CANON / B_IN / B_PASS / GS_PASS   bounds of canonical input, of a forward transform's input (canonical, or below 2 q as the
-//                       tensor-core conversion leaves it), of what a forward / an inverse pass stores
+//   B_CANON / B_WORDS / B_PASS / GS_PASS   bounds of canonical input, of words below 2 q as the tensor-core conversion leaves them,
+//                       of what a forward / an inverse pass stores
 constexpr uint64_t FP_SMALL_LIMIT = 1ull << 41;
 constexpr uint64_t FP_LIMIT = 1ull << 50;
 constexpr uint64_t INT_LAZY_LIMIT = 1ull << 60;
@@ -281,7 +281,7 @@ struct ArithIntLazy {
         uint64_t q, nq;   // nq = -q mod 2^64
         uint32_t m, s;    // floor(2^(64 + s) / q), normalised to 32 bits
     };
-    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_IN = 2, B_PASS = 16, GS_PASS = 6, B_BCONV = RED;
+    static constexpr int LIM = 16, RED = 2, PROD = 3, B_CANON = 1, B_WORDS = 2, B_PASS = 16, GS_PASS = 6, B_BCONV = RED;
     __device__ __forceinline__ static K make(const Mod &md, int) {
         const uint32_t s = __clz((uint32_t)md.r1);  // r1 = floor(2^64 / q), in [2^4, 2^14]
         return K{md.q, 0 - md.q, (uint32_t)((md.r1 << s) | (md.r0 >> (64 - s))), s};
@@ -352,7 +352,7 @@ struct ArithInt {
     struct K {
         uint64_t q, q2;
     };
-    static constexpr int B_CANON = 0, B_IN = 0, B_PASS = 0, GS_PASS = 0, B_BCONV = 0;
+    static constexpr int B_CANON = 0, B_WORDS = 0, B_PASS = 0, GS_PASS = 0, B_BCONV = 0;
     __device__ __forceinline__ static K make(const Mod &md, int) { return K{md.q, 2 * md.q}; }
     using TwRaw = W2;
     static constexpr int TW_RUN = 2;  // twiddles in 32 bytes
@@ -397,7 +397,7 @@ struct ArithFp {
         double q, qinv;
     };
     static constexpr int FACTOR = 32, LIM = 128, RED = 9;
-    static constexpr int B_CANON = BIG ? 16 : 0, B_IN = 2 * B_CANON, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0, B_BCONV = BIG ? RED : 0;
+    static constexpr int B_CANON = BIG ? 16 : 0, B_WORDS = 2 * B_CANON, B_PASS = BIG ? LIM : 0, GS_PASS = BIG ? RED : 0, B_BCONV = BIG ? RED : 0;
     static constexpr bool IS_BIG = BIG;
     __host__ __device__ static constexpr int prod(int B) { return 9 + (B + 3) / 4; }
     // table entry i of an FP64 prime is one double (8 bytes); w / q is rebuilt as w * (1/q), whose
@@ -601,7 +601,7 @@ __device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a
                                          size_t step, const Mod &md, const typename A::K &k) {
     if constexpr (SRC & SRC_REM) {
         if constexpr (SRC & SRC_CONV) load_src<A, SRC_CONV>(x, a, bc, src, nullptr, N, n0, step, md, k);
-        else if constexpr (SRC & SRC_WORDS) load_src<A, 0>(x, a, bc, src, nullptr, N, n0, step, md, k);
+        else if constexpr (SRC & SRC_WORDS) load_src<A, SRC_WORDS>(x, a, bc, src, nullptr, N, n0, step, md, k);
         const uint64_t q_red = SRC == SRC_REM ? 0 : barrett64(a.rem_q, md.q, md.r1);
         uint64_t v[E];
 #pragma unroll
@@ -612,7 +612,7 @@ __device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a
             if (SRC != SRC_REM && v[i] > a.rem_half) r = sub_mod(r, q_red, md.q);
             x[i] = SRC & (SRC_CONV | SRC_WORDS) ? x[i] + A::from_u64(r, k) : A::from_u64(r, k);
         }
-    } else if constexpr (SRC == 0) {
+    } else if constexpr (!(SRC & SRC_CONV)) {
 #pragma unroll
         for (int i = 0; i < E; i++) x[i] = A::from_u64(src[n0 + i * step], k);
     } else {
@@ -642,15 +642,18 @@ __device__ __forceinline__ void load_src(typename A::T (&x)[E], const NttArgs &a
     }
 }
 
-// bound of what load_src gives
+// bound of what load_src gives. Canonical words have their own: a 50-bit prime with twice the bound asks for a reduction of the factor
+// from the second stage on instead of the third (B200, eight limbs forward in one launch, us on the device: 2^14 5.98 instead of 5.96,
+// 2^13 6.06 instead of 6.04)
 template <class A, int SRC>
 __host__ __device__ constexpr int src_bound() {
-    return (SRC & SRC_REM ? A::B_CANON : 0) + (SRC & SRC_CONV ? A::B_BCONV : (SRC & SRC_WORDS) || SRC == 0 ? A::B_IN : 0);
+    if (SRC == 0) return A::B_CANON;
+    return (SRC & SRC_REM ? A::B_CANON : 0) + (SRC & SRC_CONV ? A::B_BCONV : SRC & SRC_WORDS ? A::B_WORDS : 0);
 }
 
 // ================================================================================================
 // forward pass: R1 strided stages, exchange, R2 contiguous stages
-// FIRST: the input holds residues within B_IN as words (else the raw lazy values of the previous pass)
+// FIRST: the input holds residues as words, SRC says which (else the raw lazy values of the previous pass)
 // ================================================================================================
 // SRC (column pass only): where the input comes from. LOG_REST: log2(N) - LOG_T where it is known; the column passes are compiled for
 // every ring, so that the rows of a column are immediate offsets of one address (sixteen key switches of 24 limbs at 2^16, forward

@@ -30,6 +30,7 @@ void launch_fwd_whole(const NttArgs &a, const Epi &epi, uint32_t njobs, uint32_t
 }
 
 template void launch_fwd_whole<EpiStore, 0>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
+template void launch_fwd_whole<EpiStore, SRC_WORDS>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
 template void launch_fwd_whole<EpiStore, SRC_CONV>(const NttArgs &, const EpiStore &, uint32_t, uint32_t, cudaStream_t);
 template void launch_fwd_whole<EpiSubFrom, SRC_CONV>(const NttArgs &, const EpiSubFrom &, uint32_t, uint32_t, cudaStream_t);
 template void launch_fwd_whole<EpiSubFromTab, SRC_CONV>(const NttArgs &, const EpiSubFromTab &, uint32_t, uint32_t, cudaStream_t);
