@@ -959,7 +959,7 @@ static int run_fwd(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
                    const Epi &epi, cudaStream_t s, uint32_t period = 0, const BatchDims &bd = BatchDims{}, const RemSrc &rem = RemSrc{}) {
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, period, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
+    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, period};
     rem.put(a);
     if constexpr (WholeHas<Epi, SRC>::value) {
         if ((SRC == 0 || c->logN == 12) && use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, period)) {
@@ -986,7 +986,7 @@ static int run_inv(const b2_ctx *c, const uint64_t *src, uint64_t *dst, const Jo
                    const W2 *fin, cudaStream_t s, const BatchDims &bd = BatchDims{}) {
     if (njobs == 0) return B2_OK;
     if (!aligned32(src) || !aligned32(dst)) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, bd.perm};
+    NttArgs a{src, dst, jobs, first_prime, (uint32_t)c->logN, c->d_itw, c->d_mod, fin, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs, 0, bd.perm};
     if (use_whole(c, (size_t)njobs * bd.batch, jobs, first_prime, njobs, 0)) {
         LaunchScope ls(c, s, "ntt_inv_whole");
         launch_inv_whole(a, njobs, bd.batch, s);
@@ -1012,7 +1012,7 @@ template <class Epi, int SRC = SRC_CONV>
 static int run_bconv_fwd(const b2_ctx *c, const uint64_t *in, uint64_t *dst, const Job *jobs, const BcJob *bc, const W2 *mat, uint32_t njobs, const Epi &epi,
                          cudaStream_t s, const BatchDims &bd = BatchDims{}, const RemSrc &rem = RemSrc{}) {
     if (!aligned32(in) || !aligned32(dst) || !epi.aligned()) return fail(B2_EINVAL, "device buffers must be 32-byte aligned (256-bit accesses)");
-    NttArgs a{in, dst, jobs, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
+    NttArgs a{in, dst, jobs, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, bd.src_lm1, bd.src_bs, bd.dst_lm1, bd.dst_bs};
     a.bc = bc, a.mat = mat;
     rem.put(a);
     switch (c->logN) {
@@ -1538,7 +1538,7 @@ static int modup_inner_fused(b2_ctx *c, size_t l, const uint64_t *c2, const uint
         }
         // ModUp up to the column pass for every limb; the row pass is stored only for the limbs the stand-alone inner
         // product still handles (wide Q primes and P); for the FP64 limbs of Q it runs inside ntt_fwd_rows_mac
-        NttArgs a{up, up, pl.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
+        NttArgs a{up, up, pl.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod};
         a.src_bs = a.dst_bs = batched ? per : 0;
         if (loading) {
             NttArgs b = a;
@@ -2974,7 +2974,7 @@ extern "C" int b2_shard_keyswitch_phase_batch(b2_ctx *c, size_t l, int phase, si
                 // rank's slice: its P limbs first), as the one-GPU batched key switch does; the P limbs go straight into the
                 // limb-major exchange buffer
                 using Cfg = PassCfg<8>;
-                NttArgs na{UP, UP, sp.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod, nullptr, 0};
+                NttArgs na{UP, UP, sp.jobs_up_ntt, 0, (uint32_t)c->logN, c->d_tw, c->d_mod};
                 na.src_bs = na.dst_bs = per;
                 if (sp.n_up_ntt) {
                     launch_fwd_cols<SRC_WORDS>(c, na, sp.n_up_ntt, s, B);
