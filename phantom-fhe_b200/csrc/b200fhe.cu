@@ -335,13 +335,9 @@ static inline uint32_t h_npieces(uint64_t q) { return q < (1ull << 42) ? 2u : 3u
 // uploads what a TcBuild holds, in device form, as one blob and points the sets' job lists (given as [first job, count) ranges)
 // into it
 static int tc_upload(const TcBuild &b, void **blob, std::initializer_list<std::pair<TcSet *, std::pair<uint32_t, uint32_t>>> sets) {
-    std::vector<TcJob> jobs = b.jobs;
+    const std::vector<TcJob> &jobs = b.jobs;
+    const std::vector<uint8_t> &images = b.images;
     std::vector<TcGroup> groups = b.groups;
-    std::vector<uint8_t> images;
-    for (size_t j = 0; j < jobs.size(); j++) {
-        jobs[j].img_off = (uint32_t)images.size();
-        tc_pair_image(b, b.jobs[j], images);
-    }
     for (auto &g : groups)
         for (auto &o : g.o) o.p = 0 - o.p;
     const size_t jb = (jobs.size() * sizeof(TcJob) + 255) & ~size_t(255), gb = (groups.size() * sizeof(TcGroup) + 255) & ~size_t(255);
@@ -364,7 +360,7 @@ static int tc_upload(const TcBuild &b, void **blob, std::initializer_list<std::p
             if (j < TC_JOBS_INLINE) ts->first[j] = job;
             ts->min_groups = std::min(ts->min_groups, job.n_groups);
             ts->max_groups = std::max(ts->max_groups, job.n_groups);
-            ts->max_slices = std::max(ts->max_slices, (job.ni + 1) & ~1u);
+            ts->max_slices = std::max(ts->max_slices, tc_slices(job.ni));
         }
     }
     return B2_OK;

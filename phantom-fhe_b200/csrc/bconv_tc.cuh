@@ -1,5 +1,5 @@
 // bconv_tc.cuh - fast base conversion on the sm_100a tensor cores (tcgen05.mma kind::i8, accumulators in TMEM).
-// The formulation, the data structures and the host-side planning are in bconv_tc_plan.h.
+// The formulation, the data structures, the reduction and the host-side planning are in bconv_tc_plan.h.
 //
 // A tile is 256 coefficients of one job: 128 rows of two coefficients, so that an input limb's share of the tile is 2 KB of
 // consecutive memory AND, as it lies there, one 16-byte K slice of all rows of A. One cp.async.bulk per limb brings it in, no
@@ -116,40 +116,15 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t (&c)[32]) {
                  : "memory");
 }
 
-// One residue below 2 p from its planes: paired with shift-adds, joined by one (7 and 8 planes: two) wide multiply-adds, the
-// quotient estimate one high multiply, v + qhat (2^64 - p) one wide multiply-add and one narrow one. tc_reduce
-// (bconv_tc_plan.h) without its last subtraction, which the forward transform that follows does not need (B_WORDS).
-// r: {2^64 - p as two words, mu, slot}
-template <int NB>
-__device__ __forceinline__ uint2 tc_residue(const uint32_t *c, const uint4 r) {
-    constexpr int SH = 8 * NB - 17;
-    const uint32_t x0 = c[0] + (c[1] << 8), x1 = c[2] + (c[3] << 8);
-    uint32_t vl, vh, vq;  // V mod 2^64 as two words; V >> SH
-    if constexpr (NB <= 6) {
-        const uint32_t x2 = NB == 4 ? 0u : (NB == 5 ? c[4] : c[4] + (c[5] << 8));
-        const uint64_t v = (uint64_t)x1 * 65536u + (((uint64_t)x2 << 32) | x0);
-        vl = (uint32_t)v, vh = (uint32_t)(v >> 32);
-        vq = __funnelshift_r(vl, vh, SH);
-    } else {
-        const uint32_t x2 = c[4] + (c[5] << 8), x3 = NB == 7 ? c[6] : c[6] + (c[7] << 8);
-        const uint64_t a = (uint64_t)x1 * 65536u + x0, b = (uint64_t)x3 * 65536u + x2;
-        const uint64_t mid = (a >> 32) + b;
-        vl = (uint32_t)a, vh = (uint32_t)mid;
-        vq = __funnelshift_r((uint32_t)mid, (uint32_t)(mid >> 32), SH - 32);
-    }
-    const uint32_t qhat = __umulhi(vq, r.z);
-    const uint64_t t = (uint64_t)qhat * r.x + (((uint64_t)vh << 32) | vl);
-    return make_uint2((uint32_t)t, (uint32_t)(t >> 32) + qhat * r.y);
-}
-
 // the NV outputs of a group, two coefficients each
 template <int NB, int NV>
 __device__ __forceinline__ void tc_group(const uint32_t (&c)[32], const TcGroup *g, uint32_t slot_words, uint64_t *__restrict__ out_n) {
 #pragma unroll
     for (int o = 0; o < NV; o++) {
         const uint4 r = *reinterpret_cast<const uint4 *>(&g->o[o]);
-        const uint2 e = tc_residue<NB>(c + 2 * NB * o, r), f = tc_residue<NB>(c + 2 * NB * o + NB, r);
-        asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(out_n + r.w * slot_words), "r"(e.x), "r"(e.y), "r"(f.x), "r"(f.y) : "memory");
+        // r: {2^64 - p as two words, mu, slot}
+        const TcWord e = tc_residue<NB>(c + 2 * NB * o, r.x, r.y, r.z), f = tc_residue<NB>(c + 2 * NB * o + NB, r.x, r.y, r.z);
+        asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(out_n + r.w * slot_words), "r"(e.lo), "r"(e.hi), "r"(f.lo), "r"(f.hi) : "memory");
     }
 }
 __device__ __forceinline__ void tc_group_any(const uint32_t (&c)[32], uint2 hdr, const TcGroup *g, uint32_t slot_words, uint64_t *__restrict__ out_n) {
@@ -178,7 +153,7 @@ struct TcArgs {
     const uint64_t *copy_src;  // optional (one set): the digit's own limbs go from here to the jobs' copy slots
     const TcJob *jobs;         // the first TC_JOBS_INLINE of them in job[] as well: a load from memory less before the first copy
     const TcGroup *groups;     // device form: o[].p holds 2^64 - p
-    const uint8_t *images;     // device form: tc_pair_image
+    const uint8_t *images;
     uint32_t *err;
     uint32_t N;
     uint32_t items, more;      // a CTA works on `items` (job part, set, tile)s, the first `more` CTAs on one more
@@ -226,7 +201,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) bconv_tc_pairs(const __grid_con
             job = tc_job(a, pi / a.parts);
             uint32_t g0, g1;
             tc_part(job, pi % a.parts, a.parts, g0, g1);
-            const uint32_t slices = (job.ni + 1) & ~1u, row = job.n_groups * 512, part_row = (g1 - g0) * 512;
+            const uint32_t slices = tc_slices(job.ni), row = job.n_groups * 512, part_row = (g1 - g0) * 512;
             if (lane == 0) tc_expect(full_b, slices * part_row);
             __syncwarp();
             if (lane < slices) tc_bulk(sB + lane * part_row, a.images + job.img_off + g0 * 512 + lane * row, part_row, full_b);

@@ -1,5 +1,5 @@
-"""Tensor-core base conversion with two coefficients a row: the device image, its parts and the operand layout, emulated on the
-CPU against 128-bit integer arithmetic (tests/bconv_pair_emul.cpp); the rules of its waits (tests/bconv_wait_emul.cpp)."""
+"""Tensor-core base conversion, host side: the planner's groups and images (bconv_tc_plan.h), their parts, the operand layout and
+the kernel's reduction, emulated on the CPU against 128-bit integer arithmetic (tests/bconv_pair_emul.cpp); the rules of its waits (tests/bconv_wait_emul.cpp)."""
 import os
 import subprocess
 
