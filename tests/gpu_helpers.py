@@ -50,6 +50,17 @@ def key_dev(key):
     return tens, np.array([t.data_ptr() for t in tens], dtype=np.uint64)
 
 
+def kernels_of(ctx, call):
+    """-> (what `call` returns, {kernel name: launches}) by the library's own record of the launches on `ctx`"""
+    check(LIB.b2_profile_start(ctx._h))
+    try:
+        res = call()
+    finally:
+        names, ms, cnt, n = ctypes.create_string_buffer(8192), (ctypes.c_float * 128)(), (ctypes.c_uint32 * 128)(), ctypes.c_size_t()
+        check(LIB.b2_profile_stop(ctx._h, names, 8192, ms, cnt, 128, ctypes.byref(n)))
+    return res, dict(zip(names.value.decode().split(";"), cnt[:n.value]))
+
+
 def hashes(t, N):
     return limb_hashes(host(t), N)
 

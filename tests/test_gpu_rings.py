@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_helpers import dev, host, make_ctx
+from gpu_helpers import dev, host, kernels_of, make_ctx
 
 ph = pytest.importorskip("pyPhantom")
 pytestmark = pytest.mark.gpu
@@ -592,15 +592,15 @@ def test_transforms_of_ranges_of_limbs(log_n, first, n):
 
 
 @pytest.mark.parametrize("log_n,special,l,below", [
-    (15, 2, 6, 10),   # three digits: three waves of the fused pass
+    (15, 2, 6, 15),   # three digits: four and a half waves of the fused pass
     (15, 1, 4, 8),    # four digits: one and a half
     (15, 3, 6, 21),   # two digits: seven
-    (16, 2, 5, 5),    # a ragged third digit
+    (16, 2, 5, 8),    # a ragged third digit
     (16, 2, 2, 6),    # one digit: never fused
 ])
 def test_batches_on_both_sides_of_the_fused_row_pass(log_n, special, l, below):
-    """products with the last batch that stores the row pass on 148 SMs and the first that fuses it: every set as it is alone, the
-    last as the oracle has it"""
+    """products with the last batch that stores the row pass on 148 SMs and the first that fuses it (which of the two ran is read
+    from the launches): every set as it is alone, the first as the oracle has it"""
     N = 1 << log_n
     ctx, o = make_ctx(N, [60, 40, 50, 36, 40, 45][:l] + [60] * (special - 1) + [59], special)
     key = o.synth_key(o.beta(l), 4, 10)
@@ -610,48 +610,59 @@ def test_batches_on_both_sides_of_the_fused_row_pass(log_n, special, l, below):
     assert np.array_equal(host(one[0]), o.rescale(l, o.multiply_and_relin(l, a, b, key)))
     for batch in (below, below + 1):
         pick = torch.arange(batch, device="cuda") % 3
-        assert torch.equal(ph.multiply_relin_rescale_batch(ctx, da[pick], db[pick], rk), one[pick])
+        got, kernels = kernels_of(ctx, lambda: ph.multiply_relin_rescale_batch(ctx, da[pick], db[pick], rk))
+        fused = batch > below and o.beta(l) > 1
+        assert ("ntt_fwd_rows_mac" in kernels, "ks_inner_prod" in kernels) == (fused, not fused), kernels
+        assert torch.equal(got, one[pick])
     assert ctx.device_status() == 0
 
 
-@pytest.mark.parametrize("log_n,bits,special,l,batch", [
-    (13, [60, 40, 50, 36, 45, 30, 60, 60, 60], 3, 6, 1),                          # every prime class, full digits
-    (13, [60, 40, 46, 36, 50, 45, 40, 60, 59, 60, 60, 60], 5, 7, 2),              # five input limbs, then two
-    (13, [60] + [40, 50] * 4 + [60] * 8, 8, 9, 2),                                # eight input limbs, then one
-    (13, [60, 40, 40, 40, 60], 1, 4, 1),                                          # one input limb
-    (14, [60, 40, 50, 36, 60, 60], 2, 3, 1),
-    (14, [60, 40, 50, 36, 60, 60], 2, 4, 3),
-    (14, [60, 40, 50, 36, 40, 60, 60, 60], 3, 5, 1),
-    (15, [60, 40, 50, 36, 60, 60], 2, 4, 1),
-    (15, [60, 40, 50, 36, 40, 60, 60], 2, 5, 12),                                 # behind it the row pass with the inner product
-    (16, [60, 40, 50, 36, 60, 60], 2, 4, 1),                                      # the same for the FP64 limbs of a single call
-    (16, [60, 40, 36, 60, 60], 2, 3, 4),
+@pytest.mark.parametrize("log_n,bits,special,l,batch,fused", [
+    (13, [60, 40, 50, 36, 45, 30, 60, 60, 60], 3, 6, 1, False),                   # every prime class, full digits
+    (13, [60, 40, 46, 36, 50, 45, 40, 60, 59, 60, 60, 60], 5, 7, 2, False),       # five input limbs, then two
+    (13, [60] + [40, 50] * 4 + [60] * 8, 8, 9, 2, False),                         # eight input limbs, then one
+    (13, [60, 40, 40, 40, 60], 1, 4, 1, False),                                   # one input limb
+    (14, [60, 40, 50, 36, 60, 60], 2, 3, 1, False),
+    (14, [60, 40, 50, 36, 60, 60], 2, 4, 3, False),
+    (14, [60, 40, 50, 36, 40, 60, 60, 60], 3, 5, 1, False),
+    (15, [60, 40, 50, 36, 60, 60], 2, 4, 1, False),
+    (15, [60, 40, 50, 36, 40, 60, 60], 2, 5, 12, False),
+    (15, [60, 40, 50, 36, 40, 60, 60], 2, 5, 18, True),                           # behind it the row pass with the inner product
+    (16, [60, 40, 50, 36, 60, 60], 2, 4, 1, True),                                # the same for the FP64 limbs of a single call
+    (16, [60, 40, 36, 60, 60], 2, 3, 4, False),
+    (16, [60, 40, 50, 36, 40, 60, 60], 2, 5, 9, True),                            # a ragged third digit
 ])
-def test_conversion_in_the_column_pass_equals_the_oracle(log_n, bits, special, l, batch):
-    """key switches whose base conversions are made while the forward transforms load, ModUp and ModDown, single and batched"""
+def test_conversion_in_the_column_pass_equals_the_oracle(log_n, bits, special, l, batch, fused):
+    """key switches whose base conversions are made while the forward transforms load, ModUp and ModDown, single and batched (that
+    no conversion kernel ran, and which row pass did, is read from the launches)"""
     ctx, o = make_ctx(1 << log_n, bits, special)
     key = o.synth_key(o.beta(l), 8, 10)
     a, b = [o.synth_ct(l, 8, 20 + i) for i in range(batch)], [o.synth_ct(l, 8, 40 + i) for i in range(batch)]
     rlk = _key(ctx, key)
     if batch == 1:
         ca, cb = (ph.ciphertext.from_numpy(ctx, v[0], ctx.size_Q - l + 1, 2.0 ** 40) for v in (a, b))
-        got = [host(ph.multiply_and_relin(ctx, ca, cb, rlk).data)]
+        res, kernels = kernels_of(ctx, lambda: ph.multiply_and_relin(ctx, ca, cb, rlk))
+        got = [host(res.data)]
     else:
         ext = dev(np.stack([o.tensor_mul(l, a[i], b[i]) for i in range(batch)]))
-        got = host(ph.relinearize_batch(ctx, ext, rlk))
+        res, kernels = kernels_of(ctx, lambda: ph.relinearize_batch(ctx, ext, rlk))
+        got = host(res)
+    assert "bconv" not in kernels and ("ntt_fwd_rows_mac" in kernels) == fused, kernels
     for i in range(batch):
         assert np.array_equal(got[i], o.multiply_and_relin(l, a[i], b[i], key)), f"set {i}"
     assert ctx.device_status() == 0
 
 
-@pytest.mark.parametrize("log_n,special,l", [(12, 7, 8), (13, 1, 5), (14, 4, 9), (14, 5, 5), (15, 8, 17), (16, 6, 7), (17, 3, 4)])
-def test_pair_conversion_edges(log_n, special, l):
+@pytest.mark.parametrize("log_n,special,l,batch", [(12, 7, 8, 7), (13, 1, 5, 0), (14, 4, 9, 3), (14, 5, 5, 3), (14, 3, 27, 3), (15, 8, 17, 3),
+                                                   (16, 6, 7, 3), (17, 3, 4, 3)])
+def test_pair_conversion_edges(log_n, special, l, batch):
     """the tensor-core conversion at odd numbers of input limbs, ragged digits and column groups that leave its items uneven:
-    ModUp (with the digits' own limbs copied) and a batch of key switches, every byte count of an output prime among them"""
+    ModUp (with the digits' own limbs copied) and a batch of key switches, every byte count of an output prime among them; nine
+    digits are more jobs than a launch carries in its parameters. Key switches with one input limb run no conversion kernel."""
     from pyPhantom import _native
     from pyPhantom._native import LIB, check
     from gpu_helpers import stream
-    bits = ([60, 30, 40, 46, 50, 55, 36, 42] * 3)[:l] + [60] * special
+    bits = ([60, 30, 40, 46, 50, 55, 36, 42] * 4)[:l] + [60] * special
     ctx, o = make_ctx(1 << log_n, bits, special)
     c2 = o.fill(1, o.primes[:l], 3, 7)[0]
     up = ctx.empty(o.beta(l), l + special)
@@ -660,11 +671,15 @@ def test_pair_conversion_edges(log_n, special, l):
     check(LIB.b2_modup(ctx._h, l, dev(c2).data_ptr(), up.data_ptr(), ws.data_ptr(), nb, stream()))
     want = o.modup(l, c2)
     assert np.array_equal(host(up).reshape(want.shape), want)
+    assert ctx.device_status() == 0
+    if not batch:
+        return
     key = o.synth_key(o.beta(l), 3, 10)
-    sets = [o.fill(3, o.primes[:l], 3, 20 + i) for i in range(3)]
-    got = host(ph.relinearize_batch(ctx, dev(np.stack(sets)), _key(ctx, key)))
+    sets = [o.fill(3, o.primes[:l], 3, 20 + i) for i in range(batch)]
+    got, kernels = kernels_of(ctx, lambda: ph.relinearize_batch(ctx, dev(np.stack(sets)), _key(ctx, key)))
+    assert kernels["bconv"] == 2, kernels  # ModUp's and ModDown's
     for i, s in enumerate(sets):
-        assert np.array_equal(got[i], o.keyswitch(l, s[2], key, s[:2])), f"set {i}"
+        assert np.array_equal(host(got[i]), o.keyswitch(l, s[2], key, s[:2])), f"set {i}"
     assert ctx.device_status() == 0
 
 
