@@ -467,11 +467,8 @@ def test_full_size_properties():
         assert int(fxh[i].max()) < int(o.primes[i])
 
 
-@pytest.mark.parametrize("env", ["B2_NTT_CLUSTER", "B2_NTT_PIPE"])
-def test_optional_transform_kernels(monkeypatch, env):
-    """the single-launch cluster transforms and the cp.async-pipelined passes (both opt-in: measured slower than the
-    default two-pass kernels) give the same limbs as the reference"""
-    monkeypatch.setenv(env, "1")
+def test_transforms_in_place_and_key_switch_of_one_digit():
+    """2^16: transforms of the whole chain in place, and a key switch whose one digit has fewer limbs than there are special primes"""
     path = [p for p in GOLDEN if p.endswith("n16_l5_a8.json")][0]
     case, ctx, o = load_case(path)
     N, l, seed, h = o.N, case["level"], case["seed"], ctx._h
@@ -511,17 +508,16 @@ def test_inner_product_inside_the_last_forward_pass(monkeypatch, name, fused):
     assert hashes(ct, N) == case["hashes"]["keyswitch"]
 
 
-@pytest.mark.parametrize("case", ["n16_headline", "n16_wide", "n16_l11", "n16_l5", "n16_l1", "n13_fallback"])
+@pytest.mark.parametrize("case", ["n16_headline", "n16_wide", "n16_l11", "n16_l5", "n16_l1", "n13"])
 def test_batched_key_switch_equals_single_ones(case, monkeypatch):
     """b2_keyswitch_batch (every kernel one launch over a batch that shares the key; strided sets) gives, set by set, the limbs
     of b2_keyswitch - at the headline shape also the oracle's - with the stand-alone inner product for the 60-bit limbs and
-    with every limb in the fused pass, at a level with a ragged last digit, and where the fused pipeline does not apply
-    (N = 2^13: the sets run one after another)"""
+    with every limb in the fused pass, at a level with a ragged last digit, and in a ring without a fused pass (N = 2^13)"""
     if case in ("n16_l11", "n16_l5", "n16_l1"):
         monkeypatch.delenv("B2_KS_FUSED_WIDE", raising=False)  # the default: every limb in the fused pass for batched calls only
     else:
         monkeypatch.setenv("B2_KS_FUSED_WIDE", "1" if case == "n16_wide" else "0")
-    if case == "n13_fallback":
+    if case == "n13":
         N, bits, special, l, batch = 8192, [55, 40, 41, 42, 43, 44, 45, 46, 58, 59, 60], 3, 7, 3
     else:
         N, bits, special, batch = 65536, [60] + [40] * 23 + [60] * 8, 8, 5
